@@ -145,12 +145,20 @@ int kda_bwd(const KdaParams *p, void *cuda_stream);
  * reference has no generation path; this is the step its final-state interface implies (the
  * third-party package it builds on ships it as fused_recurrent_kda).
  *   q, k, g : [N, H, dk]     v, o : [N, H, dv]     beta : [N, H]     states : [N, H, dk, dv] float
- * state_out may equal state_in (updated in place).  status may be NULL, else a device word that
- * receives a non-zero code if the bounded wait for the state copy gives up. */
+ * state_out may equal state_in (updated in place).  status is not used (the kernel waits for
+ * nothing) and may be NULL. */
 int kda_recurrent_step(const void *q, const void *k, const void *v, const void *g, const void *beta,
                        const float *A_log, const float *dt_bias, const float *state_in, float *state_out,
                        void *o, int32_t N, int32_t H, int32_t dk, int32_t dv, int32_t dtype, int32_t flags,
                        float scale, int32_t *status, void *cuda_stream);
+
+/* The same recurrence over T tokens per sequence in one launch, the state held on chip in between.
+ *   q, k, g : [N, T, H, dk]     v, o : [N, T, H, dv]     beta : [N, T, H]
+ * state_in NULL: zero initial state; state_out NULL: no final state; they may be equal. */
+int kda_recurrent_fwd(const void *q, const void *k, const void *v, const void *g, const void *beta,
+                      const float *A_log, const float *dt_bias, const float *state_in, float *state_out,
+                      void *o, int32_t N, int32_t T, int32_t H, int32_t dk, int32_t dv, int32_t dtype,
+                      int32_t flags, float scale, void *cuda_stream);
 
 /* Causal depthwise short convolution + SiLU over [B, T, C] (k3mini/model.py:76-88; the
  * fast path's fla.modules.ShortConvolution at k3mini/model.py:147-155).  weight is

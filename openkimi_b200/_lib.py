@@ -62,6 +62,7 @@ EXPORTS = {
     "kda_fwd": (C.c_int, [C.POINTER(KdaParams), C.c_void_p]),
     "kda_bwd": (C.c_int, [C.POINTER(KdaParams), C.c_void_p]),
     "kda_recurrent_step": (C.c_int, [C.c_void_p] * 10 + [C.c_int32] * 6 + [C.c_float, C.c_void_p, C.c_void_p]),
+    "kda_recurrent_fwd": (C.c_int, [C.c_void_p] * 10 + [C.c_int32] * 7 + [C.c_float, C.c_void_p]),
     "kda_short_conv_fwd": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32,
                                      C.c_int32, C.c_int32, C.c_void_p, C.c_int32, C.c_void_p]),
     "kda_short_conv_bwd": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,

@@ -390,38 +390,59 @@ def recurrent_kda_step(q, k, v, g, beta, state, *, scale=None, A_log=None, dt_bi
         raise ValueError(f"state must be float32 [N,H,{K},{K}], got {state.dtype} {tuple(state.shape)}")
     if use_gate_in_kernel and (A_log is None or A_log.numel() != H or (dt_bias is not None and dt_bias.numel() != H * K)):
         raise ValueError("use_gate_in_kernel=True needs A_log with H entries (and dt_bias with H*K entries)")
-    dt = q.dtype
-    q, k, v, g, beta = (t.detach().to(dt).contiguous() for t in (q, k, v, g, beta))
-    a = A_log.detach().float().contiguous() if use_gate_in_kernel else None
-    b = dt_bias.detach().float().contiguous() if (use_gate_in_kernel and dt_bias is not None) else None
     s_in = state.detach().contiguous()
     s_out = s_in if inplace and s_in.data_ptr() == state.data_ptr() else torch.empty_like(s_in)
-    o = torch.empty_like(v)
-    flags = ((_lib.FLAG_QK_L2NORM if use_qk_l2norm_in_kernel else 0) | (_lib.FLAG_GATE if use_gate_in_kernel else 0)
-             | (_lib.FLAG_BETA_SIGMOID if use_beta_sigmoid_in_kernel else 0)
-             | (_lib.FLAG_STATE_V_FIRST if state_v_first else 0))
-    with torch.cuda.device(q.device):
-        st = _DeviceStatus.get(q.device)
-        st.poll()
-        rc = _lib.load().kda_recurrent_step(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(),
-                                            _ptr(a), _ptr(b), s_in.data_ptr(), s_out.data_ptr(), o.data_ptr(), N, H, K, K,
-                                            _DTYPES[dt], flags, float(K ** -0.5 if scale is None else scale),
-                                            st.dev.data_ptr(), C.c_void_p(torch.cuda.current_stream(q.device).cuda_stream))
-        _lib.check(rc, "kda_recurrent_step")
+    o = _recurrent(q, k, v, g, beta, s_in, s_out, (N, 1, H, K), scale, A_log, dt_bias, use_qk_l2norm_in_kernel,
+                   use_gate_in_kernel, use_beta_sigmoid_in_kernel, state_v_first)
     return o, s_out
 
 
-def fused_recurrent_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_state=False, **kw):
-    """Token-by-token KDA over ``[B, T, H, K]`` inputs through ``recurrent_kda_step`` (the decoding
-    counterpart of ``chunk_kda``, same prologue keywords; meant for the few tokens of a decode loop).
-    Returns ``(o [B, T, H, V], final_state or None)``."""
+def _recurrent(q, k, v, g, beta, s_in, s_out, sizes, scale, A_log, dt_bias, l2norm, gate, sigmoid, state_v_first):
+    """One launch of the recurrent kernel over ``sizes`` = (sequences, tokens, heads, channels)."""
+    N, T, H, K = sizes
+    dt = q.dtype
+    q, k, v, g, beta = (t.detach().to(dt).contiguous() for t in (q, k, v, g, beta))
+    a = A_log.detach().float().contiguous() if gate else None
+    b = dt_bias.detach().float().contiguous() if (gate and dt_bias is not None) else None
+    o = torch.empty_like(v)
+    flags = ((_lib.FLAG_QK_L2NORM if l2norm else 0) | (_lib.FLAG_GATE if gate else 0)
+             | (_lib.FLAG_BETA_SIGMOID if sigmoid else 0) | (_lib.FLAG_STATE_V_FIRST if state_v_first else 0))
+    with torch.cuda.device(q.device):
+        _DeviceStatus.get(q.device).poll()
+        rc = _lib.load().kda_recurrent_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(),
+                                           _ptr(a), _ptr(b), _ptr(s_in), _ptr(s_out), o.data_ptr(), N, T, H, K, K,
+                                           _DTYPES[dt], flags, float(K ** -0.5 if scale is None else scale),
+                                           C.c_void_p(torch.cuda.current_stream(q.device).cuda_stream))
+        _lib.check(rc, "kda_recurrent_fwd")
+    return o
+
+
+def fused_recurrent_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_state=False, *, A_log=None,
+                        dt_bias=None, use_qk_l2norm_in_kernel=False, use_gate_in_kernel=False,
+                        use_beta_sigmoid_in_kernel=False, state_v_first=False):
+    """Token-by-token KDA over ``[B, T, H, K]`` inputs (the decoding counterpart of ``chunk_kda``, same prologue
+    keywords; meant for the few tokens of a decode loop): the recurrence of ``recurrent_kda_step`` in one launch,
+    the state on chip from the first token to the last.  Returns ``(o [B, T, H, V], final_state or None)``."""
+    for t in (q, k, v, g, beta):
+        _require_cuda(t)
+    if q.dim() != 4 or q.shape != k.shape or g.shape != q.shape:
+        raise ValueError(f"q, k, g must share one shape [B,T,H,K], got {tuple(q.shape)}, {tuple(k.shape)}, {tuple(g.shape)}")
     B, T, H, K = q.shape
-    vfirst = bool(kw.get("state_v_first", False))
-    state = (initial_state.detach().clone() if initial_state is not None
-             else torch.zeros(B, H, K, K, dtype=torch.float32, device=q.device))
-    outs = []
-    for t in range(T):
-        o, state = recurrent_kda_step(q[:, t], k[:, t], v[:, t], g[:, t], beta[:, t], state, scale=scale, inplace=True, **kw)
-        outs.append(o)
-    o = torch.stack(outs, dim=1) if outs else v.new_zeros(B, 0, H, K)
-    return o, (state if output_final_state else None)
+    if v.shape != q.shape or K not in (64, 128):
+        raise ValueError(f"the B200 KDA kernels need K == V in (64, 128), got K={K}, v={tuple(v.shape)}")
+    if beta.shape != (B, T, H):
+        raise ValueError(f"beta must have shape {[B, T, H]}, got {list(beta.shape)}")
+    if q.dtype not in _DTYPES:
+        raise TypeError(f"q/k/v must be float32 or bfloat16, got {q.dtype}")
+    if initial_state is not None and (initial_state.dtype != torch.float32 or tuple(initial_state.shape) != (B, H, K, K)):
+        raise ValueError(f"initial_state must be float32 [B,H,{K},{K}], got {initial_state.dtype} {tuple(initial_state.shape)}")
+    if use_gate_in_kernel and (A_log is None or A_log.numel() != H or (dt_bias is not None and dt_bias.numel() != H * K)):
+        raise ValueError("use_gate_in_kernel=True needs A_log with H entries (and dt_bias with H*K entries)")
+    if T == 0:
+        state = initial_state.detach().clone() if initial_state is not None else q.new_zeros(B, H, K, K, dtype=torch.float32)
+        return v.new_zeros(B, 0, H, K), (state if output_final_state else None)
+    s_in = initial_state.detach().contiguous() if initial_state is not None else None
+    s_out = torch.empty(B, H, K, K, dtype=torch.float32, device=q.device) if output_final_state else None
+    o = _recurrent(q, k, v, g, beta, s_in, s_out, (B, T, H, K), scale, A_log, dt_bias, use_qk_l2norm_in_kernel,
+                   use_gate_in_kernel, use_beta_sigmoid_in_kernel, state_v_first)
+    return o, s_out
