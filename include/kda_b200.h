@@ -160,6 +160,17 @@ int kda_recurrent_fwd(const void *q, const void *k, const void *v, const void *g
                       void *o, int32_t N, int32_t T, int32_t H, int32_t dk, int32_t dv, int32_t dtype,
                       int32_t flags, float scale, void *cuda_stream);
 
+/* Up to KDA_PACK_MAX arrays (FP32 or BF16) converted to BF16 in one launch; `zeros` elements of 0 follow
+ * each.  Weights of the sublayer as GEMM operands. */
+#define KDA_PACK_MAX 16
+typedef struct KdaPackSegment {
+    const void *src;
+    void *dst;
+    int64_t count, zeros;
+    int32_t dtype; /* of src: KDA_DTYPE_* */
+} KdaPackSegment;
+int kda_pack_bf16(const KdaPackSegment *segments, int32_t n, void *cuda_stream);
+
 /* Causal depthwise short convolution + SiLU over [B, T, C] (k3mini/model.py:76-88; the
  * fast path's fla.modules.ShortConvolution at k3mini/model.py:147-155).  weight is
  * [C, 1, ksize] float, ksize <= 4; cu_seqlens as above (no tap crosses a document). */

@@ -63,6 +63,7 @@ EXPORTS = {
     "kda_bwd": (C.c_int, [C.POINTER(KdaParams), C.c_void_p]),
     "kda_recurrent_step": (C.c_int, [C.c_void_p] * 10 + [C.c_int32] * 6 + [C.c_float, C.c_void_p, C.c_void_p]),
     "kda_recurrent_fwd": (C.c_int, [C.c_void_p] * 10 + [C.c_int32] * 7 + [C.c_float, C.c_void_p]),
+    "kda_pack_bf16": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p]),
     "kda_short_conv_fwd": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32,
                                      C.c_int32, C.c_int32, C.c_void_p, C.c_int32, C.c_void_p]),
     "kda_short_conv_bwd": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
@@ -95,6 +96,25 @@ def load() -> C.CDLL:
             fn.restype, fn.argtypes = res, args
         _lib = lib
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (``_host.so``: argument checks, memory, autograd and launches in C++)."""
+    global _host
+    if _host is None:
+        load()  # a missing kernel library is reported first, by its own message
+        try:
+            from . import _host as mod
+        except ImportError as e:
+            raise RuntimeError("openkimi_b200/_host.so is missing or does not load: build it with "
+                               f"`python -m openkimi_b200.build` ({e})") from e
+        from . import chunk_intra, ops
+        mod.set_callbacks(ops._DeviceStatus.of_index, ops._DeviceStatus.report, chunk_intra.current_guard_span)
+        _host = mod
+    return _host
 
 
 def check(status: int, what: str) -> None:

@@ -366,6 +366,37 @@ __global__ void __launch_bounds__(256) gate_tile_spans_kernel(const T* __restric
     }
 }
 
+// Conversion of several arrays to BF16: a grid row per segment, eight elements per thread and step where both ends
+// allow 16-byte accesses.
+struct PackSegments { KdaPackSegment s[KDA_PACK_MAX]; };
+__global__ void __launch_bounds__(256) pack_bf16_kernel(const __grid_constant__ PackSegments segs) {
+    const KdaPackSegment sg = segs.s[blockIdx.y];
+    __nv_bfloat16* dst = (__nv_bfloat16*)sg.dst;
+    const long long first = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8, step = (long long)gridDim.x * blockDim.x * 8;
+    const bool vec = (((uintptr_t)sg.src | (uintptr_t)sg.dst) & 15) == 0;
+    for (long long i = first; i < sg.count + sg.zeros; i += step) {
+        if (vec && i + 8 <= sg.count) {
+            if (sg.dtype == KDA_DTYPE_F32) {
+                const float* p = (const float*)sg.src + i;
+                float v[8], lo[4], hi[4];
+                Vec<float>::load(p, lo);
+                Vec<float>::load(p + 4, hi);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { v[j] = lo[j]; v[4 + j] = hi[j]; }
+                Vec<__nv_bfloat16>::store(dst + i, v);
+            } else {
+                *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)sg.src + i);
+            }
+        } else {
+            for (long long j = i; j < i + 8 && j < sg.count + sg.zeros; ++j) {
+                float v = 0.f;
+                if (j < sg.count) v = sg.dtype == KDA_DTYPE_F32 ? ((const float*)sg.src)[j] : ldf((const __nv_bfloat16*)sg.src + j);
+                stf(dst + j, v);
+            }
+        }
+    }
+}
+
 }  // namespace kda
 
 using namespace kda;
@@ -431,6 +462,24 @@ int kda_short_conv_bwd(const void* x, const float* weight, const void* dy, void*
                                                             total, T, Cch, ksize, cu_seqlens, N);
     int n = Cch * ksize;
     partial_reduce_kernel<<<(n + 31) / 32, 256, 0, s>>>(partial, dweight, n_partial, n);
+    return launch_status();
+}
+
+int kda_pack_bf16(const KdaPackSegment* segments, int32_t n, void* stream) {
+    if (!segments) return KDA_ERR_NULL;
+    if (n < 1 || n > KDA_PACK_MAX) return KDA_ERR_SHAPE;
+    PackSegments ps = {};
+    long long most = 0;
+    for (int i = 0; i < n; ++i) {
+        ps.s[i] = segments[i];
+        if (!ps.s[i].src || !ps.s[i].dst) return KDA_ERR_NULL;
+        if (ps.s[i].count < 0 || ps.s[i].zeros < 0) return KDA_ERR_SHAPE;
+        if (ps.s[i].dtype != KDA_DTYPE_F32 && ps.s[i].dtype != KDA_DTYPE_BF16) return KDA_ERR_DTYPE;
+        if (ps.s[i].count + ps.s[i].zeros > most) most = ps.s[i].count + ps.s[i].zeros;
+    }
+    if (most == 0) return KDA_OK;
+    const long long blocks = (most + 2047) / 2048;
+    pack_bf16_kernel<<<dim3((unsigned)(blocks < 148 ? blocks : 148), n), 256, 0, (cudaStream_t)stream>>>(ps);
     return launch_status();
 }
 

@@ -12,7 +12,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib
-from .ops import chunk_kda, _DTYPES, _require_cuda
+from .ops import chunk_kda, _DTYPES, _packed_tables, _require_cuda
 
 
 def _stream(t):
@@ -212,7 +212,36 @@ class KimiDeltaAttention(nn.Module):
     def _heads(self, x):
         return x.view(*x.shape[:2], self.n_heads, self.head_dim)
 
+    def _native_parameters(self, x):
+        """The parameters in the order the native node takes them, if it computes what the modules below would: BF16
+        activations with d = 128 and the fused short convolution, plain parts (nothing replaced, no hooks)."""
+        if self.head_dim != 128 or not self.fuse_short_conv or not x.is_cuda or x.dim() != 3 or x.numel() == 0:
+            return None
+        parts = (self.q_proj, self.k_proj, self.v_proj, self.f_a_proj, self.f_b_proj, self.beta_proj, self.out_gate_a,
+                 self.out_gate_b, self.out_proj)
+        for m in parts:
+            if type(m) is not nn.Linear or m.bias is not None or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks \
+                    or m._backward_pre_hooks:
+                return None
+        norm = self.out_norm_gate
+        if type(norm) is not FusedRMSNormGated or norm._forward_hooks or norm._forward_pre_hooks or norm._backward_hooks \
+                or norm._backward_pre_hooks:
+            return None
+        if torch.is_autocast_enabled("cuda"):
+            if torch.get_autocast_dtype("cuda") != torch.bfloat16 or x.dtype not in (torch.bfloat16, torch.float32):
+                return None
+        elif x.dtype != torch.bfloat16 or any(m.weight.dtype != torch.bfloat16 for m in parts):
+            return None
+        prm = (self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.q_conv.weight, self.k_conv.weight,
+               self.v_conv.weight, self.A_log, self.f_a_proj.weight, self.f_b_proj.weight, self.dt_bias,
+               self.beta_proj.weight, self.out_gate_a.weight, self.out_gate_b.weight, norm.weight, self.out_proj.weight)
+        return prm if all(p.is_cuda for p in prm) else None
+
     def forward(self, x, cu_seqlens=None):
+        prm = self._native_parameters(x)
+        if prm is not None and not _lib.host().env_flags():
+            return _lib.host().layer(x, prm, self.n_heads, self.scale, self.out_norm_gate.eps, self.disable_recompute,
+                                     *_packed_tables(cu_seqlens, None, x.device))
         # The three narrow projections of x (decay rank, output-gate rank, beta) share one GEMM: x is
         # read once instead of three times.  Same parameters, same arithmetic per output column.  All four
         # projections of x form one autograd node (see _InputProjections).
