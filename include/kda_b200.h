@@ -125,6 +125,9 @@ typedef struct KdaParams {
      * slightly larger backward scratch.  When NULL, grad_q/k/v are gradients of the convolved rows as
      * before (feed them to kda_short_conv_bwd). */
     float *grad_conv_q, *grad_conv_k, *grad_conv_v;
+    int32_t max_chunks;         /* chunks of the longest sequence; 0: not known (with cu_seqlens the mean is
+                                   assumed).  Only a hint how to split the state recurrence over the chip;
+                                   the same value for kda_workspace_bytes, kda_fwd and kda_bwd of a call */
 } KdaParams;
 
 /* Bytes of forward workspace (saved for the backward) and of backward scratch for these

@@ -41,6 +41,7 @@ class KdaParams(C.Structure):
         ("chunk_tab", C.c_void_p),
         ("status_host", C.c_void_p),
         ("grad_conv_q", C.c_void_p), ("grad_conv_k", C.c_void_p), ("grad_conv_v", C.c_void_p),
+        ("max_chunks", C.c_int32),
     ]
 
 

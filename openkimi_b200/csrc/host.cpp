@@ -173,7 +173,8 @@ struct Spec {
     double scale = 1.0;
     int flags = 0;
     bool output_final_state = false, keep = false;
-    int64_t NT = 0;  // chunks over all sequences
+    int64_t NT = 0;       // chunks over all sequences
+    int64_t longest = 0;  // chunks of the longest packed document
 };
 struct Inputs {
     Tensor q, k, v, g, beta, A_log, dt_bias, h0, conv_q, conv_k, conv_v;  // contiguous; undefined where absent
@@ -195,6 +196,7 @@ Prepared prepare(const Inputs& in, const Spec& sp, int flags) {
     r.N = in.cu.defined() ? in.cu.numel() - 1 : q.size(0);
     r.empty = sp.NT == 0;
     p.N = (int)r.N;
+    p.max_chunks = (int)sp.longest;
     p.NT = (int)std::max<int64_t>(sp.NT, 1);
     p.dtype = q.scalar_type() == at::kBFloat16 ? KDA_DTYPE_BF16 : KDA_DTYPE_F32;
     p.flags = flags;
@@ -327,17 +329,19 @@ variable_list to_list(const Inputs& in, const Tensor& ws) {
 Inputs from_list(const variable_list& s) {
     return {s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7], s[8], s[9], s[10], s[11], s[12], s[13], s[14]};
 }
-void save_spec(AutogradContext* ctx, double scale, int flags, int64_t NT, bool keep) {
-    ctx->saved_data["scale"] = scale;
-    ctx->saved_data["flags"] = (int64_t)flags;
-    ctx->saved_data["NT"] = NT;
-    ctx->saved_data["keep"] = keep;
+void save_spec(AutogradContext* ctx, const Spec& sp) {
+    ctx->saved_data["scale"] = sp.scale;
+    ctx->saved_data["flags"] = (int64_t)sp.flags;
+    ctx->saved_data["NT"] = sp.NT;
+    ctx->saved_data["longest"] = sp.longest;
+    ctx->saved_data["keep"] = sp.keep;
 }
 Spec load_spec(AutogradContext* ctx) {
     Spec sp;
     sp.scale = ctx->saved_data["scale"].toDouble();
     sp.flags = (int)ctx->saved_data["flags"].toInt();
     sp.NT = ctx->saved_data["NT"].toInt();
+    sp.longest = ctx->saved_data["longest"].toInt();
     sp.keep = ctx->saved_data["keep"].toBool();
     return sp;
 }
@@ -353,7 +357,8 @@ struct ChunkKda : torch::autograd::Function<ChunkKda> {
         const Inputs in = gather(q, k, v, g, beta, val(A_log), val(dt_bias), val(h0), val(cq), val(ck), val(cv), tables);
         FwdOut f = run_fwd(in, sp);
         ctx->save_for_backward(to_list(in, sp.keep ? f.ws : Tensor()));
-        save_spec(ctx, sp.scale, sp.flags, sp.NT, sp.keep);
+        ctx->set_materialize_grads(false);  // an unused final state has no gradient, rather than one of zeros
+        save_spec(ctx, sp);
         if (f.ht.defined()) return {f.o, f.ht};
         return {f.o};
     }
@@ -379,7 +384,7 @@ void take_tables(Inputs& tables, const OptTensor& cu, const OptTensor& chunk_seq
 std::tuple<Tensor, OptTensor> chunk_kda(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta,
                                         OptTensor A_log, OptTensor dt_bias, OptTensor h0, OptTensor cq, OptTensor ck, OptTensor cv,
                                         std::optional<double> scale, int64_t flags, bool output_final_state, bool disable_recompute,
-                                        OptTensor cu, OptTensor chunk_seq, OptTensor seq_off, OptTensor chunk_tab, int64_t NT) {
+                                        OptTensor cu, OptTensor chunk_seq, OptTensor seq_off, OptTensor chunk_tab, int64_t NT, int64_t longest) {
     for (const Tensor* t : {&q, &k, &v, &g, &beta}) require_cuda(*t);
     if (q.dim() != 4 || q.sizes() != k.sizes())
         value_error("q and k must have the same shape [B,T,H,K], got q=" + shape_of(q) + " vs k=" + shape_of(k));
@@ -401,6 +406,7 @@ std::tuple<Tensor, OptTensor> chunk_kda(const Tensor& q, const Tensor& k, const 
             value_error("The number of initial states is expected to be equal to the number of input sequences, i.e., " +
                         std::to_string(n_seq) + " rather than " + std::to_string(h0->size(0)) + ".");
         sp.NT = NT;
+        sp.longest = longest;
     } else {
         sp.NT = B * ((T + CHUNK - 1) / CHUNK);
     }
@@ -447,10 +453,9 @@ std::tuple<Tensor, OptTensor> chunk_kda(const Tensor& q, const Tensor& k, const 
 //   * weight gradients leave the GEMMs in FP32, the parameters' type, instead of BF16 plus a conversion;
 //   * no Python between the launches.
 struct LayerSpec {
-    int64_t H = 0, NT = 0;
-    double scale = 1.0, eps = 1e-6;
-    bool keep = false;
-    int flags = 0;
+    Spec op;
+    int64_t H = 0;
+    double eps = 1e-6;
 };
 enum { P_WQ, P_WK, P_WV, P_CQ, P_CK, P_CV, P_ALOG, P_FA, P_FB, P_DTB, P_BETA, P_GA, P_GB, P_NORM, P_WO, P_COUNT };
 constexpr int64_t HD = 128;
@@ -507,14 +512,9 @@ Tensor layer_fwd(const Tensor& x, const variable_list& prm, const LayerSpec& ls,
     auto heads = [&](const Tensor& t) { return t.view({B, T, H, HD}); };
     st.gates = ab[1];
     const Tensor beta = st.narrow.narrow(1, 2 * HD, H).contiguous().view({B, T, H});
-    Spec sp;
-    sp.scale = ls.scale;
-    sp.flags = ls.flags;
-    sp.keep = ls.keep;
-    sp.NT = ls.NT;
     st.in = gather(heads(qkv[0]), heads(qkv[1]), heads(qkv[2]), heads(ab[0]), beta, prm[P_ALOG], prm[P_DTB].reshape({proj}), Tensor(),
                    prm[P_CQ], prm[P_CK], prm[P_CV], tables);
-    FwdOut f = run_fwd(st.in, sp);
+    FwdOut f = run_fwd(st.in, ls.op);
     st.o = f.o;
     st.ws = f.ws;
     st.norm_w = ready(prm[P_NORM], at::kFloat);
@@ -532,11 +532,11 @@ struct Layer : torch::autograd::Function<Layer> {
         const variable_list prm = {p0, p1, p2, p3, p4, p5, p6, p7, p8, p9, p10, p11, p12, p13, p14};
         LayerState st;
         const Tensor out = layer_fwd(x, prm, ls, tables, st);
-        variable_list keep = to_list(st.in, ls.keep ? st.ws : Tensor());
+        variable_list keep = to_list(st.in, ls.op.keep ? st.ws : Tensor());
         for (const Tensor& t : {st.x2, st.narrow, st.gates, st.o, st.y, st.w.qkv, st.w.narrow, st.w.ab, st.w.out, st.norm_w})
             keep.push_back(t);
         ctx->save_for_backward(std::move(keep));
-        save_spec(ctx, ls.scale, ls.flags, ls.NT, ls.keep);
+        save_spec(ctx, ls.op);
         ctx->saved_data["eps"] = ls.eps;
         std::vector<int64_t> f32;  // which parameters want an FP32 gradient
         for (const Tensor& t : prm) f32.push_back(t.scalar_type() == at::kFloat);
@@ -618,15 +618,16 @@ struct Layer : torch::autograd::Function<Layer> {
 };
 
 Tensor layer(const Tensor& x, const std::vector<Tensor>& prm, int64_t H, double scale, double eps, bool disable_recompute,
-             OptTensor cu, OptTensor chunk_seq, OptTensor seq_off, OptTensor chunk_tab, int64_t NT) {
+             OptTensor cu, OptTensor chunk_seq, OptTensor seq_off, OptTensor chunk_tab, int64_t NT, int64_t longest) {
     require_cuda(x);
     TORCH_CHECK(prm.size() == P_COUNT, "expected the sublayer's parameters");
     LayerSpec ls;
     ls.H = H;
-    ls.scale = scale;
     ls.eps = eps;
-    ls.flags = KDA_FLAG_QK_L2NORM | KDA_FLAG_GATE | KDA_FLAG_BETA_SIGMOID | KDA_FLAG_STATE_V_FIRST;
-    ls.NT = cu ? NT : x.size(0) * ((x.size(1) + CHUNK - 1) / CHUNK);
+    ls.op.scale = scale;
+    ls.op.flags = KDA_FLAG_QK_L2NORM | KDA_FLAG_GATE | KDA_FLAG_BETA_SIGMOID | KDA_FLAG_STATE_V_FIRST;
+    ls.op.longest = longest;
+    ls.op.NT = cu ? NT : x.size(0) * ((x.size(1) + CHUNK - 1) / CHUNK);
     Inputs tables;
     if (cu) take_tables(tables, cu, chunk_seq, seq_off, chunk_tab, x.size(0));
     bool grad = false;
@@ -642,7 +643,7 @@ Tensor layer(const Tensor& x, const std::vector<Tensor>& prm, int64_t H, double 
         LayerState st;
         return layer_fwd(x, prm, ls, tables, st);
     }
-    ls.keep = disable_recompute;
+    ls.op.keep = disable_recompute;
     return Layer::apply(x, prm[0], prm[1], prm[2], prm[3], prm[4], prm[5], prm[6], prm[7], prm[8], prm[9], prm[10], prm[11], prm[12],
                         prm[13], prm[14], tables, ls)[0];
 }

@@ -13,6 +13,14 @@ cudaError_t simt_bwd(const KdaParams& p, cudaStream_t s);
 cudaError_t tc_fwd(const KdaParams& p, cudaStream_t s);
 cudaError_t tc_bwd(const KdaParams& p, cudaStream_t s);
 bool tc_supported(const KdaParams& p);
+int segment_count(const KdaParams& p);
+
+// bytes of the segment buffers behind the workspace (state at every border, transitions, their transposes for the
+// backward) and behind the backward scratch
+static size_t segment_bytes(const KdaParams& p, bool bwd) {
+    const size_t m = seg_matrix_floats(segment_count(p), p.H, p.dk) * sizeof(float);
+    return bwd ? m : m * ((p.flags & KDA_FLAG_NO_SAVE) ? 2 : 3);
+}
 
 static thread_local char g_last_error[256] = "";
 
@@ -105,14 +113,14 @@ static int validate(const KdaParams* p, bool bwd) {
     }
     const bool nosave = p->flags & KDA_FLAG_NO_SAVE;
     if (bwd && nosave) return KDA_ERR_WORKSPACE;  // the records of a forward-only call do not exist
-    if (p->workspace_bytes < (nosave ? L.total_nosave : conv ? L.total_conv : L.total) || ((uintptr_t)p->workspace & 255))
+    if (p->workspace_bytes < (nosave ? L.total_nosave : conv ? L.total_conv : L.total) + segment_bytes(*p, false) || ((uintptr_t)p->workspace & 255))
         return KDA_ERR_WORKSPACE;
     if (bwd) {
         if (!p->grad_o || !p->grad_q || !p->grad_k || !p->grad_v || !p->grad_g || !p->grad_beta || !p->bwd_scratch) return KDA_ERR_NULL;
         if ((p->flags & KDA_FLAG_GATE) && !p->grad_A_log) return KDA_ERR_NULL;
         const bool cvb = p->grad_conv_q || p->grad_conv_k || p->grad_conv_v;
         if (cvb && (!conv || !p->grad_conv_q || !p->grad_conv_k || !p->grad_conv_v)) return KDA_ERR_NULL;
-        if (p->bwd_scratch_bytes < (cvb ? L.bwd_total_conv : L.bwd_total) || ((uintptr_t)p->bwd_scratch & 255))
+        if (p->bwd_scratch_bytes < (conv ? L.bwd_total_conv : L.bwd_total) + segment_bytes(*p, true) || ((uintptr_t)p->bwd_scratch & 255))
             return KDA_ERR_WORKSPACE;
         const void* bp[] = {p->grad_o, p->grad_q, p->grad_k, p->grad_v, p->grad_g, p->grad_ht, p->grad_h0};
         for (const void* x : bp)
@@ -157,6 +165,8 @@ int kda_workspace_bytes(const KdaParams* p, size_t* fwd_bytes, size_t* bwd_bytes
     WsLayout L = ws_layout(p->NT, p->H, p->dk, p->dv, p->dtype);
     if (fwd_bytes) *fwd_bytes = (p->flags & KDA_FLAG_NO_SAVE) ? L.total_nosave : p->conv_q ? L.total_conv : L.total;
     if (bwd_bytes) *bwd_bytes = p->conv_q ? L.bwd_total_conv : L.bwd_total;
+    if (fwd_bytes) *fwd_bytes += segment_bytes(*p, false);
+    if (bwd_bytes) *bwd_bytes += segment_bytes(*p, true);
     return KDA_OK;
 }
 

@@ -126,15 +126,6 @@ __device__ __forceinline__ void seq_tokens(const KdaParams& p, int n, long long&
         end = first + p.T;
     }
 }
-__device__ __forceinline__ ChunkInfo chunk_of_seq(int n, int lc, long long first, long long end) {
-    ChunkInfo ci;
-    ci.seq = n;
-    ci.lc = lc;
-    ci.tok0 = first + (long long)lc * C;
-    const long long rem = end - ci.tok0;
-    ci.len = rem < C ? (int)rem : C;
-    return ci;
-}
 
 // ---------------------------------------------------------------------------------------
 // workspace layout (byte offsets).  All per-(chunk, head) records are stored
@@ -147,6 +138,39 @@ __device__ __forceinline__ ChunkInfo chunk_of_seq(int n, int lc, long long first
 // gamC is a plain float[dk]; aux is a plain row-major array; Gc, Qn, Kn are row-major with their
 // 16-byte chunks XOR-swizzled by the row when dk = 128 (swz_f32 / swz_bf16 in kda_tc.cuh).
 // ---------------------------------------------------------------------------------------
+// Sequence segments of the two state kernels (see kda_state_seg.cu).  len > 0: a CTA walks `len` consecutive chunks of
+// the global chunk numbering, whatever sequences they belong to; len == 0: a CTA walks one whole sequence.
+struct StateSegs {
+    int len, count;
+    float* E;   // [count][H][dv][dk]: transposed state at the end of the segment (backward: at its start)
+    float* X;   // [count][H][dk][dk]: transition of a segment that lies inside one sequence, S_end^T = S_begin^T X + E_local
+    float* XT;  // its transpose, for the backward; NULL when nothing is kept
+};
+
+// sequence of a chunk and the ranges a walk along the chunks needs; reloaded only where the walk enters another sequence
+struct SeqCursor {
+    int n, c_begin, c_end;       // sequence and its chunks [c_begin, c_end)
+    long long tok_begin, tok_end;
+    __device__ __forceinline__ void load(const KdaParams& p, int seq) {
+        n = seq;
+        int nc;
+        seq_chunks(p, n, c_begin, nc);
+        c_end = c_begin + nc;
+        seq_tokens(p, n, tok_begin, tok_end);
+    }
+    __device__ __forceinline__ void load_of_chunk(const KdaParams& p, int c) {
+        load(p, p.cu_seqlens != nullptr ? p.chunk_seq[c] : c / ((p.T + C - 1) / C));
+    }
+    __device__ __forceinline__ void move_to(const KdaParams& p, int c) {
+        if (c < c_begin || c >= c_end) load_of_chunk(p, c);
+    }
+    __device__ __forceinline__ long long tok(int c) const { return tok_begin + (long long)(c - c_begin) * C; }
+    __device__ __forceinline__ int rows(int c) const {
+        const long long rem = tok_end - tok(c);
+        return rem < C ? (int)rem : C;
+    }
+};
+
 struct WsLayout {
     size_t W, U, Aqk, Qt, Kh, gamC, total_nosave;       // what fwd_state consumes (all a forward-only call needs)
     size_t Tm, S0;                                      // kept for the backward only
@@ -217,6 +241,9 @@ __host__ __device__ inline WsLayout ws_layout(int NT, int H, int dk, int dv, int
     w.bwd_total_conv = off;
     return w;
 }
+
+// floats of the segment buffers behind the workspace / scratch of a call with `count` segments
+__host__ __device__ inline size_t seg_matrix_floats(int count, int H, int d) { return (size_t)count * H * d * d; }
 
 // state element index for logical (d, e) of a [dk, dv] state, honouring the v-first layout
 __device__ __forceinline__ size_t state_idx(const KdaParams& p, int d, int e) {

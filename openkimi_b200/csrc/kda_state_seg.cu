@@ -1,0 +1,338 @@
+// The state recurrence of long sequences in parallel segments (BF16 path, d = 128).
+//
+// kda_fwd_state_tc / kda_bwd_state_tc walk the chunks of a sequence one after the other: a chain of dependent MMA
+// round trips (about 2 us per chunk) on ONE SM per (sequence, head), while a batch of few or unevenly long sequences
+// leaves most of the 148 SMs idle.  A chunk maps its entering state linearly,
+//     S1^T = S0^T M + (U^T Kh),        M = diag(gamma) - W^T Kh,
+// so the chunks are cut into segments of equal length (in the global chunk numbering, across sequence borders):
+//   1  every segment runs the recurrence from a zero state -> its own contribution E, and, if it lies inside one
+//      sequence, from the identity -> its transition X = M_1 M_2 ... (both at once, two halves of one CTA)
+//   2  the states at the segment borders follow one after the other, S = S X + E, in FP32 on the CUDA cores
+//      (the rows of S^T are independent: 16 CTAs per chain, eight rows each)
+//   3  every segment runs as before, from its true entering state
+// X carries the same BF16 operands and FP32 accumulators as the state itself; step 2 rounds nothing.  The backward
+// walks the other way with X^T.  Work doubles (and X costs as much again, on warps that would idle), the chain shrinks
+// from n chunks to 2 len + n / len short steps.
+#include <math.h>
+
+#include <algorithm>
+
+#include "kda_common.cuh"
+#include "kda_tc.cuh"
+
+namespace kda {
+
+using namespace tc;
+
+namespace sg {
+constexpr int D = 128, NTHR = 512;
+constexpr uint32_t WT = 0, UT = 16384, KH = 32768, GAM = 49152, STAGE = 49664, TOTAL = 2 * STAGE;
+// tensor memory of one half: state, BF16 copy (V' takes its place once the first product has read it), first product
+constexpr uint32_t SACC = 0, SBF = 128, WSACC = 192, HALF_COLS = 256, TMEM_COLS = 512;
+}  // namespace sg
+
+__global__ void __launch_bounds__(sg::NTHR, 1) kda_fwd_segment_tc(const KdaParams p, const StateSegs segs) {
+    using namespace sg;
+    extern __shared__ __align__(128) unsigned char dyn[];
+    __shared__ uint64_t full[2], mmabar;
+    __shared__ uint32_t tmem_s;
+    // part 0 carries the state, part 1 the transition; inside a part as in kda_fwd_state_tc
+    const int tid = threadIdx.x, warp = tid >> 5, e = tid & 127, half = (tid >> 7) & 1, part = tid >> 8;
+    const int h = blockIdx.x, seg = blockIdx.y;
+    int cb = seg * segs.len;
+    const int ce = min(cb + segs.len, p.NT);
+    SeqCursor sq;
+    sq.load_of_chunk(p, ce - 1);
+    if (sq.c_end == ce) return;                // nobody needs the state at the end of this segment
+    const bool inside = sq.c_begin < cb;       // the sequence came in from the previous segment
+    cb = max(cb, sq.c_begin);
+    const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
+    const char* ws = (const char*)p.workspace;
+    if (warp == 0) {
+        tmem_alloc(&tmem_s, TMEM_COLS);
+        tmem_relinquish();
+    }
+    if (tid == 0) {
+        mbar_init(&full[0], 1);
+        mbar_init(&full[1], 1);
+        mbar_init(&mmabar, inside ? 2 : 1);
+        mbar_fence_init();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem0 = tmem_s + part * HALF_COLS;
+    const uint32_t tmem = tmem0 + ((uint32_t)((warp & 3) * 32) << 16);
+    const bool on = part == 0 || inside;
+    if (on) {
+        const size_t sbase = ((size_t)sq.n * p.H + h) * D * D;
+        for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
+            uint32_t r[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                float v = 0.f;
+                if (part == 1) v = d0 + j == e ? 1.f : 0.f;
+                else if (!inside && p.h0) v = p.h0[sbase + state_idx(p, d0 + j, e)];
+                r[j] = __float_as_uint(v);
+            }
+            tmem_st16(tmem + SACC + d0, r);
+        }
+        tmem_wait_st();
+    }
+    auto issue_loads = [&](int c, int stage) {
+        if ((tid & 31) != 0 || warp >= 4) return;
+        const size_t rec = (size_t)c * p.H + h;
+        unsigned char* b = dyn + stage * STAGE;
+        if (warp == 0) {
+            mbar_expect_tx(&full[stage], STAGE);
+            tma_load_1d(b + WT, (const __nv_bfloat16*)(ws + L.W) + rec * C * D, 16384, &full[stage]);
+        } else if (warp == 1) {
+            tma_load_1d(b + UT, (const __nv_bfloat16*)(ws + L.U) + rec * C * D, 16384, &full[stage]);
+        } else if (warp == 2) {
+            tma_load_1d(b + KH, (const __nv_bfloat16*)(ws + L.Kh) + rec * C * D, 16384, &full[stage]);
+        } else {
+            tma_load_1d(b + GAM, (const float*)(ws + L.gamC) + rec * D, 512, &full[stage]);
+        }
+    };
+    issue_loads(cb, 0);
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int c = cb; c < ce; ++c) {
+        const int stage = (c - cb) & 1;
+        unsigned char* b = dyn + stage * STAGE;
+        if (c + 1 < ce) issue_loads(c + 1, stage ^ 1);
+        ok = mbar_wait(&full[stage], ((c - cb) >> 1) & 1, p, 2);
+        if (!__syncthreads_and(ok)) { ok = false; break; }
+        if (on) {  // BF16 copy of the entering state, decay
+            const float* gam = reinterpret_cast<const float*>(b + GAM);
+            for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
+                uint32_t r[16], pk[8];
+                tmem_ld16(tmem + SACC + d0, r);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 8; ++j) pk[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+                tmem_st8(tmem + SBF + d0 / 2, pk);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * gam[d0 + j]);
+                tmem_st16(tmem + SACC + d0, r);
+            }
+            tmem_wait_st();
+        }
+        tc_fence_before();
+        __syncthreads();
+        const uint32_t sb = smem_u32(b);
+        if ((tid & 255) == 0 && on) {
+            tc_fence_after();
+            constexpr uint32_t id_mn = make_idesc(128, 64, false, true);
+#pragma unroll
+            for (int s = 0; s < 8; ++s)  // (W S)^T = Sbf (K = d) * W^T record
+                mma_ts(tmem0 + WSACC, tmem0 + SBF + s * 8, make_desc(sb + WT + s * 2048, 1024, 128), id_mn, s > 0);
+            mma_commit(&mmabar);
+        }
+        ok = mbar_wait(&mmabar, phase, p, 4);
+        phase ^= 1;
+        tc_fence_after();
+        if (!__syncthreads_and(ok)) { ok = false; break; }
+        if (on) {  // V'^T = U^T - (W S)^T; the transition has no U
+            const __nv_bfloat16* sU = reinterpret_cast<const __nv_bfloat16*>(b + UT);
+            for (int i0 = 32 * half; i0 < 32 * half + 32; i0 += 16) {
+                uint32_t r[16], pk[8];
+                float u[16];
+                tmem_ld16(tmem + WSACC + i0, r);
+                tmem_wait_ld();
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    float t8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                    if (part == 0) bf16x8_to_f32(*reinterpret_cast<const uint4*>(sU + cm_idx(e, i0 + 8 * g, C)), t8);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) u[8 * g + j] = t8[j];
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    pk[j] = pack_bf16(u[2 * j] - __uint_as_float(r[2 * j]), u[2 * j + 1] - __uint_as_float(r[2 * j + 1]));
+                tmem_st8(tmem + SBF + i0 / 2, pk);
+            }
+            tmem_wait_st();
+        }
+        tc_fence_before();
+        __syncthreads();
+        if ((tid & 255) == 0 && on) {
+            tc_fence_after();
+            constexpr uint32_t id_s = make_idesc(128, 128, false, true);
+#pragma unroll
+            for (int s = 0; s < 4; ++s)  // Sacc += V'^T (K = i) * Kh
+                mma_ts(tmem0 + SACC, tmem0 + SBF + s * 8, make_desc(sb + KH + s * 4096, 2048, 128), id_s, true);
+            mma_commit(&mmabar);
+        }
+        ok = mbar_wait(&mmabar, phase, p, 4);
+        phase ^= 1;
+        tc_fence_after();
+        if (!__syncthreads_and(ok)) { ok = false; break; }
+    }
+    if (ok && on) {
+        const size_t base = ((size_t)seg * p.H + h) * D * D;
+        float* dst = (part == 0 ? segs.E : segs.X) + base + (size_t)e * D;
+        for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
+            uint32_t r[16];
+            tmem_ld16(tmem + SACC + d0, r);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<uint4*>(dst + d0 + 4 * j) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+            if (part == 1 && segs.XT) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) segs.XT[base + (size_t)(d0 + j) * D + e] = __uint_as_float(r[j]);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem_s, TMEM_COLS);
+}
+
+// Step 2.  One CTA per (sequence, head, eight rows of S^T): E of every segment that a sequence leaves becomes the true
+// state there.  Thread = two columns x a quarter of the inner index; X arrives by bulk copies, two segments in flight
+// (64 KB per step and CTA from L2: about 0.7 us, as long as the arithmetic).
+namespace sc {
+constexpr int D = 128, ROWS = 8, NTHR = 256;
+constexpr uint32_t XT0 = 0, XBYTES = D * D * 4, ST = 2 * XBYTES, PART = ST + D * ROWS * 4, TOTAL = PART + 4 * ROWS * D * 4;
+}  // namespace sc
+
+template <bool BWD>
+__global__ void __launch_bounds__(sc::NTHR, 1) kda_seg_combine(const KdaParams p, const StateSegs segs) {
+    using namespace sc;
+    extern __shared__ __align__(128) unsigned char dyn[];
+    __shared__ uint64_t full[2];
+    const int tid = threadIdx.x, h = blockIdx.y, n = blockIdx.z, e0 = blockIdx.x * ROWS;
+    int c0, nc;
+    seq_chunks(p, n, c0, nc);
+    if (nc == 0) {  // no chunk of this sequence is visited by any segment: its state passes through here
+        const float* src = BWD ? p.grad_ht : p.h0;
+        float* dst = BWD ? p.grad_h0 : p.ht;
+        if (dst)
+            for (int i = tid; i < ROWS * D; i += NTHR) {
+                const size_t at = ((size_t)n * p.H + h) * D * D + state_idx(p, i & (D - 1), e0 + i / D);
+                dst[at] = src ? src[at] : 0.f;
+            }
+        return;
+    }
+    const int sa = c0 / segs.len, sz = (c0 + nc - 1) / segs.len;  // first and last segment of the sequence
+    const int steps = sz - sa - 1;                                // transitions to apply
+    if (steps <= 0) return;
+    if (tid == 0) {
+        mbar_init(&full[0], 1);
+        mbar_init(&full[1], 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+    const float* X = BWD ? segs.XT : segs.X;
+    auto mat = [&](int k) { return ((size_t)(BWD ? sz - k : sa + k) * p.H + h) * D * D; };  // k-th segment from the known end
+    auto issue = [&](int k) {
+        if (tid == 0) {
+            mbar_expect_tx(&full[k & 1], XBYTES);
+            tma_load_1d(dyn + XT0 + (k & 1) * XBYTES, X + mat(k), XBYTES, &full[k & 1]);
+        }
+    };
+    float* S = reinterpret_cast<float*>(dyn + ST);      // [d][row]
+    float* part = reinterpret_cast<float*>(dyn + PART);  // [quarter][row][column]
+    issue(1);
+    if (steps > 1) issue(2);
+    for (int i = tid; i < ROWS * D; i += NTHR) S[(i & (D - 1)) * ROWS + i / D] = segs.E[mat(0) + (size_t)(e0 + i / D) * D + (i & (D - 1))];
+    const int col = 2 * (tid & 63), quarter = tid >> 6;
+    for (int k = 1; k <= steps; ++k) {
+        float* E = segs.E + mat(k) + (size_t)e0 * D;
+        float own[ROWS * D / NTHR];
+#pragma unroll
+        for (int i = 0; i < ROWS * D / NTHR; ++i) own[i] = E[tid + NTHR * i];
+        const bool ok = mbar_wait(&full[k & 1], ((k - 1) >> 1) & 1, p, 2);
+        if (!__syncthreads_and(ok)) {
+            if (k < steps) mbar_wait(&full[(k + 1) & 1], (k >> 1) & 1, p, 2);  // the other copy in flight
+            return;
+        }
+        const float* x = reinterpret_cast<const float*>(dyn + XT0 + (k & 1) * XBYTES);
+        float acc[ROWS][2];
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) acc[r][0] = acc[r][1] = 0.f;
+#pragma unroll 8
+        for (int d = quarter * (D / 4); d < (quarter + 1) * (D / 4); ++d) {
+            const float2 xv = *reinterpret_cast<const float2*>(x + d * D + col);
+            const float4 s0 = *reinterpret_cast<const float4*>(S + d * ROWS), s1 = *reinterpret_cast<const float4*>(S + d * ROWS + 4);
+            const float sv[ROWS] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                acc[r][0] = fmaf(sv[r], xv.x, acc[r][0]);
+                acc[r][1] = fmaf(sv[r], xv.y, acc[r][1]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r)
+            *reinterpret_cast<float2*>(part + (quarter * ROWS + r) * D + col) = make_float2(acc[r][0], acc[r][1]);
+        __syncthreads();
+        if (k + 2 <= steps) issue(k + 2);
+#pragma unroll
+        for (int i = 0; i < ROWS * D / NTHR; ++i) {
+            const int at = tid + NTHR * i, r = at / D, d = at & (D - 1);
+            float v = own[i];
+#pragma unroll
+            for (int g = 0; g < 4; ++g) v += part[(g * ROWS + r) * D + d];
+            E[at] = v;
+            S[d * ROWS + r] = v;
+        }
+        __syncthreads();
+    }
+}
+
+// Segment length, 0 for whole sequences.  Estimated in chunk steps of 2.3 us: a whole-sequence walk takes as many as
+// the longest sequence has chunks, times the waves of sequences; segments of `len` take 1.8 len (both passes) plus a
+// third of a step per segment border of the longest sequence plus the launches.  len is what one wave of the chip needs,
+// but no shorter than what balances the border steps.
+static int segment_length(const KdaParams& p) {
+    if (p.NT < 8) return 0;
+    const int sms = sm_count();
+    const double longest = p.max_chunks > 0 ? p.max_chunks : (double)p.NT / p.N;
+    const double whole = std::max(longest, (double)p.NT * p.H / sms);
+    int len = (int)(((long long)p.NT * p.H + sms - 1) / sms);
+    len = std::max(len, (int)ceil(sqrt(longest / 6.0)));
+    const double split = 1.8 * len + longest / len / 3.0 + 4.0;
+    return split < 0.9 * whole ? len : 0;
+}
+
+int segment_count(const KdaParams& p) {
+    if (p.dtype != KDA_DTYPE_BF16 || p.dk != 128 || p.dv != 128 || p.NT <= 0 || p.N <= 0) return 0;
+    if (p.flags & (KDA_FLAG_FORCE_SIMT | (3 << 6))) return 0;  // a state stage in FP32 arithmetic
+    const int len = segment_length(p);
+    return len > 0 ? (p.NT + len - 1) / len : 0;
+}
+
+StateSegs state_segs(const KdaParams& p, bool bwd) {
+    StateSegs r = {};
+    r.count = segment_count(p);
+    if (r.count == 0) return r;
+    r.len = segment_length(p);
+    const size_t m = seg_matrix_floats(r.count, p.H, p.dk);
+    const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
+    const bool nosave = p.flags & KDA_FLAG_NO_SAVE;
+    float* f = (float*)((char*)p.workspace + (nosave ? L.total_nosave : p.conv_q ? L.total_conv : L.total));
+    r.E = f;
+    r.X = f + m;
+    r.XT = nosave ? nullptr : f + 2 * m;
+    if (bwd) r.E = (float*)((char*)p.bwd_scratch + (p.conv_q ? L.bwd_total_conv : L.bwd_total));
+    return r;
+}
+
+cudaError_t launch_seg_combine(const KdaParams& p, const StateSegs& segs, bool bwd, cudaStream_t s) {
+    auto kern = bwd ? kda_seg_combine<true> : kda_seg_combine<false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc::TOTAL);
+    if (e != cudaSuccess) return e;
+    kern<<<dim3(sc::D / sc::ROWS, p.H, p.N), sc::NTHR, sc::TOTAL, s>>>(p, segs);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fwd_segments(const KdaParams& p, const StateSegs& segs, cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(kda_fwd_segment_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sg::TOTAL);
+    if (e != cudaSuccess) return e;
+    kda_fwd_segment_tc<<<dim3(p.H, segs.count), sg::NTHR, sg::TOTAL, s>>>(p, segs);
+    return launch_seg_combine(p, segs, false, s);
+}
+
+}  // namespace kda

@@ -165,7 +165,8 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
     }
 }
 
-__global__ void __launch_bounds__(fs::NTHR, 1) kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps) {
+__global__ void __launch_bounds__(fs::NTHR, 1)
+kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const StateSegs segs) {
     using namespace fs;
     extern __shared__ __align__(128) unsigned char dyn[];
     __shared__ uint64_t full[2];
@@ -174,11 +175,19 @@ __global__ void __launch_bounds__(fs::NTHR, 1) kda_fwd_state_tc(const KdaParams 
     // thread (half, e) = (tid / 128, tid % 128): TMEM lane e (value column e), and half of the accumulator
     // columns in every conversion phase (two warps share a lane quadrant)
     const int tid = threadIdx.x, warp = tid >> 5, e = tid & 127, half = tid >> 7;
-    const int h = blockIdx.x, n = blockIdx.y;
-    int c0, nc;
-    seq_chunks(p, n, c0, nc);
-    long long tok_first, tok_end;
-    seq_tokens(p, n, tok_first, tok_end);
+    const int h = blockIdx.x;
+    // the chunks of this CTA: one sequence, or one segment of the chunk numbering
+    SeqCursor sq;
+    int cb, ce;
+    if (segs.len > 0) {
+        cb = blockIdx.y * segs.len;
+        ce = min(cb + segs.len, p.NT);
+        sq.load_of_chunk(p, cb);
+    } else {
+        sq.load(p, blockIdx.y);
+        cb = sq.c_begin;
+        ce = sq.c_end;
+    }
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     char* ws = (char*)p.workspace;
     if (warp == 0) {
@@ -197,22 +206,45 @@ __global__ void __launch_bounds__(fs::NTHR, 1) kda_fwd_state_tc(const KdaParams 
     tc_fence_after();
     const uint32_t tmem = tmem_s + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's lane quadrant
     const uint32_t tmem0 = tmem_s;
-    const size_t sbase = ((size_t)n * p.H + h) * D * D;
     const bool save = !(p.flags & KDA_FLAG_NO_SAVE);  // forward-only calls write no checkpoint and no V' record
 
-    for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
-        uint32_t r[16];
+    // state entering a sequence (h0 or zero), or the segment (what the previous one ended with)
+    auto init_state = [&](bool carried) {
+        const size_t sbase = ((size_t)sq.n * p.H + h) * D * D;
+        const float* E = carried ? segs.E + (((size_t)blockIdx.y - 1) * p.H + h) * D * D + (size_t)e * D : nullptr;
+        for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
+            uint32_t r[16];
+            if (carried) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(p.h0 ? p.h0[sbase + state_idx(p, d0 + j, e)] : 0.f);
-        tmem_st16(tmem + SACC + d0, r);
-    }
-    tmem_wait_st();
+                for (int j = 0; j < 4; ++j) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(E + d0 + 4 * j);
+                    r[4 * j] = x.x; r[4 * j + 1] = x.y; r[4 * j + 2] = x.z; r[4 * j + 3] = x.w;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(p.h0 ? p.h0[sbase + state_idx(p, d0 + j, e)] : 0.f);
+            }
+            tmem_st16(tmem + SACC + d0, r);
+        }
+        tmem_wait_st();
+    };
+    auto write_final = [&]() {
+        const size_t sbase = ((size_t)sq.n * p.H + h) * D * D;
+        for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
+            uint32_t r[16];
+            tmem_ld16(tmem + SACC + d0, r);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) p.ht[sbase + state_idx(p, d0 + j, e)] = __uint_as_float(r[j]);
+        }
+    };
+    init_state(cb > sq.c_begin);
 
     // the six records of a chunk: one copy each from lane 0 of six warps (a thread spends ~30 ns on every bulk
     // copy it issues, and the chunk step waits for the slowest thread)
-    auto issue_loads = [&](int lc, int stage) {
+    auto issue_loads = [&](int c, int stage) {
         if ((tid & 31) != 0 || warp >= 6) return;
-        const size_t rec = (size_t)(c0 + lc) * p.H + h;
+        const size_t rec = (size_t)c * p.H + h;
         unsigned char* b = dyn + stage * STAGE;
         if (warp == 0) {
             mbar_expect_tx(&full[stage], STAGE);
@@ -229,22 +261,25 @@ __global__ void __launch_bounds__(fs::NTHR, 1) kda_fwd_state_tc(const KdaParams 
             tma_load_1d(b + GAM, (const float*)(ws + L.gamC) + rec * D, 512, &full[stage]);
         }
     };
-    if (nc > 0) issue_loads(0, 0);
+    if (cb < ce) issue_loads(cb, 0);
 
     uint32_t mma_phase = 0;
     bool ok = true;
     KDA_PHASE_BEGIN();
     __nv_bfloat16* o = (__nv_bfloat16*)p.o;
-    for (int lc = 0; lc < nc; ++lc) {
-        const int stage = lc & 1;
+    for (int c = cb; c < ce; ++c) {
+        const int stage = (c - cb) & 1;
         unsigned char* b = dyn + stage * STAGE;
-        const ChunkInfo ci = chunk_of_seq(n, lc, tok_first, tok_end);
-        const size_t rec = (size_t)(c0 + lc) * p.H + h;
+        const size_t rec = (size_t)c * p.H + h;
         // the next chunk's records are requested first thing (the other stage was last read by the previous
         // chunk's MMAs, which completed before that chunk's iteration ended): a whole chunk step ahead of their use
-        if (lc + 1 < nc) issue_loads(lc + 1, stage ^ 1);
+        if (c + 1 < ce) issue_loads(c + 1, stage ^ 1);
         tma_store_wait_read();  // the previous chunk's output rows have left the staging tile
-        ok = mbar_wait(&full[stage], (lc >> 1) & 1, p, 2);
+        if (c == sq.c_end) {  // (segments only) the walk enters the next sequence
+            sq.load_of_chunk(p, c);
+            init_state(false);
+        }
+        ok = mbar_wait(&full[stage], ((c - cb) >> 1) & 1, p, 2);
         if (!__syncthreads_and(ok)) { ok = false; break; }
         KDA_PHASE(0);
 
@@ -362,27 +397,22 @@ __global__ void __launch_bounds__(fs::NTHR, 1) kda_fwd_state_tc(const KdaParams 
             }
             fence_async_smem();
             __syncthreads();
-            if (maps.ok && ci.len == C) {  // the whole tile with one bulk-tensor store
+            const long long tok0 = sq.tok(c);
+            const int len = sq.rows(c);
+            if (maps.ok && len == C) {  // the whole tile with one bulk-tensor store
                 if (tid == 0) {
-                    tma_store_tile(&maps.m[0], h * D, (int)ci.tok0, sO);
+                    tma_store_tile(&maps.m[0], h * D, (int)tok0, sO);
                     tma_store_commit();
                 }
-            } else if (tid < ci.len) {
-                tma_store_1d(o + ((size_t)(ci.tok0 + tid) * p.H + h) * D, sO + tid * D, D * 2);
+            } else if (tid < len) {
+                tma_store_1d(o + ((size_t)(tok0 + tid) * p.H + h) * D, sO + tid * D, D * 2);
                 tma_store_commit();
             }
         }
+        if (c + 1 == sq.c_end && p.ht) write_final();
         KDA_PHASE(5);
     }
-    if (ok && p.ht) {
-        for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
-            uint32_t r[16];
-            tmem_ld16(tmem + SACC + d0, r);
-            tmem_wait_ld();
-#pragma unroll
-            for (int j = 0; j < 16; ++j) p.ht[sbase + state_idx(p, d0 + j, e)] = __uint_as_float(r[j]);
-        }
-    }
+    if (ok && cb == ce && p.ht) write_final();  // a sequence without tokens hands its initial state on
     tma_store_wait_all();
     tc_fence_before();
     __syncthreads();
@@ -403,7 +433,10 @@ constexpr uint32_t TMA_BYTES = 16384 * 3 + 8192 + 512;
 constexpr uint32_t SACC = 0, SBF = 128, VACC = 192, VBF = 256, TMEM_COLS = 512;
 }  // namespace bs
 
-__global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams p) {
+// PARTIAL (segments only): the contribution of the segment's own dO to the dS at its start, from a zero dS at its end where
+// the sequence goes on behind it; nothing else is stored.
+template <bool PARTIAL>
+__global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams p, const StateSegs segs) {
     using namespace bs;
     extern __shared__ __align__(128) unsigned char dyn[];
     __shared__ uint64_t full[3];  // three stages: the records of a chunk are requested two chunk steps ahead of their use
@@ -411,11 +444,26 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
     __shared__ uint32_t tmem_s;
     // thread (half, e) = (tid / 128, tid % 128): TMEM lane e, and half of the columns of every conversion phase
     const int tid = threadIdx.x, warp = tid >> 5, e = tid & 127, half = tid >> 7;
-    const int h = blockIdx.x, n = blockIdx.y;
-    int c0, nc;
-    seq_chunks(p, n, c0, nc);
-    long long tok_first, tok_end;
-    seq_tokens(p, n, tok_first, tok_end);
+    const int h = blockIdx.x;
+    // the chunks of this CTA, walked from the last to the first: one sequence, or one segment of the chunk numbering
+    SeqCursor sq;  // sequence of the current chunk
+    int cb, ce;
+    if (segs.len > 0) {
+        cb = blockIdx.y * segs.len;
+        ce = min(cb + segs.len, p.NT);
+        if (PARTIAL) {  // only the sequence that the segment's first chunk continues has anyone to hand its dS to
+            sq.load_of_chunk(p, cb);
+            if (sq.c_begin == cb) return;
+            ce = min(ce, sq.c_end);
+        } else {
+            sq.load_of_chunk(p, ce - 1);
+        }
+    } else {
+        sq.load(p, blockIdx.y);
+        cb = sq.c_begin;
+        ce = sq.c_end;
+    }
+    const int nc = ce - cb;
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     const char* ws = (const char*)p.workspace;
     char* sc = (char*)p.bwd_scratch;
@@ -437,20 +485,46 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
     tc_fence_after();
     const uint32_t tmem = tmem_s + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t tmem0 = tmem_s;
-    const size_t sbase = ((size_t)n * p.H + h) * D * D;
 
-    for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
-        uint32_t r[16];
+    // dS at the end of a sequence (grad_ht or zero), or of the segment (what the next one found at its start)
+    auto init_state = [&](bool carried) {
+        const size_t sbase = ((size_t)sq.n * p.H + h) * D * D;
+        const float* E = carried ? segs.E + (((size_t)blockIdx.y + 1) * p.H + h) * D * D + (size_t)e * D : nullptr;
+        for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
+            uint32_t r[16];
+            if (carried && !PARTIAL) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(p.grad_ht ? p.grad_ht[sbase + state_idx(p, d0 + j, e)] : 0.f);
-        tmem_st16(tmem + SACC + d0, r);
-    }
-    tmem_wait_st();
+                for (int j = 0; j < 4; ++j) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(E + d0 + 4 * j);
+                    r[4 * j] = x.x; r[4 * j + 1] = x.y; r[4 * j + 2] = x.z; r[4 * j + 3] = x.w;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    r[j] = __float_as_uint(p.grad_ht && !carried ? p.grad_ht[sbase + state_idx(p, d0 + j, e)] : 0.f);
+            }
+            tmem_st16(tmem + SACC + d0, r);
+        }
+        tmem_wait_st();
+    };
+    auto write_dh0 = [&]() {
+        const size_t sbase = ((size_t)sq.n * p.H + h) * D * D;
+        for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
+            uint32_t r[16];
+            tmem_ld16(tmem + SACC + d0, r);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) p.grad_h0[sbase + state_idx(p, d0 + j, e)] = __uint_as_float(r[j]);
+        }
+    };
+    init_state(ce < sq.c_end);
 
-    // step k = 0..nc-1 processes chunk lc = nc-1-k
+    // step k = 0..nc-1 processes chunk ce-1-k
+    SeqCursor sl = sq;  // sequence of the chunk whose loads are issued
     auto issue_loads = [&](int k, int stage) {
-        const int lc = nc - 1 - k;
-        const size_t rec = (size_t)(c0 + lc) * p.H + h;
+        const int c = ce - 1 - k;
+        const size_t rec = (size_t)c * p.H + h;
+        sl.move_to(p, c);
         unsigned char* b = dyn + stage * STAGE;
         if ((tid & 31) == 0) {  // one bulk copy each from lane 0 of five warps
             if (warp == 0) {
@@ -467,12 +541,13 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
             }
         }
         // dO tile -> core-matrix layout cm(i, e; 128), 16-byte chunks, zero rows past the end
-        const ChunkInfo ci = chunk_of_seq(n, lc, tok_first, tok_end);
+        const long long tok0 = sl.tok(c);
+        const int len = sl.rows(c);
         __nv_bfloat16* sdo = reinterpret_cast<__nv_bfloat16*>(b + DO);
         for (int q = tid; q < C * (D / 8); q += NTHR) {
             const int i = q >> 4, e8 = (q & 15) * 8;
-            const bool valid = i < ci.len;
-            const size_t row = (size_t)(ci.tok0 + (valid ? i : 0)) * p.H + h;
+            const bool valid = i < len;
+            const size_t row = (size_t)(tok0 + (valid ? i : 0)) * p.H + h;
             cp_async16_z(sdo + cm_idx(i, e8, D), dO + row * D + e8, valid);
         }
         cp_async_commit();
@@ -484,9 +559,13 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
     int stage = 0;
     uint32_t ring_phase = 0;  // parity of full[stage]: flips every time the ring wraps
     for (int k = 0; k < nc; ++k) {
-        const int lc = nc - 1 - k;
+        const int c = ce - 1 - k;
         unsigned char* b = dyn + stage * STAGE;
-        const size_t rec = (size_t)(c0 + lc) * p.H + h;
+        const size_t rec = (size_t)c * p.H + h;
+        if (c < sq.c_begin) {  // (segments only) the walk enters the previous sequence
+            sq.load_of_chunk(p, c);
+            init_state(false);
+        }
         if (k + 2 < nc) {  // (the stage behind this one was last read by the previous step's MMAs, which have completed)
             issue_loads(k + 2, stage == 0 ? 2 : stage - 1);
             cp_async_wait<2>();
@@ -509,8 +588,10 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
 #pragma unroll
                 for (int j = 0; j < 8; ++j) pk[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
                 tmem_st8(tmem + SBF + d0 / 2, pk);
-                *reinterpret_cast<uint4*>(gdS + cm_idx(e, d0, D)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                *reinterpret_cast<uint4*>(gdS + cm_idx(e, d0 + 8, D)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                if (!PARTIAL) {
+                    *reinterpret_cast<uint4*>(gdS + cm_idx(e, d0, D)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                    *reinterpret_cast<uint4*>(gdS + cm_idx(e, d0 + 8, D)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                }
 #pragma unroll
                 for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * gam[d0 + j]);
                 tmem_st16(tmem + SACC + d0, r);
@@ -554,8 +635,10 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
 #pragma unroll
                 for (int j = 0; j < 8; ++j) pk[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
                 tmem_st8(tmem + VBF + i0 / 2, pk);
-                *reinterpret_cast<uint4*>(gdV + cm_idx(e, i0, C)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                *reinterpret_cast<uint4*>(gdV + cm_idx(e, i0 + 8, C)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                if (!PARTIAL) {
+                    *reinterpret_cast<uint4*>(gdV + cm_idx(e, i0, C)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                    *reinterpret_cast<uint4*>(gdV + cm_idx(e, i0 + 8, C)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                }
             }
             tmem_wait_st();
         }
@@ -573,18 +656,22 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
         ok = mbar_wait(&mmabar2, k & 1, p, 4);
         tc_fence_after();
         if (!__syncthreads_and(ok)) { ok = false; break; }
+        if (!PARTIAL && c == sq.c_begin && p.grad_h0) write_dh0();
         if (++stage == 3) {
             stage = 0;
             ring_phase ^= 1;
         }
     }
-    if (ok && p.grad_h0) {
+    if (!PARTIAL && ok && nc == 0 && p.grad_h0) write_dh0();  // a sequence without tokens
+    if (PARTIAL && ok) {
+        float* E = segs.E + ((size_t)blockIdx.y * p.H + h) * D * D + (size_t)e * D;
         for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
             uint32_t r[16];
             tmem_ld16(tmem + SACC + d0, r);
             tmem_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 16; ++j) p.grad_h0[sbase + state_idx(p, d0 + j, e)] = __uint_as_float(r[j]);
+            for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<uint4*>(E + d0 + 4 * j) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
         }
     }
     cp_async_wait<0>();
@@ -597,6 +684,9 @@ cudaError_t simt_stage(const KdaParams& p, int stage, cudaStream_t s);
 cudaError_t launch_fwd_intra_tc(const KdaParams& p, cudaStream_t s);
 cudaError_t launch_bwd_intra(const KdaParams& p, cudaStream_t s);
 cudaError_t launch_bwd_wy_tc(const KdaParams& p, cudaStream_t s);
+StateSegs state_segs(const KdaParams& p, bool bwd);
+cudaError_t launch_fwd_segments(const KdaParams& p, const StateSegs& segs, cudaStream_t s);
+cudaError_t launch_seg_combine(const KdaParams& p, const StateSegs& segs, bool bwd, cudaStream_t s);
 void prof_mark(cudaStream_t s);
 
 enum { ST_FWD_INTRA = 0, ST_FWD_STATE = 1, ST_BWD_STATE = 2, ST_BWD_CHUNK = 3, ST_PARAM_REDUCE = 4 };
@@ -612,12 +702,14 @@ cudaError_t tc_fwd(const KdaParams& p, cudaStream_t s) {
     if (stage_simt(p, ST_FWD_STATE)) {
         if ((e = simt_stage(p, ST_FWD_STATE, s)) != cudaSuccess) return e;
     } else {
+        const StateSegs segs = state_segs(p, false);
+        if (segs.len > 0 && (e = launch_fwd_segments(p, segs, s)) != cudaSuccess) return e;
         constexpr int smem = fs::TOTAL;
         if ((e = cudaFuncSetAttribute(kda_fwd_state_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
             return e;
         RowMaps maps = {};
         maps.ok = !(p.flags & KDA_FLAG_ROW_COPIES) && make_row_map(&maps.m[0], p.o, (long long)p.B * p.T, p.H, C);
-        kda_fwd_state_tc<<<dim3(p.H, p.N), fs::NTHR, smem, s>>>(p, maps);
+        kda_fwd_state_tc<<<dim3(p.H, segs.len > 0 ? segs.count : p.N), fs::NTHR, smem, s>>>(p, maps, segs);
     }
     prof_mark(s);
     return cudaGetLastError();
@@ -629,9 +721,16 @@ cudaError_t tc_bwd(const KdaParams& p, cudaStream_t s) {
         if ((e = simt_stage(p, ST_BWD_STATE, s)) != cudaSuccess) return e;
     } else {
         constexpr int smem = 3 * bs::STAGE;
-        if ((e = cudaFuncSetAttribute(kda_bwd_state_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
+        if ((e = cudaFuncSetAttribute(kda_bwd_state_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
             return e;
-        kda_bwd_state_tc<<<dim3(p.H, p.N), bs::NTHR, smem, s>>>(p);
+        const StateSegs segs = state_segs(p, true);
+        if (segs.len > 0) {
+            if ((e = cudaFuncSetAttribute(kda_bwd_state_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
+                return e;
+            kda_bwd_state_tc<true><<<dim3(p.H, segs.count), bs::NTHR, smem, s>>>(p, segs);
+            if ((e = launch_seg_combine(p, segs, true, s)) != cudaSuccess) return e;
+        }
+        kda_bwd_state_tc<false><<<dim3(p.H, segs.len > 0 ? segs.count : p.N), bs::NTHR, smem, s>>>(p, segs);
     }
     prof_mark(s);
     if (stage_simt(p, ST_BWD_CHUNK)) {  // fused FP32-math kernel

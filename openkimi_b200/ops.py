@@ -34,7 +34,7 @@ def _chunk_tables_cached(cu: tuple, device_index: int):
     dev = torch.device("cuda", device_index)
     return (torch.tensor(seq if seq else [0], dtype=torch.int32, device=dev),
             torch.tensor(off, dtype=torch.int32, device=dev), off[-1],
-            torch.tensor(tab if tab else [(0, 0, 0, 0)], dtype=torch.int32, device=dev))
+            torch.tensor(tab if tab else [(0, 0, 0, 0)], dtype=torch.int32, device=dev), max(counts, default=0))
 
 
 def _chunk_tables(cu_seqlens, cu_seqlens_cpu, device):
@@ -46,11 +46,12 @@ def _chunk_tables(cu_seqlens, cu_seqlens_cpu, device):
 
 
 def _packed_tables(cu_seqlens, cu_seqlens_cpu, device):
-    """(cu_seqlens, chunk_seq, seq_chunk_off, chunk_tab, number of chunks) as the native calls take them."""
+    """(cu_seqlens, chunk_seq, seq_chunk_off, chunk_tab, number of chunks, chunks of the longest document) as the native
+    calls take them."""
     if cu_seqlens is None:
-        return None, None, None, None, 0
-    seq, off, nt, tab = _chunk_tables(cu_seqlens, cu_seqlens_cpu, device)
-    return cu_seqlens.to(device=device, dtype=torch.int64).contiguous(), seq, off, tab, nt
+        return None, None, None, None, 0, 0
+    seq, off, nt, tab, longest = _chunk_tables(cu_seqlens, cu_seqlens_cpu, device)
+    return cu_seqlens.to(device=device, dtype=torch.int64).contiguous(), seq, off, tab, nt, longest
 
 
 class _DeviceStatus:
