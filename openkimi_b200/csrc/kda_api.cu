@@ -15,11 +15,10 @@ cudaError_t tc_bwd(const KdaParams& p, cudaStream_t s);
 bool tc_supported(const KdaParams& p);
 int segment_count(const KdaParams& p);
 
-// bytes of the segment buffers behind the workspace (state at every border, transitions, their transposes for the
-// backward) and behind the backward scratch
+// bytes of the segment buffers behind the workspace (state at every border, transitions) and behind the backward scratch
 static size_t segment_bytes(const KdaParams& p, bool bwd) {
     const size_t m = seg_matrix_floats(segment_count(p), p.H, p.dk) * sizeof(float);
-    return bwd ? m : m * ((p.flags & KDA_FLAG_NO_SAVE) ? 2 : 3);
+    return bwd ? m : 2 * m;
 }
 
 static thread_local char g_last_error[256] = "";

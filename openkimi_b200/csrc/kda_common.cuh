@@ -142,9 +142,9 @@ __device__ __forceinline__ void seq_tokens(const KdaParams& p, int n, long long&
 // the global chunk numbering, whatever sequences they belong to; len == 0: a CTA walks one whole sequence.
 struct StateSegs {
     int len, count;
-    float* E;   // [count][H][dv][dk]: transposed state at the end of the segment (backward: at its start)
-    float* X;   // [count][H][dk][dk]: transition of a segment that lies inside one sequence, S_end^T = S_begin^T X + E_local
-    float* XT;  // its transpose, for the backward; NULL when nothing is kept
+    float* E;   // [count][H][dk][dv]: state at the end of the segment (backward: at its start)
+    float* X;   // [count][H] transitions of the segments that lie inside one sequence, S_end^T = S_begin^T X + E_local^T,
+                // as X^T with the 16-byte chunks of row r XOR-swizzled by r mod 32
 };
 
 // sequence of a chunk and the ranges a walk along the chunks needs; reloaded only where the walk enters another sequence

@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "kda_common.cuh"
+#include "kda_state.cuh"
 #include "kda_tc.cuh"
 
 namespace kda {
@@ -30,6 +31,11 @@ constexpr uint32_t WT = 0, UT = 16384, KH = 32768, GAM = 49152, STAGE = 49664, T
 // tensor memory of one half: state, BF16 copy (V' takes its place once the first product has read it), first product
 constexpr uint32_t SACC = 0, SBF = 128, WSACC = 192, HALF_COLS = 256, TMEM_COLS = 512;
 }  // namespace sg
+
+// X is kept as X^T, chunks of row r swizzled by r: consecutive lanes write it coalesced (lane = row of X), and it can be
+// read from a linear copy in shared memory without bank conflicts both along rows (backward) and by threads that own
+// one row each (forward)
+__device__ __forceinline__ int xt_idx(int r, int c) { return r * 128 + ((((c >> 2) ^ (r & 31)) << 2) | (c & 3)); }
 
 __global__ void __launch_bounds__(sg::NTHR, 1) kda_fwd_segment_tc(const KdaParams p, const StateSegs segs) {
     using namespace sg;
@@ -64,20 +70,16 @@ __global__ void __launch_bounds__(sg::NTHR, 1) kda_fwd_segment_tc(const KdaParam
     const uint32_t tmem0 = tmem_s + part * HALF_COLS;
     const uint32_t tmem = tmem0 + ((uint32_t)((warp & 3) * 32) << 16);
     const bool on = part == 0 || inside;
-    if (on) {
-        const size_t sbase = ((size_t)sq.n * p.H + h) * D * D;
+    if (part == 1) {  // identity
         for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
             uint32_t r[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                float v = 0.f;
-                if (part == 1) v = d0 + j == e ? 1.f : 0.f;
-                else if (!inside && p.h0) v = p.h0[sbase + state_idx(p, d0 + j, e)];
-                r[j] = __float_as_uint(v);
-            }
+            for (int j = 0; j < 16; ++j) r[j] = d0 + j == e ? __float_as_uint(1.f) : 0u;
             tmem_st16(tmem + SACC + d0, r);
         }
         tmem_wait_st();
+    } else {
+        state_fill(tmem + SACC, inside ? nullptr : state_of(p.h0, p, sq.n, h), p.flags & KDA_FLAG_STATE_V_FIRST, nullptr, tid, e, half);
     }
     auto issue_loads = [&](int c, int stage) {
         if ((tid & 31) != 0 || warp >= 4) return;
@@ -171,17 +173,15 @@ __global__ void __launch_bounds__(sg::NTHR, 1) kda_fwd_segment_tc(const KdaParam
     }
     if (ok && on) {
         const size_t base = ((size_t)seg * p.H + h) * D * D;
-        float* dst = (part == 0 ? segs.E : segs.X) + base + (size_t)e * D;
-        for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
-            uint32_t r[16];
-            tmem_ld16(tmem + SACC + d0, r);
-            tmem_wait_ld();
+        if (part == 0) {
+            state_drain(tmem + SACC, segs.E + base, false, nullptr, tid, e, half);
+        } else {
+            for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
+                uint32_t r[16];
+                tmem_ld16(tmem + SACC + d0, r);
+                tmem_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                *reinterpret_cast<uint4*>(dst + d0 + 4 * j) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-            if (part == 1 && segs.XT) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) segs.XT[base + (size_t)(d0 + j) * D + e] = __uint_as_float(r[j]);
+                for (int j = 0; j < 16; ++j) segs.X[base + xt_idx(d0 + j, e)] = __uint_as_float(r[j]);
             }
         }
     }
@@ -192,10 +192,10 @@ __global__ void __launch_bounds__(sg::NTHR, 1) kda_fwd_segment_tc(const KdaParam
 
 // Step 2.  One CTA per (sequence, head, eight rows of S^T): E of every segment that a sequence leaves becomes the true
 // state there.  Thread = two columns x a quarter of the inner index; X arrives by bulk copies, two segments in flight
-// (64 KB per step and CTA from L2: about 0.7 us, as long as the arithmetic).
+// (64 KB per step and CTA from L2 take about as long as the arithmetic, in packed FP32 pairs).
 namespace sc {
 constexpr int D = 128, ROWS = 8, NTHR = 256;
-constexpr uint32_t XT0 = 0, XBYTES = D * D * 4, ST = 2 * XBYTES, PART = ST + D * ROWS * 4, TOTAL = PART + 4 * ROWS * D * 4;
+constexpr uint32_t XBYTES = D * D * 4, ST = 2 * XBYTES, PART = ST + D * ROWS * 4, TOTAL = PART + 4 * ROWS * D * 4;
 }  // namespace sc
 
 template <bool BWD>
@@ -225,59 +225,76 @@ __global__ void __launch_bounds__(sc::NTHR, 1) kda_seg_combine(const KdaParams p
         mbar_fence_init();
     }
     __syncthreads();
-    const float* X = BWD ? segs.XT : segs.X;
     auto mat = [&](int k) { return ((size_t)(BWD ? sz - k : sa + k) * p.H + h) * D * D; };  // k-th segment from the known end
     auto issue = [&](int k) {
         if (tid == 0) {
             mbar_expect_tx(&full[k & 1], XBYTES);
-            tma_load_1d(dyn + XT0 + (k & 1) * XBYTES, X + mat(k), XBYTES, &full[k & 1]);
+            tma_load_1d(dyn + (k & 1) * XBYTES, segs.X + mat(k), XBYTES, &full[k & 1]);
         }
     };
-    float* S = reinterpret_cast<float*>(dyn + ST);      // [d][row]
-    float* part = reinterpret_cast<float*>(dyn + PART);  // [quarter][row][column]
+    float* S = reinterpret_cast<float*>(dyn + ST);       // [d][row]
+    float* part = reinterpret_cast<float*>(dyn + PART);  // [quarter][column][row]
     issue(1);
     if (steps > 1) issue(2);
-    for (int i = tid; i < ROWS * D; i += NTHR) S[(i & (D - 1)) * ROWS + i / D] = segs.E[mat(0) + (size_t)(e0 + i / D) * D + (i & (D - 1))];
-    const int col = 2 * (tid & 63), quarter = tid >> 6;
+    // thread's share of the eight rows: four of one column d
+    const int md = tid >> 1, mr = 4 * (tid & 1);
+    *reinterpret_cast<float4*>(S + md * ROWS + mr) = *reinterpret_cast<const float4*>(segs.E + mat(0) + (size_t)md * D + e0 + mr);
+    const int lane64 = tid & 63, quarter = tid >> 6;
     for (int k = 1; k <= steps; ++k) {
-        float* E = segs.E + mat(k) + (size_t)e0 * D;
-        float own[ROWS * D / NTHR];
-#pragma unroll
-        for (int i = 0; i < ROWS * D / NTHR; ++i) own[i] = E[tid + NTHR * i];
+        float4* E = reinterpret_cast<float4*>(segs.E + mat(k) + (size_t)md * D + e0 + mr);
+        const float4 own = *E;
         const bool ok = mbar_wait(&full[k & 1], ((k - 1) >> 1) & 1, p, 2);
         if (!__syncthreads_and(ok)) {
             if (k < steps) mbar_wait(&full[(k + 1) & 1], (k >> 1) & 1, p, 2);  // the other copy in flight
             return;
         }
-        const float* x = reinterpret_cast<const float*>(dyn + XT0 + (k & 1) * XBYTES);
-        float acc[ROWS][2];
+        const float* x = reinterpret_cast<const float*>(dyn + (k & 1) * XBYTES);
+        float2 acc[2][ROWS / 2];  // two columns, pairs of rows
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) acc[r][0] = acc[r][1] = 0.f;
-#pragma unroll 8
-        for (int d = quarter * (D / 4); d < (quarter + 1) * (D / 4); ++d) {
-            const float2 xv = *reinterpret_cast<const float2*>(x + d * D + col);
-            const float4 s0 = *reinterpret_cast<const float4*>(S + d * ROWS), s1 = *reinterpret_cast<const float4*>(S + d * ROWS + 4);
-            const float sv[ROWS] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+        for (int r = 0; r < ROWS / 2; ++r) acc[0][r] = acc[1][r] = make_float2(0.f, 0.f);
+        const int colA = BWD ? 2 * lane64 : lane64, colB = BWD ? 2 * lane64 + 1 : lane64 + 64;
+#pragma unroll 2
+        for (int d = quarter * (D / 4); d < (quarter + 1) * (D / 4); d += 4) {
+            float xa[4], xb[4];
+            if (BWD) {
 #pragma unroll
-            for (int r = 0; r < ROWS; ++r) {
-                acc[r][0] = fmaf(sv[r], xv.x, acc[r][0]);
-                acc[r][1] = fmaf(sv[r], xv.y, acc[r][1]);
+                for (int j = 0; j < 4; ++j) {
+                    const float2 v = *reinterpret_cast<const float2*>(x + xt_idx(d + j, colA));
+                    xa[j] = v.x; xb[j] = v.y;
+                }
+            } else {
+                const float4 va = *reinterpret_cast<const float4*>(x + xt_idx(colA, d)), vb = *reinterpret_cast<const float4*>(x + xt_idx(colB, d));
+                xa[0] = va.x; xa[1] = va.y; xa[2] = va.z; xa[3] = va.w;
+                xb[0] = vb.x; xb[1] = vb.y; xb[2] = vb.z; xb[3] = vb.w;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 s0 = *reinterpret_cast<const float4*>(S + (d + j) * ROWS), s1 = *reinterpret_cast<const float4*>(S + (d + j) * ROWS + 4);
+                const float2 sv[4] = {make_float2(s0.x, s0.y), make_float2(s0.z, s0.w), make_float2(s1.x, s1.y), make_float2(s1.z, s1.w)};
+                const float2 a2 = make_float2(xa[j], xa[j]), b2 = make_float2(xb[j], xb[j]);
+#pragma unroll
+                for (int r = 0; r < ROWS / 2; ++r) {
+                    acc[0][r] = __ffma2_rn(sv[r], a2, acc[0][r]);
+                    acc[1][r] = __ffma2_rn(sv[r], b2, acc[1][r]);
+                }
             }
         }
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r)
-            *reinterpret_cast<float2*>(part + (quarter * ROWS + r) * D + col) = make_float2(acc[r][0], acc[r][1]);
+        for (int c = 0; c < 2; ++c) {
+            float* dst = part + (quarter * D + (c ? colB : colA)) * ROWS;
+            *reinterpret_cast<float4*>(dst) = make_float4(acc[c][0].x, acc[c][0].y, acc[c][1].x, acc[c][1].y);
+            *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[c][2].x, acc[c][2].y, acc[c][3].x, acc[c][3].y);
+        }
         __syncthreads();
         if (k + 2 <= steps) issue(k + 2);
+        float4 v = own;
 #pragma unroll
-        for (int i = 0; i < ROWS * D / NTHR; ++i) {
-            const int at = tid + NTHR * i, r = at / D, d = at & (D - 1);
-            float v = own[i];
-#pragma unroll
-            for (int g = 0; g < 4; ++g) v += part[(g * ROWS + r) * D + d];
-            E[at] = v;
-            S[d * ROWS + r] = v;
+        for (int g = 0; g < 4; ++g) {
+            const float4 t = *reinterpret_cast<const float4*>(part + (g * D + md) * ROWS + mr);
+            v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
         }
+        *E = v;
+        *reinterpret_cast<float4*>(S + md * ROWS + mr) = v;
         __syncthreads();
     }
 }
@@ -315,7 +332,6 @@ StateSegs state_segs(const KdaParams& p, bool bwd) {
     float* f = (float*)((char*)p.workspace + (nosave ? L.total_nosave : p.conv_q ? L.total_conv : L.total));
     r.E = f;
     r.X = f + m;
-    r.XT = nosave ? nullptr : f + 2 * m;
     if (bwd) r.E = (float*)((char*)p.bwd_scratch + (p.conv_q ? L.bwd_total_conv : L.bwd_total));
     return r;
 }

@@ -1,5 +1,6 @@
 // Tensor-core (tcgen05 / TMEM) stages of the KDA op for BF16 operands.
 #include "kda_common.cuh"
+#include "kda_state.cuh"
 #include "kda_tc.cuh"
 #include "kda_tmap.cuh"
 
@@ -208,37 +209,13 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
     const uint32_t tmem0 = tmem_s;
     const bool save = !(p.flags & KDA_FLAG_NO_SAVE);  // forward-only calls write no checkpoint and no V' record
 
-    // state entering a sequence (h0 or zero), or the segment (what the previous one ended with)
-    auto init_state = [&](bool carried) {
-        const size_t sbase = ((size_t)sq.n * p.H + h) * D * D;
-        const float* E = carried ? segs.E + (((size_t)blockIdx.y - 1) * p.H + h) * D * D + (size_t)e * D : nullptr;
-        for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
-            uint32_t r[16];
-            if (carried) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint4 x = *reinterpret_cast<const uint4*>(E + d0 + 4 * j);
-                    r[4 * j] = x.x; r[4 * j + 1] = x.y; r[4 * j + 2] = x.z; r[4 * j + 3] = x.w;
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(p.h0 ? p.h0[sbase + state_idx(p, d0 + j, e)] : 0.f);
-            }
-            tmem_st16(tmem + SACC + d0, r);
-        }
-        tmem_wait_st();
-    };
-    auto write_final = [&]() {
-        const size_t sbase = ((size_t)sq.n * p.H + h) * D * D;
-        for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
-            uint32_t r[16];
-            tmem_ld16(tmem + SACC + d0, r);
-            tmem_wait_ld();
-#pragma unroll
-            for (int j = 0; j < 16; ++j) p.ht[sbase + state_idx(p, d0 + j, e)] = __uint_as_float(r[j]);
-        }
-    };
-    init_state(cb > sq.c_begin);
+    const bool vfirst = p.flags & KDA_FLAG_STATE_V_FIRST;
+    float* stage_space = reinterpret_cast<float*>(dyn);  // before the first and after the last chunk's copies
+    // state entering the segment (what the previous one ended with), or a sequence (h0 or zero)
+    if (cb > sq.c_begin)
+        state_fill(tmem + SACC, segs.E + (((size_t)blockIdx.y - 1) * p.H + h) * D * D, false, nullptr, tid, e, half);
+    else
+        state_fill(tmem + SACC, state_of(p.h0, p, sq.n, h), vfirst, stage_space, tid, e, half);
 
     // the six records of a chunk: one copy each from lane 0 of six warps (a thread spends ~30 ns on every bulk
     // copy it issues, and the chunk step waits for the slowest thread)
@@ -277,7 +254,7 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
         tma_store_wait_read();  // the previous chunk's output rows have left the staging tile
         if (c == sq.c_end) {  // (segments only) the walk enters the next sequence
             sq.load_of_chunk(p, c);
-            init_state(false);
+            state_fill(tmem + SACC, state_of(p.h0, p, sq.n, h), vfirst, nullptr, tid, e, half);
         }
         ok = mbar_wait(&full[stage], ((c - cb) >> 1) & 1, p, 2);
         if (!__syncthreads_and(ok)) { ok = false; break; }
@@ -409,10 +386,13 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
                 tma_store_commit();
             }
         }
-        if (c + 1 == sq.c_end && p.ht) write_final();
+        if (c + 1 == sq.c_end && c + 1 < ce && p.ht)
+            state_drain(tmem + SACC, const_cast<float*>(state_of(p.ht, p, sq.n, h)), vfirst, nullptr, tid, e, half);
         KDA_PHASE(5);
     }
-    if (ok && cb == ce && p.ht) write_final();  // a sequence without tokens hands its initial state on
+    // the sequence that ends with the last chunk (one without tokens hands its initial state on)
+    if (ok && ce == sq.c_end && p.ht)
+        state_drain(tmem + SACC, const_cast<float*>(state_of(p.ht, p, sq.n, h)), vfirst, stage_space, tid, e, half);
     tma_store_wait_all();
     tc_fence_before();
     __syncthreads();
@@ -486,38 +466,13 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
     const uint32_t tmem = tmem_s + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t tmem0 = tmem_s;
 
-    // dS at the end of a sequence (grad_ht or zero), or of the segment (what the next one found at its start)
-    auto init_state = [&](bool carried) {
-        const size_t sbase = ((size_t)sq.n * p.H + h) * D * D;
-        const float* E = carried ? segs.E + (((size_t)blockIdx.y + 1) * p.H + h) * D * D + (size_t)e * D : nullptr;
-        for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
-            uint32_t r[16];
-            if (carried && !PARTIAL) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint4 x = *reinterpret_cast<const uint4*>(E + d0 + 4 * j);
-                    r[4 * j] = x.x; r[4 * j + 1] = x.y; r[4 * j + 2] = x.z; r[4 * j + 3] = x.w;
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    r[j] = __float_as_uint(p.grad_ht && !carried ? p.grad_ht[sbase + state_idx(p, d0 + j, e)] : 0.f);
-            }
-            tmem_st16(tmem + SACC + d0, r);
-        }
-        tmem_wait_st();
-    };
-    auto write_dh0 = [&]() {
-        const size_t sbase = ((size_t)sq.n * p.H + h) * D * D;
-        for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
-            uint32_t r[16];
-            tmem_ld16(tmem + SACC + d0, r);
-            tmem_wait_ld();
-#pragma unroll
-            for (int j = 0; j < 16; ++j) p.grad_h0[sbase + state_idx(p, d0 + j, e)] = __uint_as_float(r[j]);
-        }
-    };
-    init_state(ce < sq.c_end);
+    const bool vfirst = p.flags & KDA_FLAG_STATE_V_FIRST;
+    float* stage_space = reinterpret_cast<float*>(dyn);  // before the first and after the last chunk's copies
+    // dS at the end of the segment (what the next one found at its start), or of a sequence (grad_ht or zero)
+    if (ce < sq.c_end)
+        state_fill(tmem + SACC, PARTIAL ? nullptr : segs.E + (((size_t)blockIdx.y + 1) * p.H + h) * D * D, false, nullptr, tid, e, half);
+    else
+        state_fill(tmem + SACC, state_of(p.grad_ht, p, sq.n, h), vfirst, stage_space, tid, e, half);
 
     // step k = 0..nc-1 processes chunk ce-1-k
     SeqCursor sl = sq;  // sequence of the chunk whose loads are issued
@@ -564,7 +519,7 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
         const size_t rec = (size_t)c * p.H + h;
         if (c < sq.c_begin) {  // (segments only) the walk enters the previous sequence
             sq.load_of_chunk(p, c);
-            init_state(false);
+            state_fill(tmem + SACC, state_of(p.grad_ht, p, sq.n, h), vfirst, nullptr, tid, e, half);
         }
         if (k + 2 < nc) {  // (the stage behind this one was last read by the previous step's MMAs, which have completed)
             issue_loads(k + 2, stage == 0 ? 2 : stage - 1);
@@ -656,25 +611,19 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
         ok = mbar_wait(&mmabar2, k & 1, p, 4);
         tc_fence_after();
         if (!__syncthreads_and(ok)) { ok = false; break; }
-        if (!PARTIAL && c == sq.c_begin && p.grad_h0) write_dh0();
+        if (!PARTIAL && c == sq.c_begin && c > cb && p.grad_h0)
+            state_drain(tmem + SACC, const_cast<float*>(state_of(p.grad_h0, p, sq.n, h)), vfirst, nullptr, tid, e, half);
         if (++stage == 3) {
             stage = 0;
             ring_phase ^= 1;
         }
     }
-    if (!PARTIAL && ok && nc == 0 && p.grad_h0) write_dh0();  // a sequence without tokens
-    if (PARTIAL && ok) {
-        float* E = segs.E + ((size_t)blockIdx.y * p.H + h) * D * D + (size_t)e * D;
-        for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
-            uint32_t r[16];
-            tmem_ld16(tmem + SACC + d0, r);
-            tmem_wait_ld();
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                *reinterpret_cast<uint4*>(E + d0 + 4 * j) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-        }
-    }
     cp_async_wait<0>();
+    if (PARTIAL) {
+        if (ok) state_drain(tmem + SACC, segs.E + ((size_t)blockIdx.y * p.H + h) * D * D, false, nullptr, tid, e, half);
+    } else if (ok && cb == sq.c_begin && p.grad_h0) {  // (a sequence without tokens hands grad_ht on)
+        state_drain(tmem + SACC, const_cast<float*>(state_of(p.grad_h0, p, sq.n, h)), vfirst, stage_space, tid, e, half);
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem0, TMEM_COLS);
