@@ -191,15 +191,17 @@ __global__ void __launch_bounds__(sg::NTHR, 1) kda_fwd_segment_tc(const KdaParam
 }
 
 // Step 2.  One CTA per (sequence, head, eight rows of S^T): E of every segment that a sequence leaves becomes the true
-// state there.  Thread = two columns x a quarter of the inner index; X arrives by bulk copies, two segments in flight
-// (64 KB per step and CTA from L2 take about as long as the arithmetic, in packed FP32 pairs).
+// state there.  Thread = two columns x a quarter of the inner index, in packed FP32 pairs; X arrives by bulk copies (64 KB
+// per step and CTA from L2, as long as the arithmetic).  Latency bound: with STAGES = 2 a CTA has the next segment's X in
+// flight, with STAGES = 1 two CTAs share an SM (more chains than one CTA per SM covers).
 namespace sc {
-constexpr int D = 128, ROWS = 8, NTHR = 256;
-constexpr uint32_t XBYTES = D * D * 4, ST = 2 * XBYTES, PART = ST + D * ROWS * 4, TOTAL = PART + 4 * ROWS * D * 4;
+constexpr int D = 128, ROWS = 8, NTHR = 256, GROUPS = NTHR / 64, OWN = D * ROWS / NTHR;
+constexpr uint32_t XBYTES = D * D * 4, SBYTES = D * ROWS * 4;
+constexpr uint32_t total(int stages) { return stages * XBYTES + SBYTES + GROUPS * SBYTES; }
 }  // namespace sc
 
-template <bool BWD>
-__global__ void __launch_bounds__(sc::NTHR, 1) kda_seg_combine(const KdaParams p, const StateSegs segs) {
+template <bool BWD, int STAGES>
+__global__ void __launch_bounds__(sc::NTHR, 3 - STAGES) kda_seg_combine(const KdaParams p, const StateSegs segs) {
     using namespace sc;
     extern __shared__ __align__(128) unsigned char dyn[];
     __shared__ uint64_t full[2];
@@ -228,33 +230,35 @@ __global__ void __launch_bounds__(sc::NTHR, 1) kda_seg_combine(const KdaParams p
     auto mat = [&](int k) { return ((size_t)(BWD ? sz - k : sa + k) * p.H + h) * D * D; };  // k-th segment from the known end
     auto issue = [&](int k) {
         if (tid == 0) {
-            mbar_expect_tx(&full[k & 1], XBYTES);
-            tma_load_1d(dyn + (k & 1) * XBYTES, segs.X + mat(k), XBYTES, &full[k & 1]);
+            const int st = STAGES == 2 ? k & 1 : 0;
+            mbar_expect_tx(&full[st], XBYTES);
+            tma_load_1d(dyn + st * XBYTES, segs.X + mat(k), XBYTES, &full[st]);
         }
     };
-    float* S = reinterpret_cast<float*>(dyn + ST);       // [d][row]
-    float* part = reinterpret_cast<float*>(dyn + PART);  // [quarter][column][row]
+    float* S = reinterpret_cast<float*>(dyn + STAGES * XBYTES);  // [d][row]
+    float* part = S + D * ROWS;                                   // [group][column][row]
     issue(1);
-    if (steps > 1) issue(2);
-    // thread's share of the eight rows: four of one column d
-    const int md = tid >> 1, mr = 4 * (tid & 1);
+    if (STAGES == 2 && steps > 1) issue(2);
+    // thread's share of the rows: OWN of one column d
+    const int md = tid / (ROWS / OWN), mr = OWN * (tid & (ROWS / OWN - 1));
+    static_assert(OWN == 4, "one 16-byte word");
     *reinterpret_cast<float4*>(S + md * ROWS + mr) = *reinterpret_cast<const float4*>(segs.E + mat(0) + (size_t)md * D + e0 + mr);
-    const int lane64 = tid & 63, quarter = tid >> 6;
+    const int lane64 = tid & 63, group = tid >> 6;
     for (int k = 1; k <= steps; ++k) {
         float4* E = reinterpret_cast<float4*>(segs.E + mat(k) + (size_t)md * D + e0 + mr);
         const float4 own = *E;
-        const bool ok = mbar_wait(&full[k & 1], ((k - 1) >> 1) & 1, p, 2);
+        const bool ok = STAGES == 2 ? mbar_wait(&full[k & 1], ((k - 1) >> 1) & 1, p, 2) : mbar_wait(&full[0], (k - 1) & 1, p, 2);
         if (!__syncthreads_and(ok)) {
-            if (k < steps) mbar_wait(&full[(k + 1) & 1], (k >> 1) & 1, p, 2);  // the other copy in flight
+            if (STAGES == 2 && k < steps) mbar_wait(&full[(k + 1) & 1], (k >> 1) & 1, p, 2);  // the other copy in flight
             return;
         }
-        const float* x = reinterpret_cast<const float*>(dyn + (k & 1) * XBYTES);
+        const float* x = reinterpret_cast<const float*>(dyn + (STAGES == 2 ? k & 1 : 0) * XBYTES);
         float2 acc[2][ROWS / 2];  // two columns, pairs of rows
 #pragma unroll
         for (int r = 0; r < ROWS / 2; ++r) acc[0][r] = acc[1][r] = make_float2(0.f, 0.f);
         const int colA = BWD ? 2 * lane64 : lane64, colB = BWD ? 2 * lane64 + 1 : lane64 + 64;
-#pragma unroll 2
-        for (int d = quarter * (D / 4); d < (quarter + 1) * (D / 4); d += 4) {
+#pragma unroll 4
+        for (int d = group * (D / GROUPS); d < (group + 1) * (D / GROUPS); d += 4) {
             float xa[4], xb[4];
             if (BWD) {
 #pragma unroll
@@ -269,8 +273,13 @@ __global__ void __launch_bounds__(sc::NTHR, 1) kda_seg_combine(const KdaParams p
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float4 s0 = *reinterpret_cast<const float4*>(S + (d + j) * ROWS), s1 = *reinterpret_cast<const float4*>(S + (d + j) * ROWS + 4);
-                const float2 sv[4] = {make_float2(s0.x, s0.y), make_float2(s0.z, s0.w), make_float2(s1.x, s1.y), make_float2(s1.z, s1.w)};
+                float2 sv[ROWS / 2];
+#pragma unroll
+                for (int r = 0; r < ROWS / 4; ++r) {
+                    const float4 t = *reinterpret_cast<const float4*>(S + (d + j) * ROWS + 4 * r);
+                    sv[2 * r] = make_float2(t.x, t.y);
+                    sv[2 * r + 1] = make_float2(t.z, t.w);
+                }
                 const float2 a2 = make_float2(xa[j], xa[j]), b2 = make_float2(xb[j], xb[j]);
 #pragma unroll
                 for (int r = 0; r < ROWS / 2; ++r) {
@@ -281,15 +290,16 @@ __global__ void __launch_bounds__(sc::NTHR, 1) kda_seg_combine(const KdaParams p
         }
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-            float* dst = part + (quarter * D + (c ? colB : colA)) * ROWS;
-            *reinterpret_cast<float4*>(dst) = make_float4(acc[c][0].x, acc[c][0].y, acc[c][1].x, acc[c][1].y);
-            *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[c][2].x, acc[c][2].y, acc[c][3].x, acc[c][3].y);
+            float* dst = part + (group * D + (c ? colB : colA)) * ROWS;
+#pragma unroll
+            for (int r = 0; r < ROWS / 4; ++r)
+                *reinterpret_cast<float4*>(dst + 4 * r) = make_float4(acc[c][2 * r].x, acc[c][2 * r].y, acc[c][2 * r + 1].x, acc[c][2 * r + 1].y);
         }
         __syncthreads();
-        if (k + 2 <= steps) issue(k + 2);
+        if (k + STAGES <= steps) issue(k + STAGES);
         float4 v = own;
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
+        for (int g = 0; g < GROUPS; ++g) {
             const float4 t = *reinterpret_cast<const float4*>(part + (g * D + md) * ROWS + mr);
             v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
         }
@@ -299,18 +309,22 @@ __global__ void __launch_bounds__(sc::NTHR, 1) kda_seg_combine(const KdaParams p
     }
 }
 
-// Segment length, 0 for whole sequences.  Estimated in chunk steps of 2.3 us: a whole-sequence walk takes as many as
-// the longest sequence has chunks, times the waves of sequences; segments of `len` take 1.8 len (both passes) plus a
-// third of a step per segment border of the longest sequence plus the launches.  len is what one wave of the chip needs,
-// but no shorter than what balances the border steps.
+// CTAs of step 2, counting one chain per sequence and head
+static long long combine_ctas(const KdaParams& p) { return (long long)p.N * p.H * (sc::D / sc::ROWS); }
+
+// Segment length, 0 for whole sequences, from the times measured on a B200 (us): a walk takes 6 plus 2.1 per chunk of the
+// longest sequence (the dependent chain) or 2.4 per chunk and SM (the records' traffic); both passes over segments of
+// `len` take 18 (three launches) plus 4.5 len plus 1.4 per segment border and wave of step 2.  len is what one wave of
+// the chip needs, but no shorter than what balances the border steps.
 static int segment_length(const KdaParams& p) {
     if (p.NT < 8) return 0;
-    const int sms = sm_count();
+    const double sms = sm_count();
     const double longest = p.max_chunks > 0 ? p.max_chunks : (double)p.NT / p.N;
-    const double whole = std::max(longest, (double)p.NT * p.H / sms);
-    int len = (int)(((long long)p.NT * p.H + sms - 1) / sms);
-    len = std::max(len, (int)ceil(sqrt(longest / 6.0)));
-    const double split = 1.8 * len + longest / len / 3.0 + 4.0;
+    const double per_sm = p.NT * (double)p.H / sms;
+    const double border = 1.4 * ceil(combine_ctas(p) / (2.0 * sms));
+    const int len = (int)ceil(std::max(per_sm, sqrt(longest * border / 4.5)));
+    const double whole = 6.0 + std::max(2.1 * longest, 2.4 * per_sm);
+    const double split = 18.0 + 4.5 * len + border * longest / len;
     return split < 0.9 * whole ? len : 0;
 }
 
@@ -337,10 +351,13 @@ StateSegs state_segs(const KdaParams& p, bool bwd) {
 }
 
 cudaError_t launch_seg_combine(const KdaParams& p, const StateSegs& segs, bool bwd, cudaStream_t s) {
-    auto kern = bwd ? kda_seg_combine<true> : kda_seg_combine<false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc::TOTAL);
+    const bool two = combine_ctas(p) > sm_count();  // two CTAs per SM
+    auto kern = bwd ? (two ? kda_seg_combine<true, 1> : kda_seg_combine<true, 2>)
+                    : (two ? kda_seg_combine<false, 1> : kda_seg_combine<false, 2>);
+    const int smem = (int)sc::total(two ? 1 : 2);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    kern<<<dim3(sc::D / sc::ROWS, p.H, p.N), sc::NTHR, sc::TOTAL, s>>>(p, segs);
+    kern<<<dim3(sc::D / sc::ROWS, p.H, p.N), sc::NTHR, smem, s>>>(p, segs);
     return cudaGetLastError();
 }
 
