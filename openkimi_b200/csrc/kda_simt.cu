@@ -19,45 +19,73 @@
 namespace kda {
 
 void prof_mark(cudaStream_t s);
+cudaError_t simt_state(const KdaParams& p, bool bwd, cudaStream_t s);  // kda_simt_state.cu
 
 constexpr int NTHREADS = 256;
 constexpr int KS = 16;  // k-slice of the tile product
+constexpr int CP = C + 4;  // row stride of the [64][64] matrices in shared memory: rows start on 16-byte boundaries
+
+// thread (ty, tx) = (tid / 16, tid % 16) owns rows 4 ty + r and columns col(tx, c) of a tile product
+__device__ __forceinline__ int tile_col(int tx, int c) { return 4 * tx + (c & 3) + 64 * (c >> 2); }
 
 // ---------------------------------------------------------------------------------------
-// acc[M/16][N/16] += A[M x K] * B[K x N], operands fetched through functors la(m,k), lb(k,n)
+// acc[4][N/16] += A[64 x K] * B[K x N], operands fetched through functors la(m,k), lb(k,n)
 // (from global or shared memory, any element type) and staged through shared memory in
-// slices of KS.  Thread (ty,tx) = (tid/16, tid%16) owns rows ty+16r and columns tx+16c.
+// slices of KS.  A thread's 4 x 4 (4 x 8) tile costs two (three) 16-byte shared loads per k;
+// the next slice is fetched into registers while the current one is worked on, and the two
+// staging buffers alternate, so that a slice costs one barrier and no exposed memory latency.
 // a_kfast / b_kfast say which index is contiguous in the operand's memory, so that the
 // staging loads coalesce.
 // ---------------------------------------------------------------------------------------
+template <int N>
+constexpr int st_floats() { return 2 * KS * (C + 4 + N + 4); }
+
 template <int M, int N, class LA, class LB>
-__device__ __forceinline__ void mm_tile(float (&acc)[M / 16][N / 16], int K, LA la, LB lb, float* st,
-                                        bool a_kfast, bool b_kfast) {
-    float* stA = st;
-    float* stB = st + KS * (M + 1);
+__device__ __forceinline__ void mm_tile(float (&acc)[4][N / 16], int K, LA la, LB lb, float* st, bool a_kfast, bool b_kfast) {
+    static_assert(M == C, "64 output rows");
+    constexpr int SA = M + 4, SB = N + 4, BUF = KS * (SA + SB), NA = M * KS / NTHREADS, NB = N * KS / NTHREADS;
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    for (int k0 = 0; k0 < K; k0 += KS) {
-        __syncthreads();
-        for (int idx = tid; idx < M * KS; idx += NTHREADS) {
-            int m, k;
-            if (a_kfast) { k = idx % KS; m = idx / KS; } else { m = idx % M; k = idx / M; }
-            stA[k * (M + 1) + m] = la(m, k0 + k);
+    float ra[NA], rb[NB];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < NA; ++u) {
+            const int idx = tid + NTHREADS * u;
+            ra[u] = a_kfast ? la(idx / KS, k0 + idx % KS) : la(idx % M, k0 + idx / M);
         }
-        for (int idx = tid; idx < N * KS; idx += NTHREADS) {
-            int n, k;
-            if (b_kfast) { k = idx % KS; n = idx / KS; } else { n = idx % N; k = idx / N; }
-            stB[k * (N + 1) + n] = lb(k0 + k, n);
+#pragma unroll
+        for (int u = 0; u < NB; ++u) {
+            const int idx = tid + NTHREADS * u;
+            rb[u] = b_kfast ? lb(k0 + idx % KS, idx / KS) : lb(k0 + idx / N, idx % N);
+        }
+    };
+    __syncthreads();  // operands in shared memory are complete
+    fetch(0);
+    for (int k0 = 0, buf = 0; k0 < K; k0 += KS, buf ^= 1) {
+        float *stA = st + buf * BUF, *stB = stA + KS * SA;
+#pragma unroll
+        for (int u = 0; u < NA; ++u) {
+            const int idx = tid + NTHREADS * u;
+            stA[a_kfast ? (idx % KS) * SA + idx / KS : (idx / M) * SA + idx % M] = ra[u];
+        }
+#pragma unroll
+        for (int u = 0; u < NB; ++u) {
+            const int idx = tid + NTHREADS * u;
+            stB[b_kfast ? (idx % KS) * SB + idx / KS : (idx / N) * SB + idx % N] = rb[u];
         }
         __syncthreads();
+        if (k0 + KS < K) fetch(k0 + KS);
 #pragma unroll
         for (int k = 0; k < KS; ++k) {
-            float a[M / 16], b[N / 16];
+            float a[4], b[N / 16];
+            const float4 av = *reinterpret_cast<const float4*>(stA + k * SA + 4 * ty);
+            a[0] = av.x; a[1] = av.y; a[2] = av.z; a[3] = av.w;
 #pragma unroll
-            for (int r = 0; r < M / 16; ++r) a[r] = stA[k * (M + 1) + ty + 16 * r];
+            for (int g = 0; g < N / 64; ++g) {
+                const float4 bv = *reinterpret_cast<const float4*>(stB + k * SB + 64 * g + 4 * tx);
+                b[4 * g] = bv.x; b[4 * g + 1] = bv.y; b[4 * g + 2] = bv.z; b[4 * g + 3] = bv.w;
+            }
 #pragma unroll
-            for (int c = 0; c < N / 16; ++c) b[c] = stB[k * (N + 1) + tx + 16 * c];
-#pragma unroll
-            for (int r = 0; r < M / 16; ++r)
+            for (int r = 0; r < 4; ++r)
 #pragma unroll
                 for (int c = 0; c < N / 16; ++c) acc[r][c] = fmaf(a[r], b[c], acc[r][c]);
         }
@@ -85,75 +113,104 @@ __device__ __forceinline__ float row16_sum(float v) {
 //   sq, sk  normalised q, k (x / max(||x||, 1e-6), k3mini/model.py:218-219) or raw
 //   sG      inclusive cumulative log2-decay of the chunk (rows >= len repeat the last value)
 //   sv      v (optional)          sbeta  beta after the optional sigmoid (0 on padding rows)
-//   srq,srk 1 / max(||x||, eps) per row (1 when the norm is not applied)
+//   srq,srk 1 / max(||x||, eps) per row (1 when the norm is not applied); scratch: 4 D floats
 // ---------------------------------------------------------------------------------------
+__device__ __forceinline__ float4 load_quad(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load_quad(const __nv_bfloat16* p) {
+    const uint2 r = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16),
+                       __uint_as_float(r.y & 0xffff0000u));
+}
+
 template <typename T, int D>
 __device__ __forceinline__ void load_prologue(const KdaParams& p, const ChunkInfo& ci, int h, float* sq, float* sk,
-                                              float* sG, float* sv, float* sbeta, float* srq, float* srk) {
+                                              float* sG, float* sv, float* sbeta, float* srq, float* srk, float* scratch) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const T* q = (const T*)p.q;
-    const T* k = (const T*)p.k;
-    const T* v = (const T*)p.v;
-    const T* g = (const T*)p.g;
-    const T* beta = (const T*)p.beta;
     const bool l2 = p.flags & KDA_FLAG_QK_L2NORM, gate = p.flags & KDA_FLAG_GATE, sig = p.flags & KDA_FLAG_BETA_SIGMOID;
     const float negA = gate ? -expf(p.A_log[h]) : 0.f;
-    for (int r = warp; r < C; r += NTHREADS / 32) {
-        const bool valid = r < ci.len;
-        const size_t row = (size_t)(ci.tok0 + r) * p.H + h;
-        float qv[D / 32], kv[D / 32];
-        float ssq = 0.f, ssk = 0.f;
+    // the rows of the chunk, four elements per access and all of a thread's accesses to a tensor in flight at once
+    constexpr int QN = C * D / 4 / NTHREADS;
+    auto rows_in = [&](const T* src, float* dst, bool is_gate) {
+        float4 x[QN];
 #pragma unroll
-        for (int m = 0; m < D / 32; ++m) {
-            int d = lane + 32 * m;
-            qv[m] = valid ? ldf(q + row * D + d) : 0.f;
-            kv[m] = valid ? ldf(k + row * D + d) : 0.f;
-            ssq += qv[m] * qv[m];
-            ssk += kv[m] * kv[m];
+        for (int u = 0; u < QN; ++u) {
+            const int idx = tid + NTHREADS * u, r = idx / (D / 4), d = idx % (D / 4) * 4;
+            x[u] = r < ci.len ? load_quad(src + ((size_t)(ci.tok0 + r) * p.H + h) * D + d) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
+#pragma unroll
+        for (int u = 0; u < QN; ++u) {
+            const int idx = tid + NTHREADS * u, r = idx / (D / 4), d = idx % (D / 4) * 4;
+            float4 y = x[u];
+            if (is_gate) {
+                float v[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (gate) v[j] = negA * softplus_f(v[j] + (p.dt_bias ? p.dt_bias[h * D + d + j] : 0.f));
+                    v[j] = r < ci.len ? v[j] * LOG2E : 0.f;
+                }
+                y = make_float4(v[0], v[1], v[2], v[3]);
+            }
+            *reinterpret_cast<float4*>(dst + r * D + d) = y;
+        }
+    };
+    rows_in((const T*)p.q, sq, false);
+    rows_in((const T*)p.k, sk, false);
+    rows_in((const T*)p.g, sG, true);
+    if (sv) rows_in((const T*)p.v, sv, false);
+    if (tid < C) {
+        float b = 0.f;
+        if (tid < ci.len) {
+            b = ldf((const T*)p.beta + (size_t)(ci.tok0 + tid) * p.H + h);
+            if (sig) b = sigmoid_f(b);
+        }
+        sbeta[tid] = b;
+    }
+    __syncthreads();
+    // cumulative gate: 16-row groups summed on their own, then the totals of the groups before are added
+    for (int it = tid; it < D * 4; it += NTHREADS) {
+        const int d = it % D, grp = it / D;
+        float run = 0.f;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            run += sG[(16 * grp + r) * D + d];
+            sG[(16 * grp + r) * D + d] = run;
+        }
+        scratch[it] = run;
+    }
+#pragma unroll 4
+    for (int r = warp; r < C; r += NTHREADS / 32) {
         float rq = 1.f, rk = 1.f;
         if (l2) {
+            float ssq = 0.f, ssk = 0.f;
+#pragma unroll
+            for (int m = 0; m < D / 32; ++m) {
+                const float a = sq[r * D + lane + 32 * m], b = sk[r * D + lane + 32 * m];
+                ssq += a * a;
+                ssk += b * b;
+            }
             ssq = warp_sum(ssq);
             ssk = warp_sum(ssk);
             rq = 1.f / fmaxf(sqrtf(ssq), 1e-6f);
             rk = 1.f / fmaxf(sqrtf(ssk), 1e-6f);
-        }
 #pragma unroll
-        for (int m = 0; m < D / 32; ++m) {
-            int d = lane + 32 * m;
-            sq[r * D + d] = qv[m] * rq;
-            sk[r * D + d] = kv[m] * rk;
-            float gl = 0.f;
-            if (valid) {
-                float x = ldf(g + row * D + d);
-                if (gate) {
-                    if (p.dt_bias) x += p.dt_bias[h * D + d];
-                    gl = negA * softplus_f(x);
-                } else {
-                    gl = x;
-                }
+            for (int m = 0; m < D / 32; ++m) {
+                sq[r * D + lane + 32 * m] *= rq;
+                sk[r * D + lane + 32 * m] *= rk;
             }
-            sG[r * D + d] = gl * LOG2E;
-            if (sv) sv[r * D + d] = valid ? ldf(v + row * D + d) : 0.f;
         }
         if (lane == 0) {
-            float b = 0.f;
-            if (valid) {
-                b = ldf(beta + row);
-                if (sig) b = sigmoid_f(b);
-            }
-            sbeta[r] = b;
             srq[r] = rq;
             srk[r] = rk;
         }
     }
     __syncthreads();
-    for (int d = tid; d < D; d += NTHREADS) {
-        float run = 0.f;
-        for (int r = 0; r < C; ++r) {
-            run += sG[r * D + d];
-            sG[r * D + d] = run;
-        }
+    for (int it = tid; it < D * 4; it += NTHREADS) {
+        const int d = it % D, grp = it / D;
+        if (grp == 0) continue;
+        float before = 0.f;
+        for (int g = 0; g < grp; ++g) before += scratch[g * D + d];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) sG[(16 * grp + r) * D + d] += before;
     }
     __syncthreads();
 }
@@ -163,15 +220,15 @@ __device__ __forceinline__ void load_prologue(const KdaParams& p, const ChunkInf
 // ---------------------------------------------------------------------------------------
 template <typename T, int D>
 __global__ void __launch_bounds__(NTHREADS, 1) kda_fwd_intra_simt(const KdaParams p) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     float* sq = smem;
     float* sk = sq + C * D;
     float* sG = sk + C * D;
     float* sv = sG + C * D;
-    float* sA = sv + C * D;       // [64][65]
-    float* sL = sA + C * 65;
-    float* sT = sL + C * 65;
-    float* sbeta = sT + C * 65;
+    float* sA = sv + C * D;       // [64][CP]
+    float* sL = sA + C * CP;
+    float* sT = sL + C * CP;
+    float* sbeta = sT + C * CP;
     float* srq = sbeta + C;
     float* srk = srq + C;
     float* st = srk + C;
@@ -190,7 +247,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_fwd_intra_simt(const KdaParam
     T* gT = (T*)(ws + L.Tm) + rec * C * C;
     float* gGam = (float*)(ws + L.gamC) + rec * D;
 
-    load_prologue<T, D>(p, ci, h, sq, sk, sG, sv, sbeta, srq, srk);
+    load_prologue<T, D>(p, ci, h, sq, sk, sG, sv, sbeta, srq, srk, st);
     const bool save = !(p.flags & KDA_FLAG_NO_SAVE);  // forward-only calls keep nothing for a backward
     if (save) {  // prologue results kept for the backward
         float* gGc = (float*)(ws + L.Gc) + rec * C * D;
@@ -211,54 +268,86 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_fwd_intra_simt(const KdaParam
         }
     }
 
-    // exact pairwise products: one warp per (i, j) pair, lanes over channels
-    for (int i = warp; i < C; i += NTHREADS / 32) {
-        float qi[D / 32], ki[D / 32], gi[D / 32];
+    // exact pairwise products.  A warp takes the rows i and 63 - i (65 pairs together, the same for every warp); its
+    // lanes are eight keys x four quarters of the channels, so that a pair costs two shuffles per product instead of five
+    {
+        constexpr int DQ = D / 4;
+        const int jl = lane >> 2, dq0 = (lane & 3) * 4;  // quarter: channels 4 (lane & 3) + 16 m + {0..3}
+        for (int it = warp; it < C; it += NTHREADS / 32) {
+            const int i = it < C / 2 ? it : C - 1 - (it - C / 2);
+            float4 qi[DQ / 4], ki[DQ / 4], gi[DQ / 4];
 #pragma unroll
-        for (int m = 0; m < D / 32; ++m) {
-            qi[m] = sq[i * D + lane + 32 * m];
-            ki[m] = sk[i * D + lane + 32 * m];
-            gi[m] = sG[i * D + lane + 32 * m];
-        }
-        for (int j = 0; j < C; ++j) {
-            float a = 0.f, l = 0.f;
-            if (j <= i) {
-#pragma unroll
-                for (int m = 0; m < D / 32; ++m) {
-                    float kd = sk[j * D + lane + 32 * m] * exp2f(gi[m] - sG[j * D + lane + 32 * m]);
-                    a = fmaf(qi[m], kd, a);
-                    l = fmaf(ki[m], kd, l);
-                }
-                a = warp_sum(a);
-                l = warp_sum(l);
+            for (int m = 0; m < DQ / 4; ++m) {
+                qi[m] = *reinterpret_cast<const float4*>(sq + i * D + dq0 + 16 * m);
+                ki[m] = *reinterpret_cast<const float4*>(sk + i * D + dq0 + 16 * m);
+                gi[m] = *reinterpret_cast<const float4*>(sG + i * D + dq0 + 16 * m);
             }
-            if (lane == 0) {
-                sA[i * 65 + j] = (j <= i) ? a * p.scale : 0.f;
-                sL[i * 65 + j] = (j < i) ? l : 0.f;
+            for (int j0 = 0; j0 < C; j0 += 8) {
+                const int j = j0 + jl, jr = j < i ? j : i;  // (lanes past the diagonal repeat it)
+                float a = 0.f, l = 0.f;
+                if (j0 <= i) {
+#pragma unroll
+                    for (int m = 0; m < DQ / 4; ++m) {
+                        const float4 kj = *reinterpret_cast<const float4*>(sk + jr * D + dq0 + 16 * m);
+                        const float4 gj = *reinterpret_cast<const float4*>(sG + jr * D + dq0 + 16 * m);
+                        float kd = kj.x * exp2f(gi[m].x - gj.x);
+                        a = fmaf(qi[m].x, kd, a);
+                        l = fmaf(ki[m].x, kd, l);
+                        kd = kj.y * exp2f(gi[m].y - gj.y);
+                        a = fmaf(qi[m].y, kd, a);
+                        l = fmaf(ki[m].y, kd, l);
+                        kd = kj.z * exp2f(gi[m].z - gj.z);
+                        a = fmaf(qi[m].z, kd, a);
+                        l = fmaf(ki[m].z, kd, l);
+                        kd = kj.w * exp2f(gi[m].w - gj.w);
+                        a = fmaf(qi[m].w, kd, a);
+                        l = fmaf(ki[m].w, kd, l);
+                    }
+#pragma unroll
+                    for (int o = 1; o <= 2; o <<= 1) {
+                        a += __shfl_xor_sync(0xffffffffu, a, o);
+                        l += __shfl_xor_sync(0xffffffffu, l, o);
+                    }
+                }
+                if ((lane & 3) == 0) {
+                    sA[i * CP + j] = (j <= i) ? a * p.scale : 0.f;
+                    sL[i * CP + j] = (j < i) ? l : 0.f;
+                }
             }
         }
     }
-    for (int idx = tid; idx < C * 65; idx += NTHREADS) sT[idx] = 0.f;
     __syncthreads();
 
-    // T = (I + diag(beta) L)^-1 by forward substitution, 4 threads per column
+    // T = (I + diag(beta) L)^-1 by forward substitution: four lanes of a warp own a column and keep it in registers, so
+    // the 64 dependent rows need no barrier
     {
         const int col = tid >> 2, part = tid & 3;
+        float t[C / 4];
+#pragma unroll
+        for (int m = 0; m < C / 4; ++m) t[m] = 0.f;
+#pragma unroll
         for (int i = 0; i < C; ++i) {
-            float s = 0.f;
-            for (int j = part; j < i; j += 4) s = fmaf(sL[i * 65 + j], sT[j * 65 + col], s);
+            float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+            for (int m = 0; 4 * m < i; m += 2) {  // (entries that are not known yet are zero)
+                s0 = fmaf(sL[i * CP + 4 * m + part], t[m], s0);
+                if (4 * m + 4 < i) s1 = fmaf(sL[i * CP + 4 * m + 4 + part], t[m + 1], s1);
+            }
+            float s = s0 + s1;
             s += __shfl_xor_sync(0xffffffffu, s, 1);
             s += __shfl_xor_sync(0xffffffffu, s, 2);
-            if (part == 0 && col <= i) sT[i * 65 + col] = (i == col ? 1.f : 0.f) - sbeta[i] * s;
-            __syncthreads();
+            const float v = col <= i ? (i == col ? 1.f : 0.f) - sbeta[i] * s : 0.f;
+            if (part == (i & 3)) t[i >> 2] = v;
+            if (part == 0) sT[i * CP + col] = v;
         }
     }
+    __syncthreads();
 
     // records that depend only on the prologue
     for (int idx = tid; idx < C * C; idx += NTHREADS) {
         int i = idx / C, j = idx % C;
-        stf(gA + tc::cm_idx(i, j, C), sA[i * 65 + j]);
-        if (save) stf(gT + tc::cm_idx(i, j, C), sT[i * 65 + j]);
+        stf(gA + tc::cm_idx(i, j, C), sA[i * CP + j]);
+        if (save) stf(gT + tc::cm_idx(i, j, C), sT[i * CP + j]);
     }
     for (int idx = tid; idx < C * D; idx += NTHREADS) {
         int i = idx / D, d = idx % D;
@@ -279,201 +368,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_fwd_intra_simt(const KdaParam
     {
         float acc[4][D / 16];
         zero_acc(acc);
-        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[m * 65 + k]; }, [&](int k, int n) { return sq[k * D + n]; },
+        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[m * CP + k]; }, [&](int k, int n) { return sq[k * D + n]; },
                       st, true, false);
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int cc = 0; cc < D / 16; ++cc) stf(gW + tc::cm_idx(tx + 16 * cc, ty + 16 * r, C), acc[r][cc]);
+            for (int cc = 0; cc < D / 16; ++cc) stf(gW + tc::cm_idx(tile_col(tx, cc), 4 * ty + r, C), acc[r][cc]);
         zero_acc(acc);
-        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[m * 65 + k]; }, [&](int k, int n) { return sv[k * D + n]; },
+        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[m * CP + k]; }, [&](int k, int n) { return sv[k * D + n]; },
                       st, true, false);
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int cc = 0; cc < D / 16; ++cc) stf(gU + tc::cm_idx(tx + 16 * cc, ty + 16 * r, C), acc[r][cc]);
-    }
-}
-
-// ---------------------------------------------------------------------------------------
-// fwd_state: sequential over the chunks of one sequence, for one head and one panel of BV
-// state columns.  Writes V' over U, the chunk-entry states, o and the final state.
-// ---------------------------------------------------------------------------------------
-template <typename T, int D, int BV>
-__global__ void __launch_bounds__(NTHREADS) kda_fwd_state_simt(const KdaParams p) {
-    extern __shared__ float smem[];
-    float* sS = smem;                  // [D][BV+1]
-    float* sVn = sS + D * (BV + 1);    // [64][BV+1]
-    float* st = sVn + C * (BV + 1);
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    const int e0 = blockIdx.x * BV, h = blockIdx.y, n = blockIdx.z;
-    const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
-    char* ws = (char*)p.workspace;
-    int c0, nc;
-    seq_chunks(p, n, c0, nc);
-    const size_t sbase = ((size_t)n * p.H + h) * D * D;
-
-    for (int idx = tid; idx < D * BV; idx += NTHREADS) {
-        int d = idx / BV, e = idx % BV;
-        sS[d * (BV + 1) + e] = p.h0 ? p.h0[sbase + state_idx(p, d, e0 + e)] : 0.f;
-    }
-    __syncthreads();
-
-    for (int lc = 0; lc < nc; ++lc) {
-        const int c = c0 + lc;
-        const ChunkInfo ci = chunk_info(p, c);
-        const size_t rec = (size_t)c * p.H + h;
-        const T* gW = (const T*)(ws + L.W) + rec * C * D;
-        T* gU = (T*)(ws + L.U) + rec * C * D;
-        const T* gA = (const T*)(ws + L.Aqk) + rec * C * C;
-        const T* gQt = (const T*)(ws + L.Qt) + rec * C * D;
-        const T* gKh = (const T*)(ws + L.Kh) + rec * C * D;
-        T* gS0 = (T*)(ws + L.S0) + rec * D * D;
-        const float* gGam = (const float*)(ws + L.gamC) + rec * D;
-        T* o = (T*)p.o;
-
-        for (int idx = tid; idx < D * BV; idx += NTHREADS) {
-            int d = idx / BV, e = idx % BV;
-            if (!(p.flags & KDA_FLAG_NO_SAVE)) stf(gS0 + tc::cm_idx(e0 + e, d, D), sS[d * (BV + 1) + e]);
-        }
-        // V' = U - W S
-        {
-            float acc[4][BV / 16];
-            zero_acc(acc);
-            mm_tile<C, BV>(acc, D, [&](int m, int k) { return ldf(gW + tc::cm_idx(k, m, C)); },
-                           [&](int k, int nn) { return sS[k * (BV + 1) + nn]; }, st, true, false);
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int cc = 0; cc < BV / 16; ++cc) {
-                    int i = ty + 16 * r, e = tx + 16 * cc;
-                    float vn = ldf(gU + tc::cm_idx(e0 + e, i, C)) - acc[r][cc];
-                    sVn[i * (BV + 1) + e] = vn;
-                    if (!(p.flags & KDA_FLAG_NO_SAVE)) stf(gU + tc::cm_idx(e0 + e, i, C), vn);
-                }
-        }
-        // O = Qt S + Aqk V'
-        {
-            float acc[4][BV / 16];
-            zero_acc(acc);
-            mm_tile<C, BV>(acc, D, [&](int m, int k) { return ldf(gQt + tc::cm_idx(m, k, D)); },
-                           [&](int k, int nn) { return sS[k * (BV + 1) + nn]; }, st, true, false);
-            mm_tile<C, BV>(acc, C, [&](int m, int k) { return ldf(gA + tc::cm_idx(m, k, C)); },
-                           [&](int k, int nn) { return sVn[k * (BV + 1) + nn]; }, st, true, false);
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int cc = 0; cc < BV / 16; ++cc) {
-                    int i = ty + 16 * r, e = tx + 16 * cc;
-                    if (i < ci.len) stf(o + ((size_t)(ci.tok0 + i) * p.H + h) * D + e0 + e, acc[r][cc]);
-                }
-        }
-        // S = diag(gamC) S + Kh^T V'
-        {
-            float acc[D / 16][BV / 16];
-            zero_acc(acc);
-            mm_tile<D, BV>(acc, C, [&](int m, int k) { return ldf(gKh + tc::cm_idx(k, m, D)); },
-                           [&](int k, int nn) { return sVn[k * (BV + 1) + nn]; }, st, false, false);
-#pragma unroll
-            for (int r = 0; r < D / 16; ++r)
-#pragma unroll
-                for (int cc = 0; cc < BV / 16; ++cc) {
-                    int d = ty + 16 * r, e = tx + 16 * cc;
-                    sS[d * (BV + 1) + e] = gGam[d] * sS[d * (BV + 1) + e] + acc[r][cc];
-                }
-        }
-        __syncthreads();
-    }
-    if (p.ht) {
-        for (int idx = tid; idx < D * BV; idx += NTHREADS) {
-            int d = idx / BV, e = idx % BV;
-            p.ht[sbase + state_idx(p, d, e0 + e)] = sS[d * (BV + 1) + e];
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------------------
-// bwd_state: reverse over the chunks.  dV' = Aqk^T dO + Kh dS,
-// dS <- diag(gamC) dS + Qt^T dO - W^T dV'.  Stores the dS entering each chunk and dV'.
-// ---------------------------------------------------------------------------------------
-template <typename T, int D, int BV>
-__global__ void __launch_bounds__(NTHREADS) kda_bwd_state_simt(const KdaParams p) {
-    extern __shared__ float smem[];
-    float* sS = smem;                  // dS [D][BV+1]
-    float* sVn = sS + D * (BV + 1);    // dV' [64][BV+1]
-    float* st = sVn + C * (BV + 1);
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    const int e0 = blockIdx.x * BV, h = blockIdx.y, n = blockIdx.z;
-    const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
-    const char* ws = (const char*)p.workspace;
-    char* sc = (char*)p.bwd_scratch;
-    int c0, nc;
-    seq_chunks(p, n, c0, nc);
-    const size_t sbase = ((size_t)n * p.H + h) * D * D;
-    const T* dO = (const T*)p.grad_o;
-
-    for (int idx = tid; idx < D * BV; idx += NTHREADS) {
-        int d = idx / BV, e = idx % BV;
-        sS[d * (BV + 1) + e] = p.grad_ht ? p.grad_ht[sbase + state_idx(p, d, e0 + e)] : 0.f;
-    }
-    __syncthreads();
-
-    for (int lc = nc - 1; lc >= 0; --lc) {
-        const int c = c0 + lc;
-        const ChunkInfo ci = chunk_info(p, c);
-        const size_t rec = (size_t)c * p.H + h;
-        const T* gW = (const T*)(ws + L.W) + rec * C * D;
-        const T* gA = (const T*)(ws + L.Aqk) + rec * C * C;
-        const T* gQt = (const T*)(ws + L.Qt) + rec * C * D;
-        const T* gKh = (const T*)(ws + L.Kh) + rec * C * D;
-        const float* gGam = (const float*)(ws + L.gamC) + rec * D;
-        T* gdS = (T*)(sc + L.dS) + rec * D * D;
-        T* gdV = (T*)(sc + L.dVn) + rec * C * D;
-        auto ldo = [&](int i, int e) {
-            return i < ci.len ? ldf(dO + ((size_t)(ci.tok0 + i) * p.H + h) * D + e0 + e) : 0.f;
-        };
-        for (int idx = tid; idx < D * BV; idx += NTHREADS) {
-            int d = idx / BV, e = idx % BV;
-            stf(gdS + tc::cm_idx(e0 + e, d, D), sS[d * (BV + 1) + e]);
-        }
-        {
-            float acc[4][BV / 16];
-            zero_acc(acc);
-            mm_tile<C, BV>(acc, C, [&](int m, int k) { return ldf(gA + tc::cm_idx(k, m, C)); },
-                           [&](int k, int nn) { return ldo(k, nn); }, st, false, false);
-            mm_tile<C, BV>(acc, D, [&](int m, int k) { return ldf(gKh + tc::cm_idx(m, k, D)); },
-                           [&](int k, int nn) { return sS[k * (BV + 1) + nn]; }, st, true, false);
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int cc = 0; cc < BV / 16; ++cc) {
-                    int i = ty + 16 * r, e = tx + 16 * cc;
-                    sVn[i * (BV + 1) + e] = acc[r][cc];
-                    stf(gdV + tc::cm_idx(e0 + e, i, C), acc[r][cc]);
-                }
-        }
-        {
-            float acc[D / 16][BV / 16];
-            zero_acc(acc);
-            mm_tile<D, BV>(acc, C, [&](int m, int k) { return ldf(gQt + tc::cm_idx(k, m, D)); },
-                           [&](int k, int nn) { return ldo(k, nn); }, st, false, false);
-            mm_tile<D, BV>(acc, C, [&](int m, int k) { return -ldf(gW + tc::cm_idx(m, k, C)); },
-                           [&](int k, int nn) { return sVn[k * (BV + 1) + nn]; }, st, false, false);
-#pragma unroll
-            for (int r = 0; r < D / 16; ++r)
-#pragma unroll
-                for (int cc = 0; cc < BV / 16; ++cc) {
-                    int d = ty + 16 * r, e = tx + 16 * cc;
-                    sS[d * (BV + 1) + e] = gGam[d] * sS[d * (BV + 1) + e] + acc[r][cc];
-                }
-        }
-        __syncthreads();
-    }
-    if (p.grad_h0) {
-        for (int idx = tid; idx < D * BV; idx += NTHREADS) {
-            int d = idx / BV, e = idx % BV;
-            p.grad_h0[sbase + state_idx(p, d, e0 + e)] = sS[d * (BV + 1) + e];
-        }
+            for (int cc = 0; cc < D / 16; ++cc) stf(gU + tc::cm_idx(tile_col(tx, cc), 4 * ty + r, C), acc[r][cc]);
     }
 }
 
@@ -496,16 +403,16 @@ __device__ __forceinline__ void store_split3(__nv_bfloat16* base, int i, int j, 
 
 template <typename T, int D, bool SPLIT = false>
 __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParams p) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     float* sq = smem;
     float* sk = sq + C * D;
     float* sG = sk + C * D;
     float* sW = sG + C * D;        // dW, later scratch
-    float* sT = sW + C * D;        // [64][65]
-    float* sdA = sT + C * 65;
-    float* sdM = sdA + C * 65;     // first holds dT
-    float* sY = sdM + C * 65;
-    float* sbeta = sY + C * 65;
+    float* sT = sW + C * D;        // [64][CP]
+    float* sdA = sT + C * CP;
+    float* sdM = sdA + C * CP;     // first holds dT
+    float* sY = sdM + C * CP;
+    float* sbeta = sY + C * CP;
     float* srq = sbeta + C;
     float* srk = srq + C;
     float* sdb = srk + C;          // dbeta accumulator
@@ -530,8 +437,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
     const T* v = (const T*)p.v;
     const float scale = p.scale;
 
-    load_prologue<T, D>(p, ci, h, sq, sk, sG, nullptr, sbeta, srq, srk);
-    for (int idx = tid; idx < C * C; idx += NTHREADS) sT[(idx / C) * 65 + idx % C] = ldf(gT + tc::cm_idx(idx / C, idx % C, C));
+    load_prologue<T, D>(p, ci, h, sq, sk, sG, nullptr, sbeta, srq, srk, st);
+    for (int idx = tid; idx < C * C; idx += NTHREADS) sT[(idx / C) * CP + idx % C] = ldf(gT + tc::cm_idx(idx / C, idx % C, C));
     if (tid < C) sdb[tid] = 0.f;
 
     auto ldo = [&](int i, int e) { return i < ci.len ? ldf(dO + ((size_t)(ci.tok0 + i) * p.H + h) * D + e) : 0.f; };
@@ -553,11 +460,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
         for (int r = 0; r < 4; ++r)
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc) {
-                int i = ty + 16 * r, j = tx + 16 * cc;
-                sdA[i * 65 + j] = (i >= j) ? acc[r][cc] : 0.f;
+                int i = 4 * ty + r, j = tile_col(tx, cc);
+                sdA[i * CP + j] = (i >= j) ? acc[r][cc] : 0.f;
                 if constexpr (SPLIT) {
-                    store_split3((__nv_bfloat16*)(sc + L.dAM) + rec * 6 * C * C, i, j, i > j ? sdA[i * 65 + j] : 0.f);
-                    if (i == j) ((float*)(sc + L.dAd))[rec * C + i] = sdA[i * 65 + j];
+                    store_split3((__nv_bfloat16*)(sc + L.dAM) + rec * 6 * C * C, i, j, i > j ? sdA[i * CP + j] : 0.f);
+                    if (i == j) ((float*)(sc + L.dAd))[rec * C + i] = sdA[i * CP + j];
                 }
             }
     }
@@ -570,7 +477,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int cc = 0; cc < D / 16; ++cc) sW[(ty + 16 * r) * D + tx + 16 * cc] = -acc[r][cc];
+            for (int cc = 0; cc < D / 16; ++cc) sW[(4 * ty + r) * D + tile_col(tx, cc)] = -acc[r][cc];
     }
     // 3. dT = tril(dW (beta K~)^T + dV' (beta V)^T)   -> sdM
     {
@@ -584,44 +491,44 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
         for (int r = 0; r < 4; ++r)
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc) {
-                int i = ty + 16 * r, j = tx + 16 * cc;
-                sdM[i * 65 + j] = (i >= j) ? acc[r][cc] : 0.f;
+                int i = 4 * ty + r, j = tile_col(tx, cc);
+                sdM[i * CP + j] = (i >= j) ? acc[r][cc] : 0.f;
             }
     }
     // 4. dM = -T^T dT T^T (strictly lower part is what the intra step uses)
     {
         float acc[4][4];
         zero_acc(acc);
-        mm_tile<C, C>(acc, C, [&](int m, int k) { return sdM[m * 65 + k]; }, [&](int k, int n) { return sT[n * 65 + k]; }, st,
+        mm_tile<C, C>(acc, C, [&](int m, int k) { return sdM[m * CP + k]; }, [&](int k, int n) { return sT[n * CP + k]; }, st,
                       true, true);
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int cc = 0; cc < 4; ++cc) sY[(ty + 16 * r) * 65 + tx + 16 * cc] = acc[r][cc];
+            for (int cc = 0; cc < 4; ++cc) sY[(4 * ty + r) * CP + tile_col(tx, cc)] = acc[r][cc];
         zero_acc(acc);
-        mm_tile<C, C>(acc, C, [&](int m, int k) { return sT[k * 65 + m]; }, [&](int k, int n) { return sY[k * 65 + n]; }, st,
+        mm_tile<C, C>(acc, C, [&](int m, int k) { return sT[k * CP + m]; }, [&](int k, int n) { return sY[k * CP + n]; }, st,
                       false, false);
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc) {
-                int i = ty + 16 * r, j = tx + 16 * cc;
-                sdM[i * 65 + j] = (i > j) ? -acc[r][cc] : 0.f;
+                int i = 4 * ty + r, j = tile_col(tx, cc);
+                sdM[i * CP + j] = (i > j) ? -acc[r][cc] : 0.f;
                 if constexpr (SPLIT)
-                    store_split3((__nv_bfloat16*)(sc + L.dAM) + rec * 6 * C * C + 3 * C * C, i, j, sdM[i * 65 + j]);
+                    store_split3((__nv_bfloat16*)(sc + L.dAM) + rec * 6 * C * C + 3 * C * C, i, j, sdM[i * CP + j]);
             }
     }
     // 5. d(beta K~) = T^T dW
     {
         float acc[4][D / 16];
         zero_acc(acc);
-        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[k * 65 + m]; }, [&](int k, int n) { return sW[k * D + n]; }, st,
+        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[k * CP + m]; }, [&](int k, int n) { return sW[k * D + n]; }, st,
                       false, false);
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
             for (int cc = 0; cc < D / 16; ++cc) {
-                int i = ty + 16 * r, d = tx + 16 * cc;
+                int i = 4 * ty + r, d = tile_col(tx, cc);
                 if constexpr (SPLIT) {
                     stf((T*)(sc + L.dKb) + rec * C * D + handover_idx(i, d), acc[r][cc]);
                     continue;
@@ -638,14 +545,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
     {
         float acc[4][D / 16];
         zero_acc(acc);
-        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[k * 65 + m]; }, [&](int k, int n) { return ldf(gdV + tc::cm_idx(n, k, C)); },
+        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[k * CP + m]; }, [&](int k, int n) { return ldf(gdV + tc::cm_idx(n, k, C)); },
                       st, false, false);
         T* dv = (T*)p.grad_v;
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
             for (int cc = 0; cc < D / 16; ++cc) {
-                int i = ty + 16 * r, e = tx + 16 * cc;
+                int i = 4 * ty + r, e = tile_col(tx, cc);
                 if (i < ci.len) {
                     stf(dv + ((size_t)(ci.tok0 + i) * p.H + h) * D + e, sbeta[i] * acc[r][cc]);
                     db_r[r] += acc[r][cc] * ldv(i, e);
@@ -662,7 +569,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
         for (int r = 0; r < 4; ++r)
 #pragma unroll
             for (int cc = 0; cc < D / 16; ++cc) {
-                int i = ty + 16 * r, d = tx + 16 * cc;
+                int i = 4 * ty + r, d = tile_col(tx, cc);
                 if constexpr (SPLIT) {
                     stf((T*)(sc + L.dQt) + rec * C * D + handover_idx(i, d), acc[r][cc]);
                     continue;
@@ -682,7 +589,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
         for (int r = 0; r < 4; ++r)
 #pragma unroll
             for (int cc = 0; cc < D / 16; ++cc) {
-                int i = ty + 16 * r, d = tx + 16 * cc;
+                int i = 4 * ty + r, d = tile_col(tx, cc);
                 if constexpr (SPLIT) {
                     stf((T*)(sc + L.dKh) + rec * C * D + handover_idx(i, d), acc[r][cc]);
                     sW[i * D + d] = 0.f;
@@ -696,11 +603,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
             }
     }
     __syncthreads();
-    for (int d = tid; d < D; d += NTHREADS) {
-        float s = 0.f;
-        for (int i = 0; i < C; ++i) s += sW[i * D + d];
-        scol[d] = s;
+    for (int it = tid; it < 4 * D; it += NTHREADS) {
+        float t = 0.f;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) t += sW[(16 * (it / D) + r) * D + it % D];
+        st[it] = t;
     }
+    __syncthreads();
+    for (int d = tid; d < D; d += NTHREADS) scol[d] = (st[d] + st[D + d]) + (st[2 * D + d] + st[3 * D + d]);
     __syncthreads();
     // 9. d(gamC)[d] = sum_e dS[d][e] S0[d][e]
     for (int d = warp; d < D; d += NTHREADS / 32) {
@@ -713,85 +623,154 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             float s = row16_sum(db_r[r]);
-            if (tx == 0) ((float*)(sc + L.dbp))[rec * C + ty + 16 * r] = s;
+            if (tx == 0) ((float*)(sc + L.dbp))[rec * C + 4 * ty + r] = s;
         }
         __syncthreads();
         for (int d = tid; d < D; d += NTHREADS) ((float*)(sc + L.gC))[rec * D + d] = scol[d];
         return;
     }
-    // 10. intra step with exact pairwise decays
+    // 10. intra step with exact pairwise decays.  A thread's tile is four rows i x four channels d (twice that for
+    //     d = 128): walking the keys j in front of the tile it needs k_j, G_j and column j of dA and dM for its rows,
+    //     walking the queries behind it q, k, G and row entries of dA and dM, four 16-byte loads per 16 pairs each way.
+    //     dA^T and beta dM^T go where T and Y were.
+    __syncthreads();
+    for (int idx = tid; idx < C * C; idx += NTHREADS) {
+        const int i = idx & 63, j = idx >> 6;
+        sT[j * CP + i] = sdA[i * CP + j];
+        sY[j * CP + i] = sdM[i * CP + j];
+    }
+    __syncthreads();
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int i = ty + 16 * r;
+    for (int g = 0; g < D / 64; ++g) {
+        const int d0 = tile_col(tx, 4 * g), i0 = 4 * ty;
+        float gi[4][4], a1[4][4], a2[4][4], c1[4][4];
 #pragma unroll
-        for (int cc = 0; cc < D / 16; ++cc) {
-            const int d = tx + 16 * cc;
-            const float gi = sG[i * D + d], qi = sq[i * D + d], ki = sk[i * D + d];
-            // strictly-lower / strictly-upper parts; the diagonal pair (j == i) has decay 1 and
-            // contributes equal and opposite amounts to dG, so it is kept out of dG exactly
-            float a1 = 0.f, a2 = 0.f;
-            for (int j = 0; j < i; ++j) {
-                float kd = sk[j * D + d] * exp2f(gi - sG[j * D + d]);
-                a1 = fmaf(sdA[i * 65 + j], kd, a1);
-                a2 = fmaf(sdM[i * 65 + j], kd, a2);
+        for (int r = 0; r < 4; ++r) {
+            const float4 v = *reinterpret_cast<const float4*>(sG + (i0 + r) * D + d0);
+            gi[r][0] = v.x; gi[r][1] = v.y; gi[r][2] = v.z; gi[r][3] = v.w;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) a1[r][c] = a2[r][c] = c1[r][c] = 0.f;
+        }
+        // `inside`: pairs of the tile's own rows, where only j < i counts (the diagonal pair has decay 1 and contributes
+        // equal and opposite amounts to dG, so it is kept out of dG exactly)
+        auto keys = [&](int j, bool inside) {
+            const float4 kv = *reinterpret_cast<const float4*>(sk + j * D + d0), gv = *reinterpret_cast<const float4*>(sG + j * D + d0);
+            const float4 av = *reinterpret_cast<const float4*>(sT + j * CP + i0), mv = *reinterpret_cast<const float4*>(sY + j * CP + i0);
+            const float kj[4] = {kv.x, kv.y, kv.z, kv.w}, gj[4] = {gv.x, gv.y, gv.z, gv.w};
+            const float da[4] = {av.x, av.y, av.z, av.w}, dm[4] = {mv.x, mv.y, mv.z, mv.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (inside && i0 + r <= j) continue;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float kd = kj[c] * exp2f(gi[r][c] - gj[c]);
+                    a1[r][c] = fmaf(da[r], kd, a1[r][c]);
+                    a2[r][c] = fmaf(dm[r], kd, a2[r][c]);
+                }
             }
-            float c1 = 0.f;
-            for (int ii = i + 1; ii < C; ++ii) {
-                float e = exp2f(sG[ii * D + d] - gi);
-                float t = scale * sdA[ii * 65 + i] * sq[ii * D + d] + sbeta[ii] * sdM[ii * 65 + i] * sk[ii * D + d];
-                c1 = fmaf(t, e, c1);
+        };
+        auto queries = [&](int ii, bool inside) {
+            const float4 qv = *reinterpret_cast<const float4*>(sq + ii * D + d0), kv = *reinterpret_cast<const float4*>(sk + ii * D + d0);
+            const float4 gv = *reinterpret_cast<const float4*>(sG + ii * D + d0);
+            const float4 av = *reinterpret_cast<const float4*>(sdA + ii * CP + i0), mv = *reinterpret_cast<const float4*>(sdM + ii * CP + i0);
+            const float q4[4] = {qv.x, qv.y, qv.z, qv.w}, k4[4] = {kv.x, kv.y, kv.z, kv.w}, g4[4] = {gv.x, gv.y, gv.z, gv.w};
+            const float b = sbeta[ii];
+            const float da[4] = {scale * av.x, scale * av.y, scale * av.z, scale * av.w}, dm[4] = {b * mv.x, b * mv.y, b * mv.z, b * mv.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (inside && ii <= i0 + r) continue;
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    c1[r][c] = fmaf(fmaf(da[r], q4[c], dm[r] * k4[c]), exp2f(g4[c] - gi[r][c]), c1[r][c]);
             }
-            const float diag = scale * sdA[i * 65 + i];
-            float dq_in = scale * a1, dk_row = sbeta[i] * a2;
-            db_r[r] += ki * a2;
-            dq_a[r][cc] += dq_in + diag * ki;
-            dk_a[r][cc] += dk_row + c1 + diag * qi;
-            dG_a[r][cc] += qi * dq_in + ki * dk_row - ki * c1;
+        };
+#pragma unroll 2
+        for (int j = 0; j < i0; ++j) keys(j, false);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) keys(i0 + j, true);
+#pragma unroll
+        for (int j = 1; j < 4; ++j) queries(i0 + j, true);
+#pragma unroll 2
+        for (int ii = i0 + 4; ii < C; ++ii) queries(ii, false);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int i = i0 + r;
+            const float diag = scale * sdA[i * CP + i], b = sbeta[i];
+            const float4 qv = *reinterpret_cast<const float4*>(sq + i * D + d0), kv = *reinterpret_cast<const float4*>(sk + i * D + d0);
+            const float qi[4] = {qv.x, qv.y, qv.z, qv.w}, ki[4] = {kv.x, kv.y, kv.z, kv.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float dq_in = scale * a1[r][c], dk_row = b * a2[r][c];
+                db_r[r] += ki[c] * a2[r][c];
+                dq_a[r][4 * g + c] += dq_in + diag * ki[c];
+                dk_a[r][4 * g + c] += dk_row + c1[r][c] + diag * qi[c];
+                dG_a[r][4 * g + c] += qi[c] * dq_in + ki[c] * dk_row - ki[c] * c1[r][c];
+            }
         }
     }
     // 11. dbeta rows
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         float s = row16_sum(db_r[r]);
-        if (tx == 0) sdb[ty + 16 * r] = s;
+        if (tx == 0) sdb[4 * ty + r] = s;
     }
     // 12. reverse cumulative sum of dG and the gate chain
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int cc = 0; cc < D / 16; ++cc) sW[(ty + 16 * r) * D + tx + 16 * cc] = dG_a[r][cc];
+        for (int cc = 0; cc < D / 16; ++cc) sW[(4 * ty + r) * D + tile_col(tx, cc)] = dG_a[r][cc];
+    __syncthreads();
+    // thread = (channel, 16-row group): group totals first, then the sums from the last row up
+    for (int it = tid; it < 4 * D; it += NTHREADS) {
+        const int d = it % D, grp = it / D;
+        float t = 0.f;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) t += sW[(16 * grp + r) * D + d];
+        st[it] = t;
+    }
     __syncthreads();
     {
         const bool gate = p.flags & KDA_FLAG_GATE;
         const float negA = gate ? -expf(p.A_log[h]) : 0.f;
         const T* g = (const T*)p.g;
         T* dg = (T*)p.grad_g;
-        float dA = 0.f;
-        for (int d = tid; d < D; d += NTHREADS) {
-            float run = scol[d], dbias = 0.f;
-            for (int i = C - 1; i >= 0; --i) {
+        float dA = 0.f, dbias[4 * D / NTHREADS];
+#pragma unroll
+        for (int u = 0; u < 4 * D / NTHREADS; ++u) {
+            const int it = tid + NTHREADS * u, d = it % D, grp = it / D;
+            float run = scol[d];
+            for (int gg = 3; gg > grp; --gg) run += st[gg * D + d];
+            float db = 0.f;
+#pragma unroll 8
+            for (int r = 15; r >= 0; --r) {
+                const int i = 16 * grp + r;
                 run += sW[i * D + d];
                 if (i < ci.len) {
-                    size_t off = ((size_t)(ci.tok0 + i) * p.H + h) * D + d;
+                    const size_t off = ((size_t)(ci.tok0 + i) * p.H + h) * D + d;
                     if (gate) {
                         float z = ldf(g + off);
                         if (p.dt_bias) z += p.dt_bias[h * D + d];
                         dA = fmaf(run, negA * softplus_f(z), dA);
-                        float dx = run * negA * sigmoid_f(z);
-                        dbias += dx;
+                        const float dx = run * negA * sigmoid_f(z);
+                        db += dx;
                         stf(dg + off, dx);
                     } else {
                         stf(dg + off, run);
                     }
                 }
             }
-            if (gate) ((float*)(sc + L.dbias_part))[rec * D + d] = dbias;
+            dbias[u] = db;
         }
+        __syncthreads();  // the group totals have been read
         if (gate) {
+#pragma unroll
+            for (int u = 0; u < 4 * D / NTHREADS; ++u) st[tid + NTHREADS * u] = dbias[u];
             dA = warp_sum(dA);
             if (lane == 0) sred[warp] = dA;
             __syncthreads();
+            for (int d = tid; d < D; d += NTHREADS)
+                ((float*)(sc + L.dbias_part))[rec * D + d] = (st[3 * D + d] + st[2 * D + d]) + (st[D + d] + st[d]);
             if (tid == 0) {
                 float s = 0.f;
                 for (int w = 0; w < NTHREADS / 32; ++w) s += sred[w];
@@ -806,13 +785,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
         T* dk = (T*)p.grad_k;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            const int i = ty + 16 * r;
+            const int i = 4 * ty + r;
             float dotq = 0.f, dotk = 0.f;
             if (l2) {
 #pragma unroll
                 for (int cc = 0; cc < D / 16; ++cc) {
-                    dotq += sq[i * D + tx + 16 * cc] * dq_a[r][cc];
-                    dotk += sk[i * D + tx + 16 * cc] * dk_a[r][cc];
+                    dotq += sq[i * D + tile_col(tx, cc)] * dq_a[r][cc];
+                    dotk += sk[i * D + tile_col(tx, cc)] * dk_a[r][cc];
                 }
                 dotq = row16_sum(dotq);
                 dotk = row16_sum(dotk);
@@ -820,7 +799,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
             if (i < ci.len) {
 #pragma unroll
                 for (int cc = 0; cc < D / 16; ++cc) {
-                    int d = tx + 16 * cc;
+                    int d = tile_col(tx, cc);
                     size_t off = ((size_t)(ci.tok0 + i) * p.H + h) * D + d;
                     float a = dq_a[r][cc], b = dk_a[r][cc];
                     if (l2) {
@@ -890,12 +869,10 @@ __global__ void __launch_bounds__(1024) kda_param_reduce(const KdaParams p) {
 // host-side launchers
 // ---------------------------------------------------------------------------------------
 template <int D>
-constexpr size_t smem_intra() { return (size_t)(4 * C * D + 3 * C * 65 + 3 * C + KS * (C + 1) + KS * (D + 1)) * 4; }
-template <int D, int BV>
-constexpr size_t smem_state() { return (size_t)(D * (BV + 1) + C * (BV + 1) + KS * (D + 1) + KS * (BV + 1)) * 4; }
+constexpr size_t smem_intra() { return (size_t)(4 * C * D + 3 * C * CP + 3 * C + st_floats<D>()) * 4; }
 template <int D>
 constexpr size_t smem_bwd_chunk() {
-    return (size_t)(4 * C * D + 4 * C * 65 + 4 * C + D + 8 + KS * (C + 1) + KS * (D + 1)) * 4;
+    return (size_t)(4 * C * D + 4 * C * CP + 4 * C + D + 8 + st_floats<D>()) * 4;
 }
 
 template <typename K>
@@ -905,21 +882,14 @@ static cudaError_t set_smem(K kernel, size_t bytes) {
 
 template <typename T, int D>
 static cudaError_t launch_stage(const KdaParams& p, int stage, cudaStream_t s) {
-    constexpr int BV = 32;
     cudaError_t e = cudaSuccess;
     switch (stage) {
         case 0:
             if ((e = set_smem(kda_fwd_intra_simt<T, D>, smem_intra<D>())) != cudaSuccess) return e;
             kda_fwd_intra_simt<T, D><<<p.NT * p.H, NTHREADS, smem_intra<D>(), s>>>(p);
             break;
-        case 1:
-            if ((e = set_smem(kda_fwd_state_simt<T, D, BV>, smem_state<D, BV>())) != cudaSuccess) return e;
-            kda_fwd_state_simt<T, D, BV><<<dim3(D / BV, p.H, p.N), NTHREADS, smem_state<D, BV>(), s>>>(p);
-            break;
-        case 2:
-            if ((e = set_smem(kda_bwd_state_simt<T, D, BV>, smem_state<D, BV>())) != cudaSuccess) return e;
-            kda_bwd_state_simt<T, D, BV><<<dim3(D / BV, p.H, p.N), NTHREADS, smem_state<D, BV>(), s>>>(p);
-            break;
+        case 1: return simt_state(p, false, s);
+        case 2: return simt_state(p, true, s);
         case 3:
             if ((e = set_smem(kda_bwd_chunk_simt<T, D>, smem_bwd_chunk<D>())) != cudaSuccess) return e;
             kda_bwd_chunk_simt<T, D><<<p.NT * p.H, NTHREADS, smem_bwd_chunk<D>(), s>>>(p);
