@@ -23,6 +23,8 @@ cudaError_t simt_state(const KdaParams& p, bool bwd, cudaStream_t s);  // kda_si
 
 constexpr int NTHREADS = 256;
 constexpr int KS = 16;  // k-slice of the tile product
+template <int D>
+__host__ __device__ constexpr int row_stride() { return D + 4; }  // rows of q, k, G, v in shared memory: no bank conflict down a column
 constexpr int CP = C + 4;  // row stride of the [64][64] matrices in shared memory: rows start on 16-byte boundaries
 
 // thread (ty, tx) = (tid / 16, tid % 16) owns rows 4 ty + r and columns col(tx, c) of a tile product
@@ -150,7 +152,7 @@ __device__ __forceinline__ void load_prologue(const KdaParams& p, const ChunkInf
                 }
                 y = make_float4(v[0], v[1], v[2], v[3]);
             }
-            *reinterpret_cast<float4*>(dst + r * D + d) = y;
+            *reinterpret_cast<float4*>(dst + r * row_stride<D>() + d) = y;
         }
     };
     rows_in((const T*)p.q, sq, false);
@@ -172,8 +174,8 @@ __device__ __forceinline__ void load_prologue(const KdaParams& p, const ChunkInf
         float run = 0.f;
 #pragma unroll
         for (int r = 0; r < 16; ++r) {
-            run += sG[(16 * grp + r) * D + d];
-            sG[(16 * grp + r) * D + d] = run;
+            run += sG[(16 * grp + r) * row_stride<D>() + d];
+            sG[(16 * grp + r) * row_stride<D>() + d] = run;
         }
         scratch[it] = run;
     }
@@ -184,7 +186,7 @@ __device__ __forceinline__ void load_prologue(const KdaParams& p, const ChunkInf
             float ssq = 0.f, ssk = 0.f;
 #pragma unroll
             for (int m = 0; m < D / 32; ++m) {
-                const float a = sq[r * D + lane + 32 * m], b = sk[r * D + lane + 32 * m];
+                const float a = sq[r * row_stride<D>() + lane + 32 * m], b = sk[r * row_stride<D>() + lane + 32 * m];
                 ssq += a * a;
                 ssk += b * b;
             }
@@ -194,8 +196,8 @@ __device__ __forceinline__ void load_prologue(const KdaParams& p, const ChunkInf
             rk = 1.f / fmaxf(sqrtf(ssk), 1e-6f);
 #pragma unroll
             for (int m = 0; m < D / 32; ++m) {
-                sq[r * D + lane + 32 * m] *= rq;
-                sk[r * D + lane + 32 * m] *= rk;
+                sq[r * row_stride<D>() + lane + 32 * m] *= rq;
+                sk[r * row_stride<D>() + lane + 32 * m] *= rk;
             }
         }
         if (lane == 0) {
@@ -210,7 +212,7 @@ __device__ __forceinline__ void load_prologue(const KdaParams& p, const ChunkInf
         float before = 0.f;
         for (int g = 0; g < grp; ++g) before += scratch[g * D + d];
 #pragma unroll
-        for (int r = 0; r < 16; ++r) sG[(16 * grp + r) * D + d] += before;
+        for (int r = 0; r < 16; ++r) sG[(16 * grp + r) * row_stride<D>() + d] += before;
     }
     __syncthreads();
 }
@@ -222,10 +224,10 @@ template <typename T, int D>
 __global__ void __launch_bounds__(NTHREADS, 1) kda_fwd_intra_simt(const KdaParams p) {
     extern __shared__ __align__(16) float smem[];
     float* sq = smem;
-    float* sk = sq + C * D;
-    float* sG = sk + C * D;
-    float* sv = sG + C * D;
-    float* sA = sv + C * D;       // [64][CP]
+    float* sk = sq + C * row_stride<D>();
+    float* sG = sk + C * row_stride<D>();
+    float* sv = sG + C * row_stride<D>();
+    float* sA = sv + C * row_stride<D>();       // [64][CP]
     float* sL = sA + C * CP;
     float* sT = sL + C * CP;
     float* sbeta = sT + C * CP;
@@ -257,9 +259,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_fwd_intra_simt(const KdaParam
         for (int idx = tid; idx < C * D; idx += NTHREADS) {
             // d = 128: the chunk-swizzled row layout the tensor-core backward reads (swz_f32 / swz_bf16)
             const int r = idx / D, dd = idx % D;
-            gGc[D == 128 ? tc::swz_f32(r, dd) : idx] = sG[idx];
-            stf(gQn + (D == 128 ? (sizeof(T) == 2 ? tc::swz_bf16(r, dd) : tc::swz_f32(r, dd)) : idx), sq[idx]);
-            stf(gKn + (D == 128 ? (sizeof(T) == 2 ? tc::swz_bf16(r, dd) : tc::swz_f32(r, dd)) : idx), sk[idx]);
+            gGc[D == 128 ? tc::swz_f32(r, dd) : idx] = sG[r * row_stride<D>() + dd];
+            stf(gQn + (D == 128 ? (sizeof(T) == 2 ? tc::swz_bf16(r, dd) : tc::swz_f32(r, dd)) : idx), sq[r * row_stride<D>() + dd]);
+            stf(gKn + (D == 128 ? (sizeof(T) == 2 ? tc::swz_bf16(r, dd) : tc::swz_f32(r, dd)) : idx), sk[r * row_stride<D>() + dd]);
         }
         if (tid < C) {
             gaux[tid] = srq[tid];
@@ -278,9 +280,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_fwd_intra_simt(const KdaParam
             float4 qi[DQ / 4], ki[DQ / 4], gi[DQ / 4];
 #pragma unroll
             for (int m = 0; m < DQ / 4; ++m) {
-                qi[m] = *reinterpret_cast<const float4*>(sq + i * D + dq0 + 16 * m);
-                ki[m] = *reinterpret_cast<const float4*>(sk + i * D + dq0 + 16 * m);
-                gi[m] = *reinterpret_cast<const float4*>(sG + i * D + dq0 + 16 * m);
+                qi[m] = *reinterpret_cast<const float4*>(sq + i * row_stride<D>() + dq0 + 16 * m);
+                ki[m] = *reinterpret_cast<const float4*>(sk + i * row_stride<D>() + dq0 + 16 * m);
+                gi[m] = *reinterpret_cast<const float4*>(sG + i * row_stride<D>() + dq0 + 16 * m);
             }
             for (int j0 = 0; j0 < C; j0 += 8) {
                 const int j = j0 + jl, jr = j < i ? j : i;  // (lanes past the diagonal repeat it)
@@ -288,8 +290,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_fwd_intra_simt(const KdaParam
                 if (j0 <= i) {
 #pragma unroll
                     for (int m = 0; m < DQ / 4; ++m) {
-                        const float4 kj = *reinterpret_cast<const float4*>(sk + jr * D + dq0 + 16 * m);
-                        const float4 gj = *reinterpret_cast<const float4*>(sG + jr * D + dq0 + 16 * m);
+                        const float4 kj = *reinterpret_cast<const float4*>(sk + jr * row_stride<D>() + dq0 + 16 * m);
+                        const float4 gj = *reinterpret_cast<const float4*>(sG + jr * row_stride<D>() + dq0 + 16 * m);
                         float kd = kj.x * exp2f(gi[m].x - gj.x);
                         a = fmaf(qi[m].x, kd, a);
                         l = fmaf(ki[m].x, kd, l);
@@ -350,32 +352,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_fwd_intra_simt(const KdaParam
         if (save) stf(gT + tc::cm_idx(i, j, C), sT[i * CP + j]);
     }
     for (int idx = tid; idx < C * D; idx += NTHREADS) {
-        int i = idx / D, d = idx % D;
-        float G = sG[idx], gl = sG[(C - 1) * D + d];
-        float gam = exp2f(G);
-        stf(gQt + tc::cm_idx(i, d, D), p.scale * sq[idx] * gam);
-        stf(gKh + tc::cm_idx(i, d, D), sk[idx] * exp2f(gl - G));
+        const int i = idx / D, d = idx % D, at = i * row_stride<D>() + d;
+        const float G = sG[at], gl = sG[(C - 1) * row_stride<D>() + d], gam = exp2f(G);
+        stf(gQt + tc::cm_idx(i, d, D), p.scale * sq[at] * gam);
+        stf(gKh + tc::cm_idx(i, d, D), sk[at] * exp2f(gl - G));
         if (i == C - 1) gGam[d] = gam;
+        // operands of the WY products, in place: beta * k * 2^G and beta * v
+        sq[at] = sbeta[i] * sk[at] * gam;
+        sv[at] = sbeta[i] * sv[at];
     }
-    __syncthreads();
-    // operands of the WY products, in place: beta * k * 2^G and beta * v
-    for (int idx = tid; idx < C * D; idx += NTHREADS) {
-        int i = idx / D;
-        sq[idx] = sbeta[i] * sk[idx] * exp2f(sG[idx]);
-        sv[idx] = sbeta[i] * sv[idx];
-    }
-    __syncthreads();
     {
         float acc[4][D / 16];
         zero_acc(acc);
-        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[m * CP + k]; }, [&](int k, int n) { return sq[k * D + n]; },
+        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[m * CP + k]; }, [&](int k, int n) { return sq[k * row_stride<D>() + n]; },
                       st, true, false);
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
             for (int cc = 0; cc < D / 16; ++cc) stf(gW + tc::cm_idx(tile_col(tx, cc), 4 * ty + r, C), acc[r][cc]);
         zero_acc(acc);
-        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[m * CP + k]; }, [&](int k, int n) { return sv[k * D + n]; },
+        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[m * CP + k]; }, [&](int k, int n) { return sv[k * row_stride<D>() + n]; },
                       st, true, false);
 #pragma unroll
         for (int r = 0; r < 4; ++r)
@@ -405,10 +401,10 @@ template <typename T, int D, bool SPLIT = false>
 __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParams p) {
     extern __shared__ __align__(16) float smem[];
     float* sq = smem;
-    float* sk = sq + C * D;
-    float* sG = sk + C * D;
-    float* sW = sG + C * D;        // dW, later scratch
-    float* sT = sW + C * D;        // [64][CP]
+    float* sk = sq + C * row_stride<D>();
+    float* sG = sk + C * row_stride<D>();
+    float* sW = sG + C * row_stride<D>();        // dW, later scratch
+    float* sT = sW + C * row_stride<D>();        // [64][CP]
     float* sdA = sT + C * CP;
     float* sdM = sdA + C * CP;     // first holds dT
     float* sY = sdM + C * CP;
@@ -477,14 +473,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int cc = 0; cc < D / 16; ++cc) sW[(4 * ty + r) * D + tile_col(tx, cc)] = -acc[r][cc];
+            for (int cc = 0; cc < D / 16; ++cc) sW[(4 * ty + r) * row_stride<D>() + tile_col(tx, cc)] = -acc[r][cc];
     }
     // 3. dT = tril(dW (beta K~)^T + dV' (beta V)^T)   -> sdM
     {
         float acc[4][4];
         zero_acc(acc);
-        mm_tile<C, C>(acc, D, [&](int m, int k) { return sW[m * D + k]; },
-                      [&](int k, int n) { return sbeta[n] * sk[n * D + k] * exp2f(sG[n * D + k]); }, st, true, true);
+        mm_tile<C, C>(acc, D, [&](int m, int k) { return sW[m * row_stride<D>() + k]; },
+                      [&](int k, int n) { return sbeta[n] * sk[n * row_stride<D>() + k] * exp2f(sG[n * row_stride<D>() + k]); }, st, true, true);
         mm_tile<C, C>(acc, D, [&](int m, int k) { return ldf(gdV + tc::cm_idx(k, m, C)); },
                       [&](int k, int n) { return sbeta[n] * ldv(n, k); }, st, true, true);
 #pragma unroll
@@ -522,7 +518,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
     {
         float acc[4][D / 16];
         zero_acc(acc);
-        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[k * CP + m]; }, [&](int k, int n) { return sW[k * D + n]; }, st,
+        mm_tile<C, D>(acc, C, [&](int m, int k) { return sT[k * CP + m]; }, [&](int k, int n) { return sW[k * row_stride<D>() + n]; }, st,
                       false, false);
 #pragma unroll
         for (int r = 0; r < 4; ++r)
@@ -533,8 +529,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
                     stf((T*)(sc + L.dKb) + rec * C * D + handover_idx(i, d), acc[r][cc]);
                     continue;
                 }
-                float gam = exp2f(sG[i * D + d]);
-                float kt = sk[i * D + d] * gam;
+                float gam = exp2f(sG[i * row_stride<D>() + d]);
+                float kt = sk[i * row_stride<D>() + d] * gam;
                 float dkt = sbeta[i] * acc[r][cc];
                 dk_a[r][cc] += dkt * gam;
                 dG_a[r][cc] += dkt * kt;
@@ -574,9 +570,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
                     stf((T*)(sc + L.dQt) + rec * C * D + handover_idx(i, d), acc[r][cc]);
                     continue;
                 }
-                float gam = exp2f(sG[i * D + d]);
+                float gam = exp2f(sG[i * row_stride<D>() + d]);
                 dq_a[r][cc] += scale * acc[r][cc] * gam;
-                dG_a[r][cc] += acc[r][cc] * scale * sq[i * D + d] * gam;
+                dG_a[r][cc] += acc[r][cc] * scale * sq[i * row_stride<D>() + d] * gam;
             }
     }
     // 8. dKh = V' dS^T ; its column sums feed the last row of dG
@@ -592,21 +588,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
                 int i = 4 * ty + r, d = tile_col(tx, cc);
                 if constexpr (SPLIT) {
                     stf((T*)(sc + L.dKh) + rec * C * D + handover_idx(i, d), acc[r][cc]);
-                    sW[i * D + d] = 0.f;
+                    sW[i * row_stride<D>() + d] = 0.f;
                     continue;
                 }
-                float dec = exp2f(sG[(C - 1) * D + d] - sG[i * D + d]);
-                float kh = sk[i * D + d] * dec;
+                float dec = exp2f(sG[(C - 1) * row_stride<D>() + d] - sG[i * row_stride<D>() + d]);
+                float kh = sk[i * row_stride<D>() + d] * dec;
                 dk_a[r][cc] += acc[r][cc] * dec;
                 dG_a[r][cc] -= acc[r][cc] * kh;
-                sW[i * D + d] = acc[r][cc] * kh;
+                sW[i * row_stride<D>() + d] = acc[r][cc] * kh;
             }
     }
     __syncthreads();
     for (int it = tid; it < 4 * D; it += NTHREADS) {
         float t = 0.f;
 #pragma unroll
-        for (int r = 0; r < 16; ++r) t += sW[(16 * (it / D) + r) * D + it % D];
+        for (int r = 0; r < 16; ++r) t += sW[(16 * (it / D) + r) * row_stride<D>() + it % D];
         st[it] = t;
     }
     __syncthreads();
@@ -646,7 +642,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
         float gi[4][4], a1[4][4], a2[4][4], c1[4][4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            const float4 v = *reinterpret_cast<const float4*>(sG + (i0 + r) * D + d0);
+            const float4 v = *reinterpret_cast<const float4*>(sG + (i0 + r) * row_stride<D>() + d0);
             gi[r][0] = v.x; gi[r][1] = v.y; gi[r][2] = v.z; gi[r][3] = v.w;
 #pragma unroll
             for (int c = 0; c < 4; ++c) a1[r][c] = a2[r][c] = c1[r][c] = 0.f;
@@ -654,7 +650,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
         // `inside`: pairs of the tile's own rows, where only j < i counts (the diagonal pair has decay 1 and contributes
         // equal and opposite amounts to dG, so it is kept out of dG exactly)
         auto keys = [&](int j, bool inside) {
-            const float4 kv = *reinterpret_cast<const float4*>(sk + j * D + d0), gv = *reinterpret_cast<const float4*>(sG + j * D + d0);
+            const float4 kv = *reinterpret_cast<const float4*>(sk + j * row_stride<D>() + d0), gv = *reinterpret_cast<const float4*>(sG + j * row_stride<D>() + d0);
             const float4 av = *reinterpret_cast<const float4*>(sT + j * CP + i0), mv = *reinterpret_cast<const float4*>(sY + j * CP + i0);
             const float kj[4] = {kv.x, kv.y, kv.z, kv.w}, gj[4] = {gv.x, gv.y, gv.z, gv.w};
             const float da[4] = {av.x, av.y, av.z, av.w}, dm[4] = {mv.x, mv.y, mv.z, mv.w};
@@ -670,8 +666,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
             }
         };
         auto queries = [&](int ii, bool inside) {
-            const float4 qv = *reinterpret_cast<const float4*>(sq + ii * D + d0), kv = *reinterpret_cast<const float4*>(sk + ii * D + d0);
-            const float4 gv = *reinterpret_cast<const float4*>(sG + ii * D + d0);
+            const float4 qv = *reinterpret_cast<const float4*>(sq + ii * row_stride<D>() + d0), kv = *reinterpret_cast<const float4*>(sk + ii * row_stride<D>() + d0);
+            const float4 gv = *reinterpret_cast<const float4*>(sG + ii * row_stride<D>() + d0);
             const float4 av = *reinterpret_cast<const float4*>(sdA + ii * CP + i0), mv = *reinterpret_cast<const float4*>(sdM + ii * CP + i0);
             const float q4[4] = {qv.x, qv.y, qv.z, qv.w}, k4[4] = {kv.x, kv.y, kv.z, kv.w}, g4[4] = {gv.x, gv.y, gv.z, gv.w};
             const float b = sbeta[ii];
@@ -696,7 +692,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
         for (int r = 0; r < 4; ++r) {
             const int i = i0 + r;
             const float diag = scale * sdA[i * CP + i], b = sbeta[i];
-            const float4 qv = *reinterpret_cast<const float4*>(sq + i * D + d0), kv = *reinterpret_cast<const float4*>(sk + i * D + d0);
+            const float4 qv = *reinterpret_cast<const float4*>(sq + i * row_stride<D>() + d0), kv = *reinterpret_cast<const float4*>(sk + i * row_stride<D>() + d0);
             const float qi[4] = {qv.x, qv.y, qv.z, qv.w}, ki[4] = {kv.x, kv.y, kv.z, kv.w};
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -719,14 +715,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int cc = 0; cc < D / 16; ++cc) sW[(4 * ty + r) * D + tile_col(tx, cc)] = dG_a[r][cc];
+        for (int cc = 0; cc < D / 16; ++cc) sW[(4 * ty + r) * row_stride<D>() + tile_col(tx, cc)] = dG_a[r][cc];
     __syncthreads();
     // thread = (channel, 16-row group): group totals first, then the sums from the last row up
     for (int it = tid; it < 4 * D; it += NTHREADS) {
         const int d = it % D, grp = it / D;
         float t = 0.f;
 #pragma unroll
-        for (int r = 0; r < 16; ++r) t += sW[(16 * grp + r) * D + d];
+        for (int r = 0; r < 16; ++r) t += sW[(16 * grp + r) * row_stride<D>() + d];
         st[it] = t;
     }
     __syncthreads();
@@ -745,7 +741,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
 #pragma unroll 8
             for (int r = 15; r >= 0; --r) {
                 const int i = 16 * grp + r;
-                run += sW[i * D + d];
+                run += sW[i * row_stride<D>() + d];
                 if (i < ci.len) {
                     const size_t off = ((size_t)(ci.tok0 + i) * p.H + h) * D + d;
                     if (gate) {
@@ -790,8 +786,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
             if (l2) {
 #pragma unroll
                 for (int cc = 0; cc < D / 16; ++cc) {
-                    dotq += sq[i * D + tile_col(tx, cc)] * dq_a[r][cc];
-                    dotk += sk[i * D + tile_col(tx, cc)] * dk_a[r][cc];
+                    dotq += sq[i * row_stride<D>() + tile_col(tx, cc)] * dq_a[r][cc];
+                    dotk += sk[i * row_stride<D>() + tile_col(tx, cc)] * dk_a[r][cc];
                 }
                 dotq = row16_sum(dotq);
                 dotk = row16_sum(dotk);
@@ -803,8 +799,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
                     size_t off = ((size_t)(ci.tok0 + i) * p.H + h) * D + d;
                     float a = dq_a[r][cc], b = dk_a[r][cc];
                     if (l2) {
-                        a = (a - sq[i * D + d] * dotq) * srq[i];
-                        b = (b - sk[i * D + d] * dotk) * srk[i];
+                        a = (a - sq[i * row_stride<D>() + d] * dotq) * srq[i];
+                        b = (b - sk[i * row_stride<D>() + d] * dotk) * srk[i];
                     }
                     stf(dq + off, a);
                     stf(dk + off, b);
@@ -869,10 +865,10 @@ __global__ void __launch_bounds__(1024) kda_param_reduce(const KdaParams p) {
 // host-side launchers
 // ---------------------------------------------------------------------------------------
 template <int D>
-constexpr size_t smem_intra() { return (size_t)(4 * C * D + 3 * C * CP + 3 * C + st_floats<D>()) * 4; }
+constexpr size_t smem_intra() { return (size_t)(4 * C * row_stride<D>() + 3 * C * CP + 3 * C + st_floats<D>()) * 4; }
 template <int D>
 constexpr size_t smem_bwd_chunk() {
-    return (size_t)(4 * C * D + 4 * C * CP + 4 * C + D + 8 + st_floats<D>()) * 4;
+    return (size_t)(4 * C * row_stride<D>() + 4 * C * CP + 4 * C + D + 8 + st_floats<D>()) * 4;
 }
 
 template <typename K>

@@ -6,8 +6,8 @@
 //
 // Bound by the dependent chain of one chunk.  The chunk's records arrive as linear 16-byte asynchronous copies, each
 // requested as soon as the previous chunk's product has consumed the same record, so that no product waits for memory;
-// every product reads its operands where they are.  A record is laid out in 8 x 8 core matrices (cm_idx), so it can be
-// read four elements at a time along its second index only.  Products whose second index is the output row give a thread
+// every product reads its operands where they are.  The copies turn the records' 8 x 8 core matrices (cm_idx) into padded
+// rows, read four elements at a time along the second index.  Products whose second index is the output row give a thread
 // four rows x two columns and split the inner index over thread groups (`rows4`); products whose second index is the
 // inner one give a thread one row and walk the inner index by fours (`dots`).
 #include "kda_common.cuh"
@@ -28,13 +28,27 @@ __device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&v)[4]) {
     v[2] = __uint_as_float(r.y << 16); v[3] = __uint_as_float(r.y & 0xffff0000u);
 }
 
-// asynchronous linear copy of `bytes` (a multiple of 16) by the whole CTA
-__device__ __forceinline__ void copy_record(void* dst, const void* src, int bytes) {
-    for (int o = threadIdx.x * 16; o < bytes; o += NT * 16) tc::cp_async16_z((char*)dst + o, (const char*)src + o, true);
+// Row stride of a record in shared memory: 16 bytes more than a row, so that neither a walk along a row nor eight rows
+// at the same column meet in a bank
+template <typename T>
+constexpr int stride(int cols) { return cols + 16 / (int)sizeof(T); }
+
+// asynchronous copy of a record cm(row, col; COLS) of R rows into plain rows, by the whole CTA
+template <int R, int COLS, typename T>
+__device__ __forceinline__ void copy_record(T* dst, const T* src) {
+    constexpr int E = 16 / sizeof(T);  // elements of a chunk: a half row (FP32) or a row (BF16) of a core matrix
+#pragma unroll
+    for (int q = threadIdx.x; q < R * COLS / E; q += NT) {
+        const int at = q * E, blk = at >> 6, r = blk / (COLS / 8) * 8 + ((at >> 3) & 7), c = blk % (COLS / 8) * 8 + (at & 7);
+        tc::cp_async16_z(dst + r * stride<T>(COLS) + c, src + at, true);
+    }
+}
+__device__ __forceinline__ void copy_floats(float* dst, const float* src, int n) {
+    for (int o = threadIdx.x * 4; o < n; o += NT * 4) tc::cp_async16_z(dst + o, src + o, true);
 }
 
 // acc[4][2] = sum over k of A(k, 4 rq + r) * B[k][2 ep + c] for this thread group's share of k.
-// A: record cm(k, row; COLS) of K rows; B: float [K][BV]; R = number of output rows
+// A: record of K rows (k) and COLS columns (output row); B: float [K][BV]; R = number of output rows
 template <int R, int COLS, int K, int BV, typename T>
 __device__ __forceinline__ void rows4(float (&acc)[4][2], const T* A, const float* B) {
     constexpr int RQ = R / 4, SPLIT = NT / (RQ * (BV / 2));
@@ -43,7 +57,7 @@ __device__ __forceinline__ void rows4(float (&acc)[4][2], const T* A, const floa
 #pragma unroll 8
     for (int k = ks * (K / SPLIT); k < (ks + 1) * (K / SPLIT); ++k) {
         float a[4];
-        load4(A + tc::cm_idx(k, 4 * rq, COLS), a);
+        load4(A + k * stride<T>(COLS) + 4 * rq, a);
         const float2 b = *reinterpret_cast<const float2*>(B + k * BV + 2 * ep);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -65,13 +79,13 @@ __device__ __forceinline__ int rows4_store(const float (&acc)[4][2], float* part
 template <int R, int BV>
 constexpr int rows4_floats() { return NT / (R / 4 * (BV / 2)) * R * BV; }
 
-// acc[NC] += sum over k of A(row, k) * B[k][col0 + c], A: record cm(row, k; K)
+// acc[NC] += sum over k of A(row, k) * B[k][col0 + c], A: record of rows (output row) and K columns (k)
 template <int K, int NC, int BV, typename T>
 __device__ __forceinline__ void dots(float (&acc)[NC], const T* A, int row, const float* B, int col0) {
 #pragma unroll 4
     for (int k = 0; k < K; k += 4) {
         float a[4];
-        load4(A + tc::cm_idx(row, k, K), a);
+        load4(A + row * stride<T>(K) + k, a);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -86,8 +100,8 @@ __device__ __forceinline__ void dots(float (&acc)[NC], const T* A, int row, cons
 // shared memory: the records W, Qt, Kh, Aqk, then S [D][BV], V' [64][BV], a second [64][BV] (U panel / dO), partial sums
 template <typename T, int D, int BV>
 struct Smem {
-    static constexpr int REC = C * D * (int)sizeof(T), AREC = C * C * (int)sizeof(T);
-    static constexpr int W = 0, QT = REC, KH = 2 * REC, AQ = 3 * REC, S = AQ + AREC, VN = S + D * BV * 4, X = VN + C * BV * 4;
+    static constexpr int WREC = D * stride<T>(C) * (int)sizeof(T), REC = C * stride<T>(D) * (int)sizeof(T);
+    static constexpr int W = 0, QT = WREC, KH = QT + REC, AQ = KH + REC, S = AQ + C * stride<T>(C) * (int)sizeof(T), VN = S + D * BV * 4, X = VN + C * BV * 4;
     static constexpr int GAM = X + C * BV * 4, PART = GAM + D * 4;
     static constexpr int PFLOATS = rows4_floats<C, BV>() > rows4_floats<D, BV>() ? rows4_floats<C, BV>() : rows4_floats<D, BV>();
     static constexpr int TOTAL = PART + PFLOATS * 4;
@@ -99,7 +113,7 @@ __global__ void __launch_bounds__(ss::NT) kda_fwd_state_simt(const KdaParams p) 
     using namespace ss;
     using M = Smem<T, D, BV>;
     extern __shared__ __align__(16) unsigned char dyn[];
-    const T *sW = (const T*)(dyn + M::W), *sQt = (const T*)(dyn + M::QT), *sKh = (const T*)(dyn + M::KH), *sA = (const T*)(dyn + M::AQ);
+    T *sW = (T*)(dyn + M::W), *sQt = (T*)(dyn + M::QT), *sKh = (T*)(dyn + M::KH), *sA = (T*)(dyn + M::AQ);
     float *sS = (float*)(dyn + M::S), *sVn = (float*)(dyn + M::VN), *sGam = (float*)(dyn + M::GAM), *part = (float*)(dyn + M::PART);
     const int tid = threadIdx.x;
     const int e0 = blockIdx.x * BV, h = blockIdx.y, n = blockIdx.z;
@@ -123,17 +137,17 @@ __global__ void __launch_bounds__(ss::NT) kda_fwd_state_simt(const KdaParams p) 
     float u[BV / 4];
     // copy groups in the order of use: W (with gamC), Qt and Aqk, Kh
     auto get_w = [&](int c) {
-        copy_record(dyn + M::W, (const T*)(ws + L.W) + rec_of(c) * C * D, M::REC);
+        copy_record<D, C>(sW, (const T*)(ws + L.W) + rec_of(c) * C * D);
         tc::cp_async_commit();
     };
     auto get_q = [&](int c) {
-        copy_record(dyn + M::QT, (const T*)(ws + L.Qt) + rec_of(c) * C * D, M::REC);
-        copy_record(dyn + M::AQ, (const T*)(ws + L.Aqk) + rec_of(c) * C * C, M::AREC);
+        copy_record<C, D>(sQt, (const T*)(ws + L.Qt) + rec_of(c) * C * D);
+        copy_record<C, C>(sA, (const T*)(ws + L.Aqk) + rec_of(c) * C * C);
         tc::cp_async_commit();
     };
     auto get_k = [&](int c) {
-        copy_record(dyn + M::KH, (const T*)(ws + L.Kh) + rec_of(c) * C * D, M::REC);
-        copy_record(dyn + M::GAM, (const float*)(ws + L.gamC) + rec_of(c) * D, D * 4);
+        copy_record<C, D>(sKh, (const T*)(ws + L.Kh) + rec_of(c) * C * D);
+        copy_floats(sGam, (const float*)(ws + L.gamC) + rec_of(c) * D, D);
         tc::cp_async_commit();
     };
     if (sq.c_begin < sq.c_end) {
@@ -207,7 +221,7 @@ __global__ void __launch_bounds__(ss::NT) kda_bwd_state_simt(const KdaParams p) 
     using namespace ss;
     using M = Smem<T, D, BV>;
     extern __shared__ __align__(16) unsigned char dyn[];
-    const T *sW = (const T*)(dyn + M::W), *sQt = (const T*)(dyn + M::QT), *sKh = (const T*)(dyn + M::KH), *sA = (const T*)(dyn + M::AQ);
+    T *sW = (T*)(dyn + M::W), *sQt = (T*)(dyn + M::QT), *sKh = (T*)(dyn + M::KH), *sA = (T*)(dyn + M::AQ);
     float *sS = (float*)(dyn + M::S), *sVn = (float*)(dyn + M::VN), *sdO = (float*)(dyn + M::X), *sGam = (float*)(dyn + M::GAM),
           *part = (float*)(dyn + M::PART);
     const int tid = threadIdx.x;
@@ -232,14 +246,14 @@ __global__ void __launch_bounds__(ss::NT) kda_bwd_state_simt(const KdaParams p) 
     }
     // copy groups in the order of use: Aqk and Kh, Qt and W (with gamC)
     auto get_a = [&](int c) {
-        copy_record(dyn + M::AQ, (const T*)(ws + L.Aqk) + rec_of(c) * C * C, M::AREC);
-        copy_record(dyn + M::KH, (const T*)(ws + L.Kh) + rec_of(c) * C * D, M::REC);
+        copy_record<C, C>(sA, (const T*)(ws + L.Aqk) + rec_of(c) * C * C);
+        copy_record<C, D>(sKh, (const T*)(ws + L.Kh) + rec_of(c) * C * D);
         tc::cp_async_commit();
     };
     auto get_w = [&](int c) {
-        copy_record(dyn + M::QT, (const T*)(ws + L.Qt) + rec_of(c) * C * D, M::REC);
-        copy_record(dyn + M::W, (const T*)(ws + L.W) + rec_of(c) * C * D, M::REC);
-        copy_record(dyn + M::GAM, (const float*)(ws + L.gamC) + rec_of(c) * D, D * 4);
+        copy_record<C, D>(sQt, (const T*)(ws + L.Qt) + rec_of(c) * C * D);
+        copy_record<D, C>(sW, (const T*)(ws + L.W) + rec_of(c) * C * D);
+        copy_floats(sGam, (const float*)(ws + L.gamC) + rec_of(c) * D, D);
         tc::cp_async_commit();
     };
     float x[BV / 4];
