@@ -76,8 +76,8 @@ __device__ __forceinline__ void mm_tile(float (&acc)[4][N / 16], int K, LA la, L
         }
         __syncthreads();
         if (k0 + KS < K) fetch(k0 + KS);
-#pragma unroll
-        for (int k = 0; k < KS; ++k) {
+#pragma unroll 4
+        for (int k = 0; k < KS; ++k) {  // (not unrolled further: a CTA runs the code of every product once)
             float a[4], b[N / 16];
             const float4 av = *reinterpret_cast<const float4*>(stA + k * SA + 4 * ty);
             a[0] = av.x; a[1] = av.y; a[2] = av.z; a[3] = av.w;
@@ -320,27 +320,33 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_fwd_intra_simt(const KdaParam
     }
     __syncthreads();
 
-    // T = (I + diag(beta) L)^-1 by forward substitution: four lanes of a warp own a column and keep it in registers, so
-    // the 64 dependent rows need no barrier
+    // T = (I + diag(beta) L)^-1 by forward substitution, 16 rows at a time: four lanes of a warp own a column, first sum
+    // what the rows before the block contribute, then solve the block in registers.  No barrier between dependent rows.
     {
         const int col = tid >> 2, part = tid & 3;
-        float t[C / 4];
+        for (int b = 0; b < C; b += 16) {
+            float s[16], t[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int m = 0; m < C / 4; ++m) t[m] = 0.f;
+            for (int r = 0; r < 16; ++r) s[r] = 0.f;
+            for (int j = part; j < b; j += 4) {
+                const float tj = sT[j * CP + col];
 #pragma unroll
-        for (int i = 0; i < C; ++i) {
-            float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-            for (int m = 0; 4 * m < i; m += 2) {  // (entries that are not known yet are zero)
-                s0 = fmaf(sL[i * CP + 4 * m + part], t[m], s0);
-                if (4 * m + 4 < i) s1 = fmaf(sL[i * CP + 4 * m + 4 + part], t[m + 1], s1);
+                for (int r = 0; r < 16; ++r) s[r] = fmaf(sL[(b + r) * CP + j], tj, s[r]);
             }
-            float s = s0 + s1;
-            s += __shfl_xor_sync(0xffffffffu, s, 1);
-            s += __shfl_xor_sync(0xffffffffu, s, 2);
-            const float v = col <= i ? (i == col ? 1.f : 0.f) - sbeta[i] * s : 0.f;
-            if (part == (i & 3)) t[i >> 2] = v;
-            if (part == 0) sT[i * CP + col] = v;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                float x = s[r];
+#pragma unroll
+                for (int m = 0; 4 * m < r; ++m) x = fmaf(sL[(b + r) * CP + b + 4 * m + part], t[m], x);  // (unknown entries are 0)
+                x += __shfl_xor_sync(0xffffffffu, x, 1);
+                x += __shfl_xor_sync(0xffffffffu, x, 2);
+                const float v = col <= b + r ? (b + r == col ? 1.f : 0.f) - sbeta[b + r] * x : 0.f;
+                if (part == (r & 3)) {
+                    t[r >> 2] = v;
+                    sT[(b + r) * CP + col] = v;
+                }
+            }
+            __syncwarp();
         }
     }
     __syncthreads();

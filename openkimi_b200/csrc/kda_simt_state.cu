@@ -8,8 +8,8 @@
 // requested as soon as the previous chunk's product has consumed the same record, so that no product waits for memory;
 // every product reads its operands where they are.  The copies turn the records' 8 x 8 core matrices (cm_idx) into padded
 // rows, read four elements at a time along the second index.  Products whose second index is the output row give a thread
-// four rows x two columns and split the inner index over thread groups (`rows4`); products whose second index is the
-// inner one give a thread one row and walk the inner index by fours (`dots`).
+// four rows x two columns (`rows4`); products whose second index is the inner one give a thread one row x eight columns
+// and walk the inner index by fours (`dots`); both split the inner index over thread groups.
 #include "kda_common.cuh"
 #include "kda_tc.cuh"
 
@@ -66,35 +66,54 @@ __device__ __forceinline__ void rows4(float (&acc)[4][2], const T* A, const floa
         }
     }
 }
-// leaves a rows4 result in part[group][R][BV]; returns the number of groups
+// leaves a rows4 result in part[group][R][BV]
 template <int R, int BV>
-__device__ __forceinline__ int rows4_store(const float (&acc)[4][2], float* part) {
-    constexpr int RQ = R / 4, SPLIT = NT / (RQ * (BV / 2));
+constexpr int rows4_groups() { return NT / (R / 4 * (BV / 2)); }
+template <int R, int BV>
+__device__ __forceinline__ void rows4_store(const float (&acc)[4][2], float* part) {
+    constexpr int RQ = R / 4;
     const int rq = threadIdx.x % RQ, ep = (threadIdx.x / RQ) % (BV / 2), ks = threadIdx.x / (RQ * (BV / 2));
 #pragma unroll
     for (int r = 0; r < 4; ++r)
         *reinterpret_cast<float2*>(part + (ks * R + 4 * rq + r) * BV + 2 * ep) = make_float2(acc[r][0], acc[r][1]);
-    return SPLIT;
 }
-template <int R, int BV>
-constexpr int rows4_floats() { return NT / (R / 4 * (BV / 2)) * R * BV; }
+// sum of the partial results of one element
+template <int R, int BV, int GROUPS>
+__device__ __forceinline__ float part_sum(const float* part, int at) {
+    float s = 0.f;
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g) s += part[g * R * BV + at];
+    return s;
+}
 
-// acc[NC] += sum over k of A(row, k) * B[k][col0 + c], A: record of rows (output row) and K columns (k)
-template <int K, int NC, int BV, typename T>
-__device__ __forceinline__ void dots(float (&acc)[NC], const T* A, int row, const float* B, int col0) {
-#pragma unroll 4
-    for (int k = 0; k < K; k += 4) {
+// acc[8] += sum over this thread's share of k of A(row, k) * B[k][8 cg + c]: thread = one of R rows x eight columns x a
+// part of the inner index.  A: record of rows (output row) and K columns (k)
+template <int R, int BV>
+constexpr int dots_groups() { return NT / (R * (BV / 8)); }
+template <int R, int K, int BV, typename T>
+__device__ __forceinline__ void dots(float (&acc)[8], const T* A, const float* B) {
+    constexpr int KN = K / dots_groups<R, BV>();
+    const int row = threadIdx.x % R, cg = (threadIdx.x / R) % (BV / 8), ks = threadIdx.x / (R * (BV / 8));
+#pragma unroll 2
+    for (int k = ks * KN; k < (ks + 1) * KN; k += 4) {
         float a[4];
         load4(A + row * stride<T>(K) + k, a);
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int c = 0; c < NC; c += 2) {
-                const float2 b = *reinterpret_cast<const float2*>(B + (k + j) * BV + col0 + c);
-                acc[c] = fmaf(a[j], b.x, acc[c]);
-                acc[c + 1] = fmaf(a[j], b.y, acc[c + 1]);
-            }
+        for (int j = 0; j < 4; ++j) {
+            const float4 b0 = *reinterpret_cast<const float4*>(B + (k + j) * BV + 8 * cg), b1 = *reinterpret_cast<const float4*>(B + (k + j) * BV + 8 * cg + 4);
+            acc[0] = fmaf(a[j], b0.x, acc[0]); acc[1] = fmaf(a[j], b0.y, acc[1]);
+            acc[2] = fmaf(a[j], b0.z, acc[2]); acc[3] = fmaf(a[j], b0.w, acc[3]);
+            acc[4] = fmaf(a[j], b1.x, acc[4]); acc[5] = fmaf(a[j], b1.y, acc[5]);
+            acc[6] = fmaf(a[j], b1.z, acc[6]); acc[7] = fmaf(a[j], b1.w, acc[7]);
+        }
     }
+}
+template <int R, int BV>
+__device__ __forceinline__ void dots_store(const float (&acc)[8], float* part) {
+    const int row = threadIdx.x % R, cg = (threadIdx.x / R) % (BV / 8), ks = threadIdx.x / (R * (BV / 8));
+    float4* dst = reinterpret_cast<float4*>(part + (ks * R + row) * BV + 8 * cg);
+    dst[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    dst[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
 }
 
 // shared memory: the records W, Qt, Kh, Aqk, then S [D][BV], V' [64][BV], a second [64][BV] (U panel / dO), partial sums
@@ -103,13 +122,14 @@ struct Smem {
     static constexpr int WREC = D * stride<T>(C) * (int)sizeof(T), REC = C * stride<T>(D) * (int)sizeof(T);
     static constexpr int W = 0, QT = WREC, KH = QT + REC, AQ = KH + REC, S = AQ + C * stride<T>(C) * (int)sizeof(T), VN = S + D * BV * 4, X = VN + C * BV * 4;
     static constexpr int GAM = X + C * BV * 4, PART = GAM + D * 4;
-    static constexpr int PFLOATS = rows4_floats<C, BV>() > rows4_floats<D, BV>() ? rows4_floats<C, BV>() : rows4_floats<D, BV>();
-    static constexpr int TOTAL = PART + PFLOATS * 4;
+    // partial sums of rows4 and of dots (the numbers of floats do not depend on R)
+    static constexpr int P4 = rows4_groups<C, BV>() * C * BV, P8 = dots_groups<C, BV>() * C * BV;
+    static constexpr int TOTAL = PART + (P4 + P8) * 4;
 };
 }  // namespace ss
 
 template <typename T, int D, int BV>
-__global__ void __launch_bounds__(ss::NT) kda_fwd_state_simt(const KdaParams p) {
+__global__ void __launch_bounds__(ss::NT, 1) kda_fwd_state_simt(const KdaParams p) {
     using namespace ss;
     using M = Smem<T, D, BV>;
     extern __shared__ __align__(16) unsigned char dyn[];
@@ -167,15 +187,13 @@ __global__ void __launch_bounds__(ss::NT) kda_fwd_state_simt(const KdaParams p) 
         {  // V' = U - W S
             float acc[4][2] = {};
             rows4<C, C, D, BV>(acc, sW, sS);
-            const int groups = rows4_store<C, BV>(acc, part);
+            rows4_store<C, BV>(acc, part);
             __syncthreads();
             if (more) get_w(c + 1);
             else tc::cp_async_commit();
 #pragma unroll
             for (int j = 0; j < BV / 4; ++j) {
-                float s = 0.f;
-                for (int g = 0; g < groups; ++g) s += part[(g * C + ui) * BV + uc + j];
-                const float vn = u[j] - s;
+                const float vn = u[j] - part_sum<C, BV, rows4_groups<C, BV>()>(part, ui * BV + uc + j);
                 sVn[ui * BV + uc + j] = vn;
                 if (save) stf(gUbase + rec_of(c) * C * D + tc::cm_idx(e0 + uc + j, ui, C), vn);
             }
@@ -183,27 +201,25 @@ __global__ void __launch_bounds__(ss::NT) kda_fwd_state_simt(const KdaParams p) 
         }
         tc::cp_async_wait<1>();  // Qt, Aqk and Kh of this chunk have landed
         __syncthreads();
-        {  // O = Qt S + Aqk V'
-            float acc[BV / 4] = {};
-            dots<D, BV / 4, BV>(acc, sQt, ui, sS, uc);
-            dots<C, BV / 4, BV>(acc, sA, ui, sVn, uc);
-            if (ui < sq.rows(c)) {
-                T* o = (T*)p.o + ((size_t)(sq.tok(c) + ui) * p.H + h) * D + e0 + uc;
-#pragma unroll
-                for (int j = 0; j < BV / 4; ++j) stf(o + j, acc[j]);
-            }
+        {
+            float acc[8] = {};  // O = Qt S + Aqk V'
+            dots<C, D, BV>(acc, sQt, sS);
+            dots<C, C, BV>(acc, sA, sVn);
+            dots_store<C, BV>(acc, part + M::P4);
+            float kacc[4][2] = {};  // Kh^T V'
+            rows4<D, D, C, BV>(kacc, sKh, sVn);
+            rows4_store<D, BV>(kacc, part);
         }
-        float kacc[4][2] = {};  // Kh^T V'
-        rows4<D, D, C, BV>(kacc, sKh, sVn);
-        const int groups = rows4_store<D, BV>(kacc, part);
         __syncthreads();
         if (more) get_q(c + 1);
         else tc::cp_async_commit();
-        for (int idx = tid; idx < D * BV; idx += NT) {
-            float s = sGam[idx / BV] * sS[idx];
-            for (int g = 0; g < groups; ++g) s += part[g * D * BV + idx];
-            sS[idx] = s;
+        if (ui < sq.rows(c)) {
+            T* o = (T*)p.o + ((size_t)(sq.tok(c) + ui) * p.H + h) * D + e0 + uc;
+#pragma unroll
+            for (int j = 0; j < BV / 4; ++j) stf(o + j, part_sum<C, BV, dots_groups<C, BV>()>(part + M::P4, ui * BV + uc + j));
         }
+        for (int idx = tid; idx < D * BV; idx += NT)
+            sS[idx] = sGam[idx / BV] * sS[idx] + part_sum<D, BV, rows4_groups<D, BV>()>(part, idx);
         __syncthreads();
         if (more) get_k(c + 1);
         else tc::cp_async_commit();
@@ -217,7 +233,7 @@ __global__ void __launch_bounds__(ss::NT) kda_fwd_state_simt(const KdaParams p) 
 
 // Stores the dS entering each chunk (from the right) and dV'.
 template <typename T, int D, int BV>
-__global__ void __launch_bounds__(ss::NT) kda_bwd_state_simt(const KdaParams p) {
+__global__ void __launch_bounds__(ss::NT, 1) kda_bwd_state_simt(const KdaParams p) {
     using namespace ss;
     using M = Smem<T, D, BV>;
     extern __shared__ __align__(16) unsigned char dyn[];
@@ -272,39 +288,35 @@ __global__ void __launch_bounds__(ss::NT) kda_bwd_state_simt(const KdaParams p) 
         T* gdS = (T*)(sc + L.dS) + rec_of(c) * D * D;
         for (int idx = tid; idx < D * BV; idx += NT) stf(gdS + tc::cm_idx(e0 + idx / D, idx % D, D), sS[(idx % D) * BV + idx / D]);
         {  // dV' = Aqk^T dO + Kh dS
-            float acc[4][2] = {}, own[BV / 4] = {};
+            float acc[4][2] = {}, own[8] = {};
             rows4<C, C, C, BV>(acc, sA, sdO);
-            const int groups = rows4_store<C, BV>(acc, part);
-            dots<D, BV / 4, BV>(own, sKh, ui, sS, uc);
+            rows4_store<C, BV>(acc, part);
+            dots<C, D, BV>(own, sKh, sS);
+            dots_store<C, BV>(own, part + M::P4);
             __syncthreads();
             if (more) get_a(c - 1);
             else tc::cp_async_commit();
             T* gdV = (T*)(sc + L.dVn) + rec_of(c) * C * D;
 #pragma unroll
             for (int j = 0; j < BV / 4; ++j) {
-                float s = own[j];
-                for (int g = 0; g < groups; ++g) s += part[(g * C + ui) * BV + uc + j];
-                sVn[ui * BV + uc + j] = s;
+                const int at = ui * BV + uc + j;
+                const float s = part_sum<C, BV, rows4_groups<C, BV>()>(part, at) + part_sum<C, BV, dots_groups<C, BV>()>(part + M::P4, at);
+                sVn[at] = s;
                 stf(gdV + tc::cm_idx(e0 + uc + j, ui, C), s);
             }
         }
         tc::cp_async_wait<1>();
         __syncthreads();
         {  // dS <- diag(gamC) dS + Qt^T dO - W^T dV'
-            float acc[4][2] = {};
+            float acc[4][2] = {}, own[8] = {};
             rows4<D, D, C, BV>(acc, sQt, sdO);
-            const int groups = rows4_store<D, BV>(acc, part);
-            constexpr int NC = D * BV / NT;                       // columns per thread of one row of dS
-            const int d = tid % D, dc = (tid / D) * NC;
-            float own[NC] = {};
-            dots<C, NC, BV>(own, sW, d, sVn, dc);
+            rows4_store<D, BV>(acc, part);
+            dots<D, C, BV>(own, sW, sVn);
+            dots_store<D, BV>(own, part + M::P4);
             __syncthreads();
-#pragma unroll
-            for (int j = 0; j < NC; ++j) {
-                float s = sGam[d] * sS[d * BV + dc + j] - own[j];
-                for (int g = 0; g < groups; ++g) s += part[(g * D + d) * BV + dc + j];
-                sS[d * BV + dc + j] = s;
-            }
+            for (int idx = tid; idx < D * BV; idx += NT)
+                sS[idx] = sGam[idx / BV] * sS[idx] + part_sum<D, BV, rows4_groups<D, BV>()>(part, idx) -
+                          part_sum<D, BV, dots_groups<D, BV>()>(part + M::P4, idx);
         }
         __syncthreads();
         if (more) get_w(c - 1);
