@@ -14,7 +14,7 @@ namespace tc {
 // where the caller has the room, and by 16-byte accesses otherwise.
 __device__ __forceinline__ int stage_idx(int e, int chunk) { return e * 128 + ((chunk ^ (e & 7)) << 2); }
 
-// src NULL: zero state.  With `stage` every thread of the CTA calls (it synchronises).
+// src NULL: zero state.  With `stage` all 256 threads call (named barrier 1).
 __device__ __forceinline__ void state_fill(uint32_t tmem_acc, const float* src, bool rows, float* stage, int tid, int e, int half) {
     const bool staged = src && rows && stage;
     if (staged) {
@@ -25,7 +25,7 @@ __device__ __forceinline__ void state_fill(uint32_t tmem_acc, const float* src, 
         }
         cp_async_commit();
         cp_async_wait<0>();
-        __syncthreads();
+        bar_sync(1, 256);
     }
     for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
         uint32_t r[16];
@@ -48,7 +48,7 @@ __device__ __forceinline__ void state_fill(uint32_t tmem_acc, const float* src, 
     tmem_wait_st();
     if (staged) {  // the caller reuses the space for bulk copies
         fence_async_smem();
-        __syncthreads();
+        bar_sync(1, 256);
     }
 }
 
@@ -71,7 +71,7 @@ __device__ __forceinline__ void state_drain(uint32_t tmem_acc, float* dst, bool 
         }
     }
     if (staged) {
-        __syncthreads();
+        bar_sync(1, 256);
 #pragma unroll 4
         for (int i = 0; i < 16; ++i) {
             const int q = tid + 256 * i, r = q >> 5, c = q & 31;

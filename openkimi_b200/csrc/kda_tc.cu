@@ -139,18 +139,21 @@ __global__ void __launch_bounds__(128, 1) wait_selftest_kernel(const float* __re
 }
 
 // ---------------------------------------------------------------------------------------
-// fwd_state on tensor cores.  One CTA per (sequence, head); thread t owns value column
-// e = t, which is TMEM lane t.  The state is kept TRANSPOSED in tensor memory for the whole
-// sequence: Sacc[e][d] (FP32, 128 columns).  Per chunk:
+// fwd_state on tensor cores.  One CTA per (sequence, head), or per segment of the chunk numbering and head; value column e
+// is TMEM lane e.  The state is kept TRANSPOSED in tensor memory for the whole walk: Sacc[e][d] (FP32, 128 columns).
+// Per chunk:
 //   A  read Sacc -> BF16 copy Sbf (MMA operand, also the chunk-entry checkpoint), decay Sacc
 //   1  WSacc = Sbf * W^T        (V'^T = U^T - WSacc)        Oacc  = Sbf * Qt^T
 //   B  V'^T -> BF16 Vbf (MMA operand) and the V' record
-//   2  Oacc += Vbf * Aqk^T      Sacc += Vbf * Kh
-//   C  o = Oacc
-// The per-chunk records arrive by linear bulk TMA copies into a two-stage ring.
+//   2  Sacc += Vbf * Kh         Oacc += Vbf * Aqk^T
+// Bound by the chain A, W S, B, K V: two MMA round trips and two conversions per chunk.  Everything else is kept off that
+// chain by giving it to other warps: a producer warp requests the records (linear bulk copies into a two-stage ring), four
+// warps turn finished Oacc tiles into output rows while the next chunk runs, records that leave the chip (checkpoint, V')
+// are stored after the MMA issue they used to precede.  One thread issues all products of one accumulator, so only the
+// products the chain needs are waited for (8 chunks of one sequence: 21.1 -> 15.9 us).
 // ---------------------------------------------------------------------------------------
 namespace fs {
-constexpr int D = 128, NTHR = 256;
+constexpr int D = 128, MAIN = 256, OUTT = 128, NTHR = MAIN + OUTT + 32;
 constexpr uint32_t WT = 0, QT = 16384, KH = 32768, UT = 49152, AQ = 65536, GAM = 73728, STAGE = 74240;
 constexpr uint32_t OUT = 2 * STAGE, TOTAL = OUT + 16384;  // output tile bf16 [64][128] behind the two stages
 constexpr uint32_t SACC = 0, SBF = 128, WSACC = 192, OACC = 256, VBF = 320, TMEM_COLS = 512;
@@ -166,15 +169,45 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
     }
 }
 
+// Phase A of both state kernels: this thread's 64 columns of the accumulator, all loads in flight at once.  pk receives
+// the BF16 copy (pairs), which also goes to `bf`; the accumulator is decayed by gam.
+__device__ __forceinline__ void state_convert(uint32_t acc, uint32_t bf, int c0, const float* gam, uint32_t (&pk)[4][8]) {
+    uint32_t r[4][16];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) tmem_ld16(acc + c0 + 16 * g, r[g]);
+    tmem_wait_ld();
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) pk[g][j] = pack_bf16(__uint_as_float(r[g][2 * j]), __uint_as_float(r[g][2 * j + 1]));
+        tmem_st8(bf + (c0 + 16 * g) / 2, pk[g]);
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) {
+            const float4 gm = *reinterpret_cast<const float4*>(gam + c0 + 16 * g + j);
+            r[g][j] = __float_as_uint(__uint_as_float(r[g][j]) * gm.x);
+            r[g][j + 1] = __float_as_uint(__uint_as_float(r[g][j + 1]) * gm.y);
+            r[g][j + 2] = __float_as_uint(__uint_as_float(r[g][j + 2]) * gm.z);
+            r[g][j + 3] = __float_as_uint(__uint_as_float(r[g][j + 3]) * gm.w);
+        }
+        tmem_st16(acc + c0 + 16 * g, r[g]);
+    }
+    tmem_wait_st();
+}
+// 16 BF16 values (columns c0 .. c0 + 15 of row e) into a core-matrix record of `cols` columns
+__device__ __forceinline__ void store_record16(__nv_bfloat16* dst, int e, int c0, int cols, const uint32_t (&pk)[8]) {
+    *reinterpret_cast<uint4*>(dst + cm_idx(e, c0, cols)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+    *reinterpret_cast<uint4*>(dst + cm_idx(e, c0 + 8, cols)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+}
+
 __global__ void __launch_bounds__(fs::NTHR, 1)
 kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const StateSegs segs) {
     using namespace fs;
     extern __shared__ __align__(128) unsigned char dyn[];
-    __shared__ uint64_t full[2];
-    __shared__ uint64_t mmabar;
+    __shared__ uint64_t full[2], empty[2], wsbar, sbar, obar, ofree;
     __shared__ uint32_t tmem_s;
-    // thread (half, e) = (tid / 128, tid % 128): TMEM lane e (value column e), and half of the accumulator
-    // columns in every conversion phase (two warps share a lane quadrant)
+    // main threads (half, e) = (tid / 128, tid % 128): TMEM lane e (value column e), and half of the accumulator
+    // columns in every conversion phase (two warps share a lane quadrant); then the output threads, lane e each; then
+    // the producer warp
     const int tid = threadIdx.x, warp = tid >> 5, e = tid & 127, half = tid >> 7;
     const int h = blockIdx.x;
     // the chunks of this CTA: one sequence, or one segment of the chunk numbering
@@ -196,10 +229,15 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
         tmem_relinquish();
     }
     if (tid == 0) {
-        mbar_init(&full[0], 1);
-        mbar_init(&full[1], 1);
-        mbar_init(&mmabar, 2);  // two issuing threads per MMA group (one accumulator each): a single thread spends
-                                // ~50 ns on every MMA it issues, which is on the critical path of the chunk loop
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 1);
+        }
+        mbar_init(&wsbar, 1);
+        mbar_init(&sbar, 1);
+        mbar_init(&obar, 1);
+        mbar_init(&ofree, OUTT / 32);
         mbar_fence_init();
     }
     tc_fence_before();
@@ -208,192 +246,189 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
     const uint32_t tmem = tmem_s + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's lane quadrant
     const uint32_t tmem0 = tmem_s;
     const bool save = !(p.flags & KDA_FLAG_NO_SAVE);  // forward-only calls write no checkpoint and no V' record
-
     const bool vfirst = p.flags & KDA_FLAG_STATE_V_FIRST;
     float* stage_space = reinterpret_cast<float*>(dyn);  // before the first and after the last chunk's copies
-    // state entering the segment (what the previous one ended with), or a sequence (h0 or zero)
-    if (cb > sq.c_begin)
-        state_fill(tmem + SACC, segs.E + (((size_t)blockIdx.y - 1) * p.H + h) * D * D, false, nullptr, tid, e, half);
-    else
-        state_fill(tmem + SACC, state_of(p.h0, p, sq.n, h), vfirst, stage_space, tid, e, half);
+    if (tid < MAIN) {
+        // state entering the segment (what the previous one ended with), or a sequence (h0 or zero)
+        if (cb > sq.c_begin)
+            state_fill(tmem + SACC, segs.E + (((size_t)blockIdx.y - 1) * p.H + h) * D * D, false, nullptr, tid, e, half);
+        else
+            state_fill(tmem + SACC, state_of(p.h0, p, sq.n, h), vfirst, stage_space, tid, e, half);
+    }
+    __syncthreads();
 
-    // the six records of a chunk: one copy each from lane 0 of six warps (a thread spends ~30 ns on every bulk
-    // copy it issues, and the chunk step waits for the slowest thread)
-    auto issue_loads = [&](int c, int stage) {
-        if ((tid & 31) != 0 || warp >= 6) return;
-        const size_t rec = (size_t)c * p.H + h;
-        unsigned char* b = dyn + stage * STAGE;
-        if (warp == 0) {
-            mbar_expect_tx(&full[stage], STAGE);
-            tma_load_1d(b + WT, (const __nv_bfloat16*)(ws + L.W) + rec * C * D, 16384, &full[stage]);
-        } else if (warp == 1) {
-            tma_load_1d(b + UT, (const __nv_bfloat16*)(ws + L.U) + rec * C * D, 16384, &full[stage]);
-        } else if (warp == 2) {
-            tma_load_1d(b + QT, (const __nv_bfloat16*)(ws + L.Qt) + rec * C * D, 16384, &full[stage]);
-        } else if (warp == 3) {
-            tma_load_1d(b + KH, (const __nv_bfloat16*)(ws + L.Kh) + rec * C * D, 16384, &full[stage]);
-        } else if (warp == 4) {
-            tma_load_1d(b + AQ, (const __nv_bfloat16*)(ws + L.Aqk) + rec * C * C, 8192, &full[stage]);
-        } else {
-            tma_load_1d(b + GAM, (const float*)(ws + L.gamC) + rec * D, 512, &full[stage]);
-        }
-    };
-    if (cb < ce) issue_loads(cb, 0);
-
-    uint32_t mma_phase = 0;
     bool ok = true;
-    KDA_PHASE_BEGIN();
-    __nv_bfloat16* o = (__nv_bfloat16*)p.o;
-    for (int c = cb; c < ce; ++c) {
-        const int stage = (c - cb) & 1;
-        unsigned char* b = dyn + stage * STAGE;
-        const size_t rec = (size_t)c * p.H + h;
-        // the next chunk's records are requested first thing (the other stage was last read by the previous
-        // chunk's MMAs, which completed before that chunk's iteration ended): a whole chunk step ahead of their use
-        if (c + 1 < ce) issue_loads(c + 1, stage ^ 1);
-        tma_store_wait_read();  // the previous chunk's output rows have left the staging tile
-        if (c == sq.c_end) {  // (segments only) the walk enters the next sequence
-            sq.load_of_chunk(p, c);
-            state_fill(tmem + SACC, state_of(p.h0, p, sq.n, h), vfirst, nullptr, tid, e, half);
-        }
-        ok = mbar_wait(&full[stage], ((c - cb) >> 1) & 1, p, 2);
-        if (!__syncthreads_and(ok)) { ok = false; break; }
-        KDA_PHASE(0);
-
-        // ---- A: BF16 copy of the entering state, checkpoint, decay
-        {
-            const float* gam = reinterpret_cast<const float*>(b + GAM);
-            __nv_bfloat16* gS0 = (__nv_bfloat16*)(ws + L.S0) + rec * D * D;
-            for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
-                uint32_t r[16], pk[8];
-                tmem_ld16(tmem + SACC + d0, r);
-                tmem_wait_ld();
-#pragma unroll
-                for (int j = 0; j < 8; ++j) pk[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-                tmem_st8(tmem + SBF + d0 / 2, pk);
-                if (save) {
-                    *reinterpret_cast<uint4*>(gS0 + cm_idx(e, d0, D)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                    *reinterpret_cast<uint4*>(gS0 + cm_idx(e, d0 + 8, D)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-                }
-#pragma unroll
-                for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * gam[d0 + j]);
-                tmem_st16(tmem + SACC + d0, r);
-            }
-            tmem_wait_st();
-        }
-        KDA_PHASE(1);
-        tc_fence_before();
-        __syncthreads();
-        if ((tid & 31) == 0 && warp < 2) {
-            tc_fence_after();
+    if (tid < MAIN) {
+        KDA_PHASE_BEGIN();
+        const bool issuer = (tid & 31) == 0 && warp < 2;  // warp 0: WSacc and Sacc, warp 1: Oacc
+        for (int c = cb; c < ce; ++c) {
+            const int i = c - cb, stage = i & 1;
+            unsigned char* b = dyn + stage * STAGE;
             const uint32_t sb = smem_u32(b);
-            constexpr uint32_t id_mn = make_idesc(128, 64, false, true);
-            constexpr uint32_t id_k = make_idesc(128, 64, false, false);
-            if (warp == 0) {
-#pragma unroll
-                for (int s = 0; s < 8; ++s)  // WSacc = Sbf (K = d) * W^T record, MN-major B
-                    mma_ts(tmem0 + WSACC, tmem0 + SBF + s * 8, make_desc(sb + WT + s * 2048, 1024, 128), id_mn, s > 0);
-            } else {
-#pragma unroll
-                for (int s = 0; s < 8; ++s)  // Oacc = Sbf * Qt^T, K-major B (rows = i)
-                    mma_ts(tmem0 + OACC, tmem0 + SBF + s * 8, make_desc(sb + QT + s * 256, 128, 2048), id_k, s > 0);
+            const size_t rec = (size_t)c * p.H + h;
+            if (c == sq.c_end) {  // (segments only) the walk enters the next sequence
+                sq.load_of_chunk(p, c);
+                state_fill(tmem + SACC, state_of(p.h0, p, sq.n, h), vfirst, nullptr, tid, e, half);
             }
-            mma_commit(&mmabar);
-        }
-        ok = mbar_wait(&mmabar, mma_phase, p, 4);
-        mma_phase ^= 1;
-        tc_fence_after();
-        if (!__syncthreads_and(ok)) { ok = false; break; }
-        KDA_PHASE(2);
-
-        // ---- B: V'^T = U^T - (W S)^T
-        {
+            ok = mbar_wait(&full[stage], (i >> 1) & 1, p, 2) && ok;
+            KDA_PHASE(0);
+            // ---- A: BF16 copy of the entering state, decay
+            uint32_t pk[4][8];
+            state_convert(tmem + SACC, tmem + SBF, 64 * half, reinterpret_cast<const float*>(b + GAM), pk);
+            KDA_PHASE(1);
+            tc_fence_before();
+            ok = bar_and(1, MAIN, ok);
+            if (!ok) break;
+            if (issuer) {
+                tc_fence_after();
+                constexpr uint32_t id_mn = make_idesc(128, 64, false, true);
+                constexpr uint32_t id_k = make_idesc(128, 64, false, false);
+                if (warp == 0) {
+#pragma unroll
+                    for (int s = 0; s < 8; ++s)  // WSacc = Sbf (K = d) * W^T record, MN-major B
+                        mma_ts(tmem0 + WSACC, tmem0 + SBF + s * 8, make_desc(sb + WT + s * 2048, 1024, 128), id_mn, s > 0);
+                    mma_commit(&wsbar);
+                } else {
+                    if (i > 0) ok = mbar_wait(&ofree, (i - 1) & 1, p, 4);  // the previous chunk's output has left Oacc
+                    tc_fence_after();
+                    if (ok) {
+#pragma unroll
+                        for (int s = 0; s < 8; ++s)  // Oacc = Sbf * Qt^T, K-major B (rows = i)
+                            mma_ts(tmem0 + OACC, tmem0 + SBF + s * 8, make_desc(sb + QT + s * 256, 128, 2048), id_k, s > 0);
+                    }
+                }
+            }
+            __syncwarp();
+            if (save) {
+                __nv_bfloat16* gS0 = (__nv_bfloat16*)(ws + L.S0) + rec * D * D;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) store_record16(gS0, e, 64 * half + 16 * g, D, pk[g]);
+            }
+            // ---- B: V'^T = U^T - (W S)^T
             const __nv_bfloat16* sU = reinterpret_cast<const __nv_bfloat16*>(b + UT);
-            __nv_bfloat16* gV = (__nv_bfloat16*)(ws + L.U) + rec * C * D;
-            for (int i0 = 32 * half; i0 < 32 * half + 32; i0 += 16) {
-                uint32_t r[16], pk[8];
-                float u[16];
-                tmem_ld16(tmem + WSACC + i0, r);
-                tmem_wait_ld();
-                {
-                    float t8[8];
-                    unpack8(*reinterpret_cast<const uint4*>(sU + cm_idx(e, i0, C)), t8);
+            float u[2][16];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) u[j] = t8[j];
-                    unpack8(*reinterpret_cast<const uint4*>(sU + cm_idx(e, i0 + 8, C)), t8);
+            for (int g = 0; g < 4; ++g) {
+                float t8[8];
+                unpack8(*reinterpret_cast<const uint4*>(sU + cm_idx(e, 32 * half + 8 * g, C)), t8);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) u[8 + j] = t8[j];
-                }
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    pk[j] = pack_bf16(u[2 * j] - __uint_as_float(r[2 * j]), u[2 * j + 1] - __uint_as_float(r[2 * j + 1]));
-                tmem_st8(tmem + VBF + i0 / 2, pk);
-                if (save) {
-                    *reinterpret_cast<uint4*>(gV + cm_idx(e, i0, C)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                    *reinterpret_cast<uint4*>(gV + cm_idx(e, i0 + 8, C)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-                }
+                for (int j = 0; j < 8; ++j) u[g >> 1][8 * (g & 1) + j] = t8[j];
             }
-            tmem_wait_st();
-        }
-        KDA_PHASE(3);
-        tc_fence_before();
-        __syncthreads();
-        if ((tid & 31) == 0 && warp < 2) {
+            ok = mbar_wait(&wsbar, i & 1, p, 4) && ok;
             tc_fence_after();
-            const uint32_t sb = smem_u32(b);
-            constexpr uint32_t id_k = make_idesc(128, 64, false, false);
-            constexpr uint32_t id_s = make_idesc(128, 128, false, true);
-            if (warp == 0) {
-#pragma unroll
-                for (int s = 0; s < 4; ++s)  // Oacc += Vbf (K = j) * Aqk^T, K-major B (rows = i)
-                    mma_ts(tmem0 + OACC, tmem0 + VBF + s * 8, make_desc(sb + AQ + s * 256, 128, 1024), id_k, true);
-            } else {
-#pragma unroll
-                for (int s = 0; s < 4; ++s)  // Sacc += Vbf (K = i) * Kh, MN-major B
-                    mma_ts(tmem0 + SACC, tmem0 + VBF + s * 8, make_desc(sb + KH + s * 4096, 2048, 128), id_s, true);
-            }
-            mma_commit(&mmabar);
-        }
-        ok = mbar_wait(&mmabar, mma_phase, p, 4);
-        mma_phase ^= 1;
-        tc_fence_after();
-        if (!__syncthreads_and(ok)) { ok = false; break; }
-        KDA_PHASE(4);
-
-        // ---- C: output rows.  The accumulator holds O^T (lane = channel), so the tile is transposed through
-        //      shared memory and goes out with one bulk-tensor store (row by row for a partial chunk)
-        {
-            __nv_bfloat16* sO = reinterpret_cast<__nv_bfloat16*>(dyn + OUT);
-#pragma unroll
-            for (int i0 = 32 * half; i0 < 32 * half + 32; i0 += 16) {
-                uint32_t r[16];
-                tmem_ld16(tmem + OACC + i0, r);
+            KDA_PHASE(2);
+            uint32_t vk[2][8];
+            {
+                uint32_t r[2][16];
+                tmem_ld16(tmem + WSACC + 32 * half, r[0]);
+                tmem_ld16(tmem + WSACC + 32 * half + 16, r[1]);
                 tmem_wait_ld();
 #pragma unroll
-                for (int j = 0; j < 16; ++j) sO[(i0 + j) * D + e] = __float2bfloat16_rn(__uint_as_float(r[j]));
+                for (int g = 0; g < 2; ++g) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        vk[g][j] = pack_bf16(u[g][2 * j] - __uint_as_float(r[g][2 * j]), u[g][2 * j + 1] - __uint_as_float(r[g][2 * j + 1]));
+                    tmem_st8(tmem + VBF + (32 * half + 16 * g) / 2, vk[g]);
+                }
+                tmem_wait_st();
             }
+            KDA_PHASE(3);
+            tc_fence_before();
+            ok = bar_and(1, MAIN, ok);
+            if (!ok) break;
+            if (issuer) {
+                tc_fence_after();
+                constexpr uint32_t id_k = make_idesc(128, 64, false, false);
+                constexpr uint32_t id_s = make_idesc(128, 128, false, true);
+                if (warp == 0) {
+#pragma unroll
+                    for (int s = 0; s < 4; ++s)  // Sacc += Vbf (K = i) * Kh, MN-major B
+                        mma_ts(tmem0 + SACC, tmem0 + VBF + s * 8, make_desc(sb + KH + s * 4096, 2048, 128), id_s, true);
+                    mma_commit(&sbar);
+                } else {
+#pragma unroll
+                    for (int s = 0; s < 4; ++s)  // Oacc += Vbf (K = j) * Aqk^T, K-major B (rows = i)
+                        mma_ts(tmem0 + OACC, tmem0 + VBF + s * 8, make_desc(sb + AQ + s * 256, 128, 1024), id_k, true);
+                    mma_commit(&obar);
+                }
+            }
+            __syncwarp();
+            if (save) {
+                __nv_bfloat16* gV = (__nv_bfloat16*)(ws + L.U) + rec * C * D;
+#pragma unroll
+                for (int g = 0; g < 2; ++g) store_record16(gV, e, 32 * half + 16 * g, C, vk[g]);
+            }
+            // (both: the next chunk overwrites the operands of the output products too)
+            ok = mbar_wait(&sbar, i & 1, p, 4) && mbar_wait(&obar, i & 1, p, 4) && ok;
+            tc_fence_after();
+            if (tid == 0) mbar_arrive(&empty[stage]);
+            KDA_PHASE(4);
+            if (c + 1 == sq.c_end && c + 1 < ce && p.ht && ok)
+                state_drain(tmem + SACC, const_cast<float*>(state_of(p.ht, p, sq.n, h)), vfirst, nullptr, tid, e, half);
+        }
+        ok = bar_and(1, MAIN, ok);
+        // the sequence that ends with the last chunk (one without tokens hands its initial state on)
+        if (ok && ce == sq.c_end && p.ht)
+            state_drain(tmem + SACC, const_cast<float*>(state_of(p.ht, p, sq.n, h)), vfirst, stage_space, tid, e, half);
+    } else if (tid < MAIN + OUTT) {
+        // ---- output rows.  The accumulator holds O^T (lane = channel): the tile is transposed through shared memory and
+        //      goes out with one bulk-tensor store (row by row for a partial chunk)
+        const int ot = tid - MAIN;
+        __nv_bfloat16* o = (__nv_bfloat16*)p.o;
+        __nv_bfloat16* sO = reinterpret_cast<__nv_bfloat16*>(dyn + OUT);
+        for (int c = cb; c < ce; ++c) {
+            sq.move_to(p, c);
+            ok = mbar_wait(&obar, (c - cb) & 1, p, 4);
+            ok = bar_and(2, OUTT, ok);
+            if (!ok) break;
+            tc_fence_after();
+            uint32_t r[4][16];
+#pragma unroll
+            for (int g = 0; g < 4; ++g) tmem_ld16(tmem + OACC + 16 * g, r[g]);
+            tmem_wait_ld();
+            tc_fence_before();
+            __syncwarp();
+            if ((tid & 31) == 0) mbar_arrive(&ofree);
+            tma_store_wait_read();  // the previous chunk's rows have left the staging tile
+            bar_sync(2, OUTT);
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) sO[(16 * g + j) * D + e] = __float2bfloat16_rn(__uint_as_float(r[g][j]));
             fence_async_smem();
-            __syncthreads();
+            bar_sync(2, OUTT);
             const long long tok0 = sq.tok(c);
             const int len = sq.rows(c);
             if (maps.ok && len == C) {  // the whole tile with one bulk-tensor store
-                if (tid == 0) {
+                if (ot == 0) {
                     tma_store_tile(&maps.m[0], h * D, (int)tok0, sO);
                     tma_store_commit();
                 }
-            } else if (tid < len) {
-                tma_store_1d(o + ((size_t)(tok0 + tid) * p.H + h) * D, sO + tid * D, D * 2);
+            } else if (ot < len) {
+                tma_store_1d(o + ((size_t)(tok0 + ot) * p.H + h) * D, sO + ot * D, D * 2);
                 tma_store_commit();
             }
         }
-        if (c + 1 == sq.c_end && c + 1 < ce && p.ht)
-            state_drain(tmem + SACC, const_cast<float*>(state_of(p.ht, p, sq.n, h)), vfirst, nullptr, tid, e, half);
-        KDA_PHASE(5);
+        tma_store_wait_all();
+    } else if ((tid & 31) == 0) {
+        // ---- the six records of every chunk, one chunk ahead of their use
+        int i = 0;
+        for (; i < ce - cb; ++i) {
+            const int stage = i & 1;
+            if (i >= 2 && !mbar_wait(&empty[stage], ((i >> 1) - 1) & 1, p, 2)) break;
+            const size_t rec = (size_t)(cb + i) * p.H + h;
+            unsigned char* b = dyn + stage * STAGE;
+            mbar_expect_tx(&full[stage], STAGE);
+            tma_load_1d(b + GAM, (const float*)(ws + L.gamC) + rec * D, 512, &full[stage]);
+            tma_load_1d(b + WT, (const __nv_bfloat16*)(ws + L.W) + rec * C * D, 16384, &full[stage]);
+            tma_load_1d(b + UT, (const __nv_bfloat16*)(ws + L.U) + rec * C * D, 16384, &full[stage]);
+            tma_load_1d(b + KH, (const __nv_bfloat16*)(ws + L.Kh) + rec * C * D, 16384, &full[stage]);
+            tma_load_1d(b + QT, (const __nv_bfloat16*)(ws + L.Qt) + rec * C * D, 16384, &full[stage]);
+            tma_load_1d(b + AQ, (const __nv_bfloat16*)(ws + L.Aqk) + rec * C * C, 8192, &full[stage]);
+        }
+        // (whatever became of the walk, no copy is in flight when the CTA leaves)
+        for (int j = i > 2 ? i - 2 : 0; j < i; ++j) mbar_wait(&full[j & 1], (j >> 1) & 1, p, 2);
     }
-    // the sequence that ends with the last chunk (one without tokens hands its initial state on)
-    if (ok && ce == sq.c_end && p.ht)
-        state_drain(tmem + SACC, const_cast<float*>(state_of(p.ht, p, sq.n, h)), vfirst, stage_space, tid, e, half);
-    tma_store_wait_all();
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem0, TMEM_COLS);
@@ -401,13 +436,16 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
 
 // ---------------------------------------------------------------------------------------
 // bwd_state on tensor cores: same organisation, reverse chunk order, dS^T resident in TMEM.
+//   0  dVacc = dO^T * Aqk (before the conversion: it needs the chunk's records only)
 //   A  dSacc -> BF16 dSbf (operand + checkpoint of the dS entering the chunk), decay dSacc
-//   1  dVacc = dO^T * Aqk + dSbf * Kh^T          dSacc += dO^T * Qt
+//   1  dVacc += dSbf * Kh^T         dSacc += dO^T * Qt
 //   B  dV'^T -> BF16 dVbf and the dV' record
 //   2  dSacc -= dVbf * W
+// Four producer warps fetch the records (bulk copies) and the dO tile (16-byte asynchronous copies into the core-matrix
+// layout) into a three-stage ring.
 // ---------------------------------------------------------------------------------------
 namespace bs {
-constexpr int D = 128, NTHR = 256;
+constexpr int D = 128, MAIN = 256, PROD = 128, NTHR = MAIN + PROD;
 constexpr uint32_t WT = 0, QT = 16384, KH = 32768, DO = 49152, AQ = 65536, GAM = 73728, STAGE = 74240;
 constexpr uint32_t TMA_BYTES = 16384 * 3 + 8192 + 512;
 constexpr uint32_t SACC = 0, SBF = 128, VACC = 192, VBF = 256, TMEM_COLS = 512;
@@ -419,10 +457,9 @@ template <bool PARTIAL>
 __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams p, const StateSegs segs) {
     using namespace bs;
     extern __shared__ __align__(128) unsigned char dyn[];
-    __shared__ uint64_t full[3];  // three stages: the records of a chunk are requested two chunk steps ahead of their use
-    __shared__ uint64_t mmabar, mmabar2;
+    __shared__ uint64_t full[3], empty[3], vbar, sbar;
     __shared__ uint32_t tmem_s;
-    // thread (half, e) = (tid / 128, tid % 128): TMEM lane e, and half of the columns of every conversion phase
+    // main threads (half, e) = (tid / 128, tid % 128): TMEM lane e, and half of the columns of every conversion phase
     const int tid = threadIdx.x, warp = tid >> 5, e = tid & 127, half = tid >> 7;
     const int h = blockIdx.x;
     // the chunks of this CTA, walked from the last to the first: one sequence, or one segment of the chunk numbering
@@ -453,11 +490,13 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
         tmem_relinquish();
     }
     if (tid == 0) {
-        mbar_init(&full[0], 1);
-        mbar_init(&full[1], 1);
-        mbar_init(&full[2], 1);
-        mbar_init(&mmabar, 2);   // first group: one issuing thread per accumulator
-        mbar_init(&mmabar2, 1);  // second group: a single product
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            mbar_init(&full[i], 1 + PROD / 32);  // the bulk copies, and the dO rows of every producer warp
+            mbar_init(&empty[i], 1);
+        }
+        mbar_init(&vbar, 1);
+        mbar_init(&sbar, 1);
         mbar_fence_init();
     }
     tc_fence_before();
@@ -465,164 +504,170 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
     tc_fence_after();
     const uint32_t tmem = tmem_s + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t tmem0 = tmem_s;
-
     const bool vfirst = p.flags & KDA_FLAG_STATE_V_FIRST;
     float* stage_space = reinterpret_cast<float*>(dyn);  // before the first and after the last chunk's copies
-    // dS at the end of the segment (what the next one found at its start), or of a sequence (grad_ht or zero)
-    if (ce < sq.c_end)
-        state_fill(tmem + SACC, PARTIAL ? nullptr : segs.E + (((size_t)blockIdx.y + 1) * p.H + h) * D * D, false, nullptr, tid, e, half);
-    else
-        state_fill(tmem + SACC, state_of(p.grad_ht, p, sq.n, h), vfirst, stage_space, tid, e, half);
-
-    // step k = 0..nc-1 processes chunk ce-1-k
-    SeqCursor sl = sq;  // sequence of the chunk whose loads are issued
-    auto issue_loads = [&](int k, int stage) {
-        const int c = ce - 1 - k;
-        const size_t rec = (size_t)c * p.H + h;
-        sl.move_to(p, c);
-        unsigned char* b = dyn + stage * STAGE;
-        if ((tid & 31) == 0) {  // one bulk copy each from lane 0 of five warps
-            if (warp == 0) {
-                mbar_expect_tx(&full[stage], TMA_BYTES);
-                tma_load_1d(b + WT, (const __nv_bfloat16*)(ws + L.W) + rec * C * D, 16384, &full[stage]);
-            } else if (warp == 1) {
-                tma_load_1d(b + QT, (const __nv_bfloat16*)(ws + L.Qt) + rec * C * D, 16384, &full[stage]);
-            } else if (warp == 2) {
-                tma_load_1d(b + KH, (const __nv_bfloat16*)(ws + L.Kh) + rec * C * D, 16384, &full[stage]);
-            } else if (warp == 3) {
-                tma_load_1d(b + AQ, (const __nv_bfloat16*)(ws + L.Aqk) + rec * C * C, 8192, &full[stage]);
-            } else if (warp == 4) {
-                tma_load_1d(b + GAM, (const float*)(ws + L.gamC) + rec * D, 512, &full[stage]);
-            }
-        }
-        // dO tile -> core-matrix layout cm(i, e; 128), 16-byte chunks, zero rows past the end
-        const long long tok0 = sl.tok(c);
-        const int len = sl.rows(c);
-        __nv_bfloat16* sdo = reinterpret_cast<__nv_bfloat16*>(b + DO);
-        for (int q = tid; q < C * (D / 8); q += NTHR) {
-            const int i = q >> 4, e8 = (q & 15) * 8;
-            const bool valid = i < len;
-            const size_t row = (size_t)(tok0 + (valid ? i : 0)) * p.H + h;
-            cp_async16_z(sdo + cm_idx(i, e8, D), dO + row * D + e8, valid);
-        }
-        cp_async_commit();
-    };
-    if (nc > 0) issue_loads(0, 0);
-    if (nc > 1) issue_loads(1, 1);
+    if (tid < MAIN) {
+        // dS at the end of the segment (what the next one found at its start), or of a sequence (grad_ht or zero)
+        if (ce < sq.c_end)
+            state_fill(tmem + SACC, PARTIAL ? nullptr : segs.E + (((size_t)blockIdx.y + 1) * p.H + h) * D * D, false, nullptr, tid, e, half);
+        else
+            state_fill(tmem + SACC, state_of(p.grad_ht, p, sq.n, h), vfirst, stage_space, tid, e, half);
+    }
+    __syncthreads();
 
     bool ok = true;
-    int stage = 0;
-    uint32_t ring_phase = 0;  // parity of full[stage]: flips every time the ring wraps
-    for (int k = 0; k < nc; ++k) {
-        const int c = ce - 1 - k;
-        unsigned char* b = dyn + stage * STAGE;
-        const size_t rec = (size_t)c * p.H + h;
-        if (c < sq.c_begin) {  // (segments only) the walk enters the previous sequence
-            sq.load_of_chunk(p, c);
-            state_fill(tmem + SACC, state_of(p.grad_ht, p, sq.n, h), vfirst, nullptr, tid, e, half);
-        }
-        if (k + 2 < nc) {  // (the stage behind this one was last read by the previous step's MMAs, which have completed)
-            issue_loads(k + 2, stage == 0 ? 2 : stage - 1);
-            cp_async_wait<2>();
-        } else if (k + 1 < nc) {
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        fence_async_smem();
-        ok = mbar_wait(&full[stage], ring_phase, p, 2);
-        if (!__syncthreads_and(ok)) { ok = false; break; }
-
-        {
-            const float* gam = reinterpret_cast<const float*>(b + GAM);
-            __nv_bfloat16* gdS = (__nv_bfloat16*)(sc + L.dS) + rec * D * D;
-            for (int d0 = 64 * half; d0 < 64 * half + 64; d0 += 16) {
-                uint32_t r[16], pk[8];
-                tmem_ld16(tmem + SACC + d0, r);
-                tmem_wait_ld();
-#pragma unroll
-                for (int j = 0; j < 8; ++j) pk[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-                tmem_st8(tmem + SBF + d0 / 2, pk);
-                if (!PARTIAL) {
-                    *reinterpret_cast<uint4*>(gdS + cm_idx(e, d0, D)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                    *reinterpret_cast<uint4*>(gdS + cm_idx(e, d0 + 8, D)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-                }
-#pragma unroll
-                for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * gam[d0 + j]);
-                tmem_st16(tmem + SACC + d0, r);
-            }
-            tmem_wait_st();
-        }
-        tc_fence_before();
-        __syncthreads();
-        if ((tid & 31) == 0 && warp < 2) {
-            tc_fence_after();
+    // step k = 0..nc-1 processes chunk ce-1-k
+    if (tid < MAIN) {
+        const bool issuer = (tid & 31) == 0 && warp < 2;  // warp 0: dVacc, warp 1: dSacc
+        int stage = 0;
+        uint32_t ring_phase = 0;  // parity of full[stage]: flips every time the ring wraps
+        for (int k = 0; k < nc; ++k) {
+            const int c = ce - 1 - k;
+            unsigned char* b = dyn + stage * STAGE;
             const uint32_t sb = smem_u32(b);
-            constexpr uint32_t id_v1 = make_idesc(128, 64, true, true);    // dO^T (MN-major A) * Aqk (MN-major B)
-            constexpr uint32_t id_v2 = make_idesc(128, 64, false, false);  // dSbf (TMEM) * Kh^T (K-major B)
-            constexpr uint32_t id_s1 = make_idesc(128, 128, true, true);   // dO^T * Qt (MN-major B)
-            if (warp == 0) {
+            const size_t rec = (size_t)c * p.H + h;
+            if (c < sq.c_begin) {  // (segments only) the walk enters the previous sequence
+                sq.load_of_chunk(p, c);
+                state_fill(tmem + SACC, state_of(p.grad_ht, p, sq.n, h), vfirst, nullptr, tid, e, half);
+            }
+            ok = mbar_wait(&full[stage], ring_phase, p, 2) && ok;
+            if (issuer && warp == 0 && ok) {
+                constexpr uint32_t id_v1 = make_idesc(128, 64, true, true);  // dO^T (MN-major A) * Aqk (MN-major B)
+                tc_fence_after();
 #pragma unroll
                 for (int s = 0; s < 4; ++s)
                     mma_ss(tmem0 + VACC, make_desc(sb + DO + s * 4096, 2048, 128), make_desc(sb + AQ + s * 2048, 1024, 128), id_v1,
                            s > 0);
-#pragma unroll
-                for (int s = 0; s < 8; ++s)
-                    mma_ts(tmem0 + VACC, tmem0 + SBF + s * 8, make_desc(sb + KH + s * 256, 128, 2048), id_v2, true);
-            } else {
-#pragma unroll
-                for (int s = 0; s < 4; ++s)
-                    mma_ss(tmem0 + SACC, make_desc(sb + DO + s * 4096, 2048, 128), make_desc(sb + QT + s * 4096, 2048, 128), id_s1,
-                           true);
             }
-            mma_commit(&mmabar);
-        }
-        ok = mbar_wait(&mmabar, k & 1, p, 4);
-        tc_fence_after();
-        if (!__syncthreads_and(ok)) { ok = false; break; }
-
-        {
-            __nv_bfloat16* gdV = (__nv_bfloat16*)(sc + L.dVn) + rec * C * D;
-            for (int i0 = 32 * half; i0 < 32 * half + 32; i0 += 16) {
-                uint32_t r[16], pk[8];
-                tmem_ld16(tmem + VACC + i0, r);
-                tmem_wait_ld();
+            __syncwarp();
+            uint32_t pk[4][8];
+            state_convert(tmem + SACC, tmem + SBF, 64 * half, reinterpret_cast<const float*>(b + GAM), pk);
+            tc_fence_before();
+            ok = bar_and(1, MAIN, ok);
+            if (!ok) break;
+            if (issuer) {
+                tc_fence_after();
+                constexpr uint32_t id_v2 = make_idesc(128, 64, false, false);  // dSbf (TMEM) * Kh^T (K-major B)
+                constexpr uint32_t id_s1 = make_idesc(128, 128, true, true);   // dO^T * Qt (MN-major B)
+                if (warp == 0) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) pk[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-                tmem_st8(tmem + VBF + i0 / 2, pk);
-                if (!PARTIAL) {
-                    *reinterpret_cast<uint4*>(gdV + cm_idx(e, i0, C)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                    *reinterpret_cast<uint4*>(gdV + cm_idx(e, i0 + 8, C)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                    for (int s = 0; s < 8; ++s)
+                        mma_ts(tmem0 + VACC, tmem0 + SBF + s * 8, make_desc(sb + KH + s * 256, 128, 2048), id_v2, true);
+                    mma_commit(&vbar);
+                } else {
+#pragma unroll
+                    for (int s = 0; s < 4; ++s)
+                        mma_ss(tmem0 + SACC, make_desc(sb + DO + s * 4096, 2048, 128), make_desc(sb + QT + s * 4096, 2048, 128), id_s1,
+                               true);
                 }
             }
-            tmem_wait_st();
-        }
-        tc_fence_before();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            const uint32_t sb = smem_u32(b);
-            constexpr uint32_t id_w = make_idesc(128, 128, false, false, true);  // -dVbf (TMEM) * W (K-major B, rows = d)
+            __syncwarp();
+            if (!PARTIAL) {
+                __nv_bfloat16* gdS = (__nv_bfloat16*)(sc + L.dS) + rec * D * D;
 #pragma unroll
-            for (int s = 0; s < 4; ++s)
-                mma_ts(tmem0 + SACC, tmem0 + VBF + s * 8, make_desc(sb + WT + s * 256, 128, 1024), id_w, true);
-            mma_commit(&mmabar2);
+                for (int g = 0; g < 4; ++g) store_record16(gdS, e, 64 * half + 16 * g, D, pk[g]);
+            }
+            ok = mbar_wait(&vbar, k & 1, p, 4) && ok;
+            tc_fence_after();
+            uint32_t vk[2][8];
+            {
+                uint32_t r[2][16];
+                tmem_ld16(tmem + VACC + 32 * half, r[0]);
+                tmem_ld16(tmem + VACC + 32 * half + 16, r[1]);
+                tmem_wait_ld();
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) vk[g][j] = pack_bf16(__uint_as_float(r[g][2 * j]), __uint_as_float(r[g][2 * j + 1]));
+                    tmem_st8(tmem + VBF + (32 * half + 16 * g) / 2, vk[g]);
+                }
+                tmem_wait_st();
+            }
+            tc_fence_before();
+            ok = bar_and(1, MAIN, ok);
+            if (!ok) break;
+            if (issuer && warp == 1) {
+                tc_fence_after();
+                constexpr uint32_t id_w = make_idesc(128, 128, false, false, true);  // -dVbf (TMEM) * W (K-major B, rows = d)
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                    mma_ts(tmem0 + SACC, tmem0 + VBF + s * 8, make_desc(sb + WT + s * 256, 128, 1024), id_w, true);
+                mma_commit(&sbar);
+            }
+            __syncwarp();
+            if (!PARTIAL) {
+                __nv_bfloat16* gdV = (__nv_bfloat16*)(sc + L.dVn) + rec * C * D;
+#pragma unroll
+                for (int g = 0; g < 2; ++g) store_record16(gdV, e, 32 * half + 16 * g, C, vk[g]);
+            }
+            ok = mbar_wait(&sbar, k & 1, p, 4) && ok;
+            tc_fence_after();
+            if (tid == 0) mbar_arrive(&empty[stage]);
+            if (!PARTIAL && c == sq.c_begin && c > cb && p.grad_h0 && ok)
+                state_drain(tmem + SACC, const_cast<float*>(state_of(p.grad_h0, p, sq.n, h)), vfirst, nullptr, tid, e, half);
+            if (++stage == 3) {
+                stage = 0;
+                ring_phase ^= 1;
+            }
         }
-        ok = mbar_wait(&mmabar2, k & 1, p, 4);
-        tc_fence_after();
-        if (!__syncthreads_and(ok)) { ok = false; break; }
-        if (!PARTIAL && c == sq.c_begin && c > cb && p.grad_h0)
-            state_drain(tmem + SACC, const_cast<float*>(state_of(p.grad_h0, p, sq.n, h)), vfirst, nullptr, tid, e, half);
-        if (++stage == 3) {
-            stage = 0;
-            ring_phase ^= 1;
+        ok = bar_and(1, MAIN, ok);
+        if (PARTIAL) {
+            if (ok) state_drain(tmem + SACC, segs.E + ((size_t)blockIdx.y * p.H + h) * D * D, false, nullptr, tid, e, half);
+        } else if (ok && cb == sq.c_begin && p.grad_h0) {  // (a sequence without tokens hands grad_ht on)
+            state_drain(tmem + SACC, const_cast<float*>(state_of(p.grad_h0, p, sq.n, h)), vfirst, stage_space, tid, e, half);
         }
-    }
-    cp_async_wait<0>();
-    if (PARTIAL) {
-        if (ok) state_drain(tmem + SACC, segs.E + ((size_t)blockIdx.y * p.H + h) * D * D, false, nullptr, tid, e, half);
-    } else if (ok && cb == sq.c_begin && p.grad_h0) {  // (a sequence without tokens hands grad_ht on)
-        state_drain(tmem + SACC, const_cast<float*>(state_of(p.grad_h0, p, sq.n, h)), vfirst, stage_space, tid, e, half);
+    } else {
+        const int pt = tid - MAIN, pw = pt >> 5;
+        auto landed = [&](int k) {  // the dO rows of step k are in place: hand them to the tensor cores' proxy
+            fence_async_smem();
+            __syncwarp();
+            if ((pt & 31) == 0) mbar_arrive(&full[k % 3]);
+        };
+        int k = 0;
+        for (; k < nc; ++k) {
+            const int stage = k % 3, c = ce - 1 - k;
+            if (k >= 3 && !bar_and(2, PROD, mbar_wait(&empty[stage], (k / 3 - 1) & 1, p, 2))) break;
+            const size_t rec = (size_t)c * p.H + h;
+            unsigned char* b = dyn + stage * STAGE;
+            if ((pt & 31) == 0) {
+                if (pw == 0) {
+                    mbar_expect_tx(&full[stage], TMA_BYTES);
+                    tma_load_1d(b + AQ, (const __nv_bfloat16*)(ws + L.Aqk) + rec * C * C, 8192, &full[stage]);
+                    tma_load_1d(b + GAM, (const float*)(ws + L.gamC) + rec * D, 512, &full[stage]);
+                } else if (pw == 1) {
+                    tma_load_1d(b + KH, (const __nv_bfloat16*)(ws + L.Kh) + rec * C * D, 16384, &full[stage]);
+                } else if (pw == 2) {
+                    tma_load_1d(b + QT, (const __nv_bfloat16*)(ws + L.Qt) + rec * C * D, 16384, &full[stage]);
+                } else {
+                    tma_load_1d(b + WT, (const __nv_bfloat16*)(ws + L.W) + rec * C * D, 16384, &full[stage]);
+                }
+            }
+            __syncwarp();
+            // dO tile -> core-matrix layout cm(i, e; 128), 16-byte chunks, zero rows past the end
+            sq.move_to(p, c);
+            const long long tok0 = sq.tok(c);
+            const int len = sq.rows(c);
+            __nv_bfloat16* sdo = reinterpret_cast<__nv_bfloat16*>(b + DO);
+#pragma unroll
+            for (int u = 0; u < C * (D / 8) / PROD; ++u) {
+                const int q = pt + PROD * u, i = q >> 4, e8 = (q & 15) * 8;
+                const bool valid = i < len;
+                const size_t row = (size_t)(tok0 + (valid ? i : 0)) * p.H + h;
+                cp_async16_z(sdo + cm_idx(i, e8, D), dO + row * D + e8, valid);
+            }
+            cp_async_commit();
+            if (k >= 1) {
+                cp_async_wait<1>();
+                landed(k - 1);
+            }
+        }
+        cp_async_wait<0>();
+        if (k == nc && nc > 0) landed(nc - 1);
+        // (whatever became of the walk, no copy is in flight when the CTA leaves)
+        if (k < nc) {
+            if (k > 0) landed(k - 1);
+            for (int j = k > 3 ? k - 3 : 0; j < k; ++j) mbar_wait(&full[j % 3], (j / 3) & 1, p, 2);
+        }
     }
     tc_fence_before();
     __syncthreads();
