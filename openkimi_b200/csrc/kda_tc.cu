@@ -260,7 +260,7 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
     bool ok = true;
     if (tid < MAIN) {
         KDA_PHASE_BEGIN();
-        const bool issuer = (tid & 31) == 0 && warp < 2;  // warp 0: WSacc and Sacc, warp 1: Oacc
+        const int wu = __shfl_sync(0xffffffffu, warp, 0);  // warp 0: WSacc and Sacc, warp 1: Oacc
         for (int c = cb; c < ce; ++c) {
             const int i = c - cb, stage = i & 1;
             unsigned char* b = dyn + stage * STAGE;
@@ -279,11 +279,11 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
             tc_fence_before();
             ok = bar_and(1, MAIN, ok);
             if (!ok) break;
-            if (issuer) {
+            if (wu < 2 && elect_one()) {
                 tc_fence_after();
                 constexpr uint32_t id_mn = make_idesc(128, 64, false, true);
                 constexpr uint32_t id_k = make_idesc(128, 64, false, false);
-                if (warp == 0) {
+                if (wu == 0) {
 #pragma unroll
                     for (int s = 0; s < 8; ++s)  // WSacc = Sbf (K = d) * W^T record, MN-major B
                         mma_ts(tmem0 + WSACC, tmem0 + SBF + s * 8, make_desc(sb + WT + s * 2048, 1024, 128), id_mn, s > 0);
@@ -336,11 +336,11 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
             tc_fence_before();
             ok = bar_and(1, MAIN, ok);
             if (!ok) break;
-            if (issuer) {
+            if (wu < 2 && elect_one()) {
                 tc_fence_after();
                 constexpr uint32_t id_k = make_idesc(128, 64, false, false);
                 constexpr uint32_t id_s = make_idesc(128, 128, false, true);
-                if (warp == 0) {
+                if (wu == 0) {
 #pragma unroll
                     for (int s = 0; s < 4; ++s)  // Sacc += Vbf (K = i) * Kh, MN-major B
                         mma_ts(tmem0 + SACC, tmem0 + VBF + s * 8, make_desc(sb + KH + s * 4096, 2048, 128), id_s, true);
@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
     bool ok = true;
     // step k = 0..nc-1 processes chunk ce-1-k
     if (tid < MAIN) {
-        const bool issuer = (tid & 31) == 0 && warp < 2;  // warp 0: dVacc, warp 1: dSacc
+        const int wu = __shfl_sync(0xffffffffu, warp, 0);  // warp 0: dVacc, warp 1: dSacc
         int stage = 0;
         uint32_t ring_phase = 0;  // parity of full[stage]: flips every time the ring wraps
         for (int k = 0; k < nc; ++k) {
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
                 state_fill(tmem + SACC, state_of(p.grad_ht, p, sq.n, h), vfirst, nullptr, tid, e, half);
             }
             ok = mbar_wait(&full[stage], ring_phase, p, 2) && ok;
-            if (issuer && warp == 0 && ok) {
+            if (wu == 0 && elect_one() && ok) {
                 constexpr uint32_t id_v1 = make_idesc(128, 64, true, true);  // dO^T (MN-major A) * Aqk (MN-major B)
                 tc_fence_after();
 #pragma unroll
@@ -545,11 +545,11 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
             tc_fence_before();
             ok = bar_and(1, MAIN, ok);
             if (!ok) break;
-            if (issuer) {
+            if (wu < 2 && elect_one()) {
                 tc_fence_after();
                 constexpr uint32_t id_v2 = make_idesc(128, 64, false, false);  // dSbf (TMEM) * Kh^T (K-major B)
                 constexpr uint32_t id_s1 = make_idesc(128, 128, true, true);   // dO^T * Qt (MN-major B)
-                if (warp == 0) {
+                if (wu == 0) {
 #pragma unroll
                     for (int s = 0; s < 8; ++s)
                         mma_ts(tmem0 + VACC, tmem0 + SBF + s * 8, make_desc(sb + KH + s * 256, 128, 2048), id_v2, true);
@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
             tc_fence_before();
             ok = bar_and(1, MAIN, ok);
             if (!ok) break;
-            if (issuer && warp == 1) {
+            if (wu == 1 && elect_one()) {
                 tc_fence_after();
                 constexpr uint32_t id_w = make_idesc(128, 128, false, false, true);  // -dVbf (TMEM) * W (K-major B, rows = d)
 #pragma unroll
