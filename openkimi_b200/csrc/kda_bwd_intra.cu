@@ -120,6 +120,7 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     float* fD = reinterpret_cast<float*>(dyn + FD);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, d = tid & 127, blk = tid >> 7, cg = warp & 3;
+    const int wu = __shfl_sync(0xffffffffu, warp, 0);  // the warp index as a warp-uniform value (MMA issue)
     const int b0 = B * blk;
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     char* sc = (char*)p.bwd_scratch;
@@ -212,14 +213,13 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     // (descriptors: one base per buffer, the tile / part / block offset is added to its 14-bit address field)
     const uint64_t dX = make_desc(sb + XB, 128, 1024), dY = make_desc(sb + YB, 128, 1024);
     const uint64_t dBk = make_desc(sb + SB, 128, 1024), dBm = make_desc(sb + SB, 1024, 128);
-    // Lane 0 of warp J issues the MMAs of accumulator block J: the blocks are independent, and no warp
+    // An elected lane of warp J issues the MMAs of accumulator block J: the blocks are independent, and no warp
     // falls a whole issue sequence behind the others.
-    const bool issuer = lane == 0 && warp < 4;
-    if (issuer && ok) {  // row side: accR_J = KN_J^T dA[i >= 16 J, J]^T (and dM), six passes each
+    if (wu < 4 && elect_one() && ok) {  // row side: accR_J = KN_J^T dA[i >= 16 J, J]^T (and dM), six passes each
         tc_fence_after();
 #pragma unroll
         for (int J = 0; J < 4; ++J)
-            if (J == warp) {
+            if (J == wu) {
                 const int N = 64 - B * J;
                 const uint32_t id = make_idesc(128, N, false, false);
 #pragma unroll
@@ -257,11 +257,11 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     tc_fence_before();
     ok = __syncthreads_and(ok);
     KDA_PHASE(2);
-    if (issuer && ok) {  // column side, first half: accC_I = QP_I^T dA[I, j < 16 (I+1)]
+    if (wu < 4 && elect_one() && ok) {  // column side, first half: accC_I = QP_I^T dA[I, j < 16 (I+1)]
         tc_fence_after();
 #pragma unroll
         for (int I = 0; I < 4; ++I)
-            if (I == warp) {
+            if (I == wu) {
                 const uint32_t id = make_idesc(128, B * (I + 1), false, true);
 #pragma unroll
                 for (int ps = 0; ps < 6; ++ps)
@@ -289,11 +289,11 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     tc_fence_before();
     ok = __syncthreads_and(ok);
     KDA_PHASE(3);
-    if (issuer && ok) {  // column side, second half: accC_I += KP_I^T dM[I, j < 16 (I+1)]
+    if (wu < 4 && elect_one() && ok) {  // column side, second half: accC_I += KP_I^T dM[I, j < 16 (I+1)]
         tc_fence_after();
 #pragma unroll
         for (int I = 0; I < 4; ++I)
-            if (I == warp) {
+            if (I == wu) {
                 const uint32_t id = make_idesc(128, B * (I + 1), false, true);
 #pragma unroll
                 for (int ps = 0; ps < 6; ++ps)

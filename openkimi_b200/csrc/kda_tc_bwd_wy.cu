@@ -108,6 +108,7 @@ __global__ void __launch_bounds__(bp::NTHR, 1) kda_bwd_wy_tc_pf(const KdaParams 
     __shared__ uint64_t fullA[2], fullS, fullD, fullW, mma1, mma2, mma3;
     __shared__ uint32_t tmem_s;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int wu = __shfl_sync(0xffffffffu, warp, 0);  // the warp index as a warp-uniform value (MMA issue)
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     const char* ws = (const char*)p.workspace;
     char* sc = (char*)p.bwd_scratch;
@@ -220,26 +221,26 @@ __global__ void __launch_bounds__(bp::NTHR, 1) kda_bwd_wy_tc_pf(const KdaParams 
     ok = __syncthreads_and(ok);
     KDA_PHASE(0);
 
-    // ---- S1: lane 0 of warps 0..4 issues the product of one accumulator each (dKh waits for dS)
-    if (lane == 0 && warp < 5 && ok) {
+    // ---- S1: an elected lane of warps 0..4 issues the product of one accumulator each (dKh waits for dS)
+    if (wu < 5 && elect_one() && ok) {
         tc_fence_after();
         constexpr uint32_t id_aqk = make_idesc(64, 64, false, true);
         constexpr uint32_t id_mm = make_idesc(128, 64, true, true);
         constexpr uint32_t id_mk = make_idesc(128, 64, true, false);
         constexpr uint32_t id_km = make_idesc(128, 64, false, true);
-        if (warp == 0) {
+        if (wu == 0) {
 #pragma unroll
             for (int s = 0; s < 8; ++s)  // dAqk = dO (K-major) * V' (MN-major view of V'^T)
                 mma_ss(tmem0 + DAQK, make_desc(sb + oDOT + s * 256, 128, 2048), make_desc(sb + oVT + s * 2048, 1024, 128), id_aqk, s > 0);
-        } else if (warp == 1) {
+        } else if (wu == 1) {
 #pragma unroll
             for (int s = 0; s < 8; ++s)  // dWn^T = S0 (MN-major view of S0^T) * dV'^T (MN-major)
                 mma_ss(tmem0 + DWN, make_desc(sb + S0T + s * 4096, 2048, 128), make_desc(sb + oDVT + s * 2048, 1024, 128), id_mm, s > 0);
-        } else if (warp == 2) {
+        } else if (wu == 2) {
 #pragma unroll
             for (int s = 0; s < 8; ++s)  // dQt^T = S0 * dO^T (K-major, rows = i)
                 mma_ss(tmem0 + DQT, make_desc(sb + S0T + s * 4096, 2048, 128), make_desc(sb + oDOT + s * 256, 128, 2048), id_mk, s > 0);
-        } else if (warp == 3) {
+        } else if (wu == 3) {
             if (mbar_wait(&fullD, par, p, 16)) {
 #pragma unroll
                 for (int s = 0; s < 8; ++s)  // dKh^T = dS * V'^T
@@ -397,11 +398,11 @@ __global__ void __launch_bounds__(bp::NTHR, 1) kda_bwd_wy_tc_pf(const KdaParams 
     KDA_PHASE(3);
 
     // ---- S2: two issuing threads (the products into dWn form one chain)
-    if (lane == 0 && warp < 2 && ok) {
+    if (wu < 2 && elect_one() && ok) {
         tc_fence_after();
         constexpr uint32_t id_neg = make_idesc(128, 64, false, true, true);  // -WBF (TMEM) * T (MN-major)
         constexpr uint32_t id_mm = make_idesc(128, 64, true, true);
-        if (warp == 0) {
+        if (wu == 0) {
 #pragma unroll
             for (int s = 0; s < 4; ++s) mma_ts(tmem0 + DKB, tmem0 + WBF + s * 8, make_desc(sb + TT + s * 2048, 1024, 128), id_neg, s > 0);
         } else {
@@ -498,10 +499,10 @@ __global__ void __launch_bounds__(bp::NTHR, 1) kda_bwd_wy_tc_pf(const KdaParams 
     KDA_PHASE(6);
 
     // ---- S3: the two products of dMn go to two accumulators (the second one where dAqk was), one issuing thread each
-    if (lane == 0 && warp < 2 && ok) {
+    if (wu < 2 && elect_one() && ok) {
         tc_fence_after();
         constexpr uint32_t id = make_idesc(64, 64, true, true);
-        if (warp == 0) {
+        if (wu == 0) {
 #pragma unroll
             for (int s = 0; s < 8; ++s)  // Z (MN-major view of Z^T) * W^T (MN-major view of the W^T record)
                 mma_ss(tmem0 + DMN, make_desc(sb + oDVT + s * 2048, 1024, 128), make_desc(sb + WT + s * 2048, 1024, 128), id, s > 0);
