@@ -140,6 +140,7 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
         mbar_init(&mma3, 4);
         mbar_fence_init();
     }
+    pdl_wait();
     tc_fence_before();
     __syncthreads();  // barrier initialisation and the TMEM base address are visible
     tc_fence_after();
@@ -655,6 +656,7 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
 // of the successor's first three, in the FMA order of conv_bwd_block.  Grid (chunk, head, tensor), thread = channel.
 __global__ void __launch_bounds__(128) conv_bwd_fixup_kernel(const KdaParams p) {
     const int c = blockIdx.x, h = blockIdx.y, t = blockIdx.z, ch = threadIdx.x;
+    pdl_wait();
     const ChunkInfo ci = chunk_info(p, c);
     int c0s, ncs;
     seq_chunks(p, ci.seq, c0s, ncs);
@@ -681,10 +683,18 @@ __global__ void __launch_bounds__(1024) conv_bwd_reduce_kernel(const KdaParams p
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     const float4* part = (const float4*)((const char*)p.bwd_scratch + L.cv_part);
     const int h = blockIdx.x, t = blockIdx.y, ch = threadIdx.x & 127, grp = threadIdx.x >> 7;
+    pdl_wait();
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int c = grp; c < p.NT; c += 8) {
-        const float4 u = part[(((size_t)c * p.H + h) * 3 + t) * 128 + ch];
-        s.x += u.x; s.y += u.y; s.z += u.z; s.w += u.w;
+    // (eight loads in flight per thread, added in chunk order: the loop is a chain of round trips otherwise)
+    for (int c0 = grp; c0 < p.NT; c0 += 8 * 8) {
+        float4 u[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int c = c0 + 8 * q;
+            u[q] = c < p.NT ? part[(((size_t)c * p.H + h) * 3 + t) * 128 + ch] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) { s.x += u[q].x; s.y += u[q].y; s.z += u[q].z; s.w += u[q].w; }
     }
     sb[grp][ch] = s;
     __syncthreads();
@@ -709,10 +719,10 @@ cudaError_t launch_bwd_intra(const KdaParams& p, cudaStream_t s) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bi::TOTAL);
     if (e != cudaSuccess) return e;
     const int units = p.NT * p.H, sms = sm_count();
-    kern<<<units < sms ? units : sms, bi::NTHR, bi::TOTAL, s>>>(p);
+    if ((e = launch_dependent(kern, units < sms ? units : sms, bi::NTHR, bi::TOTAL, s, p)) != cudaSuccess) return e;
     if (convb) {
-        conv_bwd_fixup_kernel<<<dim3(p.NT, p.H, 3), 128, 0, s>>>(p);
-        conv_bwd_reduce_kernel<<<dim3(p.H, 3), 1024, 0, s>>>(p);
+        if ((e = launch_dependent(conv_bwd_fixup_kernel, dim3(p.NT, p.H, 3), 128, 0, s, p)) != cudaSuccess) return e;
+        if ((e = launch_dependent(conv_bwd_reduce_kernel, dim3(p.H, 3), 1024, 0, s, p)) != cudaSuccess) return e;
     }
     return cudaGetLastError();
 }

@@ -32,6 +32,29 @@ inline int sm_count() {
     return n;
 }
 
+// The kernels of a call follow one another in the stream as programmatic dependents: the next kernel's CTAs are placed as
+// SMs come free and set themselves up (barriers, tensor memory) while the last CTAs of the one before still run.
+// pdl_wait() returns when that kernel, and through it every earlier one, has completed and its writes are visible: every
+// kernel launched with launch_dependent() calls it before its first access to global memory, in every thread.
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 // The units a CTA of a unit-walking kernel visits: first, first + stride, ...  Unit u is chunk u / H with
 // the head skewed by the chunk, (u % H + chunk) % H, so that the units of one CTA cycle through all heads
 // whatever the stride (heads differ in cost).  Stepping costs additions only: the integer divisions, which

@@ -102,6 +102,7 @@ __global__ void __launch_bounds__(32 * dec::NW) kda_recurrent_kernel(
     auto chn = [&](int j) { return VF ? 4 * ld + j : ld + LD * j; };
     const bool l2 = flags & KDA_FLAG_QK_L2NORM, gate = flags & KDA_FLAG_GATE, sig = flags & KDA_FLAG_BETA_SIGMOID;
     const size_t sbase = (size_t)nh * D * D;
+    pdl_wait();
 
     // the state is requested first; it arrives behind the prologue
     float S[NE][ND];
@@ -271,10 +272,9 @@ template <typename T, int D, bool VF, int R>
 static cudaError_t launch_recurrent(const RecurrentArgs& a, cudaStream_t s) {
     const int tb = a.T < dec::TB ? a.T : dec::TB;
     const size_t smem = (size_t)tb * dec::tok_floats(D) * sizeof(float);
-    kda_recurrent_kernel<T, D, VF, R><<<a.N * a.H * (D / (R * dec::NW)), 32 * dec::NW, smem, s>>>(
-        (const T*)a.q, (const T*)a.k, (const T*)a.v, (const T*)a.g, (const T*)a.beta, a.A_log, a.dt_bias, a.state_in,
+    return launch_dependent(
+        kda_recurrent_kernel<T, D, VF, R>, a.N * a.H * (D / (R * dec::NW)), 32 * dec::NW, smem, s, (const T*)a.q, (const T*)a.k, (const T*)a.v, (const T*)a.g, (const T*)a.beta, a.A_log, a.dt_bias, a.state_in,
         a.state_out, (T*)a.o, a.H, a.T, a.flags, a.scale, a.vec);
-    return cudaGetLastError();
 }
 
 // Columns per warp: eight (D / 32 CTAs per unit, short dependent chains per token) until the CTAs fill the chip twice

@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_fwd_intra_simt(const KdaParam
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ty = tid >> 4, tx = tid & 15;
     const int c = blockIdx.x / p.H, h = blockIdx.x % p.H;
+    pdl_wait();
     const ChunkInfo ci = chunk_info(p, c);
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     char* ws = (char*)p.workspace;
@@ -424,6 +425,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ty = tid >> 4, tx = tid & 15;
     const int c = blockIdx.x / p.H, h = blockIdx.x % p.H;
+    pdl_wait();
     const ChunkInfo ci = chunk_info(p, c);
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     const char* ws = (const char*)p.workspace;
@@ -827,6 +829,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
 __global__ void __launch_bounds__(1024) kda_param_reduce(const KdaParams p) {
     __shared__ float sb[8][128];
     __shared__ float sa[8][32];
+    pdl_wait();
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     const char* sc = (const char*)p.bwd_scratch;
     const int h = blockIdx.x, d = threadIdx.x & 127, grp = threadIdx.x >> 7;
@@ -888,22 +891,18 @@ static cudaError_t launch_stage(const KdaParams& p, int stage, cudaStream_t s) {
     switch (stage) {
         case 0:
             if ((e = set_smem(kda_fwd_intra_simt<T, D>, smem_intra<D>())) != cudaSuccess) return e;
-            kda_fwd_intra_simt<T, D><<<p.NT * p.H, NTHREADS, smem_intra<D>(), s>>>(p);
-            break;
+            return launch_dependent(kda_fwd_intra_simt<T, D>, p.NT * p.H, NTHREADS, smem_intra<D>(), s, p);
         case 1: return simt_state(p, false, s);
         case 2: return simt_state(p, true, s);
         case 3:
             if ((e = set_smem(kda_bwd_chunk_simt<T, D>, smem_bwd_chunk<D>())) != cudaSuccess) return e;
-            kda_bwd_chunk_simt<T, D><<<p.NT * p.H, NTHREADS, smem_bwd_chunk<D>(), s>>>(p);
-            break;
+            return launch_dependent(kda_bwd_chunk_simt<T, D, false>, p.NT * p.H, NTHREADS, smem_bwd_chunk<D>(), s, p);
         case 5:
             if ((e = set_smem(kda_bwd_chunk_simt<T, D, true>, smem_bwd_chunk<D>())) != cudaSuccess) return e;
-            kda_bwd_chunk_simt<T, D, true><<<p.NT * p.H, NTHREADS, smem_bwd_chunk<D>(), s>>>(p);
-            break;
+            return launch_dependent(kda_bwd_chunk_simt<T, D, true>, p.NT * p.H, NTHREADS, smem_bwd_chunk<D>(), s, p);
         default:
-            kda_param_reduce<<<p.H, 1024, 0, s>>>(p);
+            return launch_dependent(kda_param_reduce, p.H, 1024, 0, s, p);
     }
-    return cudaGetLastError();
 }
 
 // stage: 0 fwd_intra, 1 fwd_state, 2 bwd_state, 3 bwd_chunk, 4 param_reduce, 5 bwd_chunk stopped after the adjoints

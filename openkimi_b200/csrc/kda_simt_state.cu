@@ -140,6 +140,7 @@ __global__ void __launch_bounds__(ss::NT, 1) kda_fwd_state_simt(const KdaParams 
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     char* ws = (char*)p.workspace;
     const bool save = !(p.flags & KDA_FLAG_NO_SAVE);
+    pdl_wait();
     SeqCursor sq;
     sq.load(p, n);
     const size_t sbase = ((size_t)n * p.H + h) * D * D;
@@ -245,6 +246,7 @@ __global__ void __launch_bounds__(ss::NT, 1) kda_bwd_state_simt(const KdaParams 
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     const char* ws = (const char*)p.workspace;
     char* sc = (char*)p.bwd_scratch;
+    pdl_wait();
     SeqCursor sq;
     sq.load(p, n);
     const size_t sbase = ((size_t)n * p.H + h) * D * D;
@@ -335,8 +337,7 @@ static cudaError_t launch_state(const KdaParams& p, bool bwd, cudaStream_t s) {
     constexpr int smem = ss::Smem<T, D, BV>::TOTAL;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    kern<<<dim3(D / BV, p.H, p.N), ss::NT, smem, s>>>(p);
-    return cudaGetLastError();
+    return launch_dependent(kern, dim3(D / BV, p.H, p.N), ss::NT, smem, s, p);
 }
 
 // Panels of eight columns while all of them are resident at once (the chunk step is a chain of latencies); wider ones

@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(sg::NTHR, 1) kda_fwd_segment_tc(const KdaParam
     // part 0 carries the state, part 1 the transition; inside a part as in kda_fwd_state_tc
     const int tid = threadIdx.x, warp = tid >> 5, e = tid & 127, half = (tid >> 7) & 1, part = tid >> 8;
     const int h = blockIdx.x, seg = blockIdx.y;
+    pdl_wait();
     int cb = seg * segs.len;
     const int ce = min(cb + segs.len, p.NT);
     SeqCursor sq;
@@ -206,6 +207,7 @@ __global__ void __launch_bounds__(sc::NTHR, 3 - STAGES) kda_seg_combine(const Kd
     extern __shared__ __align__(128) unsigned char dyn[];
     __shared__ uint64_t full[2];
     const int tid = threadIdx.x, h = blockIdx.y, n = blockIdx.z, e0 = blockIdx.x * ROWS;
+    pdl_wait();
     int c0, nc;
     seq_chunks(p, n, c0, nc);
     if (nc == 0) {  // no chunk of this sequence is visited by any segment: its state passes through here
@@ -357,14 +359,13 @@ cudaError_t launch_seg_combine(const KdaParams& p, const StateSegs& segs, bool b
     const int smem = (int)sc::total(two ? 1 : 2);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    kern<<<dim3(sc::D / sc::ROWS, p.H, p.N), sc::NTHR, smem, s>>>(p, segs);
-    return cudaGetLastError();
+    return launch_dependent(kern, dim3(sc::D / sc::ROWS, p.H, p.N), sc::NTHR, smem, s, p, segs);
 }
 
 cudaError_t launch_fwd_segments(const KdaParams& p, const StateSegs& segs, cudaStream_t s) {
     cudaError_t e = cudaFuncSetAttribute(kda_fwd_segment_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sg::TOTAL);
     if (e != cudaSuccess) return e;
-    kda_fwd_segment_tc<<<dim3(p.H, segs.count), sg::NTHR, sg::TOTAL, s>>>(p, segs);
+    if ((e = launch_dependent(kda_fwd_segment_tc, dim3(p.H, segs.count), sg::NTHR, sg::TOTAL, s, p, segs)) != cudaSuccess) return e;
     return launch_seg_combine(p, segs, false, s);
 }
 

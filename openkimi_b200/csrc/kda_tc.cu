@@ -210,20 +210,6 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
     // the producer warp
     const int tid = threadIdx.x, warp = tid >> 5, e = tid & 127, half = tid >> 7;
     const int h = blockIdx.x;
-    // the chunks of this CTA: one sequence, or one segment of the chunk numbering
-    SeqCursor sq;
-    int cb, ce;
-    if (segs.len > 0) {
-        cb = blockIdx.y * segs.len;
-        ce = min(cb + segs.len, p.NT);
-        sq.load_of_chunk(p, cb);
-    } else {
-        sq.load(p, blockIdx.y);
-        cb = sq.c_begin;
-        ce = sq.c_end;
-    }
-    const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
-    char* ws = (char*)p.workspace;
     if (warp == 0) {
         tmem_alloc(&tmem_s, TMEM_COLS);
         tmem_relinquish();
@@ -240,6 +226,21 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
         mbar_init(&ofree, OUTT / 32);
         mbar_fence_init();
     }
+    pdl_wait();
+    // the chunks of this CTA: one sequence, or one segment of the chunk numbering
+    SeqCursor sq;
+    int cb, ce;
+    if (segs.len > 0) {
+        cb = blockIdx.y * segs.len;
+        ce = min(cb + segs.len, p.NT);
+        sq.load_of_chunk(p, cb);
+    } else {
+        sq.load(p, blockIdx.y);
+        cb = sq.c_begin;
+        ce = sq.c_end;
+    }
+    const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
+    char* ws = (char*)p.workspace;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -462,6 +463,7 @@ __global__ void __launch_bounds__(bs::NTHR, 1) kda_bwd_state_tc(const KdaParams 
     // main threads (half, e) = (tid / 128, tid % 128): TMEM lane e, and half of the columns of every conversion phase
     const int tid = threadIdx.x, warp = tid >> 5, e = tid & 127, half = tid >> 7;
     const int h = blockIdx.x;
+    pdl_wait();
     // the chunks of this CTA, walked from the last to the first: one sequence, or one segment of the chunk numbering
     SeqCursor sq;  // sequence of the current chunk
     int cb, ce;
@@ -703,7 +705,8 @@ cudaError_t tc_fwd(const KdaParams& p, cudaStream_t s) {
             return e;
         RowMaps maps = {};
         maps.ok = !(p.flags & KDA_FLAG_ROW_COPIES) && make_row_map(&maps.m[0], p.o, (long long)p.B * p.T, p.H, C);
-        kda_fwd_state_tc<<<dim3(p.H, segs.len > 0 ? segs.count : p.N), fs::NTHR, smem, s>>>(p, maps, segs);
+        if ((e = launch_dependent(kda_fwd_state_tc, dim3(p.H, segs.len > 0 ? segs.count : p.N), fs::NTHR, smem, s, p, maps, segs)) != cudaSuccess)
+            return e;
     }
     prof_mark(s);
     return cudaGetLastError();
@@ -721,10 +724,11 @@ cudaError_t tc_bwd(const KdaParams& p, cudaStream_t s) {
         if (segs.len > 0) {
             if ((e = cudaFuncSetAttribute(kda_bwd_state_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
                 return e;
-            kda_bwd_state_tc<true><<<dim3(p.H, segs.count), bs::NTHR, smem, s>>>(p, segs);
+            if ((e = launch_dependent(kda_bwd_state_tc<true>, dim3(p.H, segs.count), bs::NTHR, smem, s, p, segs)) != cudaSuccess) return e;
             if ((e = launch_seg_combine(p, segs, true, s)) != cudaSuccess) return e;
         }
-        kda_bwd_state_tc<false><<<dim3(p.H, segs.len > 0 ? segs.count : p.N), bs::NTHR, smem, s>>>(p, segs);
+        if ((e = launch_dependent(kda_bwd_state_tc<false>, dim3(p.H, segs.len > 0 ? segs.count : p.N), bs::NTHR, smem, s, p, segs)) != cudaSuccess)
+            return e;
     }
     prof_mark(s);
     if (stage_simt(p, ST_BWD_CHUNK)) {  // fused FP32-math kernel

@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(bp::NTHR, 1) kda_bwd_wy_tc_pf(const KdaParams 
         mbar_init(&mma3, 2);
         mbar_fence_init();
     }
+    pdl_wait();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -558,8 +559,7 @@ cudaError_t launch_bwd_wy_tc(const KdaParams& p, cudaStream_t s) {
     const int smem = convb ? (int)bp::TOTAL_CONVB : (int)bp::TOTAL;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    kern<<<units < sms ? units : sms, bp::NTHR, smem, s>>>(p, maps);
-    return cudaGetLastError();
+    return launch_dependent(kern, units < sms ? units : sms, bp::NTHR, smem, s, p, maps);
 }
 
 }  // namespace kda

@@ -205,6 +205,7 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
         mbar_init(&vbar, 1);
         mbar_fence_init();
     }
+    pdl_wait();
     __syncthreads();
 
     // ---- 0: a unit's inputs arrive as bulk-tensor tile copies (row by row for partial chunks), completing on two
@@ -858,8 +859,7 @@ cudaError_t launch_fwd_intra_tc(const KdaParams& p, cudaStream_t s) {
     const long long tokens = (long long)p.B * p.T;
     maps.ok = !(p.flags & KDA_FLAG_ROW_COPIES) && make_row_map(&maps.m[0], p.q, tokens, p.H, C) && make_row_map(&maps.m[1], p.k, tokens, p.H, C) &&
               make_row_map(&maps.m[2], p.v, tokens, p.H, C) && make_row_map(&maps.m[3], p.g, tokens, p.H, C);
-    kern<<<units < sms ? units : sms, fi::NTHR, fi::TOTAL, s>>>(p, maps);
-    return cudaGetLastError();
+    return launch_dependent(kern, units < sms ? units : sms, fi::NTHR, fi::TOTAL, s, p, maps);
 }
 
 }  // namespace kda
