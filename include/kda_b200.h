@@ -48,7 +48,12 @@ enum {
     /* Move the [64 x 128] tiles of the token-major tensors (q, k, v, g in, o and dv out) row by row instead of
      * with one bulk-tensor copy per tile.  Same bytes either way; the library falls back to this by itself
      * where the driver's tensor-map encoder is not available, and uses it for partial chunks. */
-    KDA_FLAG_ROW_COPIES = 2048
+    KDA_FLAG_ROW_COPIES = 2048,
+    /* A forward run for its records only (the second forward of the recompute policy): o is not computed (the
+     * pointer is not used but must be valid), and with BORDERS_READY `borders` already holds what an earlier
+     * forward of the same call left there. */
+    KDA_FLAG_NO_OUTPUT = 4096,
+    KDA_FLAG_BORDERS_READY = 8192
 };
 
 enum {
@@ -128,11 +133,18 @@ typedef struct KdaParams {
     int32_t max_chunks;         /* chunks of the longest sequence; 0: not known (with cu_seqlens the mean is
                                    assumed).  Only a hint how to split the state recurrence over the chip;
                                    the same value for kda_workspace_bytes, kda_fwd and kda_bwd of a call */
+    float *borders;             /* optional, kda_border_bytes() long, 256-byte aligned: where a forward that splits its
+                                   sequences leaves the states at the split points and the transitions between
+                                   them, instead of at the end of the workspace.  A caller that drops the
+                                   workspace and runs the forward again for the backward keeps this (a few KB
+                                   per chunk) and sets KDA_FLAG_BORDERS_READY for the second run. */
 } KdaParams;
 
 /* Bytes of forward workspace (saved for the backward) and of backward scratch for these
  * sizes.  Replaces the torch.empty calls inside the reference's third-party op. */
 int kda_workspace_bytes(const KdaParams *p, size_t *fwd_bytes, size_t *bwd_bytes);
+/* Size of KdaParams.borders for this call; 0 where the forward does not split its sequences. */
+int kda_border_bytes(const KdaParams *p, size_t *bytes);
 
 /* Forward of chunk_kda (k3mini/model.py:200-216): o, optional final state, and the
  * per-chunk intermediates in the workspace. */

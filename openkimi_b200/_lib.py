@@ -42,6 +42,7 @@ class KdaParams(C.Structure):
         ("status_host", C.c_void_p),
         ("grad_conv_q", C.c_void_p), ("grad_conv_k", C.c_void_p), ("grad_conv_v", C.c_void_p),
         ("max_chunks", C.c_int32),
+        ("borders", C.c_void_p),
     ]
 
 
@@ -60,6 +61,7 @@ EXPORTS = {
     "kda_selftest_mma": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p] + [C.c_int] * 12 + [C.c_void_p, C.c_void_p]),
     "kda_selftest_wait": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p]),
     "kda_workspace_bytes": (C.c_int, [C.POINTER(KdaParams), C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]),
+    "kda_border_bytes": (C.c_int, [C.POINTER(KdaParams), C.POINTER(C.c_size_t)]),
     "kda_fwd": (C.c_int, [C.POINTER(KdaParams), C.c_void_p]),
     "kda_bwd": (C.c_int, [C.POINTER(KdaParams), C.c_void_p]),
     "kda_recurrent_step": (C.c_int, [C.c_void_p] * 10 + [C.c_int32] * 6 + [C.c_float, C.c_void_p, C.c_void_p]),

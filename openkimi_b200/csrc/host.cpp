@@ -4,6 +4,7 @@
 //
 // No tensor is kept from one call for the next; the only state here is the table of the devices' status words.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/extension.h>
@@ -108,7 +109,11 @@ Tensor ready(const Tensor& t, at::ScalarType dt) {
     if (!r.is_contiguous()) r = r.contiguous();
     return (reinterpret_cast<uintptr_t>(r.data_ptr()) & 15) == 0 ? r : r.clone();
 }
-Tensor ready_f32(const OptTensor& t) { return t && t->defined() ? ready(t->detach(), at::kFloat) : Tensor(); }
+Tensor ready_f32(const OptTensor& t) { return t && t->defined() ? ready(*t, at::kFloat) : Tensor(); }
+// a new tensor without the dispatcher's detour (half of what at::empty costs)
+Tensor fresh(at::IntArrayRef sizes, at::ScalarType dt, const Tensor& like) {
+    return Tensor(at::detail::empty_cuda(sizes, dt, like.device(), std::nullopt));
+}
 template <class T>
 T* ptr(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr; }
 
@@ -144,12 +149,12 @@ std::tuple<Tensor, OptTensor> recurrent(const Tensor& q, const Tensor& k, const 
     const Tensor qc = ready(q, dt), kc = ready(k, dt), vc = ready(v, dt), gc = ready(g, dt), bc = ready(beta, dt);
     const Tensor a = gate ? ready_f32(A_log) : Tensor(), b = gate ? ready_f32(dt_bias) : Tensor();
     Tensor s_in, s_out;
-    if (state) s_in = ready(state->detach(), at::kFloat);
+    if (state) s_in = ready(*state, at::kFloat);
     if (want_state) {
-        if (inplace && s_in.data_ptr() == state->data_ptr()) s_out = s_in;
-        else s_out = at::empty(want, q.options().dtype(at::kFloat));
+        if (inplace && s_in.data_ptr() == state->data_ptr()) s_out = s_in.requires_grad() ? s_in.detach() : s_in;
+        else s_out = fresh(want, at::kFloat, q);
     }
-    Tensor o = at::empty(q.sizes(), q.options());
+    Tensor o = fresh(q.sizes(), dt, q);
     status_word(q.device().index());
     if (N * T * H == 0) {
         if (s_out.defined() && !s_out.is_same(s_in)) {
@@ -219,7 +224,8 @@ Prepared prepare(const Inputs& in, const Spec& sp, int flags) {
     return r;
 }
 
-Tensor bytes(size_t n, const Tensor& like) { return at::empty({(int64_t)n}, like.options().dtype(at::kByte)); }
+Tensor bytes(size_t n, const Tensor& like) { return fresh({(int64_t)n}, at::kByte, like); }
+Tensor fresh_like(const Tensor& t) { return fresh(t.sizes(), t.scalar_type(), t); }
 
 std::array<int64_t, 4> state_shape(const Inputs& in, const Spec& sp, int64_t N) {
     const int64_t H = in.q.size(2), dk = in.q.size(3), dv = in.v.size(3);
@@ -227,16 +233,26 @@ std::array<int64_t, 4> state_shape(const Inputs& in, const Spec& sp, int64_t N) 
     return {N, H, dk, dv};
 }
 
-struct FwdOut { Tensor o, ht, ws; };
+struct FwdOut { Tensor o, ht, ws, borders; };
 
-FwdOut run_fwd(const Inputs& in, const Spec& sp) {
+// recompute: the backward will rebuild the records; the states at the split points of long sequences are kept for it
+FwdOut run_fwd(const Inputs& in, const Spec& sp, bool recompute = false) {
     // The forward-only kernels skip every record that only the backward reads: when nobody will differentiate this
     // call, or the backward rebuilds the records anyway (recompute policy).
     Prepared pr = prepare(in, sp, sp.keep ? sp.flags : sp.flags | KDA_FLAG_NO_SAVE);
     FwdOut out;
     const Tensor& q = in.q;
-    out.o = at::empty_like(in.v);
-    if (sp.output_final_state) out.ht = at::empty(state_shape(in, sp, pr.N), q.options().dtype(at::kFloat));
+    if (recompute && !pr.empty) {
+        size_t n = 0;
+        check_rc(kda_border_bytes(&pr.p, &n), "kda_border_bytes");
+        if (n) {
+            out.borders = bytes(n, q);
+            pr.p.borders = ptr<float>(out.borders);
+            check_rc(kda_workspace_bytes(&pr.p, &pr.fwd_bytes, &pr.bwd_bytes), "kda_workspace_bytes");
+        }
+    }
+    out.o = fresh_like(in.v);
+    if (sp.output_final_state) out.ht = fresh(state_shape(in, sp, pr.N), at::kFloat, q);
     out.ws = bytes(pr.fwd_bytes, q);
     if (pr.empty) {
         if (out.ht.defined()) {
@@ -254,35 +270,39 @@ FwdOut run_fwd(const Inputs& in, const Spec& sp) {
 struct Grads { Tensor q, k, v, g, beta, A_log, dt_bias, h0, conv_q, conv_k, conv_v; };
 
 // out: where dq, dk, dv, dg go if the caller has a place for them
-Grads run_bwd(const Inputs& in, const Spec& sp, Tensor ws, const Tensor& grad_o, const Tensor& grad_ht, Grads out = {}) {
+Grads run_bwd(const Inputs& in, const Spec& sp, Tensor ws, const Tensor& borders, const Tensor& grad_o, const Tensor& grad_ht, Grads out = {}) {
     Prepared pr = prepare(in, sp, sp.flags);
+    if (borders.defined()) {
+        pr.p.borders = ptr<float>(borders);
+        check_rc(kda_workspace_bytes(&pr.p, &pr.fwd_bytes, &pr.bwd_bytes), "kda_workspace_bytes");
+    }
     const Tensor& q = in.q;
     const int64_t H = q.size(2), dk = q.size(3);
     void* stream = stream_of(q);
     KdaParams& p = pr.p;
     if (!ws.defined()) {  // recompute policy: rebuild the per-chunk records instead of keeping them
         ws = bytes(pr.fwd_bytes, q);
-        Tensor o_tmp = at::empty_like(in.v);
-        p.o = o_tmp.data_ptr();
+        p.o = q.data_ptr();  // (not written)
         p.workspace = ws.data_ptr(); p.workspace_bytes = pr.fwd_bytes;
+        p.flags |= KDA_FLAG_NO_OUTPUT | (borders.defined() ? KDA_FLAG_BORDERS_READY : 0);
         if (!pr.empty) check_rc(kda_fwd(&p, stream), "kda_fwd (recompute)");
+        p.flags = sp.flags;
     }
-    const auto f32 = q.options().dtype(at::kFloat);
     const Tensor go = grad_o.defined() ? ready(grad_o, q.scalar_type()) : at::zeros_like(in.v);
     const Tensor ght = grad_ht.defined() ? ready(grad_ht, at::kFloat) : Tensor();
-    if (!out.q.defined()) out.q = at::empty_like(q);
-    if (!out.k.defined()) out.k = at::empty_like(in.k);
-    if (!out.v.defined()) out.v = at::empty_like(in.v);
-    if (!out.g.defined()) out.g = at::empty_like(in.g);
-    if (!out.beta.defined()) out.beta = at::empty_like(in.beta);
+    if (!out.q.defined()) out.q = fresh_like(q);
+    if (!out.k.defined()) out.k = fresh_like(in.k);
+    if (!out.v.defined()) out.v = fresh_like(in.v);
+    if (!out.g.defined()) out.g = fresh_like(in.g);
+    if (!out.beta.defined()) out.beta = fresh_like(in.beta);
     const bool gate = sp.flags & KDA_FLAG_GATE;
     // written in full by the fixed-order reduction kernel (no zero fill needed)
-    if (gate) out.A_log = at::empty({H}, f32);
-    if (gate && in.dt_bias.defined()) out.dt_bias = at::empty({H * dk}, f32);
-    if (in.h0.defined()) out.h0 = at::empty(state_shape(in, sp, pr.N), f32);
+    if (gate) out.A_log = fresh({H}, at::kFloat, q);
+    if (gate && in.dt_bias.defined()) out.dt_bias = fresh({H * dk}, at::kFloat, q);
+    if (in.h0.defined()) out.h0 = fresh(state_shape(in, sp, pr.N), at::kFloat, q);
     if (in.conv_q.defined()) {
         const std::array<int64_t, 2> sh = {H * dk, in.conv_q.size(-1)};
-        out.conv_q = at::empty(sh, f32); out.conv_k = at::empty(sh, f32); out.conv_v = at::empty(sh, f32);
+        out.conv_q = fresh(sh, at::kFloat, q); out.conv_k = fresh(sh, at::kFloat, q); out.conv_v = fresh(sh, at::kFloat, q);
     }
     if (pr.empty) {
         for (Tensor* t : {&out.q, &out.k, &out.v, &out.g, &out.beta, &out.A_log, &out.dt_bias, &out.conv_q, &out.conv_k, &out.conv_v})
@@ -322,9 +342,9 @@ Inputs gather(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g
     return in;
 }
 
-variable_list to_list(const Inputs& in, const Tensor& ws) {
+variable_list to_list(const Inputs& in, const Tensor& ws, const Tensor& borders) {
     return {in.q, in.k, in.v, in.g, in.beta, in.A_log, in.dt_bias, in.h0, in.conv_q, in.conv_k, in.conv_v,
-            in.cu, in.chunk_seq, in.seq_off, in.chunk_tab, ws};
+            in.cu, in.chunk_seq, in.seq_off, in.chunk_tab, ws, borders};
 }
 Inputs from_list(const variable_list& s) {
     return {s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7], s[8], s[9], s[10], s[11], s[12], s[13], s[14]};
@@ -355,8 +375,8 @@ struct ChunkKda : torch::autograd::Function<ChunkKda> {
                                  OptTensor dt_bias, OptTensor h0, OptTensor cq, OptTensor ck, OptTensor cv, const Inputs& tables,
                                  const Spec& sp) {
         const Inputs in = gather(q, k, v, g, beta, val(A_log), val(dt_bias), val(h0), val(cq), val(ck), val(cv), tables);
-        FwdOut f = run_fwd(in, sp);
-        ctx->save_for_backward(to_list(in, sp.keep ? f.ws : Tensor()));
+        FwdOut f = run_fwd(in, sp, !sp.keep);
+        ctx->save_for_backward(to_list(in, sp.keep ? f.ws : Tensor(), f.borders));
         ctx->set_materialize_grads(false);  // an unused final state has no gradient, rather than one of zeros
         save_spec(ctx, sp);
         if (f.ht.defined()) return {f.o, f.ht};
@@ -366,7 +386,7 @@ struct ChunkKda : torch::autograd::Function<ChunkKda> {
         const variable_list s = ctx->get_saved_variables();
         const Inputs in = from_list(s);
         c10::cuda::CUDAGuard guard(in.q.device());
-        Grads r = run_bwd(in, load_spec(ctx), s[15], grads[0], grads.size() > 1 ? grads[1] : Tensor());
+        Grads r = run_bwd(in, load_spec(ctx), s[15], s[16], grads[0], grads.size() > 1 ? grads[1] : Tensor());
         // (the engine casts every gradient to its input's dtype)
         return {r.q, r.k, r.v, r.g, r.beta, r.A_log, r.dt_bias, r.h0, as_filter(r.conv_q), as_filter(r.conv_k), as_filter(r.conv_v),
                 Tensor(), Tensor()};
@@ -464,7 +484,7 @@ struct Weights { Tensor qkv, narrow, ab, out; };  // views of one BF16 buffer
 
 struct LayerState {
     Inputs in;  // q, k, v, decay, beta and the parameters of the op
-    Tensor x2, narrow, gates, o, y, ws, norm_w;
+    Tensor x2, narrow, gates, o, y, ws, borders, norm_w;
     Weights w;
 };
 
@@ -501,7 +521,7 @@ Tensor rank_pair(const Tensor& narrow) {
     return narrow.as_strided({2, narrow.size(0), HD}, {HD, narrow.size(1), 1}, narrow.storage_offset());
 }
 
-Tensor layer_fwd(const Tensor& x, const variable_list& prm, const LayerSpec& ls, const Inputs& tables, LayerState& st) {
+Tensor layer_fwd(const Tensor& x, const variable_list& prm, const LayerSpec& ls, const Inputs& tables, LayerState& st, bool recompute = false) {
     const int64_t H = ls.H, proj = H * HD, width = x.size(-1), wide = (2 * HD + H + 7) / 8 * 8;
     const int64_t B = x.size(0), T = x.size(1), n = B * T;
     st.x2 = ready(x, at::kBFloat16).view({n, width});
@@ -514,9 +534,10 @@ Tensor layer_fwd(const Tensor& x, const variable_list& prm, const LayerSpec& ls,
     const Tensor beta = st.narrow.narrow(1, 2 * HD, H).contiguous().view({B, T, H});
     st.in = gather(heads(qkv[0]), heads(qkv[1]), heads(qkv[2]), heads(ab[0]), beta, prm[P_ALOG], prm[P_DTB].reshape({proj}), Tensor(),
                    prm[P_CQ], prm[P_CK], prm[P_CV], tables);
-    FwdOut f = run_fwd(st.in, ls.op);
+    FwdOut f = run_fwd(st.in, ls.op, recompute);
     st.o = f.o;
     st.ws = f.ws;
+    st.borders = f.borders;
     st.norm_w = ready(prm[P_NORM], at::kFloat);
     st.y = at::empty({n, proj}, st.x2.options());
     check_rc(kda_norm_gate_fwd(st.o.data_ptr(), st.gates.data_ptr(), ptr<float>(st.norm_w), st.y.data_ptr(), nullptr, n * H, (int)HD,
@@ -531,8 +552,8 @@ struct Layer : torch::autograd::Function<Layer> {
                                  const Inputs& tables, const LayerSpec& ls) {
         const variable_list prm = {p0, p1, p2, p3, p4, p5, p6, p7, p8, p9, p10, p11, p12, p13, p14};
         LayerState st;
-        const Tensor out = layer_fwd(x, prm, ls, tables, st);
-        variable_list keep = to_list(st.in, ls.op.keep ? st.ws : Tensor());
+        const Tensor out = layer_fwd(x, prm, ls, tables, st, !ls.op.keep);
+        variable_list keep = to_list(st.in, ls.op.keep ? st.ws : Tensor(), st.borders);
         for (const Tensor& t : {st.x2, st.narrow, st.gates, st.o, st.y, st.w.qkv, st.w.narrow, st.w.ab, st.w.out, st.norm_w})
             keep.push_back(t);
         ctx->save_for_backward(std::move(keep));
@@ -546,8 +567,8 @@ struct Layer : torch::autograd::Function<Layer> {
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const variable_list s = ctx->get_saved_variables();
         const Inputs in = from_list(s);
-        const Tensor &x2 = s[16], &narrow = s[17], &gates = s[18], &o = s[19], &y = s[20], &norm_w = s[25];
-        const Weights w = {s[21], s[22], s[23], s[24]};
+        const Tensor &x2 = s[17], &narrow = s[18], &gates = s[19], &o = s[20], &y = s[21], &norm_w = s[26];
+        const Weights w = {s[22], s[23], s[24], s[25]};
         const std::vector<int64_t> f32 = ctx->saved_data["f32"].toIntVector();
         variable_list r(1 + P_COUNT + 2);
         if (!grads[0].defined()) return r;
@@ -577,7 +598,7 @@ struct Layer : torch::autograd::Function<Layer> {
         const Tensor dqkv = at::empty({3, n, proj}, bf);
         Grads gr;
         gr.q = dqkv[0]; gr.k = dqkv[1]; gr.v = dqkv[2]; gr.g = dab[0];
-        gr = run_bwd(in, load_spec(ctx), s[15], d_o, Tensor(), gr);
+        gr = run_bwd(in, load_spec(ctx), s[15], s[16], d_o, Tensor(), gr);
         r[1 + P_CQ] = as_filter(gr.conv_q);
         r[1 + P_CK] = as_filter(gr.conv_k);
         r[1 + P_CV] = as_filter(gr.conv_v);

@@ -18,7 +18,7 @@ int segment_count(const KdaParams& p);
 // bytes of the segment buffers behind the workspace (state at every border, transitions) and behind the backward scratch
 static size_t segment_bytes(const KdaParams& p, bool bwd) {
     const size_t m = seg_matrix_floats(segment_count(p), p.H, p.dk) * sizeof(float);
-    return bwd ? m : 2 * m;
+    return bwd ? m : p.borders ? 0 : 2 * m;
 }
 
 static thread_local char g_last_error[256] = "";
@@ -97,6 +97,8 @@ static int validate(const KdaParams* p, bool bwd) {
     }
     if (!p->q || !p->k || !p->v || !p->g || !p->beta || !p->o || !p->workspace) return KDA_ERR_NULL;
     if ((p->flags & KDA_FLAG_GATE) && !p->A_log) return KDA_ERR_NULL;
+    if ((p->flags & KDA_FLAG_BORDERS_READY) && !p->borders) return KDA_ERR_NULL;
+    if ((uintptr_t)p->borders & 255) return KDA_ERR_ALIGN;
     if (!(p->guard_span < 0.f) && !(isfinite(p->guard_span) && p->guard_span <= kda_guard_max_span()))
         return KDA_ERR_GUARD;
     const void* ptrs[] = {p->q, p->k, p->v, p->g, p->o, p->workspace, p->h0, p->ht, p->chunk_tab};
@@ -166,6 +168,13 @@ int kda_workspace_bytes(const KdaParams* p, size_t* fwd_bytes, size_t* bwd_bytes
     if (bwd_bytes) *bwd_bytes = p->conv_q ? L.bwd_total_conv : L.bwd_total;
     if (fwd_bytes) *fwd_bytes += segment_bytes(*p, false);
     if (bwd_bytes) *bwd_bytes += segment_bytes(*p, true);
+    return KDA_OK;
+}
+
+int kda_border_bytes(const KdaParams* p, size_t* bytes) {
+    if (!p || !bytes) return KDA_ERR_NULL;
+    if (p->NT <= 0 || p->H <= 0 || p->dk <= 0 || p->dv <= 0) return KDA_ERR_SHAPE;
+    *bytes = 2 * seg_matrix_floats(segment_count(*p), p->H, p->dk) * sizeof(float);
     return KDA_OK;
 }
 

@@ -36,10 +36,7 @@ inline int sm_count() {
 // SMs come free and set themselves up (barriers, tensor memory) while the last CTAs of the one before still run.
 // pdl_wait() returns when that kernel, and through it every earlier one, has completed and its writes are visible: every
 // kernel launched with launch_dependent() calls it before its first access to global memory, in every thread.
-__device__ __forceinline__ void pdl_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class... P, class... A>
 inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
     cudaLaunchAttribute at;

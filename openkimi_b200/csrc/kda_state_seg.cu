@@ -345,7 +345,7 @@ StateSegs state_segs(const KdaParams& p, bool bwd) {
     const size_t m = seg_matrix_floats(r.count, p.H, p.dk);
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     const bool nosave = p.flags & KDA_FLAG_NO_SAVE;
-    float* f = (float*)((char*)p.workspace + (nosave ? L.total_nosave : p.conv_q ? L.total_conv : L.total));
+    float* f = p.borders ? p.borders : (float*)((char*)p.workspace + (nosave ? L.total_nosave : p.conv_q ? L.total_conv : L.total));
     r.E = f;
     r.X = f + m;
     if (bwd) r.E = (float*)((char*)p.bwd_scratch + (p.conv_q ? L.bwd_total_conv : L.bwd_total));

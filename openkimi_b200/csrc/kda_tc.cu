@@ -246,7 +246,8 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
     tc_fence_after();
     const uint32_t tmem = tmem_s + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's lane quadrant
     const uint32_t tmem0 = tmem_s;
-    const bool save = !(p.flags & KDA_FLAG_NO_SAVE);  // forward-only calls write no checkpoint and no V' record
+    const bool save = !(p.flags & KDA_FLAG_NO_SAVE);     // forward-only calls write no checkpoint and no V' record
+    const bool with_o = !(p.flags & KDA_FLAG_NO_OUTPUT);  // a walk for the records only leaves the output products out
     const bool vfirst = p.flags & KDA_FLAG_STATE_V_FIRST;
     float* stage_space = reinterpret_cast<float*>(dyn);  // before the first and after the last chunk's copies
     if (tid < MAIN) {
@@ -289,7 +290,7 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
                     for (int s = 0; s < 8; ++s)  // WSacc = Sbf (K = d) * W^T record, MN-major B
                         mma_ts(tmem0 + WSACC, tmem0 + SBF + s * 8, make_desc(sb + WT + s * 2048, 1024, 128), id_mn, s > 0);
                     mma_commit(&wsbar);
-                } else {
+                } else if (with_o) {
                     if (i > 0) ok = mbar_wait(&ofree, (i - 1) & 1, p, 4);  // the previous chunk's output has left Oacc
                     tc_fence_after();
                     if (ok) {
@@ -346,7 +347,7 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
                     for (int s = 0; s < 4; ++s)  // Sacc += Vbf (K = i) * Kh, MN-major B
                         mma_ts(tmem0 + SACC, tmem0 + VBF + s * 8, make_desc(sb + KH + s * 4096, 2048, 128), id_s, true);
                     mma_commit(&sbar);
-                } else {
+                } else if (with_o) {
 #pragma unroll
                     for (int s = 0; s < 4; ++s)  // Oacc += Vbf (K = j) * Aqk^T, K-major B (rows = i)
                         mma_ts(tmem0 + OACC, tmem0 + VBF + s * 8, make_desc(sb + AQ + s * 256, 128, 1024), id_k, true);
@@ -360,7 +361,7 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
                 for (int g = 0; g < 2; ++g) store_record16(gV, e, 32 * half + 16 * g, C, vk[g]);
             }
             // (both: the next chunk overwrites the operands of the output products too)
-            ok = mbar_wait(&sbar, i & 1, p, 4) && mbar_wait(&obar, i & 1, p, 4) && ok;
+            ok = mbar_wait(&sbar, i & 1, p, 4) && (!with_o || mbar_wait(&obar, i & 1, p, 4)) && ok;
             tc_fence_after();
             if (tid == 0) mbar_arrive(&empty[stage]);
             KDA_PHASE(4);
@@ -377,7 +378,7 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
         const int ot = tid - MAIN;
         __nv_bfloat16* o = (__nv_bfloat16*)p.o;
         __nv_bfloat16* sO = reinterpret_cast<__nv_bfloat16*>(dyn + OUT);
-        for (int c = cb; c < ce; ++c) {
+        for (int c = cb; c < ce && with_o; ++c) {
             sq.move_to(p, c);
             ok = mbar_wait(&obar, (c - cb) & 1, p, 4);
             ok = bar_and(2, OUTT, ok);
@@ -419,11 +420,12 @@ kda_fwd_state_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const 
             if (i >= 2 && !mbar_wait(&empty[stage], ((i >> 1) - 1) & 1, p, 2)) break;
             const size_t rec = (size_t)(cb + i) * p.H + h;
             unsigned char* b = dyn + stage * STAGE;
-            mbar_expect_tx(&full[stage], STAGE);
+            mbar_expect_tx(&full[stage], with_o ? STAGE : STAGE - 16384 - 8192);
             tma_load_1d(b + GAM, (const float*)(ws + L.gamC) + rec * D, 512, &full[stage]);
             tma_load_1d(b + WT, (const __nv_bfloat16*)(ws + L.W) + rec * C * D, 16384, &full[stage]);
             tma_load_1d(b + UT, (const __nv_bfloat16*)(ws + L.U) + rec * C * D, 16384, &full[stage]);
             tma_load_1d(b + KH, (const __nv_bfloat16*)(ws + L.Kh) + rec * C * D, 16384, &full[stage]);
+            if (!with_o) continue;
             tma_load_1d(b + QT, (const __nv_bfloat16*)(ws + L.Qt) + rec * C * D, 16384, &full[stage]);
             tma_load_1d(b + AQ, (const __nv_bfloat16*)(ws + L.Aqk) + rec * C * C, 8192, &full[stage]);
         }
@@ -699,7 +701,7 @@ cudaError_t tc_fwd(const KdaParams& p, cudaStream_t s) {
         if ((e = simt_stage(p, ST_FWD_STATE, s)) != cudaSuccess) return e;
     } else {
         const StateSegs segs = state_segs(p, false);
-        if (segs.len > 0 && (e = launch_fwd_segments(p, segs, s)) != cudaSuccess) return e;
+        if (segs.len > 0 && !(p.flags & KDA_FLAG_BORDERS_READY) && (e = launch_fwd_segments(p, segs, s)) != cudaSuccess) return e;
         constexpr int smem = fs::TOTAL;
         if ((e = cudaFuncSetAttribute(kda_fwd_state_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
             return e;
