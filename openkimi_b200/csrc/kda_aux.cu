@@ -246,34 +246,26 @@ __global__ void __launch_bounds__(256) norm_gate_fwd_kernel(const T* __restrict_
     float wv[V];
 #pragma unroll
     for (int i = 0; i < V; ++i) wv[i] = w[sub * V + i];
-    // (two rows' loads in flight per thread: with one the kernel ran at 4.1 TB/s)
-    for (long long r0 = warp * RPW; r0 < rows; r0 += 2 * nw * RPW) {
-        float xv[2][V], gv[2][V];
+    for (long long r0 = warp * RPW; r0 < rows; r0 += nw * RPW) {
+        const long long r = r0 + rsub;
+        const bool ok = r < rows;
+        float xv[V], gv[V], out[V], ss = 0.f;
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const long long r = r0 + u * nw * RPW + rsub;
-#pragma unroll
-            for (int i = 0; i < V; ++i) xv[u][i] = gv[u][i] = 0.f;
-            if (r < rows) {
-                Vec<T>::load(x + r * DIM + sub * V, xv[u]);
-                Vec<T>::load(gate + r * DIM + sub * V, gv[u]);
-            }
+        for (int i = 0; i < V; ++i) xv[i] = gv[i] = 0.f;
+        if (ok) {
+            Vec<T>::load(x + r * DIM + sub * V, xv);
+            Vec<T>::load(gate + r * DIM + sub * V, gv);
         }
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const long long r = r0 + u * nw * RPW + rsub;
-            float out[V], ss = 0.f;
+        for (int i = 0; i < V; ++i) ss += xv[i] * xv[i];
 #pragma unroll
-            for (int i = 0; i < V; ++i) ss += xv[u][i] * xv[u][i];
+        for (int o = LPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        const float rs = rsqrtf(ss / DIM + eps);
+        if (ok) {
+            if (sub == 0 && rstd) rstd[r] = rs;
 #pragma unroll
-            for (int o = LPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            const float rs = rsqrtf(ss / DIM + eps);
-            if (r < rows) {
-                if (sub == 0 && rstd) rstd[r] = rs;
-#pragma unroll
-                for (int i = 0; i < V; ++i) out[i] = xv[u][i] * rs * wv[i] * sigmoid_f(gv[u][i]);
-                Vec<T>::store(y + r * DIM + sub * V, out);
-            }
+            for (int i = 0; i < V; ++i) out[i] = xv[i] * rs * wv[i] * sigmoid_f(gv[i]);
+            Vec<T>::store(y + r * DIM + sub * V, out);
         }
     }
 }
@@ -294,48 +286,42 @@ __global__ void __launch_bounds__(256) norm_gate_bwd_kernel(const T* __restrict_
         wv[i] = w[sub * V + i];
         dwv[i] = 0.f;
     }
-    for (long long r0 = warp * RPW; r0 < rows; r0 += 2 * nw * RPW) {  // (two rows in flight, as in the forward)
-        float xv[2][V], gv[2][V], gy[2][V];
+    for (long long r0 = warp * RPW; r0 < rows; r0 += nw * RPW) {
+        const long long r = r0 + rsub;
+        const bool ok = r < rows;
+        float xv[V], gv[V], gy[V], dn[V], ss = 0.f, dot = 0.f;
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const long long r = r0 + u * nw * RPW + rsub;
-#pragma unroll
-            for (int i = 0; i < V; ++i) xv[u][i] = gv[u][i] = gy[u][i] = 0.f;
-            if (r < rows) {
-                Vec<T>::load(x + r * DIM + sub * V, xv[u]);
-                Vec<T>::load(gate + r * DIM + sub * V, gv[u]);
-                Vec<T>::load(dy + r * DIM + sub * V, gy[u]);
-            }
+        for (int i = 0; i < V; ++i) xv[i] = gv[i] = gy[i] = 0.f;
+        if (ok) {
+            Vec<T>::load(x + r * DIM + sub * V, xv);
+            Vec<T>::load(gate + r * DIM + sub * V, gv);
+            Vec<T>::load(dy + r * DIM + sub * V, gy);
         }
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const long long r = r0 + u * nw * RPW + rsub;
-            float dn[V], dg[V], ss = 0.f, dot = 0.f;
+        for (int i = 0; i < V; ++i) ss += xv[i] * xv[i];
 #pragma unroll
-            for (int i = 0; i < V; ++i) ss += xv[u][i] * xv[u][i];
+        for (int o = LPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        const float rs = rsqrtf(ss / DIM + eps);
+        float dg[V];
 #pragma unroll
-            for (int o = LPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            const float rs = rsqrtf(ss / DIM + eps);
+        for (int i = 0; i < V; ++i) {
+            const float sgm = sigmoid_f(gv[i]);
+            const float xh = xv[i] * rs;
+            dg[i] = gy[i] * xh * wv[i] * sgm * (1.f - sgm);
+            dn[i] = gy[i] * sgm;
+            dwv[i] += dn[i] * xh;
+            dn[i] *= wv[i];
+            dot += dn[i] * xh;
+        }
 #pragma unroll
-            for (int i = 0; i < V; ++i) {
-                const float sgm = sigmoid_f(gv[u][i]);
-                const float xh = xv[u][i] * rs;
-                dg[i] = gy[u][i] * xh * wv[i] * sgm * (1.f - sgm);
-                dn[i] = gy[u][i] * sgm;
-                dwv[i] += dn[i] * xh;
-                dn[i] *= wv[i];
-                dot += dn[i] * xh;
-            }
+        for (int o = LPR / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        dot /= DIM;
+        if (ok) {
+            float out[V];
 #pragma unroll
-            for (int o = LPR / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-            dot /= DIM;
-            if (r < rows) {
-                float out[V];
-#pragma unroll
-                for (int i = 0; i < V; ++i) out[i] = rs * (dn[i] - xv[u][i] * rs * dot);
-                Vec<T>::store(dx + r * DIM + sub * V, out);
-                Vec<T>::store(dgate + r * DIM + sub * V, dg);
-            }
+            for (int i = 0; i < V; ++i) out[i] = rs * (dn[i] - xv[i] * rs * dot);
+            Vec<T>::store(dx + r * DIM + sub * V, out);
+            Vec<T>::store(dgate + r * DIM + sub * V, dg);
         }
     }
 #pragma unroll

@@ -679,30 +679,30 @@ __global__ void __launch_bounds__(128) conv_bwd_fixup_kernel(const KdaParams p) 
 // Filter gradients: fixed-order sum of the per-chunk shares.  Grid (head, tensor), 8 groups of 128 threads sum
 // every 8th chunk, then the 8 group sums are added in order (the scheme of kda_param_reduce).
 __global__ void __launch_bounds__(1024) conv_bwd_reduce_kernel(const KdaParams p) {
-    __shared__ float4 sb[8][128];
+    constexpr int CH = 16, G = 64;  // channels of a CTA (256 contiguous bytes of a record), groups of chunks
+    __shared__ float4 sb[G][CH];
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     const float4* part = (const float4*)((const char*)p.bwd_scratch + L.cv_part);
-    const int h = blockIdx.x, t = blockIdx.y, ch = threadIdx.x & 127, grp = threadIdx.x >> 7;
+    const int h = blockIdx.x, t = blockIdx.y, cl = threadIdx.x % CH, ch = CH * blockIdx.z + cl, grp = threadIdx.x / CH;
     pdl_wait();
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
     // (eight loads in flight per thread, added in chunk order: the loop is a chain of round trips otherwise)
-    for (int c0 = grp; c0 < p.NT; c0 += 8 * 8) {
+    for (int c0 = grp; c0 < p.NT; c0 += G * 8) {
         float4 u[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const int c = c0 + 8 * q;
+            const int c = c0 + G * q;
             u[q] = c < p.NT ? part[(((size_t)c * p.H + h) * 3 + t) * 128 + ch] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int q = 0; q < 8; ++q) { s.x += u[q].x; s.y += u[q].y; s.z += u[q].z; s.w += u[q].w; }
     }
-    sb[grp][ch] = s;
+    sb[grp][cl] = s;
     __syncthreads();
     if (grp == 0) {
-        float4 a = sb[0][ch];
-#pragma unroll
-        for (int gi = 1; gi < 8; ++gi) {
-            a.x += sb[gi][ch].x; a.y += sb[gi][ch].y; a.z += sb[gi][ch].z; a.w += sb[gi][ch].w;
+        float4 a = sb[0][cl];
+        for (int gi = 1; gi < G; ++gi) {
+            a.x += sb[gi][cl].x; a.y += sb[gi][cl].y; a.z += sb[gi][cl].z; a.w += sb[gi][cl].w;
         }
         const int K = p.conv_ksize;
         float* dst = (t == 0 ? p.grad_conv_q : t == 1 ? p.grad_conv_k : p.grad_conv_v) + (size_t)(h * 128 + ch) * K;
@@ -722,7 +722,7 @@ cudaError_t launch_bwd_intra(const KdaParams& p, cudaStream_t s) {
     if ((e = launch_dependent(kern, units < sms ? units : sms, bi::NTHR, bi::TOTAL, s, p)) != cudaSuccess) return e;
     if (convb) {
         if ((e = launch_dependent(conv_bwd_fixup_kernel, dim3(p.NT, p.H, 3), 128, 0, s, p)) != cudaSuccess) return e;
-        if ((e = launch_dependent(conv_bwd_reduce_kernel, dim3(p.H, 3), 1024, 0, s, p)) != cudaSuccess) return e;
+        if ((e = launch_dependent(conv_bwd_reduce_kernel, dim3(p.H, 3, 8), 1024, 0, s, p)) != cudaSuccess) return e;
     }
     return cudaGetLastError();
 }

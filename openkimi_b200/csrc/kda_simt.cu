@@ -823,48 +823,47 @@ __global__ void __launch_bounds__(NTHREADS, 1) kda_bwd_chunk_simt(const KdaParam
     }
 }
 
-// deterministic reduction of the per-chunk partial parameter gradients: one block per head,
-// 8 groups of 128 threads each sum every 8th chunk in order, then the 8 group sums are added
-// in a fixed order
+// deterministic reduction of the per-chunk partial parameter gradients: one block per head and 32 channels; 32 groups of
+// 32 threads each sum every 32nd chunk in order, then the group sums are added in a fixed order
 __global__ void __launch_bounds__(1024) kda_param_reduce(const KdaParams p) {
-    __shared__ float sb[8][128];
-    __shared__ float sa[8][32];
+    __shared__ float sb[32][33];
+    __shared__ float sa[32];
     pdl_wait();
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     const char* sc = (const char*)p.bwd_scratch;
-    const int h = blockIdx.x, d = threadIdx.x & 127, grp = threadIdx.x >> 7;
+    const int h = blockIdx.x, lane = threadIdx.x & 31, d = 32 * blockIdx.y + lane, grp = threadIdx.x >> 5;
     const float* pb = (const float*)(sc + L.dbias_part);
     const float* pa = (const float*)(sc + L.dA_part);
     // (sixteen loads in flight per thread, added in chunk order: the loop is a chain of round trips otherwise)
     float s = 0.f;
-    if (d < p.dk)
-        for (int c0 = grp; c0 < p.NT; c0 += 8 * 16) {
-            float v[16];
+    for (int c0 = grp; c0 < p.NT; c0 += 32 * 16) {
+        float v[16];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                const int c = c0 + 8 * u;
-                v[u] = c < p.NT ? pb[((size_t)c * p.H + h) * p.dk + d] : 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < 16; ++u) s += v[u];
+        for (int u = 0; u < 16; ++u) {
+            const int c = c0 + 32 * u;
+            v[u] = c < p.NT ? pb[((size_t)c * p.H + h) * p.dk + d] : 0.f;
         }
-    sb[grp][d] = s;
-    // dA_log: lanes 0..31 of every group take every 32nd of the group's chunks
-    float a = 0.f;
-    if (d < 32)
-        for (int c = grp + 8 * d; c < p.NT; c += 256) a += pa[(size_t)c * p.H + h];
-    if (d < 32) sa[grp][d] = a;
+#pragma unroll
+        for (int u = 0; u < 16; ++u) s += v[u];
+    }
+    sb[grp][lane] = s;
+    if (blockIdx.y == 0) {  // dA_log: thread t takes every 1024th chunk
+        float a = 0.f;
+        for (int c = threadIdx.x; c < p.NT; c += 1024) a += pa[(size_t)c * p.H + h];
+        a = warp_sum(a);
+        if (lane == 0) sa[grp] = a;
+    }
     __syncthreads();
     if (grp == 0) {
-        if (d < p.dk && p.grad_dt_bias) {
+        if (p.grad_dt_bias) {
             float t = 0.f;
-            for (int gidx = 0; gidx < 8; ++gidx) t += sb[gidx][d];
+#pragma unroll
+            for (int g = 0; g < 32; ++g) t += sb[g][lane];
             p.grad_dt_bias[h * p.dk + d] = t;
         }
-        if (d == 0 && p.grad_A_log) {
+        if (blockIdx.y == 0 && lane == 0 && p.grad_A_log) {
             float t = 0.f;
-            for (int gidx = 0; gidx < 8; ++gidx)
-                for (int l = 0; l < 32; ++l) t += sa[gidx][l];
+            for (int g = 0; g < 32; ++g) t += sa[g];
             p.grad_A_log[h] = t;
         }
     }
@@ -901,7 +900,7 @@ static cudaError_t launch_stage(const KdaParams& p, int stage, cudaStream_t s) {
             if ((e = set_smem(kda_bwd_chunk_simt<T, D, true>, smem_bwd_chunk<D>())) != cudaSuccess) return e;
             return launch_dependent(kda_bwd_chunk_simt<T, D, true>, p.NT * p.H, NTHREADS, smem_bwd_chunk<D>(), s, p);
         default:
-            return launch_dependent(kda_param_reduce, p.H, 1024, 0, s, p);
+            return launch_dependent(kda_param_reduce, dim3(p.H, p.dk / 32), 1024, 0, s, p);
     }
 }
 

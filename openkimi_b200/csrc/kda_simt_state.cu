@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(ss::NT, 1) kda_fwd_state_simt(const KdaParams 
     const int e0 = blockIdx.x * BV, h = blockIdx.y, n = blockIdx.z;
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     char* ws = (char*)p.workspace;
-    const bool save = !(p.flags & KDA_FLAG_NO_SAVE);
+    const bool save = !(p.flags & KDA_FLAG_NO_SAVE), with_o = !(p.flags & KDA_FLAG_NO_OUTPUT);
     pdl_wait();
     SeqCursor sq;
     sq.load(p, n);
@@ -203,10 +203,12 @@ __global__ void __launch_bounds__(ss::NT, 1) kda_fwd_state_simt(const KdaParams 
         tc::cp_async_wait<1>();  // Qt, Aqk and Kh of this chunk have landed
         __syncthreads();
         {
-            float acc[8] = {};  // O = Qt S + Aqk V'
-            dots<C, D, BV>(acc, sQt, sS);
-            dots<C, C, BV>(acc, sA, sVn);
-            dots_store<C, BV>(acc, part + M::P4);
+            if (with_o) {
+                float acc[8] = {};  // O = Qt S + Aqk V'
+                dots<C, D, BV>(acc, sQt, sS);
+                dots<C, C, BV>(acc, sA, sVn);
+                dots_store<C, BV>(acc, part + M::P4);
+            }
             float kacc[4][2] = {};  // Kh^T V'
             rows4<D, D, C, BV>(kacc, sKh, sVn);
             rows4_store<D, BV>(kacc, part);
@@ -214,7 +216,7 @@ __global__ void __launch_bounds__(ss::NT, 1) kda_fwd_state_simt(const KdaParams 
         __syncthreads();
         if (more) get_q(c + 1);
         else tc::cp_async_commit();
-        if (ui < sq.rows(c)) {
+        if (with_o && ui < sq.rows(c)) {
             T* o = (T*)p.o + ((size_t)(sq.tok(c) + ui) * p.H + h) * D + e0 + uc;
 #pragma unroll
             for (int j = 0; j < BV / 4; ++j) stf(o + j, part_sum<C, BV, dots_groups<C, BV>()>(part + M::P4, ui * BV + uc + j));
