@@ -32,10 +32,12 @@ inline int sm_count() {
     return n;
 }
 
-// The kernels of a call follow one another in the stream as programmatic dependents: the next kernel's CTAs are placed as
-// SMs come free and set themselves up (barriers, tensor memory) while the last CTAs of the one before still run.
+// The kernels of a call follow one another in the stream as programmatic dependents: a kernel is launched, and sets itself
+// up (barriers, tensor memory), as soon as the last CTA of the one before has exited, ahead of the end of that grid.
 // pdl_wait() returns when that kernel, and through it every earlier one, has completed and its writes are visible: every
 // kernel launched with launch_dependent() calls it before its first access to global memory, in every thread.
+// No kernel triggers its successor earlier: with CTAs of the next grid placed as single SMs came free the large kernels
+// lost 2 us each.  Ten kernels of one 2047-token sequence: 210 -> 190 us; 16 x 2048 tokens: 1011 -> 996 us.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class... P, class... A>
 inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {

@@ -14,6 +14,9 @@
 //   * [dv][dk] states: a lane holds four consecutive key channels of every column (a row is one 512-byte line);
 //   * [dk][dv] states: a lane holds four consecutive value columns at every (128 / lanes)th key channel.
 // The tokens' prologue (L2 norm, gate, sigmoid) is evaluated once per CTA, a warp per token, into shared memory.
+//
+// 1536 units, one token: 48.2 us with the state in shared memory -> 36.1 us, 5.6 TB/s; one sequence of six heads:
+// 6.6 -> 3.6 us; eight tokens of four sequences: eight launches of 7 us -> 7.0 us.
 #include "kda_common.cuh"
 
 namespace kda {
@@ -278,7 +281,8 @@ static cudaError_t launch_recurrent(const RecurrentArgs& a, cudaStream_t s) {
 }
 
 // Columns per warp: eight (D / 32 CTAs per unit, short dependent chains per token) until the CTAs fill the chip twice
-// over, then sixteen (half as many CTAs evaluate the same token's prologue).
+// over, then sixteen (half as many CTAs evaluate the same token's prologue; 36.3 against 36.1 us at 1536 units, so the
+// line could lie anywhere above it).
 template <typename T, int D>
 static cudaError_t launch_columns(const RecurrentArgs& a, cudaStream_t s) {
     const bool vf = a.flags & KDA_FLAG_STATE_V_FIRST;

@@ -13,6 +13,10 @@
 // X carries the same BF16 operands and FP32 accumulators as the state itself; step 2 rounds nothing.  The backward
 // walks the other way with X^T.  Work doubles (and X costs as much again, on warps that would idle), the chain shrinks
 // from n chunks to 2 len + n / len short steps.
+//
+// Measured (six heads): one sequence of 256 chunks, forward, 24 segments: 498 -> 32 + 32 + 28 us (at 148 busy SMs the walks
+// are bound by the records' traffic, 5.5 TB/s); 16 documents of 65536 tokens, both directions: 838 -> 520 us; 4 sequences
+// of 64 chunks: 454 -> 237 us.
 #include <math.h>
 
 #include <algorithm>
@@ -193,7 +197,8 @@ __global__ void __launch_bounds__(sg::NTHR, 1) kda_fwd_segment_tc(const KdaParam
 
 // Step 2.  One CTA per (sequence, head, eight rows of S^T): E of every segment that a sequence leaves becomes the true
 // state there.  Thread = two columns x a quarter of the inner index, in packed FP32 pairs; X arrives by bulk copies (64 KB
-// per step and CTA from L2, as long as the arithmetic).  Latency bound: with STAGES = 2 a CTA has the next segment's X in
+// per step and CTA from L2, as long as the arithmetic); 1.3 us a step, twice that with sixteen rows per CTA and no less
+// with 512 threads.  Latency bound: with STAGES = 2 a CTA has the next segment's X in
 // flight, with STAGES = 1 two CTAs share an SM (more chains than one CTA per SM covers).
 namespace sc {
 constexpr int D = 128, ROWS = 8, NTHR = 256, GROUPS = NTHR / 64, OWN = D * ROWS / NTHR;
