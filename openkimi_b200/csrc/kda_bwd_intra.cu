@@ -59,14 +59,18 @@ constexpr uint32_t SSCR = STOT + 2048;       // f32 [4][128]
 constexpr uint32_t SRED = SSCR + 2048;       // f32 [16]
 constexpr uint32_t SREJ = SRED + 64;         // int [4][4]: tile (block, channel group) rejected
 constexpr uint32_t FD = SREJ + 64;           // f32 [2][4][16][16] diagonal blocks of dAqk, dM rebuilt for rejected tiles
-constexpr uint32_t TOTAL = FD + 8192;
+constexpr uint32_t SAUX2 = FD + 8192;        // the aux record of every other unit (requests ahead, CONVB)
+constexpr uint32_t TOTAL = SAUX2 + 768;
+static_assert(TOTAL <= 232448, "shared memory of a CTA");
 // later uses of the dead operand space
 constexpr uint32_t PF = YB;                  // bf16 [3][64][128]: dQt, dKh, dKb (after the MMAs that read Y)
 constexpr uint32_t STG = SB;                 // f32 [3][64][128] staging of dq, dk, dbeta terms over SB and X (after all MMAs)
 // fused short-convolution backward (CONVB): once their first users are done, Y holds the pre-convolution q and
-// k rows -3 .. 63 (bf16 [67][128] each), the G tile holds dq and dk of the convolved rows (bf16 [64][128] each)
-// and the staging area the four blocks' filter-gradient shares
-constexpr uint32_t CXQ = YB, CXK = YB + 67 * 256, CTAPS = CXK + 67 * 256, CDY = SG, CDW = STG;  // CTAPS: f32 [2][128][4] padded filter taps
+// k rows -3 .. 63 (bf16 [67][128] each), and the staging area dq and dk of the convolved rows (bf16, every row in the
+// first half of the FP32 row it was made from) and the four blocks' filter-gradient shares
+constexpr uint32_t CXQ = YB, CXK = YB + 67 * 256, CTAPS = CXK + 67 * 256;  // CTAPS: f32 [2][128][4] padded filter taps
+constexpr uint32_t CDYQ = STG, CDYK = STG + 64 * 128 * 4, CDW = STG + 2 * 64 * 128 * 4;
+constexpr int CDS = 256;                     // row stride of dq, dk in elements
 static_assert(CTAPS + 2 * 128 * 16 <= YB + 49152, "the projection rows and the taps share the Y buffer");
 constexpr uint32_t TMEM_COLS = 512;
 // The midpoint factors reach 2^(+-span/2) and the third BF16 part of an operand sits 2^-16 below its
@@ -107,9 +111,6 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     const __nv_bfloat16* sB = reinterpret_cast<const __nv_bfloat16*>(dyn + SB);
     float* stg = reinterpret_cast<float*>(dyn + STG);
     const __nv_bfloat16* spf = reinterpret_cast<const __nv_bfloat16*>(dyn + PF);
-    float* srq = reinterpret_cast<float*>(dyn + SAUX);  // aux record order: 1/|q|, 1/|k|, beta
-    float* srk = srq + 64;
-    float* sbeta = srq + 128;
     float* sdb = reinterpret_cast<float*>(dyn + SDB);
     float* sdiag = reinterpret_cast<float*>(dyn + SDIAG);
     float* smid = reinterpret_cast<float*>(dyn + SMID);
@@ -151,12 +152,32 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     // The CTA walks the units blockIdx.x, blockIdx.x + gridDim.x, ...: tensor memory, barriers and the CTA itself
     // are set up once.  Unit u = (chunk u / H, head (u + chunk) % H), so that the units of one CTA cycle through
     // all heads whatever the stride (heads differ in cost: rejected tiles take the exact path).
+    // What the operands are built from: G, the normalised q and k, the row norms and beta kept by the forward.  With the
+    // convolution fused, the NEXT unit's are requested as soon as this one has them in registers or is done with them, a
+    // third of a unit ahead (1667 -> 1595 us at 12288 units; without the convolution that third is too short for the
+    // copies to land, and the registers it takes cost more than it gives: 335 -> 341 us at 3072 units).
+    constexpr bool AHEAD = CONVB;
+    auto request_A = [&](size_t r, bool second) {
+        const char* ws = (const char*)p.workspace;
+        mbar_expect_tx(&barA, C * D * 4 + 2 * C * D * 2 + 3 * C * 4);
+        tma_load_1d(dyn + SG, (const float*)(ws + L.Gc) + r * C * D, C * D * 4, &barA);
+        tma_load_1d(dyn + SQ, (const __nv_bfloat16*)(ws + L.Qn) + r * C * D, C * D * 2, &barA);
+        tma_load_1d(dyn + SK, (const __nv_bfloat16*)(ws + L.Kn) + r * C * D, C * D * 2, &barA);
+        tma_load_1d(dyn + (second ? SAUX2 : SAUX), (const float*)(ws + L.aux) + r * 3 * C, 3 * C * 4, &barA);
+    };
     const int n_units = p.NT * p.H;
+    bool ok = true, ahead = false;
     uint32_t it = 0;
     UnitWalk uw;
     uw.init(blockIdx.x, gridDim.x, p.H);
     for (; uw.unit < n_units; uw.next(), ++it) {
     const uint32_t par = it & 1;
+    const float* srq = reinterpret_cast<const float*>(dyn + (AHEAD && par ? SAUX2 : SAUX));  // aux record order: 1/|q|, 1/|k|, beta
+    const float* srk = srq + 64;
+    const float* sbeta = srq + 128;
+    UnitWalk un = uw;  // the next unit of this CTA (without the requests ahead it is worked out where the hints need it)
+    if constexpr (AHEAD) un.next();
+    ahead = false;
     const int c = uw.c, hd = uw.head();
     const ChunkInfo ci = chunk_info(p, c);
     const size_t rec = (size_t)c * p.H + hd;
@@ -167,19 +188,14 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     //      dAqk / dM tiles and the diagonal of dAqk from bwd_wy; the three [64][128] hand-over arrays
     //      that only the assembly needs follow on barH once an operand buffer is free
     if (tid == 0) {
-        const char* ws = (const char*)p.workspace;
-        mbar_expect_tx(&barA, C * D * 4 + 2 * C * D * 2 + 3 * C * 4);
-        tma_load_1d(dyn + SG, (const float*)(ws + L.Gc) + rec * C * D, C * D * 4, &barA);
-        tma_load_1d(dyn + SQ, (const __nv_bfloat16*)(ws + L.Qn) + rec * C * D, C * D * 2, &barA);
-        tma_load_1d(dyn + SK, (const __nv_bfloat16*)(ws + L.Kn) + rec * C * D, C * D * 2, &barA);
-        tma_load_1d(srq, (const float*)(ws + L.aux) + rec * 3 * C, 3 * C * 4, &barA);  // 1/|q|, 1/|k|, beta
+        if (!AHEAD || it == 0) request_A(rec, false);
         mbar_expect_tx(&barB, 6 * C * C * 2 + C * 4);
         tma_load_1d(dyn + SB, (const __nv_bfloat16*)(sc + L.dAM) + rec * 6 * C * C, 6 * C * C * 2, &barB);
         tma_load_1d(sdiag, (const float*)(sc + L.dAd) + rec * C, C * 4, &barB);
     }
     if (tid < C) sdb[tid] = ((const float*)(sc + L.dbp))[rec * C + tid];
     const float carry_in = ((const float*)(sc + L.gC))[rec * D + d];
-    bool ok = mbar_wait(&barA, par, p, 64);
+    ok = mbar_wait(&barA, par, p, 64);
     KDA_PHASE(0);
 
     // ---- my block: G of my channel, guard and references; operand step 1: KN_j = k_j 2^(ref - G_j) -> X
@@ -336,8 +352,10 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     // The next unit of this CTA finds what it needs first in L2: the hints go out here, in the middle of the unit,
     // when the copy unit has nothing else to do (there is no shared memory left to receive the records themselves).
     if (tid == 5 * 32) {
-        UnitWalk un = uw;
-        un.next();
+        if constexpr (!AHEAD) {
+            un = uw;
+            un.next();
+        }
         if (un.unit < n_units) {
             const char* ws = (const char*)p.workspace;
             const size_t rn = un.rec();
@@ -449,7 +467,23 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
             sscr[blk * D + d] = tail;
         }
         KDA_PHASE(9);
+        const int c4 = (tid & 15) * 4;
+        uint2 qrow[2][2], krow[2][2];  // q^ and k^ of the two rows this half warp finishes below
+        if constexpr (AHEAD) {
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    qrow[m][hf] = *reinterpret_cast<const uint2*>(sQ + swz_bf16((tid >> 4) + 32 * m, 64 * hf + c4));
+                    krow[m][hf] = *reinterpret_cast<const uint2*>(sK + swz_bf16((tid >> 4) + 32 * m, 64 * hf + c4));
+                }
+            fence_async_smem();
+        }
         __syncthreads();
+        if constexpr (AHEAD) {
+            ahead = un.unit < n_units;
+            if (ahead && tid == NTHR - 32) request_A(un.rec(), par == 0);
+        }
         KDA_PHASE(10);
         if constexpr (CONVB) {  // the hand-over arrays in Y are dead: fetch the projection rows the convolution backward needs
             const __nv_bfloat16* xq = (const __nv_bfloat16*)p.q;
@@ -500,7 +534,6 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
         {
             __nv_bfloat16* dq_out = (__nv_bfloat16*)p.grad_q;
             __nv_bfloat16* dk_out = (__nv_bfloat16*)p.grad_k;
-            const int c4 = (tid & 15) * 4;
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 const int ii = (tid >> 4) + 32 * m;
@@ -511,8 +544,8 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
                     const float4 a = *reinterpret_cast<const float4*>(stg + (0 * C + ii) * D + ch);
                     const float4 b = *reinterpret_cast<const float4*>(stg + (1 * C + ii) * D + ch);
                     const float4 e = *reinterpret_cast<const float4*>(stg + (2 * C + ii) * D + ch);
-                    const uint2 qu = *reinterpret_cast<const uint2*>(sQ + swz_bf16(ii, ch));
-                    const uint2 ku = *reinterpret_cast<const uint2*>(sK + swz_bf16(ii, ch));
+                    const uint2 qu = AHEAD ? qrow[m][hf] : *reinterpret_cast<const uint2*>(sQ + swz_bf16(ii, ch));
+                    const uint2 ku = AHEAD ? krow[m][hf] : *reinterpret_cast<const uint2*>(sK + swz_bf16(ii, ch));
                     const float2 q01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qu.x));
                     const float2 q23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qu.y));
                     const float2 k01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ku.x));
@@ -540,15 +573,16 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
                     }
                 }
                 if constexpr (CONVB) {  // rows of the convolved tensors' gradients stay on chip (zero past the end)
-                    __nv_bfloat16* sdyq = reinterpret_cast<__nv_bfloat16*>(dyn + CDY);
-                    __nv_bfloat16* sdyk = sdyq + C * D;
+                    __nv_bfloat16* sdyq = reinterpret_cast<__nv_bfloat16*>(dyn + CDYQ);
+                    __nv_bfloat16* sdyk = reinterpret_cast<__nv_bfloat16*>(dyn + CDYK);
                     const bool valid = ii < ci.len;
+                    __syncwarp();  // every lane has read its part of the staged rows that are overwritten here
 #pragma unroll
                     for (int hf = 0; hf < 2; ++hf) {
-                        *reinterpret_cast<uint2*>(sdyq + ii * D + 64 * hf + c4) =
+                        *reinterpret_cast<uint2*>(sdyq + ii * CDS + 64 * hf + c4) =
                             valid ? make_uint2(pack_bf16(dq8[4 * hf], dq8[4 * hf + 1]), pack_bf16(dq8[4 * hf + 2], dq8[4 * hf + 3]))
                                   : make_uint2(0u, 0u);
-                        *reinterpret_cast<uint2*>(sdyk + ii * D + 64 * hf + c4) =
+                        *reinterpret_cast<uint2*>(sdyk + ii * CDS + 64 * hf + c4) =
                             valid ? make_uint2(pack_bf16(dk8[4 * hf], dk8[4 * hf + 1]), pack_bf16(dk8[4 * hf + 2], dk8[4 * hf + 3]))
                                   : make_uint2(0u, 0u);
                     }
@@ -580,8 +614,8 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
             __syncthreads();  // the projection rows have landed, dq / dk of the convolved rows are complete
             const __nv_bfloat16* sxq = reinterpret_cast<const __nv_bfloat16*>(dyn + CXQ);
             const __nv_bfloat16* sxk = reinterpret_cast<const __nv_bfloat16*>(dyn + CXK);
-            __nv_bfloat16* sdyq = reinterpret_cast<__nv_bfloat16*>(dyn + CDY);
-            __nv_bfloat16* sdyk = sdyq + C * D;
+            __nv_bfloat16* sdyq = reinterpret_cast<__nv_bfloat16*>(dyn + CDYQ);
+            __nv_bfloat16* sdyk = reinterpret_cast<__nv_bfloat16*>(dyn + CDYK);
             float* sdw = reinterpret_cast<float*>(dyn + CDW);  // [2][4][128][4]
             int c0s, ncs;
             seq_chunks(p, ci.seq, c0s, ncs);
@@ -594,15 +628,15 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
             }
             float* cvh = (float*)(sc + L.cv_head) + (rec * 3 * 3) * D;
             float* cvt = (float*)(sc + L.cv_tail) + (rec * 3 * 3) * D;
-            conv_bwd_block(sxq, sxq + 3 * D, sdyq, wq, d, blk, cvh, cvt, dwq, oq);
-            conv_bwd_block(sxk, sxk + 3 * D, sdyk, wk, d, blk, cvh + 3 * D, cvt + 3 * D, dwk, ok_);
+            conv_bwd_block<CDS>(sxq, sxq + 3 * D, sdyq, wq, d, blk, cvh, cvt, dwq, oq);
+            conv_bwd_block<CDS>(sxk, sxk + 3 * D, sdyk, wk, d, blk, cvh + 3 * D, cvt + 3 * D, dwk, ok_);
             *reinterpret_cast<float4*>(sdw + (blk * D + d) * 4) = make_float4(dwq[0], dwq[1], dwq[2], dwq[3]);
             *reinterpret_cast<float4*>(sdw + ((4 + blk) * D + d) * 4) = make_float4(dwk[0], dwk[1], dwk[2], dwk[3]);
             __syncthreads();  // every read of dy is done, the filter-gradient shares are visible
 #pragma unroll
             for (int r = 0; r < B; ++r) {
-                sdyq[(b0 + r) * D + d] = __float2bfloat16_rn(oq[r]);
-                sdyk[(b0 + r) * D + d] = __float2bfloat16_rn(ok_[r]);
+                sdyq[(b0 + r) * CDS + d] = __float2bfloat16_rn(oq[r]);
+                sdyk[(b0 + r) * CDS + d] = __float2bfloat16_rn(ok_[r]);
             }
             if (blk < 2) {  // block 0 threads reduce the q filter, block 1 threads the k filter (fixed order)
                 const float* src = sdw + (4 * blk * D + d) * 4;
@@ -623,8 +657,8 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
                 const int ii = (tid >> 4) + 32 * m, e8 = (tid & 15) * 8;
                 if (ii < lim) {
                     const size_t row = tok(ii);
-                    *reinterpret_cast<uint4*>(dq_o + row * D + e8) = *reinterpret_cast<const uint4*>(sdyq + ii * D + e8);
-                    *reinterpret_cast<uint4*>(dk_o + row * D + e8) = *reinterpret_cast<const uint4*>(sdyk + ii * D + e8);
+                    *reinterpret_cast<uint4*>(dq_o + row * D + e8) = *reinterpret_cast<const uint4*>(sdyq + ii * CDS + e8);
+                    *reinterpret_cast<uint4*>(dk_o + row * D + e8) = *reinterpret_cast<const uint4*>(sdyk + ii * CDS + e8);
                 }
             }
         }
@@ -647,6 +681,7 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     ok = __syncthreads_and(ok);
     if (!ok) break;  // a wait gave up (recorded in the status word): no further unit is started
     }
+    if (!ok && ahead) mbar_wait(&barA, (it + 1) & 1, p, 64);  // the next unit's copies are in flight
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem0, TMEM_COLS);

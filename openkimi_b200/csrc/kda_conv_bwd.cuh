@@ -23,11 +23,12 @@ __device__ __forceinline__ float dsilu_f(float x) {
 // Thread = (channel ch, 16-row block blk) of a 512-thread CTA.
 //   sxh  [3][128] BF16: rows -3 .. -1 of the pre-convolution tensor, sx [64][128]: rows 0 .. 63 (zero where a
 //        row does not exist); the two may be one [67][128] array (sx = sxh + 3 * 128)
-//   sdy  [64][128] BF16: gradient of the convolved rows (zero past the end of a partial chunk)
+//   sdy  [64][128] BF16, rows SD elements apart: gradient of the convolved rows (zero past the end of a partial chunk)
 //   w    the four padded taps of this channel
 // Returns dx of the block's 16 rows in out[] (rows 61..63 are incomplete when the chunk has a
 // successor), adds the block's share of dw, and hands dpre of rows 0..2 / 61..63 to head / tail
 // ([3][128] FP32 each, written by block 0 / block 3).
+template <int SD = 128>
 __device__ __forceinline__ void conv_bwd_block(const __nv_bfloat16* __restrict__ sxh, const __nv_bfloat16* __restrict__ sx,
                                                const __nv_bfloat16* __restrict__ sdy,
                                                const float (&w)[4], int ch, int blk, float* __restrict__ head,
@@ -39,7 +40,7 @@ __device__ __forceinline__ void conv_bwd_block(const __nv_bfloat16* __restrict__
     for (int sI = 0; sI < 19; ++sI) {
         const int s = b0 + sI;
         const bool in = s < 64;  // rows of the next chunk: their dpre arrives through the fix-up
-        const float xd = in ? X(in ? s : 0) : 0.f, gy = in ? __bfloat162float(sdy[(in ? s : 0) * 128 + ch]) : 0.f;
+        const float xd = in ? X(in ? s : 0) : 0.f, gy = in ? __bfloat162float(sdy[(in ? s : 0) * SD + ch]) : 0.f;
         const float pd = gy * dsilu_f(conv_pre(w[0], w[1], w[2], w[3], xa, xb, xc, xd));
         if (sI < 16) {
             dw[0] = fmaf(pd, xa, dw[0]);
