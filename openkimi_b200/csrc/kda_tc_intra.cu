@@ -14,8 +14,8 @@
 //      the factorised operands  k_j 2^(r_I - G_j) (j < 16 I)  and  x_i 2^(G_i - r_I) (i in I),
 //      r_I = G at the first row of block I, so that every exponent is <= 0; off-diagonal blocks of
 //      Aqk and L as tcgen05 MMAs (M = 64 keys, N = 32 = q and k rows of block I, K = 128)
-//   3  T = (I + diag(beta) L)^-1: forward substitution inside the diagonal blocks, block
-//      forward substitution for the rest (FP32)
+//   3  T = (I + diag(beta) L)^-1: forward substitution inside the diagonal blocks, products for the
+//      rest (FP32)
 //   4  Aqk and T records; 5  W^T = (beta k 2^G)^T T^T and U^T = (beta v)^T T^T as tcgen05 MMAs
 //      (M = 128 channels); 6  W, U, gamC records.
 #include "kda_common.cuh"
@@ -49,92 +49,100 @@ constexpr uint32_t T_D = 0, T_W = 96, T_U = 160, TMEM_COLS = 256;
 }  // namespace fi
 using fi::LDR;
 
-// One block column J of T = (I + diag(beta) L)^-1 (see stage 3 of the kernel).  sL holds L
-// (strictly lower, row stride LDR: rows start on 16-byte boundaries and are read four floats at a time), sT
-// receives T; sT must be zero above the diagonal blocks.
-// Eight warps work (the column solve is a dependent chain: more lanes only add redundancy):
-// warp (J, cw) owns columns 8 cw + lane % 8 of block column J, and its four lane groups (lane / 8)
-// split the 16 rows of every block below the diagonal, four rows each.
-// J is uniform over the warp; the loops run over all blocks with warp-uniform skips so that the
-// register arrays keep compile-time indices in a single copy of the code.
-__device__ __forceinline__ void solve_block_column(const float* sL, float* sT, const float* sbeta, int J, int cw, int lane,
-                                                   bool active) {
-    if (!active) {
-        __syncthreads();  // (matches the barrier below)
-        return;
-    }
-    const int col = 8 * cw + (lane & 7), rq = lane >> 3, gc = 16 * J + col;
-    float t[4][16];
-    // diagonal block: forward substitution down the column (every lane group does all 16 rows)
+// T = (I + diag(beta) L)^-1 by blocks, FP32.  sL holds L (strictly lower), sT receives T (zero above the diagonal blocks on
+// entry); both have rows of LDR floats on 16-byte boundaries.  The four 16 x 16 diagonal blocks are inverted by forward
+// substitution, one warp each (one per scheduler: a dependent chain of 16 rows, lane = column); everything below them is
+// products on all 16 warps: T_ba = -T_bb (beta L)_ba T_aa for the block pairs (0, 1) and (2, 3), then the same with 32 x 32
+// halves.  A thread's tile is 2 x 2 with the inner index split over neighbouring lanes; sY (32 rows of LDY floats) takes
+// the inner products between two barriers.  (One column after the other down all blocks, on eight warps, was a chain three
+// block levels long: 2.6 us of a unit's 15.5.)
+constexpr int LDY = 36;
+
+// acc[2][2] over `K4` groups of four inner elements: rows of A (float4 along k), rows k of B (two columns)
+template <int K4>
+__device__ __forceinline__ void tile22(float (&acc)[2][2], const float* A0, const float* A1, const float* B, int ldb, int kstep) {
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
-        const float* lrow = sL + (16 * J + r) * LDR + 16 * J;
-        float s0 = 0.f, s1 = 0.f;
+    for (int m = 0; m < K4; ++m) {
+        const float4 a0 = *reinterpret_cast<const float4*>(A0 + m * kstep), a1 = *reinterpret_cast<const float4*>(A1 + m * kstep);
+        const float x0[4] = {a0.x, a0.y, a0.z, a0.w}, x1[4] = {a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-        for (int j = 0; j < r; j += 4) {
-            const float4 l = *reinterpret_cast<const float4*>(lrow + j);
-            s0 = fmaf(l.x, t[0][j], s0);
-            if (j + 1 < r) s1 = fmaf(l.y, t[0][j + 1], s1);
-            if (j + 2 < r) s0 = fmaf(l.z, t[0][j + 2], s0);
-            if (j + 3 < r) s1 = fmaf(l.w, t[0][j + 3], s1);
+        for (int j = 0; j < 4; ++j) {
+            const float2 b = *reinterpret_cast<const float2*>(B + (m * kstep + j) * ldb);
+            acc[0][0] = fmaf(x0[j], b.x, acc[0][0]);
+            acc[0][1] = fmaf(x0[j], b.y, acc[0][1]);
+            acc[1][0] = fmaf(x1[j], b.x, acc[1][0]);
+            acc[1][1] = fmaf(x1[j], b.y, acc[1][1]);
         }
-        t[0][r] = (r == col ? 1.f : 0.f) - sbeta[16 * J + r] * (s0 + s1);
-        if (r < col) t[0][r] = 0.f;
     }
-    if (rq == 0) {
+}
+template <int LANES>
+__device__ __forceinline__ void sum22(float (&acc)[2][2]) {
 #pragma unroll
-        for (int r = 0; r < 16; ++r) sT[(16 * J + r) * LDR + gc] = t[0][r];
-    }
-    __syncthreads();  // every diagonal block of T is in shared memory
-    // t[n] is the column restricted to block J + n.  Lane group rq owns rows rq, rq + 4, rq + 8, rq + 12 of a
-    // block: the four rows one load instruction touches are adjacent, LDR floats apart, in four different banks.
+    for (int o = 1; o < LANES; o <<= 1)
 #pragma unroll
-    for (int n = 1; n < 4; ++n) {
-        const int I = J + n;
-        if (I > 3) break;
-        // y = sum_K (beta L)_IK t_K for my four rows, then all 16 entries from the lane groups
-        float y4[4], y[16];
+        for (int i = 0; i < 4; ++i) acc[i >> 1][i & 1] += __shfl_xor_sync(0xffffffffu, acc[i >> 1][i & 1], o);
+}
+
+__device__ __forceinline__ void invert_blocks(const float* sL, float* sT, const float* sbeta, float* sY, int tid) {
+    const int warp = tid >> 5, lane = tid & 31;
+    if (warp < 4) {
+        const int col = lane & 15;
+        float t[16];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int r = 16 * I + rq + 4 * q;
-            float s = 0.f;
+        for (int r = 0; r < 16; ++r) {
+            const float* lrow = sL + (16 * warp + r) * LDR + 16 * warp;
+            float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-            for (int kn = 0; kn < n; ++kn)
-#pragma unroll
-                for (int m = 0; m < 16; m += 4) {
-                    const float4 l = *reinterpret_cast<const float4*>(sL + r * LDR + 16 * (J + kn) + m);
-                    s = fmaf(l.x, t[kn][m], s);
-                    s = fmaf(l.y, t[kn][m + 1], s);
-                    s = fmaf(l.z, t[kn][m + 2], s);
-                    s = fmaf(l.w, t[kn][m + 3], s);
-                }
-            y4[q] = sbeta[r] * s;
-        }
-#pragma unroll
-        for (int g4 = 0; g4 < 4; ++g4)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) y[g4 + 4 * q] = __shfl_sync(0xffffffffu, y4[q], (lane & 7) + 8 * g4);
-        // t_I = -T_II y for my four rows, shared the same way
-        float n4[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int r = 16 * I + rq + 4 * q;
-            float s = 0.f;
-#pragma unroll
-            for (int m = 0; m < 16; m += 4) {
-                const float4 l = *reinterpret_cast<const float4*>(sT + r * LDR + 16 * I + m);
-                s = fmaf(l.x, y[m], s);
-                s = fmaf(l.y, y[m + 1], s);
-                s = fmaf(l.z, y[m + 2], s);
-                s = fmaf(l.w, y[m + 3], s);
+            for (int j = 0; j < r; j += 4) {
+                const float4 l = *reinterpret_cast<const float4*>(lrow + j);
+                s0 = fmaf(l.x, t[j], s0);
+                if (j + 1 < r) s1 = fmaf(l.y, t[j + 1], s1);
+                if (j + 2 < r) s0 = fmaf(l.z, t[j + 2], s0);
+                if (j + 3 < r) s1 = fmaf(l.w, t[j + 3], s1);
             }
-            n4[q] = -s;
-            sT[r * LDR + gc] = -s;
+            t[r] = (r == col ? 1.f : 0.f) - sbeta[16 * warp + r] * (s0 + s1);
+            if (r < col) t[r] = 0.f;
         }
+        if (lane < 16) {
 #pragma unroll
-        for (int g4 = 0; g4 < 4; ++g4)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) t[n][g4 + 4 * q] = __shfl_sync(0xffffffffu, n4[q], (lane & 7) + 8 * g4);
+            for (int r = 0; r < 16; ++r) sT[(16 * warp + r) * LDR + 16 * warp + col] = t[r];
+        }
+    }
+    __syncthreads();
+    {   // pairs of 16 x 16 blocks: eight warps each, inner index over four lanes
+        const int pr = tid >> 8, a = 32 * pr, b = a + 16, r0 = 2 * (warp & 7), c0 = 2 * (lane >> 2), k0 = 4 * (lane & 3);
+        float acc[2][2] = {};
+        tile22<1>(acc, sL + (b + r0) * LDR + a + k0, sL + (b + r0 + 1) * LDR + a + k0, sT + (a + k0) * LDR + a + c0, LDR, 0);
+        sum22<4>(acc);
+        if ((lane & 3) < 2) {
+            const int i = lane & 1;
+            const float be = sbeta[b + r0 + i];
+            *reinterpret_cast<float2*>(sY + (16 * pr + r0 + i) * LDY + c0) =
+                make_float2(be * (i ? acc[1][0] : acc[0][0]), be * (i ? acc[1][1] : acc[0][1]));
+        }
+        __syncthreads();
+        acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = 0.f;
+        tile22<1>(acc, sT + (b + r0) * LDR + b + k0, sT + (b + r0 + 1) * LDR + b + k0, sY + (16 * pr + k0) * LDY + c0, LDY, 0);
+        sum22<4>(acc);
+        if ((lane & 3) < 2) {
+            const int i = lane & 1;
+            *reinterpret_cast<float2*>(sT + (b + r0 + i) * LDR + a + c0) =
+                make_float2(-(i ? acc[1][0] : acc[0][0]), -(i ? acc[1][1] : acc[0][1]));
+        }
+        __syncthreads();
+    }
+    {   // the 32 x 32 halves: a warp has two rows, inner index over two lanes (alternating groups of four)
+        const int r0 = 2 * warp, c0 = 2 * (lane >> 1), k0 = 4 * (lane & 1), i = lane & 1;
+        float acc[2][2] = {};
+        tile22<4>(acc, sL + (32 + r0) * LDR + k0, sL + (33 + r0) * LDR + k0, sT + k0 * LDR + c0, LDR, 8);
+        sum22<2>(acc);
+        const float be = sbeta[32 + r0 + i];
+        *reinterpret_cast<float2*>(sY + (r0 + i) * LDY + c0) = make_float2(be * (i ? acc[1][0] : acc[0][0]), be * (i ? acc[1][1] : acc[0][1]));
+        __syncthreads();
+        acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = 0.f;
+        tile22<4>(acc, sT + (32 + r0) * LDR + 32 + k0, sT + (33 + r0) * LDR + 32 + k0, sY + k0 * LDY + c0, LDY, 8);
+        sum22<2>(acc);
+        *reinterpret_cast<float2*>(sT + (32 + r0 + i) * LDR + c0) = make_float2(-(i ? acc[1][0] : acc[0][0]), -(i ? acc[1][1] : acc[0][1]));
     }
 }
 
@@ -233,7 +241,7 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
     const bool tiles = maps.ok != 0;  // whole [64 x 128] tiles with one bulk-tensor copy each (full chunks only)
     auto row_src = [&](const __nv_bfloat16* base, const ChunkInfo& ci, int h, int i) { return base + ((size_t)(ci.tok0 + i) * p.H + h) * D; };
     auto request_rows = [&](const ChunkInfo& ci, int h) {  // gate, q, k (and every halo row)
-        // (issued from the last warp, which has no share in the column solve that follows the in-loop request: the
+        // (issued from the last warp, which has no diagonal block to invert after the in-loop request: the
         //  issuing warp is held up while the copy unit works through its requests)
         if (tid == NTHR - 32) mbar_expect_tx(&rowbar, (uint32_t)(3 * ci.len + ((CONV && ci.lc > 0) ? 9 : 0)) * 256u);
         if (tiles && ci.len == C) {
@@ -445,7 +453,7 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
     tc_fence_after();
     // A and T must read zero above the diagonal: the stages below write A for j <= i only and T from the diagonal
     // block down, and the records carry whole 64 x 64 tiles.  Row i is cleared from its diagonal block on, four
-    // floats at a time.  (L needs no clearing: the solve reads its diagonal blocks for j < i only, which the
+    // floats at a time.  (L needs no clearing: the solve uses its diagonal blocks for j < i only, which the
     // diagonal walks write, and the blocks below them whole, which the accumulator read-back writes.)
 #pragma unroll
     for (int idx = tid; idx < C * 16; idx += NTHR) {
@@ -747,7 +755,7 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
     KDA_PHASE(12);
     tc_fence_before();
     __syncthreads();
-    if (more) {  // the operand tiles of the off-diagonal products are dead; the scalars have the whole solve to arrive
+    if (more) {  // the operand tiles of the off-diagonal products are dead; the scalars have the inversion to arrive
         ci_nx = chunk_info(p, un.c);
         request_rows(ci_nx, un.head());
         request_scalars(ci_nx, un.head(), nx);
@@ -757,7 +765,7 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
     KDA_PHASE(5);
     // (issued here rather than before the operand stage, whose shared-memory traffic they would share)
     if (tid == NTHR - 64 && save) {  // prologue results for the backward: bulk stores straight from shared memory, issued by a
-                                     // thread of a warp that has no share in the solve
+                                     // thread of a warp that has no diagonal block to invert
         tma_store_1d((float*)(ws + L.Gc) + rec * C * D, sG, C * D * 4);
         tma_store_1d((__nv_bfloat16*)(ws + L.Qn) + rec * C * D, sQ, C * D * 2);
         tma_store_1d((__nv_bfloat16*)(ws + L.Kn) + rec * C * D, sK, C * D * 2);
@@ -765,12 +773,8 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
         tma_store_commit();
     }
 
-    // ---- 3: T = (I + diag(beta) L)^-1, column by column.  Column c of T depends only on
-    //      column c of the blocks above it, so one lane carries a whole column in registers:
-    //      warp w < 8 owns columns 8 (w / 4) + lane % 8 of block column J = w % 4 (w < 4) or 3 - w % 4 (w >= 4),
-    //      and its four lane groups (lane / 8) split the 16 rows of every block below the diagonal.  Warps w and
-    //      w + 4 issue from the same scheduler: with J and 3 - J they bring it 3 block levels whatever J is.
-    solve_block_column(sL, sT, sbeta, (warp & 4) ? 3 - (warp & 3) : (warp & 3), (warp >> 2) & 1, lane, warp < 8);
+    // ---- 3: T = (I + diag(beta) L)^-1; the inner products pass through the space behind T's operand tile
+    invert_blocks(sL, sT, sbeta, reinterpret_cast<float*>(dyn + KSC + 8192), tid);
     fence_async_smem();
     __syncthreads();
     if (more) request_v(ci_nx, un.head());  // L is dead: its tile receives the next unit's v rows
