@@ -108,41 +108,37 @@ __device__ __forceinline__ void invert_blocks(const float* sL, float* sT, const 
             for (int r = 0; r < 16; ++r) sT[(16 * warp + r) * LDR + 16 * warp + col] = t[r];
         }
     }
-    __syncthreads();
-    {   // pairs of 16 x 16 blocks: eight warps each, inner index over four lanes
-        const int pr = tid >> 8, a = 32 * pr, b = a + 16, r0 = 2 * (warp & 7), c0 = 2 * (lane >> 2), k0 = 4 * (lane & 3);
-        float acc[2][2] = {};
-        tile22<1>(acc, sL + (b + r0) * LDR + a + k0, sL + (b + r0 + 1) * LDR + a + k0, sT + (a + k0) * LDR + a + c0, LDR, 0);
-        sum22<4>(acc);
-        if ((lane & 3) < 2) {
-            const int i = lane & 1;
-            const float be = sbeta[b + r0 + i];
-            *reinterpret_cast<float2*>(sY + (16 * pr + r0 + i) * LDY + c0) =
-                make_float2(be * (i ? acc[1][0] : acc[0][0]), be * (i ? acc[1][1] : acc[0][1]));
-        }
-        __syncthreads();
+    if (warp >= 8) return;
+    bar_sync(1, 256);
+    float acc[2][2] = {};
+    {   // pairs of 16 x 16 blocks: four warps each, inner index over two lanes (alternating groups of four)
+        const int pr = warp >> 2, a = 32 * pr, b = a + 16, i = lane & 1;
+        const int r0 = 4 * (warp & 3) + 2 * (lane >> 4), c0 = 2 * ((lane >> 1) & 7), k0 = 4 * i;
+        tile22<2>(acc, sL + (b + r0) * LDR + a + k0, sL + (b + r0 + 1) * LDR + a + k0, sT + (a + k0) * LDR + a + c0, LDR, 8);
+        sum22<2>(acc);
+        const float be = sbeta[b + r0 + i];
+        *reinterpret_cast<float2*>(sY + (16 * pr + r0 + i) * LDY + c0) = make_float2(be * (i ? acc[1][0] : acc[0][0]), be * (i ? acc[1][1] : acc[0][1]));
+        bar_sync(1, 256);
         acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = 0.f;
-        tile22<1>(acc, sT + (b + r0) * LDR + b + k0, sT + (b + r0 + 1) * LDR + b + k0, sY + (16 * pr + k0) * LDY + c0, LDY, 0);
-        sum22<4>(acc);
-        if ((lane & 3) < 2) {
-            const int i = lane & 1;
-            *reinterpret_cast<float2*>(sT + (b + r0 + i) * LDR + a + c0) =
-                make_float2(-(i ? acc[1][0] : acc[0][0]), -(i ? acc[1][1] : acc[0][1]));
-        }
-        __syncthreads();
+        tile22<2>(acc, sT + (b + r0) * LDR + b + k0, sT + (b + r0 + 1) * LDR + b + k0, sY + (16 * pr + k0) * LDY + c0, LDY, 8);
+        sum22<2>(acc);
+        *reinterpret_cast<float2*>(sT + (b + r0 + i) * LDR + a + c0) = make_float2(-(i ? acc[1][0] : acc[0][0]), -(i ? acc[1][1] : acc[0][1]));
+        bar_sync(1, 256);
     }
-    {   // the 32 x 32 halves: a warp has two rows, inner index over two lanes (alternating groups of four)
-        const int r0 = 2 * warp, c0 = 2 * (lane >> 1), k0 = 4 * (lane & 1), i = lane & 1;
-        float acc[2][2] = {};
-        tile22<4>(acc, sL + (32 + r0) * LDR + k0, sL + (33 + r0) * LDR + k0, sT + k0 * LDR + c0, LDR, 8);
-        sum22<2>(acc);
-        const float be = sbeta[32 + r0 + i];
-        *reinterpret_cast<float2*>(sY + (r0 + i) * LDY + c0) = make_float2(be * (i ? acc[1][0] : acc[0][0]), be * (i ? acc[1][1] : acc[0][1]));
-        __syncthreads();
+    {   // the 32 x 32 halves: a warp has four rows
+        const int r0 = 4 * warp + 2 * (lane >> 4), c0 = 2 * (lane & 15);
         acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = 0.f;
-        tile22<4>(acc, sT + (32 + r0) * LDR + 32 + k0, sT + (33 + r0) * LDR + 32 + k0, sY + k0 * LDY + c0, LDY, 8);
-        sum22<2>(acc);
-        *reinterpret_cast<float2*>(sT + (32 + r0 + i) * LDR + c0) = make_float2(-(i ? acc[1][0] : acc[0][0]), -(i ? acc[1][1] : acc[0][1]));
+        tile22<8>(acc, sL + (32 + r0) * LDR, sL + (33 + r0) * LDR, sT + c0, LDR, 4);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float be = sbeta[32 + r0 + i];
+            *reinterpret_cast<float2*>(sY + (r0 + i) * LDY + c0) = make_float2(be * acc[i][0], be * acc[i][1]);
+        }
+        bar_sync(1, 256);
+        acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = 0.f;
+        tile22<8>(acc, sT + (32 + r0) * LDR + 32, sT + (33 + r0) * LDR + 32, sY + c0, LDY, 4);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) *reinterpret_cast<float2*>(sT + (32 + r0 + i) * LDR + c0) = make_float2(-acc[i][0], -acc[i][1]);
     }
 }
 
