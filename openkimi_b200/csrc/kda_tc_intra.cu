@@ -10,13 +10,13 @@
 //   1  the four diagonal 16x16 blocks of Aqk and L on the CUDA cores: where all four [16 x 32] tiles
 //      of a block pass the span guard, with the FP32 midpoint factorisation (pre-scaled key rows, no
 //      exponential per pair), otherwise with exact pairwise decays
-//   2  decay-scaled operands: Qt, Kh records; beta*k*2^G; and for every 16-row block I >= 1
-//      the factorised operands  k_j 2^(r_I - G_j) (j < 16 I)  and  x_i 2^(G_i - r_I) (i in I),
-//      r_I = G at the first row of block I, so that every exponent is <= 0; off-diagonal blocks of
-//      Aqk and L as tcgen05 MMAs (M = 64 keys, N = 32 = q and k rows of block I, K = 128)
-//   3  T = (I + diag(beta) L)^-1: forward substitution inside the diagonal blocks, products for the
-//      rest (FP32)
-//   4  Aqk and T records; 5  W^T = (beta k 2^G)^T T^T and U^T = (beta v)^T T^T as tcgen05 MMAs
+//   2  decay-scaled operands: for every 16-row block I >= 1 the factorised operands
+//      k_j 2^(r_I - G_j) (j < 16 I)  and  x_i 2^(G_i - r_I) (i in I),  r_I = G at the first row of block I, so that every exponent is <= 0; off-diagonal blocks of
+//      Aqk and L as tcgen05 MMAs (M = 64 keys, N = 32 = q and k rows of block I, K = 128); the Qt,
+//      Kh records and beta*k*2^G are made while these run
+//   3  T = (I + diag(beta) L)^-1: forward substitution inside the diagonal blocks (beside the
+//      accumulator read-back), products for the rest (FP32); Aqk record
+//   4  T record; 5  W^T = (beta k 2^G)^T T^T and U^T = (beta v)^T T^T as tcgen05 MMAs
 //      (M = 128 channels); 6  W, U, gamC records.
 #include "kda_common.cuh"
 #include "kda_tc.cuh"
@@ -51,94 +51,95 @@ using fi::LDR;
 
 // T = (I + diag(beta) L)^-1 by blocks, FP32.  sL holds L (strictly lower), sT receives T (zero above the diagonal blocks on
 // entry); both have rows of LDR floats on 16-byte boundaries.  The four 16 x 16 diagonal blocks are inverted by forward
-// substitution, one warp each (one per scheduler: a dependent chain of 16 rows, lane = column); everything below them is
-// products on all 16 warps: T_ba = -T_bb (beta L)_ba T_aa for the block pairs (0, 1) and (2, 3), then the same with 32 x 32
-// halves.  A thread's tile is 2 x 2 with the inner index split over neighbouring lanes; sY (32 rows of LDY floats) takes
-// the inner products between two barriers.  (One column after the other down all blocks, on eight warps, was a chain three
-// block levels long: 2.6 us of a unit's 15.5.)
+// substitution, one warp each (a dependent chain of 16 rows, lane = column), by the four warps that have no share in the
+// accumulator read-back; everything below them is products: T_ba = -T_bb (beta L)_ba T_aa for the block pairs (0, 1) and
+// (2, 3), then the same with 32 x 32 halves.  A thread's tile is 2 x 2, in the small products with the inner index split
+// over two lanes; sY (32 rows of LDY floats) takes the inner products between two barriers.  Eight warps do them: the
+// others write the Aqk record and issue the next unit's copies, which hold an issuing warp up for 0.7-0.9 us.  (One
+// column after the other down all blocks was a chain three block levels long, 2.6 us of a unit's 15.5; with all sixteen
+// warps in the products a training step's stores delayed them: 978 us against 988 for 3072 units, forward and backward.)
 constexpr int LDY = 36;
 
-// acc[2][2] over `K4` groups of four inner elements: rows of A (float4 along k), rows k of B (two columns)
+// a 2 x 2 tile over `K4` groups of four inner elements: rows of A (float4 along k), rows k of B (two columns)
 template <int K4>
-__device__ __forceinline__ void tile22(float (&acc)[2][2], const float* A0, const float* A1, const float* B, int ldb, int kstep) {
-#pragma unroll
+__device__ __forceinline__ void tile22(float2 (&acc)[2], const float* A0, const float* A1, const float* B, int ldb, int kstep) {
+#pragma unroll 2
     for (int m = 0; m < K4; ++m) {
         const float4 a0 = *reinterpret_cast<const float4*>(A0 + m * kstep), a1 = *reinterpret_cast<const float4*>(A1 + m * kstep);
         const float x0[4] = {a0.x, a0.y, a0.z, a0.w}, x1[4] = {a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float2 b = *reinterpret_cast<const float2*>(B + (m * kstep + j) * ldb);
-            acc[0][0] = fmaf(x0[j], b.x, acc[0][0]);
-            acc[0][1] = fmaf(x0[j], b.y, acc[0][1]);
-            acc[1][0] = fmaf(x1[j], b.x, acc[1][0]);
-            acc[1][1] = fmaf(x1[j], b.y, acc[1][1]);
+            acc[0] = __ffma2_rn(make_float2(x0[j], x0[j]), b, acc[0]);
+            acc[1] = __ffma2_rn(make_float2(x1[j], x1[j]), b, acc[1]);
         }
     }
 }
 template <int LANES>
-__device__ __forceinline__ void sum22(float (&acc)[2][2]) {
+__device__ __forceinline__ void sum22(float2 (&acc)[2]) {
 #pragma unroll
     for (int o = 1; o < LANES; o <<= 1)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[i >> 1][i & 1] += __shfl_xor_sync(0xffffffffu, acc[i >> 1][i & 1], o);
+        for (int i = 0; i < 2; ++i) {
+            acc[i].x += __shfl_xor_sync(0xffffffffu, acc[i].x, o);
+            acc[i].y += __shfl_xor_sync(0xffffffffu, acc[i].y, o);
+        }
 }
 
-__device__ __forceinline__ void invert_blocks(const float* sL, float* sT, const float* sbeta, float* sY, int tid) {
-    const int warp = tid >> 5, lane = tid & 31;
-    if (warp < 4) {
-        const int col = lane & 15;
-        float t[16];
+__device__ __forceinline__ void invert_diagonal(const float* sL, float* sT, const float* sbeta, int blk, int lane) {
+    const int col = lane & 15;
+    float t[16];
 #pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            const float* lrow = sL + (16 * warp + r) * LDR + 16 * warp;
-            float s0 = 0.f, s1 = 0.f;
+    for (int r = 0; r < 16; ++r) {
+        const float* lrow = sL + (16 * blk + r) * LDR + 16 * blk;
+        float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-            for (int j = 0; j < r; j += 4) {
-                const float4 l = *reinterpret_cast<const float4*>(lrow + j);
-                s0 = fmaf(l.x, t[j], s0);
-                if (j + 1 < r) s1 = fmaf(l.y, t[j + 1], s1);
-                if (j + 2 < r) s0 = fmaf(l.z, t[j + 2], s0);
-                if (j + 3 < r) s1 = fmaf(l.w, t[j + 3], s1);
-            }
-            t[r] = (r == col ? 1.f : 0.f) - sbeta[16 * warp + r] * (s0 + s1);
-            if (r < col) t[r] = 0.f;
+        for (int j = 0; j < r; j += 4) {
+            const float4 l = *reinterpret_cast<const float4*>(lrow + j);
+            s0 = fmaf(l.x, t[j], s0);
+            if (j + 1 < r) s1 = fmaf(l.y, t[j + 1], s1);
+            if (j + 2 < r) s0 = fmaf(l.z, t[j + 2], s0);
+            if (j + 3 < r) s1 = fmaf(l.w, t[j + 3], s1);
         }
-        if (lane < 16) {
-#pragma unroll
-            for (int r = 0; r < 16; ++r) sT[(16 * warp + r) * LDR + 16 * warp + col] = t[r];
-        }
+        t[r] = (r == col ? 1.f : 0.f) - sbeta[16 * blk + r] * (s0 + s1);
+        if (r < col) t[r] = 0.f;
     }
-    if (warp >= 8) return;
-    bar_sync(1, 256);
-    float acc[2][2] = {};
+    if (lane < 16) {
+#pragma unroll
+        for (int r = 0; r < 16; ++r) sT[(16 * blk + r) * LDR + 16 * blk + col] = t[r];
+    }
+}
+
+__device__ __forceinline__ void invert_products(const float* sL, float* sT, const float* sbeta, float* sY, int warp, int lane) {
+    float2 acc[2] = {};
     {   // pairs of 16 x 16 blocks: four warps each, inner index over two lanes (alternating groups of four)
         const int pr = warp >> 2, a = 32 * pr, b = a + 16, i = lane & 1;
         const int r0 = 4 * (warp & 3) + 2 * (lane >> 4), c0 = 2 * ((lane >> 1) & 7), k0 = 4 * i;
         tile22<2>(acc, sL + (b + r0) * LDR + a + k0, sL + (b + r0 + 1) * LDR + a + k0, sT + (a + k0) * LDR + a + c0, LDR, 8);
         sum22<2>(acc);
         const float be = sbeta[b + r0 + i];
-        *reinterpret_cast<float2*>(sY + (16 * pr + r0 + i) * LDY + c0) = make_float2(be * (i ? acc[1][0] : acc[0][0]), be * (i ? acc[1][1] : acc[0][1]));
+        *reinterpret_cast<float2*>(sY + (16 * pr + r0 + i) * LDY + c0) = make_float2(be * (i ? acc[1].x : acc[0].x), be * (i ? acc[1].y : acc[0].y));
         bar_sync(1, 256);
-        acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = 0.f;
+        acc[0] = acc[1] = make_float2(0.f, 0.f);
         tile22<2>(acc, sT + (b + r0) * LDR + b + k0, sT + (b + r0 + 1) * LDR + b + k0, sY + (16 * pr + k0) * LDY + c0, LDY, 8);
         sum22<2>(acc);
-        *reinterpret_cast<float2*>(sT + (b + r0 + i) * LDR + a + c0) = make_float2(-(i ? acc[1][0] : acc[0][0]), -(i ? acc[1][1] : acc[0][1]));
+        *reinterpret_cast<float2*>(sT + (b + r0 + i) * LDR + a + c0) = make_float2(-(i ? acc[1].x : acc[0].x), -(i ? acc[1].y : acc[0].y));
         bar_sync(1, 256);
     }
     {   // the 32 x 32 halves: a warp has four rows
         const int r0 = 4 * warp + 2 * (lane >> 4), c0 = 2 * (lane & 15);
-        acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = 0.f;
+        acc[0] = acc[1] = make_float2(0.f, 0.f);
         tile22<8>(acc, sL + (32 + r0) * LDR, sL + (33 + r0) * LDR, sT + c0, LDR, 4);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const float be = sbeta[32 + r0 + i];
-            *reinterpret_cast<float2*>(sY + (r0 + i) * LDY + c0) = make_float2(be * acc[i][0], be * acc[i][1]);
+            *reinterpret_cast<float2*>(sY + (r0 + i) * LDY + c0) = make_float2(be * acc[i].x, be * acc[i].y);
         }
         bar_sync(1, 256);
-        acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = 0.f;
+        acc[0] = acc[1] = make_float2(0.f, 0.f);
         tile22<8>(acc, sT + (32 + r0) * LDR + 32, sT + (33 + r0) * LDR + 32, sY + c0, LDY, 4);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) *reinterpret_cast<float2*>(sT + (32 + r0 + i) * LDR + c0) = make_float2(-acc[i][0], -acc[i][1]);
+        for (int i = 0; i < 2; ++i) *reinterpret_cast<float2*>(sT + (32 + r0 + i) * LDR + c0) = make_float2(-acc[i].x, -acc[i].y);
     }
 }
 
@@ -650,73 +651,50 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
     }
     __syncthreads();  // the pre-scaled key rows are dead: their space becomes operand space
     KDA_PHASE(10);
-    // ---- 1: decay-scaled operands.  A warp takes 8 rows x 4 channel groups at a time, so that its
-    //      16-byte stores into the core-matrix tiles cover four whole 128-byte core matrices
+    // ---- 1: decay-scaled operands of the off-diagonal products.  A warp takes 8 rows x 4 channel groups at a
+    //      time, so that its 16-byte stores into the core-matrix tiles cover four whole 128-byte core matrices
     //      (no bank conflicts; the row-major loads of q^, k^, G take the conflicts instead, and
-    //      there are five times fewer of them)
-    {
+    //      there are fewer of them).  A block's rows serve as queries for their own block and as keys for the later
+    //      ones, so a warp pairs an early combination of rows and channels with a late one.  (Key rows >= 16 I of
+    //      block I's operand keep what was there: their accumulator rows are not read.)
+    auto combo_rows = [&](int it) {
+        const int combo = it ? 31 - warp : warp;
+        return make_int2(8 * (combo >> 2) + (lane & 7), 8 * (4 * (combo & 3) + (lane >> 3)));
+    };
+    auto load_g8 = [&](int i, int c8, float (&x)[8]) {
+        const float4 a = *reinterpret_cast<const float4*>(sG + swz_f32(i, c8));
+        const float4 b = *reinterpret_cast<const float4*>(sG + swz_f32(i, c8 + 4));
+        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+    };
 #pragma unroll 1
-        for (int it = 0; it < 2; ++it) {
-            const int combo = 2 * warp + it;
-            const int i = 8 * (combo >> 2) + (lane & 7), c8 = 8 * (4 * (combo & 3) + (lane >> 3)), m = i >> 4;
-            float G8[8], qf[8], kf[8], o8[8], gl[8];
-            {
-                const float4 a = *reinterpret_cast<const float4*>(sG + swz_f32(C - 1, c8));
-                const float4 b = *reinterpret_cast<const float4*>(sG + swz_f32(C - 1, c8 + 4));
-                gl[0] = a.x; gl[1] = a.y; gl[2] = a.z; gl[3] = a.w; gl[4] = b.x; gl[5] = b.y; gl[6] = b.z; gl[7] = b.w;
-            }
-            {
-                const float4 a = *reinterpret_cast<const float4*>(sG + swz_f32(i, c8));
-                const float4 b = *reinterpret_cast<const float4*>(sG + swz_f32(i, c8 + 4));
-                G8[0] = a.x; G8[1] = a.y; G8[2] = a.z; G8[3] = a.w; G8[4] = b.x; G8[5] = b.y; G8[6] = b.z; G8[7] = b.w;
-            }
+    for (int it = 0; it < 2; ++it) {
+        const int2 ic = combo_rows(it);
+        const int i = ic.x, c8 = ic.y, m = i >> 4;
+        float G8[8], kf[8], o8[8], r[8];
+        load_g8(i, c8, G8);
+        bf16x8_to_f32(*reinterpret_cast<const uint4*>(sK + swz_bf16(i, c8)), kf);
+        if (m >= 1) {  // rows of block m as the N operand of block m's products
+            float qf[8];
             bf16x8_to_f32(*reinterpret_cast<const uint4*>(sQ + swz_bf16(i, c8)), qf);
-            bf16x8_to_f32(*reinterpret_cast<const uint4*>(sK + swz_bf16(i, c8)), kf);
-            const float bi = sbeta[i];
-            float eg[8];
+            load_g8(16 * m, c8, r);
+            __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(dyn + XSC + (m - 1) * 8192);
+            float f[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) eg[j] = ex2_approx(G8[j]);
+            for (int j = 0; j < 8; ++j) f[j] = ex2_approx(G8[j] - r[j]);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) o8[j] = p.scale * qf[j] * eg[j];
-            *reinterpret_cast<uint4*>(gQt + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
+            for (int j = 0; j < 8; ++j) o8[j] = qf[j] * f[j];
+            *reinterpret_cast<uint4*>(xs + cm_idx(i - 16 * m, c8, D)) = f32_to_bf16x8(o8);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) o8[j] = bi * kf[j] * eg[j];
-            *reinterpret_cast<uint4*>(sKB + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o8[j] = kf[j] * ex2_approx(gl[j] - G8[j]);
-            *reinterpret_cast<uint4*>(gKh + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
-            if (m >= 1) {  // rows of block m as the N operand of block m's products
-                float r[8];
-                {
-                    const float4 a = *reinterpret_cast<const float4*>(sG + swz_f32(16 * m, c8));
-                    const float4 b = *reinterpret_cast<const float4*>(sG + swz_f32(16 * m, c8 + 4));
-                    r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w; r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
-                }
-                __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(dyn + XSC + (m - 1) * 8192);
-                float f[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) f[j] = ex2_approx(G8[j] - r[j]);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) o8[j] = qf[j] * f[j];
-                *reinterpret_cast<uint4*>(xs + cm_idx(i - 16 * m, c8, D)) = f32_to_bf16x8(o8);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) o8[j] = kf[j] * f[j];
-                *reinterpret_cast<uint4*>(xs + cm_idx(16 + i - 16 * m, c8, D)) = f32_to_bf16x8(o8);
-            }
+            for (int j = 0; j < 8; ++j) o8[j] = kf[j] * f[j];
+            *reinterpret_cast<uint4*>(xs + cm_idx(16 + i - 16 * m, c8, D)) = f32_to_bf16x8(o8);
+        }
 #pragma unroll 1
-            for (int I = 1; I <= 3; ++I) {  // keys scaled for the later blocks
-                __nv_bfloat16* ks = reinterpret_cast<__nv_bfloat16*>(dyn + KSC + (I - 1) * 16384);
-                if (m < I) {
-                    const float4 a = *reinterpret_cast<const float4*>(sG + swz_f32(16 * I, c8));
-                    const float4 b = *reinterpret_cast<const float4*>(sG + swz_f32(16 * I, c8 + 4));
-                    const float r[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        for (int I = m + 1; I <= 3; ++I) {  // keys scaled for the later blocks
+            __nv_bfloat16* ks = reinterpret_cast<__nv_bfloat16*>(dyn + KSC + (I - 1) * 16384);
+            load_g8(16 * I, c8, r);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) o8[j] = kf[j] * ex2_approx(r[j] - G8[j]);
-                    *reinterpret_cast<uint4*>(ks + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
-                } else {
-                    *reinterpret_cast<uint4*>(ks + cm_idx(i, c8, D)) = make_uint4(0, 0, 0, 0);
-                }
-            }
+            for (int j = 0; j < 8; ++j) o8[j] = kf[j] * ex2_approx(r[j] - G8[j]);
+            *reinterpret_cast<uint4*>(ks + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
         }
     }
     fence_async_smem();
@@ -738,6 +716,30 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
                    make_desc(sb + XSC + (I - 1) * 8192 + s * 256, 128, 2048), id, s > 0);
         mma_commit(&bar);
     }
+    if (more) ci_nx = chunk_info(p, un.c);  // (dependent loads: issued well ahead of the requests that need them)
+    // ---- meanwhile: the Qt and Kh records and the operand beta k 2^G of the W product
+#pragma unroll 1
+    for (int it = 0; it < 2; ++it) {
+        const int2 ic = combo_rows(it);
+        const int i = ic.x, c8 = ic.y;
+        float G8[8], qf[8], kf[8], o8[8], eg[8], gl[8];
+        load_g8(i, c8, G8);
+        load_g8(C - 1, c8, gl);
+        bf16x8_to_f32(*reinterpret_cast<const uint4*>(sQ + swz_bf16(i, c8)), qf);
+        bf16x8_to_f32(*reinterpret_cast<const uint4*>(sK + swz_bf16(i, c8)), kf);
+        const float bi = sbeta[i];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) eg[j] = ex2_approx(G8[j]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o8[j] = p.scale * qf[j] * eg[j];
+        *reinterpret_cast<uint4*>(gQt + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o8[j] = bi * kf[j] * eg[j];
+        *reinterpret_cast<uint4*>(sKB + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o8[j] = kf[j] * ex2_approx(gl[j] - G8[j]);
+        *reinterpret_cast<uint4*>(gKh + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
+    }
     KDA_PHASE(4);
     ok = mbar_wait(&bar, it & 1, p, 8) && ok;
     tc_fence_after();
@@ -747,12 +749,12 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
         if (grp == 0) read_offdiag<0>(tmem0 + T_D, warp & 3, lane, sA, sL, p.scale);
         else if (grp == 1) read_offdiag<32>(tmem0 + T_D, warp & 3, lane, sA, sL, p.scale);
         else if (grp == 2) read_offdiag<64>(tmem0 + T_D, warp & 3, lane, sA, sL, p.scale);
+        else invert_diagonal(sL, sT, sbeta, warp & 3, lane);
     }
     KDA_PHASE(12);
     tc_fence_before();
     __syncthreads();
     if (more) {  // the operand tiles of the off-diagonal products are dead; the scalars have the inversion to arrive
-        ci_nx = chunk_info(p, un.c);
         request_rows(ci_nx, un.head());
         request_scalars(ci_nx, un.head(), nx);
     }
@@ -770,27 +772,37 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
     }
 
     // ---- 3: T = (I + diag(beta) L)^-1; the inner products pass through the space behind T's operand tile
-    invert_blocks(sL, sT, sbeta, reinterpret_cast<float*>(dyn + KSC + 8192), tid);
+    if (warp < 8) {
+        invert_products(sL, sT, sbeta, reinterpret_cast<float*>(dyn + KSC + 8192), warp, lane);
+    } else if (warp < 14) {  // the Aqk record; eight lanes = eight adjacent rows of one 8-column group, as below
+        for (int x = tid - 256; x < C * C / 8; x += 192) {
+            const int i = (x & 7) | ((x >> 6) << 3), j8 = ((x >> 3) & 7) * 8;
+            float a8[8];
+#pragma unroll
+            for (int j = 0; j < 8; j += 4) {
+                const float4 a = *reinterpret_cast<const float4*>(sA + i * LDR + j8 + j);
+                a8[j] = a.x, a8[j + 1] = a.y, a8[j + 2] = a.z, a8[j + 3] = a.w;
+            }
+            *reinterpret_cast<uint4*>(gA + cm_idx(i, j8, C)) = f32_to_bf16x8(a8);
+        }
+    }
     fence_async_smem();
     __syncthreads();
     if (more) request_v(ci_nx, un.head());  // L is dead: its tile receives the next unit's v rows
 
     KDA_PHASE(6);
-    // ---- 4: Aqk and T records; T as the B operand of the WY products
+    // ---- 4: T record; T as the B operand of the WY products
     {
         __nv_bfloat16* sTB = reinterpret_cast<__nv_bfloat16*>(dyn + KSC);
         // eight lanes = eight adjacent rows of one 8-column group: one core matrix of the records, 32 distinct banks
         const int i = (tid & 7) | ((tid >> 6) << 3), j8 = ((tid >> 3) & 7) * 8;
-        float a8[8], t8[8];
+        float t8[8];
 #pragma unroll
         for (int j = 0; j < 8; j += 4) {
-            const float4 a = *reinterpret_cast<const float4*>(sA + i * LDR + j8 + j);
             const float4 t = *reinterpret_cast<const float4*>(sT + i * LDR + j8 + j);
-            a8[j] = a.x, a8[j + 1] = a.y, a8[j + 2] = a.z, a8[j + 3] = a.w;
             t8[j] = t.x, t8[j + 1] = t.y, t8[j + 2] = t.z, t8[j + 3] = t.w;
         }
         const uint4 tb = f32_to_bf16x8(t8);
-        *reinterpret_cast<uint4*>(gA + cm_idx(i, j8, C)) = f32_to_bf16x8(a8);
         if (save) *reinterpret_cast<uint4*>(gT + cm_idx(i, j8, C)) = tb;
         *reinterpret_cast<uint4*>(sTB + cm_idx(i, j8, C)) = tb;
     }
