@@ -16,7 +16,7 @@
 namespace kda {
 
 __device__ __forceinline__ float dsilu_f(float x) {
-    const float s = __fdividef(1.f, 1.f + __expf(-x));
+    const float s = rcp_ftz(1.f + exp_ftz(-x));
     return s * (1.f + x * (1.f - s));
 }
 

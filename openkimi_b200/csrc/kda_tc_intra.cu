@@ -365,9 +365,6 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
         const float4* sW = reinterpret_cast<const float4*>(dyn + TAPS);
         // row x of a tensor's window (x = 0 .. 66 stands for token x - 3 of the chunk); the halo rows of v sit apart
         auto conv_rows = [&](uint4(&out)[2], int tensor) {
-            float4 w[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) w[j] = sW[tensor * D + j * 16 + (c8 >> 3)];
             float win[5][8];
 #pragma unroll
             for (int r = 0; r < 5; ++r) {
@@ -375,12 +372,23 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
                 const __nv_bfloat16* row = tensor == 0 ? sRq + x * D : tensor == 1 ? sRk + x * D : (x < 3 ? sRvh + x * D : sRv + (x - 3) * D);
                 bf16x8_to_f32(*reinterpret_cast<const uint4*>(row + c8), win[r]);
             }
+            float y2[2][8];
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {  // two channels in packed FMAs (the order of conv_pre)
+                const float4 wa = sW[tensor * D + j * 16 + (c8 >> 3)], wb = sW[tensor * D + (j + 1) * 16 + (c8 >> 3)];
+                auto x2 = [&](int r) { return make_float2(win[r][j], win[r][j + 1]); };
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    const float2 pre = __ffma2_rn(make_float2(wa.w, wb.w), x2(m + 3),
+                                                  __ffma2_rn(make_float2(wa.z, wb.z), x2(m + 2),
+                                                             __ffma2_rn(make_float2(wa.y, wb.y), x2(m + 1), __fmul2_rn(make_float2(wa.x, wb.x), x2(m)))));
+                    y2[m][j] = silu_f(pre.x);
+                    y2[m][j + 1] = silu_f(pre.y);
+                }
+            }
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
-                float y[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    y[j] = silu_f(conv_pre(w[j].x, w[j].y, w[j].z, w[j].w, win[m][j], win[m + 1][j], win[m + 2][j], win[m + 3][j]));
+                const float (&y)[8] = y2[m];
                 out[m] = 2 * hw + m < ci.len ? f32_to_bf16x8(y) : make_uint4(0, 0, 0, 0);
             }
         };
@@ -401,47 +409,66 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
             rv4[m] = *reinterpret_cast<const uint4*>(sRv + off);
         }
     }
-    // ---- 0b: q, k, v, beta row-wise: a half warp owns two rows, lane c8 the channels 8 c8 ..
+    // ---- 0b: q, k, v, beta row-wise: a half warp owns two rows, lane c8 the channels 8 c8 ..  The four sums of squares
+    //      (row m, tensor t) are reduced by a transposing exchange (5 shuffles instead of 16, the same additions), after
+    //      which lane 8 m + 4 t of the half warp turns its own into 1 / norm: one square root and one division, long
+    //      instruction sequences, per thread instead of four.  Likewise one sigmoid for the two betas.
     {
+        auto row_of = [&](int m) { return CONV ? 2 * hw + m : hw + 32 * m; };
+        const int m_l = (lane >> 3) & 1, t_l = (lane >> 2) & 1, base = lane & 16;
+        float qf[2][8], kf[2][8], rn = 1.f;
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
-            const int i = CONV ? 2 * hw + m : hw + 32 * m;
-            const bool valid = i < ci.len;
-            float qf[8], kf[8], vf[8];
-            bf16x8_to_f32(rq4[m], qf);
-            bf16x8_to_f32(rk4[m], kf);
-            bf16x8_to_f32(rv4[m], vf);
-            float b = rb[m];
-            if ((tid & 15) == 0 && valid && sig) b = sigmoid_f(b);
-            b = __shfl_sync(0xffffffffu, b, lane & 16);
-            float rq = 1.f, rk = 1.f;
-            if (l2) {
-                float ssq = 0.f, ssk = 0.f;
+            bf16x8_to_f32(rq4[m], qf[m]);
+            bf16x8_to_f32(rk4[m], kf[m]);
+        }
+        float b_l;  // beta of row m_l
+        {
+            const float b0 = __shfl_sync(0xffffffffu, rb[0], base), b1 = __shfl_sync(0xffffffffu, rb[1], base);
+            b_l = m_l ? b1 : b0;
+            if (sig) b_l = row_of(m_l) < ci.len ? sigmoid_f(b_l) : 0.f;
+        }
+        if (l2) {
+            float ss[2][2];  // [row][tensor]
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                ss[m][0] = ss[m][1] = 0.f;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    ssq = fmaf(qf[j], qf[j], ssq);  // explicit: both instantiations must round alike
-                    ssk = fmaf(kf[j], kf[j], ssk);
+                    ss[m][0] = fmaf(qf[m][j], qf[m][j], ss[m][0]);  // explicit: both instantiations must round alike
+                    ss[m][1] = fmaf(kf[m][j], kf[m][j], ss[m][1]);
                 }
-                ssq = half_warp_sum(ssq);
-                ssk = half_warp_sum(ssk);
-                rq = 1.f / fmaxf(sqrtf(ssq), 1e-6f);
-                rk = 1.f / fmaxf(sqrtf(ssk), 1e-6f);
+            }
+            float s2[2], s1;
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+                s2[t] = (m_l ? ss[1][t] : ss[0][t]) + __shfl_xor_sync(0xffffffffu, m_l ? ss[0][t] : ss[1][t], 8);
+            s1 = (t_l ? s2[1] : s2[0]) + __shfl_xor_sync(0xffffffffu, t_l ? s2[0] : s2[1], 4);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
+            rn = 1.f / fmaxf(sqrtf(s1), 1e-6f);
+        }
+        if ((lane & 3) == 0) saux[t_l * C + row_of(m_l)] = rn;
+        if ((lane & 7) == 0) sbeta[row_of(m_l)] = b_l;
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            const int i = row_of(m);
+            const float rq = __shfl_sync(0xffffffffu, rn, base + 8 * m), rk = __shfl_sync(0xffffffffu, rn, base + 8 * m + 4);
+            const float b = __shfl_sync(0xffffffffu, b_l, base + 8 * m);
+            float vf[8];
+            bf16x8_to_f32(rv4[m], vf);
+            if (l2) {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    qf[j] *= rq;
-                    kf[j] *= rk;
+                    qf[m][j] *= rq;
+                    kf[m][j] *= rk;
                 }
             }
 #pragma unroll
             for (int j = 0; j < 8; ++j) vf[j] *= b;
-            *reinterpret_cast<uint4*>(sQ + swz_bf16(i, c8)) = f32_to_bf16x8(qf);
-            *reinterpret_cast<uint4*>(sK + swz_bf16(i, c8)) = f32_to_bf16x8(kf);
+            *reinterpret_cast<uint4*>(sQ + swz_bf16(i, c8)) = f32_to_bf16x8(qf[m]);
+            *reinterpret_cast<uint4*>(sK + swz_bf16(i, c8)) = f32_to_bf16x8(kf[m]);
             *reinterpret_cast<uint4*>(sBV + cm_idx(i, c8, D)) = f32_to_bf16x8(vf);
-            if ((tid & 15) == 0) {
-                sbeta[i] = b;
-                saux[i] = rq;
-                saux[C + i] = rk;
-            }
         }
     }
     KDA_PHASE(1);
