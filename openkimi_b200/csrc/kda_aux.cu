@@ -234,6 +234,28 @@ __global__ void __launch_bounds__(256) partial_reduce_kernel(const float* __rest
 }
 
 // ---- RMSNorm(x) * w * sigmoid(gate): DIM / 8 (BF16) or DIM / 4 (FP32) lanes per row, 16-byte accesses
+// Both kernels were bound by instruction issue: an accurate expf and an IEEE division cost some 20 instructions per
+// element.  For BF16 tensors the exponential is taken with its argument's rounding error made good, e^-g =
+// 2^t (1 + (rest of -g log2 e) ln 2) with t = fl(-g log2 e), and the reciprocal from the hardware (1 ulp), two elements at a
+// time in packed arithmetic: within 4 ulp, far below the BF16 rounding of the result.  786432 rows of 128:
+// forward 147 -> 116 us (5.2 TB/s), backward 205 -> 170 (5.9 TB/s).
+__device__ __forceinline__ float clamp_nan(float x, float lim) {  // into [-lim, lim]; a NaN stays one
+    asm("min.NaN.f32 %0, %0, %1;\n\tmax.NaN.f32 %0, %0, %2;" : "+f"(x) : "f"(lim), "f"(-lim));
+    return x;
+}
+template <typename T>
+__device__ __forceinline__ float2 sigmoid2(float2 g) {
+    if constexpr (sizeof(T) == 4) return make_float2(sigmoid_f(g.x), sigmoid_f(g.y));
+    g = make_float2(clamp_nan(g.x, 100.f), clamp_nan(g.y, 100.f));  // (0 or 1 there; an infinite product has no rest)
+    constexpr float LOG2E_REST = 1.9259629911e-8f, LN2 = 0.6931471805599453f;  // log2 e = LOG2E + LOG2E_REST
+    const float2 nl = make_float2(-LOG2E, -LOG2E), nr = make_float2(-LOG2E_REST, -LOG2E_REST), one = make_float2(1.f, 1.f);
+    const float2 t = __fmul2_rn(g, nl);
+    const float2 rest = __ffma2_rn(g, nr, __ffma2_rn(g, nl, make_float2(-t.x, -t.y)));
+    const float2 corr = __ffma2_rn(rest, make_float2(LN2, LN2), one);
+    const float2 d = __ffma2_rn(make_float2(ex2_ftz(t.x), ex2_ftz(t.y)), corr, one);
+    return make_float2(rcp_ftz(d.x), rcp_ftz(d.y));
+}
+
 template <typename T, int DIM>
 __global__ void __launch_bounds__(256) norm_gate_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gate,
                                                             const float* __restrict__ w, T* __restrict__ y,
@@ -264,7 +286,11 @@ __global__ void __launch_bounds__(256) norm_gate_fwd_kernel(const T* __restrict_
         if (ok) {
             if (sub == 0 && rstd) rstd[r] = rs;
 #pragma unroll
-            for (int i = 0; i < V; ++i) out[i] = xv[i] * rs * wv[i] * sigmoid_f(gv[i]);
+            for (int i = 0; i < V; i += 2) {
+                const float2 sg = sigmoid2<T>(make_float2(gv[i], gv[i + 1]));
+                out[i] = xv[i] * rs * wv[i] * sg.x;
+                out[i + 1] = xv[i + 1] * rs * wv[i + 1] * sg.y;
+            }
             Vec<T>::store(y + r * DIM + sub * V, out);
         }
     }
@@ -304,8 +330,14 @@ __global__ void __launch_bounds__(256) norm_gate_bwd_kernel(const T* __restrict_
         const float rs = rsqrtf(ss / DIM + eps);
         float dg[V];
 #pragma unroll
+        for (int i = 0; i < V; i += 2) {
+            const float2 sg = sigmoid2<T>(make_float2(gv[i], gv[i + 1]));
+            gv[i] = sg.x;
+            gv[i + 1] = sg.y;
+        }
+#pragma unroll
         for (int i = 0; i < V; ++i) {
-            const float sgm = sigmoid_f(gv[i]);
+            const float sgm = gv[i];
             const float xh = xv[i] * rs;
             dg[i] = gy[i] * xh * wv[i] * sgm * (1.f - sgm);
             dn[i] = gy[i] * sgm;

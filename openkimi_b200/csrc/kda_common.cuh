@@ -293,13 +293,14 @@ __device__ __forceinline__ void split3_bf16(float x0, float x1, uint32_t& p0, ui
     p2 = *reinterpret_cast<uint32_t*>(&h);
 }
 
-// e^x, 1 / x and ln x by the hardware approximations alone, for arguments and results that are normal numbers or may as
+// 2^x, e^x, 1 / x and ln x by the hardware approximations alone, for arguments and results that are normal numbers or may as
 // well be zero: __expf, __fdividef and __logf use the same instructions, in rescalings for denormal operands
-__device__ __forceinline__ float exp_ftz(float x) {
+__device__ __forceinline__ float ex2_ftz(float x) {
     float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * LOG2E));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+__device__ __forceinline__ float exp_ftz(float x) { return ex2_ftz(x * LOG2E); }
 __device__ __forceinline__ float rcp_ftz(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
