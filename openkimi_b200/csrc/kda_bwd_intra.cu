@@ -688,10 +688,12 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
 }
 
 // The rows a chunk could not finish (61..63 when it has a successor): dx from dpre of its last three rows and
-// of the successor's first three, in the FMA order of conv_bwd_block.  Grid (chunk, head, tensor), thread = channel.
+// of the successor's first three, in the FMA order of conv_bwd_block.  Warp = (chunk, head, tensor), lane = four
+// channels.  (One channel per thread and a CTA per chunk was bound by starting CTAs: 2048 chunks x 6 heads, three tensors 47 -> 23 us.)
 __global__ void __launch_bounds__(128) conv_bwd_fixup_kernel(const KdaParams p) {
-    const int c = blockIdx.x, h = blockIdx.y, t = blockIdx.z, ch = threadIdx.x;
+    const int c = blockIdx.x * 4 + (threadIdx.x >> 5), h = blockIdx.y, t = blockIdx.z, ch = (threadIdx.x & 31) * 4;
     pdl_wait();
+    if (c >= p.NT) return;
     const ChunkInfo ci = chunk_info(p, c);
     int c0s, ncs;
     seq_chunks(p, ci.seq, c0s, ncs);
@@ -701,14 +703,22 @@ __global__ void __launch_bounds__(128) conv_bwd_fixup_kernel(const KdaParams p) 
     const size_t rec = (size_t)c * p.H + h, nxt = (size_t)(c + 1) * p.H + h;
     const float* tl = (const float*)(sc + L.cv_tail) + ((rec * 3 + t) * 3) * 128 + ch;
     const float* hdp = (const float*)(sc + L.cv_head) + ((nxt * 3 + t) * 3) * 128 + ch;
-    float w[4];
-    conv_taps(t == 0 ? p.conv_q : t == 1 ? p.conv_k : p.conv_v, h, ch, p.conv_ksize, w);
-    const float p61 = tl[0], p62 = tl[128], p63 = tl[256], p64 = hdp[0], p65 = hdp[128], p66 = hdp[256];
-    __nv_bfloat16* dst = (__nv_bfloat16*)(t == 0 ? p.grad_q : t == 1 ? p.grad_k : p.grad_v);
-    const size_t row = ((size_t)(ci.tok0 + 61) * p.H + h) * 128 + ch, rs = (size_t)p.H * 128;
-    dst[row] = __float2bfloat16_rn(fmaf(w[0], p64, fmaf(w[1], p63, fmaf(w[2], p62, w[3] * p61))));
-    dst[row + rs] = __float2bfloat16_rn(fmaf(w[0], p65, fmaf(w[1], p64, fmaf(w[2], p63, w[3] * p62))));
-    dst[row + 2 * rs] = __float2bfloat16_rn(fmaf(w[0], p66, fmaf(w[1], p65, fmaf(w[2], p64, w[3] * p63))));
+    float dp[6][4], w[4][4];  // dpre of rows 61 .. 66; taps [channel][tap]
+#pragma unroll
+    for (int r = 0; r < 6; ++r) {
+        const float4 v = *reinterpret_cast<const float4*>(r < 3 ? tl + r * 128 : hdp + (r - 3) * 128);
+        dp[r][0] = v.x; dp[r][1] = v.y; dp[r][2] = v.z; dp[r][3] = v.w;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) conv_taps(t == 0 ? p.conv_q : t == 1 ? p.conv_k : p.conv_v, h, ch + j, p.conv_ksize, w[j]);
+    __nv_bfloat16* dst = (__nv_bfloat16*)(t == 0 ? p.grad_q : t == 1 ? p.grad_k : p.grad_v) + ((size_t)(ci.tok0 + 61) * p.H + h) * 128 + ch;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        float o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[j] = fmaf(w[j][0], dp[r + 3][j], fmaf(w[j][1], dp[r + 2][j], fmaf(w[j][2], dp[r + 1][j], w[j][3] * dp[r][j])));
+        *reinterpret_cast<uint2*>(dst + (size_t)r * p.H * 128) = make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
+    }
 }
 
 // Filter gradients: fixed-order sum of the per-chunk shares.  Grid (head, tensor), 8 groups of 128 threads sum
@@ -756,7 +766,7 @@ cudaError_t launch_bwd_intra(const KdaParams& p, cudaStream_t s) {
     const int units = p.NT * p.H, sms = sm_count();
     if ((e = launch_dependent(kern, units < sms ? units : sms, bi::NTHR, bi::TOTAL, s, p)) != cudaSuccess) return e;
     if (convb) {
-        if ((e = launch_dependent(conv_bwd_fixup_kernel, dim3(p.NT, p.H, 3), 128, 0, s, p)) != cudaSuccess) return e;
+        if ((e = launch_dependent(conv_bwd_fixup_kernel, dim3((p.NT + 3) / 4, p.H, 3), 128, 0, s, p)) != cudaSuccess) return e;
         if ((e = launch_dependent(conv_bwd_reduce_kernel, dim3(p.H, 3, 8), 1024, 0, s, p)) != cudaSuccess) return e;
     }
     return cudaGetLastError();

@@ -74,6 +74,11 @@ __device__ __forceinline__ void stage_taps(float4* dst, const float* __restrict_
 // the padded taps of channel (head h, ch): tap j multiplies x[s - 3 + j]
 __device__ __forceinline__ void conv_taps(const float* __restrict__ wsrc, int h, int ch, int K, float (&w)[4]) {
     const float* p = wsrc + (size_t)(h * 128 + ch) * K;
+    if (K == 4 && (reinterpret_cast<uintptr_t>(wsrc) & 15) == 0) {
+        const float4 v = *reinterpret_cast<const float4*>(p);
+        w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+        return;
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) w[j] = j >= 4 - K ? p[j - (4 - K)] : 0.f;
 }
