@@ -650,10 +650,31 @@ struct Layer : torch::autograd::Function<Layer> {
     }
 };
 
-Tensor layer(const Tensor& x, const std::vector<Tensor>& prm, int64_t H, double scale, double eps, bool disable_recompute,
-             OptTensor cu, OptTensor chunk_seq, OptTensor seq_off, OptTensor chunk_tab, int64_t NT, int64_t longest) {
+// The node derives every size from x and H and hands raw pointers on, so it takes only plain tensors of exactly those sizes
+// on x's device.
+bool layer_takes(const Tensor& x, const std::vector<Tensor>& prm, int64_t H) {
+    if (x.dim() != 3 || prm.size() != P_COUNT || H < 1) return false;
+    for (const Tensor& t : prm)
+        if (t.device() != x.device() || t.layout() != at::kStrided || t.unsafeGetTensorImpl()->is_python_dispatch()) return false;
+    const int64_t width = x.size(2), proj = H * HD, ksize = prm[P_CQ].dim() == 3 ? prm[P_CQ].size(2) : 0;
+    if (ksize < 1 || ksize > 4) return false;
+    auto is = [&](int which, at::IntArrayRef sizes) { return prm[which].sizes() == sizes; };
+    for (int i : {P_WQ, P_WK, P_WV})
+        if (!is(i, {proj, width})) return false;
+    for (int i : {P_CQ, P_CK, P_CV})
+        if (!is(i, {proj, 1, ksize})) return false;
+    for (int i : {P_FA, P_GA})
+        if (!is(i, {HD, width})) return false;
+    for (int i : {P_FB, P_GB})
+        if (!is(i, {proj, HD})) return false;
+    return is(P_ALOG, {H}) && is(P_DTB, {H, HD}) && is(P_BETA, {H, width}) && is(P_NORM, {HD}) && is(P_WO, {width, proj});
+}
+
+// nothing where the node does not take these tensors: the module's parts then compute what they can, or say what is wrong
+OptTensor layer(const Tensor& x, const std::vector<Tensor>& prm, int64_t H, double scale, double eps, bool disable_recompute,
+                OptTensor cu, OptTensor chunk_seq, OptTensor seq_off, OptTensor chunk_tab, int64_t NT, int64_t longest) {
     require_cuda(x);
-    TORCH_CHECK(prm.size() == P_COUNT, "expected the sublayer's parameters");
+    if (!layer_takes(x, prm, H)) return std::nullopt;
     LayerSpec ls;
     ls.H = H;
     ls.eps = eps;
@@ -690,4 +711,5 @@ PYBIND11_MODULE(_host, m) {
     m.def("recurrent", &recurrent);
     m.def("chunk_kda", &chunk_kda);
     m.def("layer", &layer);
+    m.def("layer_takes", &layer_takes);
 }

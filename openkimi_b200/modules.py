@@ -232,16 +232,17 @@ class KimiDeltaAttention(nn.Module):
                 return None
         elif x.dtype != torch.bfloat16 or any(m.weight.dtype != torch.bfloat16 for m in parts):
             return None
-        prm = (self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.q_conv.weight, self.k_conv.weight,
-               self.v_conv.weight, self.A_log, self.f_a_proj.weight, self.f_b_proj.weight, self.dt_bias,
-               self.beta_proj.weight, self.out_gate_a.weight, self.out_gate_b.weight, norm.weight, self.out_proj.weight)
-        return prm if all(p.is_cuda for p in prm) else None
+        return (self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.q_conv.weight, self.k_conv.weight,
+                self.v_conv.weight, self.A_log, self.f_a_proj.weight, self.f_b_proj.weight, self.dt_bias,
+                self.beta_proj.weight, self.out_gate_a.weight, self.out_gate_b.weight, norm.weight, self.out_proj.weight)
 
     def forward(self, x, cu_seqlens=None):
         prm = self._native_parameters(x)
         if prm is not None and not _lib.host().env_flags():
-            return _lib.host().layer(x, prm, self.n_heads, self.scale, self.out_norm_gate.eps, self.disable_recompute,
-                                     *_packed_tables(cu_seqlens, None, x.device))
+            out = _lib.host().layer(x, prm, self.n_heads, self.scale, self.out_norm_gate.eps, self.disable_recompute,
+                                    *_packed_tables(cu_seqlens, None, x.device))
+            if out is not None:
+                return out
         # The three narrow projections of x (decay rank, output-gate rank, beta) share one GEMM: x is
         # read once instead of three times.  Same parameters, same arithmetic per output column.  All four
         # projections of x form one autograd node (see _InputProjections).
