@@ -221,7 +221,8 @@ int kda_short_conv_bwd_static(const void *x, const float *weight, const void *dy
                               const int64_t *cu_seqlens, int32_t N, void *cuda_stream);
 
 /* Headwise RMSNorm(x) * sigmoid(gate) over [rows, dim] (k3mini/model.py:91-98; the fast
- * path's fla.modules.FusedRMSNormGated at k3mini/model.py:171-175). */
+ * path's fla.modules.FusedRMSNormGated at k3mini/model.py:171-175).  All row tensors start on
+ * 16-byte boundaries. */
 int kda_norm_gate_fwd(const void *x, const void *gate, const float *weight, void *y, float *rstd,
                       int64_t rows, int32_t dim, float eps, int32_t dtype, void *cuda_stream);
 /* dweight [dim] is reduced in a fixed order from partial [n_partial, dim] (caller scratch). */

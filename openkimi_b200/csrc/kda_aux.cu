@@ -520,6 +520,7 @@ int kda_norm_gate_fwd(const void* x, const void* gate, const float* weight, void
     if (!x || !gate || !weight || !y) return KDA_ERR_NULL;
     if (rows <= 0 || (dim != 64 && dim != 128)) return KDA_ERR_SHAPE;
     if (dtype != KDA_DTYPE_BF16 && dtype != KDA_DTYPE_F32) return KDA_ERR_DTYPE;
+    if (((uintptr_t)x | (uintptr_t)gate | (uintptr_t)y) & 15) return KDA_ERR_ALIGN;
     cudaStream_t s = (cudaStream_t)stream;
     int grid = (int)((rows + 15) / 16 < 148 * 8 ? (rows + 15) / 16 : 148 * 8);
 #define NG_FWD(TT, DD) \
@@ -536,6 +537,7 @@ int kda_norm_gate_bwd(const void* x, const void* gate, const float* weight, cons
     if (!x || !gate || !weight || !dy || !dx || !dgate || !dweight || !partial) return KDA_ERR_NULL;
     if (rows <= 0 || (dim != 64 && dim != 128) || n_partial < 1 || n_partial > 65535) return KDA_ERR_SHAPE;
     if (dtype != KDA_DTYPE_BF16 && dtype != KDA_DTYPE_F32) return KDA_ERR_DTYPE;
+    if (((uintptr_t)x | (uintptr_t)gate | (uintptr_t)dy | (uintptr_t)dx | (uintptr_t)dgate) & 15) return KDA_ERR_ALIGN;
     cudaStream_t s = (cudaStream_t)stream;
 #define NG_BWD(TT, DD)                                                                                               \
     norm_gate_bwd_kernel<TT, DD><<<n_partial, 256, 0, s>>>((const TT*)x, (const TT*)gate, weight, (const TT*)dy, (TT*)dx, \

@@ -19,10 +19,25 @@ def _stream(t):
     return C.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
 
 
+def _require_device(device, **tensors):
+    for name, t in tensors.items():
+        if t is not None and t.device != device:
+            raise RuntimeError(f"expected {name} on {device}, but it is on {t.device}")
+
+
+def _rows(t):
+    """``t`` contiguous and on a 16-byte boundary (the kernels load 16 bytes at a time)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class _ShortConvFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, cu_seqlens):
+        if weight.dim() != 3 or weight.numel() != x.shape[-1] * weight.shape[-1]:
+            raise ValueError(f"expected a filter of shape [{x.shape[-1]}, 1, ksize], got {list(weight.shape)}")
         _require_cuda(x)
+        _require_device(x.device, weight=weight, cu_seqlens=cu_seqlens)
         lib = _lib.load()
         x = x.contiguous()
         w = weight.float().contiguous()
@@ -59,6 +74,8 @@ class _ShortConvFn(torch.autograd.Function):
 
 def short_convolution(x, weight, cu_seqlens=None):
     """Causal depthwise convolution + SiLU over x [B, T, C] with filter [C, 1, ksize]."""
+    if cu_seqlens is not None:
+        cu_seqlens = cu_seqlens.to(device=x.device, dtype=torch.int64).contiguous()
     return _ShortConvFn.apply(x, weight, cu_seqlens)
 
 
@@ -79,17 +96,19 @@ class ShortConvolution(nn.Module):
     def forward(self, x, cu_seqlens=None, **unused):
         if x.shape[-1] != self.hidden_size:
             raise ValueError(f"expected last dimension {self.hidden_size}, got {x.shape[-1]}")
-        if cu_seqlens is not None:
-            cu_seqlens = cu_seqlens.to(device=x.device, dtype=torch.int64).contiguous()
-        return _ShortConvFn.apply(x, self.weight, cu_seqlens), None
+        return short_convolution(x, self.weight, cu_seqlens), None
 
 
 class _NormGateFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gate, weight, eps):
+        if gate.numel() != x.numel() or weight.numel() != x.shape[-1]:
+            raise ValueError(f"expected a gate of shape {list(x.shape)} and a weight of shape [{x.shape[-1]}], got "
+                             f"{list(gate.shape)} and {list(weight.shape)}")
         _require_cuda(x)
+        _require_device(x.device, gate=gate, weight=weight)
         lib = _lib.load()
-        x, gate = x.contiguous(), gate.to(x.dtype).contiguous()
+        x, gate = _rows(x), _rows(gate.to(x.dtype))
         w = weight.float().contiguous()
         dim = x.shape[-1]
         rows = x.numel() // dim
@@ -105,7 +124,7 @@ class _NormGateFn(torch.autograd.Function):
     def backward(ctx, dy):
         lib = _lib.load()
         x, gate, w = ctx.saved_tensors
-        dy = dy.contiguous()
+        dy = _rows(dy)
         dim = x.shape[-1]
         rows = x.numel() // dim
         n_partial = 592
