@@ -97,6 +97,14 @@ void require_cuda(const Tensor& t) {
     if (!t.is_cuda()) throw std::runtime_error("chunk_kda runs only on a CUDA device (sm_100a); there is no CPU fallback");
 }
 
+// the kernels follow raw pointers: every tensor of a call has to be where q is
+void require_device(const Tensor& q, std::initializer_list<std::pair<const char*, const Tensor*>> others) {
+    for (const auto& [name, t] : others)
+        if (t->defined() && t->device() != q.device())
+            throw std::runtime_error(std::string("expected ") + name + " on " + q.device().str() + ", the device of q, but it is on " +
+                                     t->device().str());
+}
+
 int dtype_code(const Tensor& t) {
     if (t.scalar_type() == at::kBFloat16) return KDA_DTYPE_BF16;
     if (t.scalar_type() == at::kFloat) return KDA_DTYPE_F32;
@@ -109,11 +117,12 @@ Tensor ready(const Tensor& t, at::ScalarType dt) {
     if (!r.is_contiguous()) r = r.contiguous();
     return (reinterpret_cast<uintptr_t>(r.data_ptr()) & 15) == 0 ? r : r.clone();
 }
-Tensor ready_f32(const OptTensor& t) { return t && t->defined() ? ready(*t, at::kFloat) : Tensor(); }
+Tensor ready_f32(const Tensor& t) { return t.defined() ? ready(t, at::kFloat) : t; }
 // a new tensor without the dispatcher's detour (half of what at::empty costs)
 Tensor fresh(at::IntArrayRef sizes, at::ScalarType dt, const Tensor& like) {
     return Tensor(at::detail::empty_cuda(sizes, dt, like.device(), std::nullopt));
 }
+Tensor val(const OptTensor& t) { return t ? *t : Tensor(); }
 template <class T>
 T* ptr(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr; }
 
@@ -143,11 +152,13 @@ std::tuple<Tensor, OptTensor> recurrent(const Tensor& q, const Tensor& k, const 
                     c10::toString(state->scalar_type()) + " " + shape_of(*state));
     if (gate && (!A_log || A_log->numel() != H || (dt_bias && dt_bias->numel() != H * K)))
         value_error("use_gate_in_kernel=True needs A_log with H entries (and dt_bias with H*K entries)");
+    const Tensor s0 = val(state), a0 = gate ? val(A_log) : Tensor(), b0 = gate ? val(dt_bias) : Tensor();
+    require_device(q, {{"k", &k}, {"v", &v}, {"g", &g}, {"beta", &beta}, {"state", &s0}, {"A_log", &a0}, {"dt_bias", &b0}});
     at::NoGradGuard no_grad;
     c10::cuda::CUDAGuard guard(q.device());
     const auto dt = q.scalar_type();
     const Tensor qc = ready(q, dt), kc = ready(k, dt), vc = ready(v, dt), gc = ready(g, dt), bc = ready(beta, dt);
-    const Tensor a = gate ? ready_f32(A_log) : Tensor(), b = gate ? ready_f32(dt_bias) : Tensor();
+    const Tensor a = ready_f32(a0), b = ready_f32(b0);
     Tensor s_in, s_out;
     if (state) s_in = ready(*state, at::kFloat);
     if (want_state) {
@@ -367,7 +378,6 @@ Spec load_spec(AutogradContext* ctx) {
 }
 Tensor as_filter(const Tensor& w) { return w.defined() ? w.view({w.size(0), 1, w.size(1)}) : w; }
 
-Tensor val(const OptTensor& t) { return t ? *t : Tensor(); }
 OptTensor opt(const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); }  // (a node's inputs must be defined tensors)
 
 struct ChunkKda : torch::autograd::Function<ChunkKda> {
@@ -449,6 +459,8 @@ std::tuple<Tensor, OptTensor> chunk_kda(const Tensor& q, const Tensor& k, const 
     sp.flags = (int)flags;
     sp.output_final_state = output_final_state;
     const Tensor h = val(h0), wq = val(cq), wk = val(ck), wv = val(cv);
+    require_device(q, {{"k", &k}, {"v", &v}, {"g", &g}, {"beta", &beta}, {"A_log", &a}, {"dt_bias", &b}, {"initial_state", &h},
+                       {"short_conv_weights[0]", &wq}, {"short_conv_weights[1]", &wk}, {"short_conv_weights[2]", &wv}});
     bool grad = false;
     if (at::GradMode::is_enabled())
         for (const Tensor* t : {&q, &k, &v, &g, &beta, (const Tensor*)&a, (const Tensor*)&b, &h, &wq, &wk, &wv})
