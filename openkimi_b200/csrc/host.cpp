@@ -9,6 +9,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/extension.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <optional>
@@ -29,7 +30,7 @@ constexpr int CHUNK = KDA_CHUNK;
 // ---- per-device status word and its pinned host mirror (owned by ops._DeviceStatus) -------------------------
 constexpr int MAX_DEVICES = 64;
 struct StatusWord {
-    int32_t* dev = nullptr;
+    std::atomic<int32_t*> dev{nullptr};  // set after host: calls of other threads look without the interpreter lock
     const volatile int32_t* host = nullptr;
 };
 StatusWord g_status[MAX_DEVICES];
@@ -41,7 +42,8 @@ py::object* g_guard_span = nullptr;
 
 void set_status(int device, int64_t dev_ptr, int64_t host_ptr) {
     TORCH_CHECK(device >= 0 && device < MAX_DEVICES, "device index out of range");
-    g_status[device] = {reinterpret_cast<int32_t*>(dev_ptr), reinterpret_cast<const volatile int32_t*>(host_ptr)};
+    g_status[device].host = reinterpret_cast<const volatile int32_t*>(host_ptr);
+    g_status[device].dev.store(reinterpret_cast<int32_t*>(dev_ptr), std::memory_order_release);
 }
 
 void set_callbacks(py::object status_of, py::object report, py::object guard_span) {
@@ -52,10 +54,10 @@ void set_callbacks(py::object status_of, py::object report, py::object guard_spa
 
 const StatusWord& status_word(int device) {
     TORCH_CHECK(device >= 0 && device < MAX_DEVICES, "device index out of range");
-    StatusWord& st = g_status[device];
-    if (!st.dev || *st.host) {
+    const StatusWord& st = g_status[device];
+    if (!st.dev.load(std::memory_order_acquire) || *st.host) {
         py::gil_scoped_acquire gil;
-        if (!st.dev) (*g_status_of)(device);
+        if (!st.dev.load(std::memory_order_relaxed)) (*g_status_of)(device);
         if (*st.host) (*g_report)(device);  // a wait that gave up in an earlier call surfaces here
     }
     return st;
@@ -229,7 +231,7 @@ Prepared prepare(const Inputs& in, const Spec& sp, int flags) {
         p.conv_ksize = (int)in.conv_q.size(-1);
     }
     const StatusWord& st = status_word(q.device().index());
-    p.status = st.dev;
+    p.status = st.dev.load(std::memory_order_relaxed);
     p.status_host = const_cast<int32_t*>(st.host);
     check_rc(kda_workspace_bytes(&p, &r.fwd_bytes, &r.bwd_bytes), "kda_workspace_bytes");
     return r;
@@ -720,8 +722,10 @@ PYBIND11_MODULE(_host, m) {
     m.def("set_status", &set_status);
     m.def("set_callbacks", &set_callbacks);
     m.def("env_flags", &env_flags);
-    m.def("recurrent", &recurrent);
-    m.def("chunk_kda", &chunk_kda);
-    m.def("layer", &layer);
+    // allocations and launches may wait for the device, so other Python threads run meanwhile
+    const py::call_guard<py::gil_scoped_release> unlocked;
+    m.def("recurrent", &recurrent, unlocked);
+    m.def("chunk_kda", &chunk_kda, unlocked);
+    m.def("layer", &layer, unlocked);
     m.def("layer_takes", &layer_takes);
 }
