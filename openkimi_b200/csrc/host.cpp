@@ -9,6 +9,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
@@ -573,8 +574,8 @@ struct Layer : torch::autograd::Function<Layer> {
         ctx->save_for_backward(std::move(keep));
         save_spec(ctx, ls.op);
         ctx->saved_data["eps"] = ls.eps;
-        std::vector<int64_t> f32;  // which parameters want an FP32 gradient
-        for (const Tensor& t : prm) f32.push_back(t.scalar_type() == at::kFloat);
+        std::vector<int64_t> f32;  // which parameters want a gradient of more than 16 bits
+        for (const Tensor& t : prm) f32.push_back(t.element_size() > 2);
         ctx->saved_data["f32"] = f32;
         return {out};
     }
@@ -591,12 +592,14 @@ struct Layer : torch::autograd::Function<Layer> {
         const auto bf = x2.options();
         const Tensor dout = ready(grads[0], at::kBFloat16).view({n, width});
         auto need = [&](int which) { return ctx->needs_input_grad(1 + which); };
-        // weight gradients in the parameters' own type, straight from the GEMM's FP32 accumulators
-        auto weight_grad = [&](const Tensor& a, const Tensor& b, int which) {
-            if (a.dim() == 3) return f32[which] ? at::bmm(a, b, at::kFloat) : at::bmm(a, b);
-            return f32[which] ? at::mm(a, b, at::kFloat) : at::mm(a, b);
+        // weight gradients straight from the GEMM's FP32 accumulators in FP32 if one of the parameters that share the product
+        // has it (the engine rounds the others' shares to their types)
+        auto weight_grad = [&](const Tensor& a, const Tensor& b, std::initializer_list<int> which) {
+            const bool wide = std::any_of(which.begin(), which.end(), [&](int i) { return f32[i]; });
+            if (a.dim() == 3) return wide ? at::bmm(a, b, at::kFloat) : at::bmm(a, b);
+            return wide ? at::mm(a, b, at::kFloat) : at::mm(a, b);
         };
-        if (need(P_WO)) r[1 + P_WO] = weight_grad(dout.t(), y, P_WO);
+        if (need(P_WO)) r[1 + P_WO] = weight_grad(dout.t(), y, {P_WO});
         const Tensor dy = at::mm(dout, w.out);
         // norm and gate
         const Tensor dab = at::empty({2, n, proj}, bf);  // gradients of the decay and of the output gate
@@ -633,22 +636,22 @@ struct Layer : torch::autograd::Function<Layer> {
                 for (int i : {0, 1}) {
                     const Tensor rows = narrow.as_strided({CUT, n / CUT, HD}, {n / CUT * wide, wide, 1}, narrow.storage_offset() + i * HD);
                     const Tensor d = at::bmm(dab[i].view({CUT, n / CUT, proj}).transpose(1, 2), rows, at::kFloat).sum(0);
-                    r[1 + (i ? P_GB : P_FB)] = f32[P_FB] ? d : d.to(at::kBFloat16);
+                    r[1 + (i ? P_GB : P_FB)] = d;
                 }
             } else {
-                const Tensor d = weight_grad(dab.transpose(1, 2), rank_pair(narrow), P_FB);
+                const Tensor d = weight_grad(dab.transpose(1, 2), rank_pair(narrow), {P_FB, P_GB});
                 r[1 + P_FB] = d[0];
                 r[1 + P_GB] = d[1];
             }
         }
         if (need(P_FA) || need(P_GA) || need(P_BETA)) {
-            const Tensor d = weight_grad(dn.t(), x2, P_FA);
+            const Tensor d = weight_grad(dn.t(), x2, {P_FA, P_GA, P_BETA});
             r[1 + P_FA] = d.narrow(0, 0, HD);
             r[1 + P_GA] = d.narrow(0, HD, HD);
             r[1 + P_BETA] = d.narrow(0, 2 * HD, H);
         }
         if (need(P_WQ) || need(P_WK) || need(P_WV)) {
-            const Tensor d = weight_grad(dqkv.transpose(1, 2), x2.unsqueeze(0).expand({3, n, width}), P_WQ);
+            const Tensor d = weight_grad(dqkv.transpose(1, 2), x2.unsqueeze(0).expand({3, n, width}), {P_WQ, P_WK, P_WV});
             r[1 + P_WQ] = d[0];
             r[1 + P_WK] = d[1];
             r[1 + P_WV] = d[2];
