@@ -536,6 +536,34 @@ Tensor rank_pair(const Tensor& narrow) {
     return narrow.as_strided({2, narrow.size(0), HD}, {HD, narrow.size(1), 1}, narrow.storage_offset());
 }
 
+// The gradients of the two weights behind the ranks, [proj x 128] each, sum over all tokens.  cuBLAS does not split the
+// inner dimension of a batch of two, so one CTA per 128 x 128 tile walks every token: 1.2 ns each however many tiles there are
+// (up to sixteen heads on 148 SMs).  Cut into pieces the products are bound by their operands, 4 (proj + 128) bytes per token
+// at 6.2 TB/s, and cost more launches, partial results and, where the tokens leave a remainder, one more product: some 14 us
+// for two to six heads, 20 with a remainder.  The line leaves a margin to that.  Batch against pieces of an eighth (us):
+//   tokens            24576        32768        49152        49149        65536       131072
+//   1 head          36 : 26      46 : 29      65 : 38      65 : 47      84 : 42     161 : 67
+//   6 heads         42 : 40      52 : 46      73 : 58      73 : 63      92 : 71     169 : 108
+//   12 heads        51 : 54      63 : 65      84 : 85      84 : 89     103 : 101    184 : 165
+//   16 heads        56 : 65      69 : 77      91 : 99      91 : 107    112 : 122    201 : 206
+bool rank_cut(int64_t n, int64_t proj) { return n * (1.2 - 4.0 * (proj + HD) / 6200.0) > 26000.0; }
+
+Tensor rank_gradients_cut(const Tensor& dab, const Tensor& narrow) {
+    constexpr int64_t CUT = 8;
+    const int64_t n = dab.size(1), proj = dab.size(2), wide = narrow.size(1), len = n / CUT, rest = n % CUT;
+    const Tensor parts = at::empty({2, CUT + (rest > 0), proj, HD}, dab.options().dtype(at::kFloat));
+    for (int i : {0, 1}) {
+        Tensor out = parts[i].narrow(0, 0, CUT);
+        const Tensor rows = narrow.as_strided({CUT, len, HD}, {len * wide, wide, 1}, narrow.storage_offset() + i * HD);
+        at::bmm_out(out, dab[i].narrow(0, 0, CUT * len).view({CUT, len, proj}).transpose(1, 2), rows, at::kFloat);
+    }
+    if (rest) {
+        Tensor out = parts.select(1, CUT);
+        at::bmm_out(out, dab.narrow(1, CUT * len, rest).transpose(1, 2), rank_pair(narrow.narrow(0, CUT * len, rest)), at::kFloat);
+    }
+    return parts.sum(1);
+}
+
 Tensor layer_fwd(const Tensor& x, const variable_list& prm, const LayerSpec& ls, const Inputs& tables, LayerState& st, bool recompute = false) {
     const int64_t H = ls.H, proj = H * HD, width = x.size(-1), wide = (2 * HD + H + 7) / 8 * 8;
     const int64_t B = x.size(0), T = x.size(1), n = B * T;
@@ -628,21 +656,10 @@ struct Layer : torch::autograd::Function<Layer> {
         dn.narrow(1, 2 * HD, H).copy_(gr.beta.view({n, H}));
         if (wide > 2 * HD + H) dn.narrow(1, 2 * HD + H, wide - 2 * HD - H).zero_();
         if (need(P_FB) || need(P_GB)) {
-            // A long inner dimension is cut into eight by hand: cuBLAS splits it over the chip for a single product, but not
-            // for a batch of two small results (2 x [768 x 128] from 131072 tokens: 157 us as a batch, 112 as two products,
-            // 95 cut into eight).  Below 65536 tokens the batch is faster (32768: 45 us against 62 and 69).
-            constexpr int64_t CUT = 8;
-            if (n >= 65536 && n % CUT == 0) {
-                for (int i : {0, 1}) {
-                    const Tensor rows = narrow.as_strided({CUT, n / CUT, HD}, {n / CUT * wide, wide, 1}, narrow.storage_offset() + i * HD);
-                    const Tensor d = at::bmm(dab[i].view({CUT, n / CUT, proj}).transpose(1, 2), rows, at::kFloat).sum(0);
-                    r[1 + (i ? P_GB : P_FB)] = d;
-                }
-            } else {
-                const Tensor d = weight_grad(dab.transpose(1, 2), rank_pair(narrow), {P_FB, P_GB});
-                r[1 + P_FB] = d[0];
-                r[1 + P_GB] = d[1];
-            }
+            const Tensor d = rank_cut(n, proj) ? rank_gradients_cut(dab, narrow)
+                                               : weight_grad(dab.transpose(1, 2), rank_pair(narrow), {P_FB, P_GB});
+            r[1 + P_FB] = d[0];
+            r[1 + P_GB] = d[1];
         }
         if (need(P_FA) || need(P_GA) || need(P_BETA)) {
             const Tensor d = weight_grad(dn.t(), x2, {P_FA, P_GA, P_BETA});

@@ -25,3 +25,26 @@ def test_gradient_of_two_halves(dtype):
     tol = 1e-3 if dtype == torch.float32 else 1e-2
     for k in whole:
         assert rel_l2(whole[k], a[k] + b[k]) < tol, k
+
+
+@pytest.mark.parametrize("heads,tokens", [(1, 15000), (1, 13000), (2, 13999), (3, 20003), (6, 20905), (6, 20951)])
+def test_rank_gradients_around_the_line(heads, tokens):
+    """Two sequences together against each alone: cut or not, with every kind of remainder.  FP32 sums over up to 42000 tokens in
+    different orders: 42000 * 2^-24 = 2.5e-3 of the sum of the terms' magnitudes at the very worst, sqrt(42000) * 2^-24 = 1.2e-5
+    expected; 1e-4 of the norm."""
+    from openkimi_b200 import KimiDeltaAttention
+    from tests.kda_testlib import rel_l2
+
+    torch.manual_seed(tokens)
+    mod = KimiDeltaAttention(128, heads).cuda()
+    x, dy = (torch.randn(2, tokens, 128, device="cuda").bfloat16() for _ in range(2))
+
+    def grads(a, d):
+        mod.zero_grad(set_to_none=True)
+        with torch.autocast("cuda", torch.bfloat16):
+            mod(a).backward(d)
+        return [mod.f_b_proj.weight.grad.double(), mod.out_gate_b.weight.grad.double()]
+
+    whole, a, b = grads(x, dy), grads(x[:1], dy[:1]), grads(x[1:], dy[1:])
+    for w, p, q in zip(whole, a, b):
+        assert rel_l2(w, p + q) < 1e-4
