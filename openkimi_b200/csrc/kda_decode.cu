@@ -275,18 +275,26 @@ template <typename T, int D, bool VF, int R>
 static cudaError_t launch_recurrent(const RecurrentArgs& a, cudaStream_t s) {
     const int tb = a.T < dec::TB ? a.T : dec::TB;
     const size_t smem = (size_t)tb * dec::tok_floats(D) * sizeof(float);
-    return launch_dependent(
-        kda_recurrent_kernel<T, D, VF, R>, a.N * a.H * (D / (R * dec::NW)), 32 * dec::NW, smem, s, (const T*)a.q, (const T*)a.k, (const T*)a.v, (const T*)a.g, (const T*)a.beta, a.A_log, a.dt_bias, a.state_in,
-        a.state_out, (T*)a.o, a.H, a.T, a.flags, a.scale, a.vec);
+    return launch_dependent(kda_recurrent_kernel<T, D, VF, R>, a.N * a.H * (D / (R * dec::NW)), 32 * dec::NW, smem, s,
+                            (const T*)a.q, (const T*)a.k, (const T*)a.v, (const T*)a.g, (const T*)a.beta, a.A_log, a.dt_bias,
+                            a.state_in, a.state_out, (T*)a.o, a.H, a.T, a.flags, a.scale, a.vec);
 }
 
-// Columns per warp: eight (D / 32 CTAs per unit, short dependent chains per token) until the CTAs fill the chip twice
-// over, then sixteen (half as many CTAs evaluate the same token's prologue; 36.3 against 36.1 us at 1536 units, so the
-// line could lie anywhere above it).
+// Columns per warp: eight give short dependent chains per token, sixteen half as many CTAs that evaluate the same token's
+// prologue, more loads in flight per warp and, for [dk][dv] states, 64 instead of 32 consecutive bytes per access.  So eight
+// until every SM has 64 KB of [dv][dk] states, or 16 KB of [dk][dv] states, to move.  Eight against sixteen (us; d = 128 unless
+// said, BF16, launches back to back):
+//   units                      6            48           148           222           592          1536
+//   [dv][dk], 1 token      3.0 : 3.5    3.6 : 3.7     4.9 : 5.0     7.5 : 5.8    14.2 : 13.4   35.8 : 36.0
+//   [dv][dk], 16 tokens   11.3 : 13.6  13.6 : 14.0   19.0 : 18.2   32.2 : 22.4   69.7 : 58.7    171 : 152
+//   [dk][dv], 1 token      3.5 : 3.7    4.4 : 3.8     5.9 : 4.9     9.5 : 6.0    19.4 : 12.8   48.1 : 36.3
+//   [dk][dv], 16 tokens   11.4 : 13.2  14.1 : 13.6   20.1 : 17.7   34.1 : 22.0   76.2 : 53.8    184 : 137
+//   d = 64, [dv][dk], 1    2.6 : 2.7    2.7 : 2.8     2.9 : 2.9     3.2 : 3.4     4.3 : 4.5     9.2 : 8.4
+//   d = 64, [dk][dv], 1    2.7 : 2.7    2.8 : 2.8     3.3 : 3.0     3.7 : 3.5     5.3 : 4.5    12.8 : 9.9
 template <typename T, int D>
 static cudaError_t launch_columns(const RecurrentArgs& a, cudaStream_t s) {
     const bool vf = a.flags & KDA_FLAG_STATE_V_FIRST;
-    if ((long long)a.N * a.H * (D / 32) < 8LL * sm_count())
+    if ((long long)a.N * a.H * D * D < (vf ? 16384LL : 4096LL) * sm_count())
         return vf ? launch_recurrent<T, D, true, 8>(a, s) : launch_recurrent<T, D, false, 8>(a, s);
     return vf ? launch_recurrent<T, D, true, 16>(a, s) : launch_recurrent<T, D, false, 16>(a, s);
 }
