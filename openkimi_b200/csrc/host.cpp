@@ -3,6 +3,7 @@
 // The Python modules keep the public signatures and everything that is not on such a path.
 //
 // No tensor is kept from one call for the next; the only state here is the table of the devices' status words.
+#include <ATen/MemoryOverlap.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -150,6 +151,7 @@ std::tuple<Tensor, OptTensor> recurrent(const Tensor& q, const Tensor& k, const 
         value_error("beta must have the shape of q without its last axis, got " + shape_of(beta));
     const int dtype = dtype_code(q);
     const std::array<int64_t, 4> want = {N, H, K, K};
+    if (!state && !multi) type_error("recurrent_kda_step needs a state");
     if (state && (state->scalar_type() != at::kFloat || state->sizes() != at::IntArrayRef(want)))
         value_error("state must be float32 [N,H," + std::to_string(K) + "," + std::to_string(K) + "], got " +
                     c10::toString(state->scalar_type()) + " " + shape_of(*state));
@@ -162,11 +164,17 @@ std::tuple<Tensor, OptTensor> recurrent(const Tensor& q, const Tensor& k, const 
     const auto dt = q.scalar_type();
     const Tensor qc = ready(q, dt), kc = ready(k, dt), vc = ready(v, dt), gc = ready(g, dt), bc = ready(beta, dt);
     const Tensor a = ready_f32(a0), b = ready_f32(b0);
-    Tensor s_in, s_out;
+    Tensor s_in, s_out, s_back;  // s_back: a state to be updated that the kernel cannot write itself
     if (state) s_in = ready(*state, at::kFloat);
     if (want_state) {
-        if (inplace && s_in.data_ptr() == state->data_ptr()) s_out = s_in.requires_grad() ? s_in.detach() : s_in;
-        else s_out = fresh(want, at::kFloat, q);
+        const Tensor own = inplace ? (state->requires_grad() ? state->detach() : *state) : Tensor();
+        if (inplace && s_in.data_ptr() == own.data_ptr()) {
+            s_out = own;
+        } else {
+            s_out = fresh(want, at::kFloat, q);
+            // (an expanded state has no memory of its own to update: the new state is returned alone)
+            if (inplace && at::has_internal_overlap(own) != at::MemOverlap::Yes) s_back = own;
+        }
     }
     Tensor o = fresh(q.sizes(), dt, q);
     status_word(q.device().index());
@@ -183,6 +191,7 @@ std::tuple<Tensor, OptTensor> recurrent(const Tensor& q, const Tensor& k, const 
                                ptr<float>(s_in), ptr<float>(s_out), o.data_ptr(), (int)N, (int)T, (int)H, (int)K, (int)K, dtype, flags,
                                (float)scale.value_or(1.0 / std::sqrt((double)K)), stream_of(q)),
              "kda_recurrent_fwd");
+    if (s_back.defined()) s_out = s_back.copy_(s_out);
     return {o, want_state ? OptTensor(s_out) : OptTensor()};
 }
 

@@ -31,3 +31,28 @@ def test_tensors_on_another_device_raise():
     y = dict(x, g=-x["g"].abs(), beta=x["beta"].sigmoid(), A_log=x["A_log"].cpu(), dt_bias=None)
     chunk_kda(**y)
     fused_recurrent_kda(**y)
+
+
+def test_in_place_states_of_any_layout():
+    """A state off a 16-byte boundary, or with strides of its own, is updated in place like any other."""
+    x = _inputs(3)
+    want = torch.randn(3, 2, 128, 128, device="cuda")
+    buf = torch.empty(1 + want.numel(), device="cuda")
+    off, strided = buf[1:].view(want.shape), torch.empty(3, 2, 128, 256, device="cuda")[..., ::2]
+    o1, s1 = recurrent_kda_step(**x, state=want, **FUSED)
+    for state in (off, strided, want.transpose(-1, -2).contiguous().transpose(-1, -2), want.clone().requires_grad_(True)):
+        with torch.no_grad():
+            state.copy_(want)
+        o2, s2 = recurrent_kda_step(**x, state=state, inplace=True, **FUSED)
+        assert torch.equal(o1, o2) and torch.equal(s1, state) and torch.equal(s1, s2)
+        assert s2.data_ptr() == state.data_ptr() and not s2.requires_grad
+    wide = want[:1].expand(3, -1, -1, -1).contiguous()
+    o3, s3 = recurrent_kda_step(**x, state=wide, **FUSED)
+    o4, s4 = recurrent_kda_step(**x, state=want[:1].expand(3, -1, -1, -1), inplace=True, **FUSED)
+    assert torch.equal(o3, o4) and torch.equal(s3, s4) and not torch.equal(want[0], s4[0])
+
+
+def test_a_step_needs_a_state():
+    for inplace in (False, True):
+        with pytest.raises(TypeError, match="state"):
+            recurrent_kda_step(**_inputs(2), state=None, inplace=inplace, **FUSED)
