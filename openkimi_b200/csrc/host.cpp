@@ -109,6 +109,14 @@ void require_device(const Tensor& q, std::initializer_list<std::pair<const char*
                                      t->device().str());
 }
 
+// A call that nobody differentiates backward does not pass through its autograd node, which refuses forward-mode inputs.
+template <class Tensors>
+void refuse_tangents(const Tensors& inputs) {
+    for (const Tensor* t : inputs)
+        if (t->defined() && t->_fw_grad(0).defined())
+            throw std::runtime_error("the KDA kernels have no forward-mode derivative (an input carries a tangent)");
+}
+
 int dtype_code(const Tensor& t) {
     if (t.scalar_type() == at::kBFloat16) return KDA_DTYPE_BF16;
     if (t.scalar_type() == at::kFloat) return KDA_DTYPE_F32;
@@ -473,10 +481,11 @@ std::tuple<Tensor, OptTensor> chunk_kda(const Tensor& q, const Tensor& k, const 
     const Tensor h = val(h0), wq = val(cq), wk = val(ck), wv = val(cv);
     require_device(q, {{"k", &k}, {"v", &v}, {"g", &g}, {"beta", &beta}, {"A_log", &a}, {"dt_bias", &b}, {"initial_state", &h},
                        {"short_conv_weights[0]", &wq}, {"short_conv_weights[1]", &wk}, {"short_conv_weights[2]", &wv}});
+    const std::array<const Tensor*, 11> inputs = {&q, &k, &v, &g, &beta, &a, &b, &h, &wq, &wk, &wv};
+    refuse_tangents(inputs);
     bool grad = false;
     if (at::GradMode::is_enabled())
-        for (const Tensor* t : {&q, &k, &v, &g, &beta, (const Tensor*)&a, (const Tensor*)&b, &h, &wq, &wk, &wv})
-            grad = grad || (t->defined() && t->requires_grad());
+        for (const Tensor* t : inputs) grad = grad || (t->defined() && t->requires_grad());
     c10::cuda::CUDAGuard guard(q.device());
     if (!grad) {
         at::NoGradGuard no_grad;
@@ -727,11 +736,12 @@ OptTensor layer(const Tensor& x, const std::vector<Tensor>& prm, int64_t H, doub
     ls.op.NT = cu ? NT : x.size(0) * ((x.size(1) + CHUNK - 1) / CHUNK);
     Inputs tables;
     if (cu) take_tables(tables, cu, chunk_seq, seq_off, chunk_tab, x.size(0));
+    std::array<const Tensor*, 1 + P_COUNT> inputs = {&x};
+    for (int i = 0; i < P_COUNT; ++i) inputs[1 + i] = &prm[i];
+    refuse_tangents(inputs);
     bool grad = false;
-    if (at::GradMode::is_enabled()) {
-        grad = x.requires_grad();
-        for (const Tensor& t : prm) grad = grad || t.requires_grad();
-    }
+    if (at::GradMode::is_enabled())
+        for (const Tensor* t : inputs) grad = grad || t->requires_grad();
     c10::cuda::CUDAGuard guard(x.device());
     // the node does its own conversions; autocast must not see its matrix products
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
