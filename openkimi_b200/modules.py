@@ -259,7 +259,7 @@ class KimiDeltaAttention(nn.Module):
         prm = self._native_parameters(x)
         if prm is not None and not _lib.host().env_flags():
             out = _lib.host().layer(x, prm, self.n_heads, self.scale, self.out_norm_gate.eps, self.disable_recompute,
-                                    *_packed_tables(cu_seqlens, None, x.device))
+                                    *_packed_tables(cu_seqlens, None, x))
             if out is not None:
                 return out
         # The three narrow projections of x (decay rank, output-gate rank, beta) share one GEMM: x is

@@ -37,21 +37,24 @@ def _chunk_tables_cached(cu: tuple, device_index: int):
             torch.tensor(tab if tab else [(0, 0, 0, 0)], dtype=torch.int32, device=dev), max(counts, default=0))
 
 
-def _chunk_tables(cu_seqlens, cu_seqlens_cpu, device):
+def _chunk_tables(cu_seqlens, cu_seqlens_cpu, device, tokens):
     """Per-chunk sequence index and per-sequence first chunk.  Chunks never straddle a
     document boundary, so the table depends on the lengths; it is built on the host
     (``cu_seqlens_cpu`` avoids the device-to-host copy) and cached per length tuple."""
     host = cu_seqlens_cpu if cu_seqlens_cpu is not None else cu_seqlens.cpu()
-    return _chunk_tables_cached(tuple(int(x) for x in host.tolist()), device.index or 0)
+    cu = tuple(int(x) for x in host.tolist())
+    if cu and (cu[0] < 0 or cu[-1] > tokens):
+        raise ValueError(f"cu_seqlens must stay within the {tokens} tokens of the batch, got {cu[0]} to {cu[-1]}")
+    return _chunk_tables_cached(cu, device.index or 0)
 
 
-def _packed_tables(cu_seqlens, cu_seqlens_cpu, device):
+def _packed_tables(cu_seqlens, cu_seqlens_cpu, x):
     """(cu_seqlens, chunk_seq, seq_chunk_off, chunk_tab, number of chunks, chunks of the longest document) as the native
-    calls take them."""
+    calls take them, for documents packed into the [B, T, ...] tensor x."""
     if cu_seqlens is None:
         return None, None, None, None, 0, 0
-    seq, off, nt, tab, longest = _chunk_tables(cu_seqlens, cu_seqlens_cpu, device)
-    return cu_seqlens.to(device=device, dtype=torch.int64).contiguous(), seq, off, tab, nt, longest
+    seq, off, nt, tab, longest = _chunk_tables(cu_seqlens, cu_seqlens_cpu, x.device, x.shape[:2].numel())
+    return cu_seqlens.to(device=x.device, dtype=torch.int64).contiguous(), seq, off, tab, nt, longest
 
 
 class _DeviceStatus:
@@ -190,7 +193,7 @@ def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_sta
                        for x, w in zip((q, k, v), (wq, wk, wv)))
             wq = wk = wv = None
     return host.chunk_kda(q, k, v, g, beta, A_log, dt_bias, initial_state, wq, wk, wv, scale, flags, output_final_state,
-                          disable_recompute, *_packed_tables(cu_seqlens, cu_seqlens_cpu, q.device))
+                          disable_recompute, *_packed_tables(cu_seqlens, cu_seqlens_cpu, q))
 
 
 def recurrent_kda_step(q, k, v, g, beta, state, *, scale=None, A_log=None, dt_bias=None,
