@@ -10,6 +10,7 @@ import math
 
 import torch
 import torch.nn as nn
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import _lib
 from .ops import chunk_kda, _DTYPES, _packed_tables, _require_cuda
@@ -197,6 +198,12 @@ class _InputProjections(torch.autograd.Function):
         return (dx, *grads, None, None)
 
 
+def _plain(m, cls):
+    """Whether calling ``m`` runs cls.forward and nothing else."""
+    return type(m) is cls and "forward" not in m.__dict__ and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks
+                                                                   or m._backward_pre_hooks)
+
+
 class KimiDeltaAttention(nn.Module):
     """The KDA sublayer of k3mini/model.py:132-227 on the B200 kernels: q/k/v projections,
     short conv + SiLU, decay and beta projections, ``chunk_kda`` with the fused L2 norm /
@@ -238,13 +245,8 @@ class KimiDeltaAttention(nn.Module):
             return None
         parts = (self.q_proj, self.k_proj, self.v_proj, self.f_a_proj, self.f_b_proj, self.beta_proj, self.out_gate_a,
                  self.out_gate_b, self.out_proj)
-        for m in parts:
-            if type(m) is not nn.Linear or m.bias is not None or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks \
-                    or m._backward_pre_hooks:
-                return None
         norm = self.out_norm_gate
-        if type(norm) is not FusedRMSNormGated or norm._forward_hooks or norm._forward_pre_hooks or norm._backward_hooks \
-                or norm._backward_pre_hooks:
+        if _has_any_global_hook() or not _plain(norm, FusedRMSNormGated) or not all(_plain(m, nn.Linear) and m.bias is None for m in parts):
             return None
         if torch.is_autocast_enabled("cuda"):
             if torch.get_autocast_dtype("cuda") != torch.bfloat16 or x.dtype not in (torch.bfloat16, torch.float32):
