@@ -43,3 +43,27 @@ def test_forward_only_segments_match_the_saving_forward():
         o, s = chunk_kda(*args, **kw)
     o2, s2 = chunk_kda(args[0].requires_grad_(True), *args[1:], **kw)
     assert torch.equal(o, o2) and torch.equal(s, s2)
+
+
+@pytest.mark.parametrize("name", ["one_ragged", "first_long", "uneven"])
+@pytest.mark.parametrize("recompute", [False, True])
+def test_segments_with_the_fused_convolution(name, recompute):
+    """The border states lie behind another workspace with the convolution, and outside it with the recompute policy."""
+    import ctypes as C
+
+    from openkimi_b200 import _lib
+    from tests.test_fused_conv_gpu import _inputs, _run, _same
+
+    lens = CASES[name]
+    p, n = _lib.KdaParams(), C.c_size_t()
+    p.B, p.T, p.H, p.N, p.dk, p.dv, p.dtype = 1, sum(lens), 2, len(lens), 128, 128, _lib.DTYPE_BF16
+    p.NT, p.max_chunks = sum(-(-l // 64) for l in lens), max(-(-l // 64) for l in lens)
+    assert _lib.load().kda_border_bytes(C.byref(p), C.byref(n)) == 0 and n.value > 0  # this size is cut into segments
+    t = _inputs(1, sum(lens), 2, 128, 4, seed=13)
+    gen = torch.Generator().manual_seed(14)
+    t["A_log"] = torch.log(torch.empty(2).uniform_(0.02, 1.0, generator=gen))  # slow decay: states last
+    kw = dict(cu=torch.tensor([0] + lens).cumsum(0), h0=torch.randn(len(lens), 2, 128, 128, generator=gen) * 0.1)
+    dev = _run(t, True, disable_recompute=not recompute, **kw)
+    _same(dev, _run(t, False, disable_recompute=not recompute, **kw))
+    ref = _run(t, False, fp32_math=True, **kw)
+    assert_rows(compare(dev, ref, tol_max=2e-2, tol_l2=1.5e-2, names=tuple(ref)))
