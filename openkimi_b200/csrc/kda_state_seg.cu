@@ -14,9 +14,9 @@
 // walks the other way with X^T.  Work doubles (and X costs as much again, on warps that would idle), the chain shrinks
 // from n chunks to 2 len + n / len short steps.
 //
-// Measured (six heads): one sequence of 256 chunks, forward, 24 segments: 498 -> 32 + 32 + 28 us (at 148 busy SMs the walks
-// are bound by the records' traffic, 5.5 TB/s); 16 documents of 65536 tokens, both directions: 838 -> 520 us; 4 sequences
-// of 64 chunks: 454 -> 237 us.
+// Measured (six heads, the launches of the stage together): one sequence of 256 chunks, forward: 503 -> 95 us, of which
+// some 30 for step 1 and 35 for step 3 (at 148 busy SMs the walks are bound by the records' traffic, 5.5 TB/s); 16 documents of
+// 65536 tokens, both directions: 905 -> 514 us; 4 sequences of 64 chunks, both directions: 339 -> 183 us.
 #include <math.h>
 
 #include <algorithm>

@@ -298,8 +298,7 @@ __device__ __forceinline__ bool guard_tile(const float (&G)[16], float limit, fl
     return __all_sync(0xffffffffu, good) && isfinite(span) && span <= limit;
 }
 
-// 2^x by the hardware approximation alone (results below 2^-126 flush to zero); exp2f wraps the
-// same instruction in a rescaling for denormal results that no decay factor here needs
+// 2^x by the hardware approximation (2 ulp; results below 2^-126 flush to zero, as no decay factor here needs them)
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

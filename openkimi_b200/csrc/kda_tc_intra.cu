@@ -11,9 +11,10 @@
 //      of a block pass the span guard, with the FP32 midpoint factorisation (pre-scaled key rows, no
 //      exponential per pair), otherwise with exact pairwise decays
 //   2  decay-scaled operands: for every 16-row block I >= 1 the factorised operands
-//      k_j 2^(r_I - G_j) (j < 16 I)  and  x_i 2^(G_i - r_I) (i in I),  r_I = G at the first row of block I, so that every exponent is <= 0; off-diagonal blocks of
-//      Aqk and L as tcgen05 MMAs (M = 64 keys, N = 32 = q and k rows of block I, K = 128); the Qt,
-//      Kh records and beta*k*2^G are made while these run
+//      k_j 2^(r_I - G_j) (j < 16 I)  and  x_i 2^(G_i - r_I) (i in I),  r_I = G at the first row of
+//      block I, so that every exponent is <= 0; off-diagonal blocks of Aqk and L as tcgen05 MMAs
+//      (M = 64 keys, N = 32 = q and k rows of block I, K = 128); the Qt, Kh records and beta*k*2^G
+//      are made while these run
 //   3  T = (I + diag(beta) L)^-1: forward substitution inside the diagonal blocks (beside the
 //      accumulator read-back), products for the rest (FP32); Aqk record
 //   4  T record; 5  W^T = (beta k 2^G)^T T^T and U^T = (beta v)^T T^T as tcgen05 MMAs
