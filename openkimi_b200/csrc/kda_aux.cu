@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(256) norm_gate_bwd_kernel(const T* __restrict_
         for (int i = 0; i < V; ++i) ss += xv[i] * xv[i];
 #pragma unroll
         for (int o = LPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        const float rs = rsqrtf(ss / DIM + eps);
+        const float rs = ok ? rsqrtf(ss / DIM + eps) : 0.f;  // (a row that does not exist adds nothing to dw, whatever eps)
         float dg[V];
 #pragma unroll
         for (int i = 0; i < V; i += 2) {
