@@ -102,11 +102,10 @@ void require_cuda(const Tensor& t) {
 }
 
 // the kernels follow raw pointers: every tensor of a call has to be where q is
-void require_device(const Tensor& q, std::initializer_list<std::pair<const char*, const Tensor*>> others) {
-    for (const auto& [name, t] : others)
-        if (t->defined() && t->device() != q.device())
-            throw std::runtime_error(std::string("expected ") + name + " on " + q.device().str() + ", the device of q, but it is on " +
-                                     t->device().str());
+void require_device(const Tensor& q, const char* name, const Tensor& t) {
+    if (t.defined() && t.device() != q.device())
+        throw std::runtime_error(std::string("expected ") + name + " on " + q.device().str() + ", the device of q, but it is on " +
+                                 t.device().str());
 }
 
 // A call that nobody differentiates backward does not pass through its autograd node, which refuses forward-mode inputs.
@@ -129,12 +128,19 @@ Tensor ready(const Tensor& t, at::ScalarType dt) {
     if (!r.is_contiguous()) r = r.contiguous();
     return (reinterpret_cast<uintptr_t>(r.data_ptr()) & 15) == 0 ? r : r.clone();
 }
-Tensor ready_f32(const Tensor& t) { return t.defined() ? ready(t, at::kFloat) : t; }
+// the same without a new reference where t is that already or undefined; copy holds what else it becomes
+const Tensor& ready(const Tensor& t, at::ScalarType dt, Tensor& copy) {
+    if (!t.defined() || (t.scalar_type() == dt && t.is_contiguous() && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0)) return t;
+    return copy = ready(t, dt);
+}
 // a new tensor without the dispatcher's detour (half of what at::empty costs)
 Tensor fresh(at::IntArrayRef sizes, at::ScalarType dt, const Tensor& like) {
     return Tensor(at::detail::empty_cuda(sizes, dt, like.device(), std::nullopt));
 }
-Tensor val(const OptTensor& t) { return t ? *t : Tensor(); }
+const Tensor& val(const OptTensor& t) {
+    static const Tensor none;
+    return t ? *t : none;
+}
 template <class T>
 T* ptr(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr; }
 
@@ -146,8 +152,10 @@ std::tuple<Tensor, OptTensor> recurrent(const Tensor& q, const Tensor& k, const 
                                         const OptTensor& state, const OptTensor& A_log, const OptTensor& dt_bias,
                                         std::optional<double> scale, bool l2norm, bool gate, bool sigmoid, bool v_first,
                                         bool inplace, bool multi, bool want_state) {
-    for (const Tensor* t : {&q, &k, &v, &g, &beta}) require_cuda(*t);
-    if (state) require_cuda(*state);
+    require_cuda(q);
+    const Tensor &a0 = gate ? val(A_log) : val(std::nullopt), &b0 = gate ? val(dt_bias) : val(std::nullopt), &s0 = val(state);
+    require_device(q, "k", k); require_device(q, "v", v); require_device(q, "g", g); require_device(q, "beta", beta);
+    require_device(q, "state", s0); require_device(q, "A_log", a0); require_device(q, "dt_bias", b0);
     const int64_t dims = multi ? 4 : 3;
     if (q.dim() != dims || q.sizes() != k.sizes() || g.sizes() != q.sizes())
         value_error("q, k, g must share one shape " + std::string(multi ? "[B,T,H,K]" : "[N,H,K]") + ", got " + shape_of(q) + ", " +
@@ -165,15 +173,14 @@ std::tuple<Tensor, OptTensor> recurrent(const Tensor& q, const Tensor& k, const 
                     c10::toString(state->scalar_type()) + " " + shape_of(*state));
     if (gate && (!A_log || A_log->numel() != H || (dt_bias && dt_bias->numel() != H * K)))
         value_error("use_gate_in_kernel=True needs A_log with H entries (and dt_bias with H*K entries)");
-    const Tensor s0 = val(state), a0 = gate ? val(A_log) : Tensor(), b0 = gate ? val(dt_bias) : Tensor();
-    require_device(q, {{"k", &k}, {"v", &v}, {"g", &g}, {"beta", &beta}, {"state", &s0}, {"A_log", &a0}, {"dt_bias", &b0}});
     at::NoGradGuard no_grad;
     c10::cuda::CUDAGuard guard(q.device());
     const auto dt = q.scalar_type();
-    const Tensor qc = ready(q, dt), kc = ready(k, dt), vc = ready(v, dt), gc = ready(g, dt), bc = ready(beta, dt);
-    const Tensor a = ready_f32(a0), b = ready_f32(b0);
-    Tensor s_in, s_out, s_back;  // s_back: a state to be updated that the kernel cannot write itself
-    if (state) s_in = ready(*state, at::kFloat);
+    Tensor copies[8];
+    const Tensor &qc = ready(q, dt, copies[0]), &kc = ready(k, dt, copies[1]), &vc = ready(v, dt, copies[2]),
+                 &gc = ready(g, dt, copies[3]), &bc = ready(beta, dt, copies[4]), &a = ready(a0, at::kFloat, copies[5]),
+                 &b = ready(b0, at::kFloat, copies[6]), &s_in = ready(s0, at::kFloat, copies[7]);
+    Tensor s_out, s_back;  // s_back: a state to be updated that the kernel cannot write itself
     if (want_state) {
         const Tensor own = inplace ? (state->requires_grad() ? state->detach() : *state) : Tensor();
         if (inplace && s_in.data_ptr() == own.data_ptr()) {
@@ -478,9 +485,11 @@ std::tuple<Tensor, OptTensor> chunk_kda(const Tensor& q, const Tensor& k, const 
     sp.scale = scale.value_or(1.0 / std::sqrt((double)K));
     sp.flags = (int)flags;
     sp.output_final_state = output_final_state;
-    const Tensor h = val(h0), wq = val(cq), wk = val(ck), wv = val(cv);
-    require_device(q, {{"k", &k}, {"v", &v}, {"g", &g}, {"beta", &beta}, {"A_log", &a}, {"dt_bias", &b}, {"initial_state", &h},
-                       {"short_conv_weights[0]", &wq}, {"short_conv_weights[1]", &wk}, {"short_conv_weights[2]", &wv}});
+    const Tensor &h = val(h0), &wq = val(cq), &wk = val(ck), &wv = val(cv);
+    require_device(q, "k", k); require_device(q, "v", v); require_device(q, "g", g); require_device(q, "beta", beta);
+    require_device(q, "A_log", a); require_device(q, "dt_bias", b); require_device(q, "initial_state", h);
+    require_device(q, "short_conv_weights[0]", wq); require_device(q, "short_conv_weights[1]", wk);
+    require_device(q, "short_conv_weights[2]", wv);
     const std::array<const Tensor*, 11> inputs = {&q, &k, &v, &g, &beta, &a, &b, &h, &wq, &wk, &wv};
     refuse_tangents(inputs);
     bool grad = false;
