@@ -9,6 +9,7 @@ of include/kda_b200.h; PyTorch only owns the memory and the stream.
 
 from __future__ import annotations
 
+import threading
 from functools import lru_cache
 
 import torch
@@ -65,6 +66,7 @@ class _DeviceStatus:
     no synchronisation on the hot path."""
 
     _per_device: dict = {}
+    _lock = threading.Lock()  # a word that kernels and the native path know is never replaced
 
     def __init__(self, device):
         self.dev = torch.zeros(1, dtype=torch.int32, device=device)
@@ -76,7 +78,10 @@ class _DeviceStatus:
         key = device.index if device.index is not None else torch.cuda.current_device()
         st = cls._per_device.get(key)
         if st is None:
-            st = cls._per_device[key] = cls(torch.device("cuda", key))
+            with cls._lock:
+                st = cls._per_device.get(key)
+                if st is None:
+                    st = cls._per_device[key] = cls(torch.device("cuda", key))
         return st
 
     @classmethod
