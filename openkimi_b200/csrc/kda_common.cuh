@@ -157,8 +157,8 @@ __device__ __forceinline__ void seq_tokens(const KdaParams& p, int n, long long&
 //   W    as W^T   cm(d, i; 64)      U / V'  as V'^T  cm(e, i; 64)     (i = token in chunk)
 //   Aqk, Tm       cm(i, j; 64)      Qt, Kh           cm(i, d; dk)
 //   S0, dS as S^T cm(e, d; dk)      dVn     as dV'^T cm(e, i; 64)
-// gamC is a plain float[dk]; aux is a plain row-major array; Gc, Qn, Kn are row-major with their
-// 16-byte chunks XOR-swizzled by the row when dk = 128 (swz_f32 / swz_bf16 in kda_tc.cuh).
+// gamC is a plain float[dk]; aux is a plain row-major array; Gc, Qn, Kn are row-major with their 16-byte chunks XOR-swizzled
+// by the row when dk = 128 (swz_f32 / swz_bf16 in kda_tc.cuh; in BF16 two halves of 64 channels one after the other).
 // ---------------------------------------------------------------------------------------
 // Sequence segments of the two state kernels (see kda_state_seg.cu).  len > 0: a CTA walks `len` consecutive chunks of
 // the global chunk numbering, whatever sequences they belong to; len == 0: a CTA walks one whole sequence.
@@ -330,6 +330,17 @@ __device__ __forceinline__ float softplus_fast(float x) {
     const float t = exp_ftz(-fabsf(x));
     const float l = t < 1e-3f ? t * fmaf(t, fmaf(0.33333334f, t, -0.5f), 1.f) : ln_ftz(1.f + t);
     return fmaxf(x, 0.f) + l;
+}
+
+__device__ __forceinline__ float2 softplus_fast2(float2 x) {  // the same of two, in packed arithmetic, bit for bit
+    const float2 u = __fmul2_rn(make_float2(-fabsf(x.x), -fabsf(x.y)), make_float2(LOG2E, LOG2E));
+    const float2 t = make_float2(ex2_ftz(u.x), ex2_ftz(u.y)), o = make_float2(1.f, 1.f), s = __fadd2_rn(o, t);
+    float a, b;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(s.x));
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(b) : "f"(s.y));
+    const float2 l = __fmul2_rn(make_float2(a, b), make_float2(0.6931471805599453f, 0.6931471805599453f));
+    const float2 q = __fmul2_rn(t, __ffma2_rn(t, __ffma2_rn(make_float2(0.33333334f, 0.33333334f), t, make_float2(-0.5f, -0.5f)), o));
+    return __fadd2_rn(make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)), make_float2(t.x < 1e-3f ? q.x : l.x, t.y < 1e-3f ? q.y : l.y));
 }
 
 }  // namespace kda

@@ -23,15 +23,17 @@ __host__ __device__ __forceinline__ int cm_idx(int r, int c, int cols) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Row-major [rows][128] tiles (the kept prologue: G in FP32, q^ and k^ in BF16) are stored with
-// their 16-byte chunks XOR-swizzled by the row: chunk c of row r sits at chunk position
-// c ^ (r & 7).  A warp that reads eight ROWS at the same channels (the operand stage of the
-// forward) then touches eight different 16-byte bank groups instead of one, while every access
-// that walks the channels of one row (thread = channel, or a half warp per row) stays
-// conflict-free, because the swizzle permutes chunks inside an aligned group of eight.
+// Row-major [64][128] tiles (the kept prologue: G in FP32, q^ and k^ in BF16) are stored with their 16-byte chunks XOR-swizzled
+// by the row: chunk c of row r sits at chunk position c ^ (r & 7).  A warp that reads eight ROWS at the same channels then
+// touches eight different 16-byte bank groups instead of one, while every access that walks the channels of one row (thread =
+// channel, or a half warp per row) stays conflict-free, because the swizzle permutes chunks inside an aligned group of eight.
+// BF16 tiles are two halves of [64][64], rows of 128 bytes: what a bulk-tensor copy with 128-byte swizzle delivers, and an
+// MN-major operand of tcgen05.mma (make_desc_sw128).
 // ---------------------------------------------------------------------------------------
 __host__ __device__ __forceinline__ int swz_f32(int r, int d) { return r * 128 + ((((d >> 2) ^ (r & 7)) << 2) | (d & 3)); }
-__host__ __device__ __forceinline__ int swz_bf16(int r, int d) { return r * 128 + ((((d >> 3) ^ (r & 7)) << 3) | (d & 7)); }
+__host__ __device__ __forceinline__ int swz_bf16(int r, int d) {
+    return ((d >> 6) << 12) + r * 64 + (((((d >> 3) & 7) ^ (r & 7)) << 3) | (d & 7));
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -43,6 +45,12 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes
     d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32;
     d |= (uint64_t)1 << 46;
     return d;
+}
+
+// the same for 128-byte swizzle, MN-major: rows (the contracted index) of 64 elements = 128 bytes, eight rows 1024 bytes; lbo:
+// the next 64 elements along M or N, sbo: the next eight rows; tile halves on 1024-byte boundaries
+__device__ __forceinline__ uint64_t make_desc_sw128(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+    return make_desc(saddr, lbo_bytes, sbo_bytes) | (uint64_t)2 << 61;
 }
 
 // instruction descriptor for kind::f16 with BF16 operands and FP32 accumulation

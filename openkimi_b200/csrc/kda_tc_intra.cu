@@ -1,25 +1,28 @@
-// fwd_intra on tensor cores (BF16 operands, d = 128).  One CTA per SM walks the (chunk, head) units
-// (UnitWalk) and requests the inputs of its next unit while it works on the current one.
+// fwd_intra (BF16 operands, d = 128): everything of a chunk that does not need the state.  Two CTAs of 256 threads per SM walk
+// the (chunk, head) units (UnitWalk); each requests the inputs of its next unit as soon as their place is free.
 //
-//   0  the unit's gate, q, k, v tiles arrive as bulk-tensor tile copies (tensor maps; row by row for
-//      partial chunks).  Gate channel-wise: activation and the within-chunk cumulative sum G (log2);
-//      q, k, v, beta row-wise: L2 norm, sigmoid, beta*v operand.
-//      The CONV instantiation reads the pre-convolution projections instead (three halo rows
-//      before the chunk included) and applies the causal depthwise filter + SiLU of
-//      k3mini/model.py:76-88,181-185 in registers before anything else sees the rows
-//   1  the four diagonal 16x16 blocks of Aqk and L on the CUDA cores: where all four [16 x 32] tiles
-//      of a block pass the span guard, with the FP32 midpoint factorisation (pre-scaled key rows, no
-//      exponential per pair), otherwise with exact pairwise decays
-//   2  decay-scaled operands: for every 16-row block I >= 1 the factorised operands
-//      k_j 2^(r_I - G_j) (j < 16 I)  and  x_i 2^(G_i - r_I) (i in I),  r_I = G at the first row of
-//      block I, so that every exponent is <= 0; off-diagonal blocks of Aqk and L as tcgen05 MMAs
-//      (M = 64 keys, N = 32 = q and k rows of block I, K = 128); the Qt, Kh records and beta*k*2^G
-//      are made while these run
-//   3  T = (I + diag(beta) L)^-1: forward substitution inside the diagonal blocks (beside the
-//      accumulator read-back), products for the rest (FP32); Aqk record
-//   4  T record; 5  W^T = (beta k 2^G)^T T^T and U^T = (beta v)^T T^T as tcgen05 MMAs
-//      (M = 128 channels); 6  W, U, gamC records.
+//   1  rows: q, k, v, gate tiles arrive as bulk-tensor tile copies.  L2 norm of the q and k rows, sigmoid, beta*v.  The
+//      CONV instantiation reads the pre-convolution projections instead (three halo rows before the chunk included) and applies
+//      the causal depthwise filter + SiLU of k3mini/model.py:76-88,181-185 before anything else sees the rows
+//   2  gate channel-wise: activation, within-chunk cumulative sum G (log2), span guard
+//   3  Aqk and L: warp = (16-row block I, 64 channels), operands made in registers for mma.sync.  Earlier blocks: x_i 2^(G_i - r_I)
+//      against k_j 2^(r_I - G_j), r_I = G at the first row of block I, every exponent <= 0, one BF16 pass.  The diagonal block, whose
+//      products stay FP32-class (three TF32 passes of split operands), by eight rows: with their midpoint m as reference,
+//      x_i 2^(G_i - m) against k_j 2^(m - G_j), where the tile passes the guard; else by halving (reference: the second half's
+//      first row, every exponent <= 0); pair by pair with one exp2 each where G is not monotone.  The two channel halves
+//      meet in shared memory.  The Qt and Kh records
+//   4  Aqk record; T = (I + diag(beta) L)^-1; the operand beta*k*2^G
+//   5  T record; W^T = (beta k 2^G)^T T^T and U^T = (beta v)^T T^T as tcgen05 MMAs (M = 128 channels); W, U records
+//
+// What bounds it: one unit is a chain of short dependent stages (a dozen barriers, 14 us alone), and at 40 000 warp
+// instructions it needs 5.3 us of the four schedulers.  Two CTAs share an SM so that one unit's waits are the other's issue
+// slots (9.4 us a unit, half of the slots used).  A unit lives in 110 KB for that: the products' operands never touch shared
+// memory, L turns into T in place, beta v and beta k 2^G are MMA operands where the tile copies left v and q, and the next unit's
+// rows are requested as their places fall free.  Operand tiles in shared memory and the diagonal blocks as FP32 FMAs took
+// one CTA of 512 threads and 14.5 us a unit (3072 units 304 -> 206 us, 1536 units of one sequence 162 -> 115, 192 units
+// 40.5 -> 24; with the convolution 12288 units 1434 -> 1052).
 #include "kda_common.cuh"
+#include "kda_conv_bwd.cuh"
 #include "kda_tc.cuh"
 #include "kda_tmap.cuh"
 
@@ -28,71 +31,44 @@ namespace kda {
 using namespace tc;
 
 namespace fi {
-constexpr int D = 128, NTHR = 512;
-constexpr uint32_t SQ = 0;                   // q^  bf16 [64][128] row-major
-constexpr uint32_t SK = SQ + 16384;          // k^  bf16 [64][128]
-constexpr uint32_t SG = SK + 16384;          // G   f32  [64][128]
-constexpr uint32_t KSC = SG + 32768;         // 3 x cm(j, d; 128) bf16; block 0 later holds T (bf16)
-constexpr uint32_t XSC = KSC + 3 * 16384;    // 3 x cm(n, d; 128) bf16, 32 rows each
-constexpr uint32_t KB = XSC + 3 * 8192;      // beta k 2^G  cm(j, d; 128)
-constexpr uint32_t BV = KB + 16384;          // beta v      cm(j, e; 128)
-constexpr int LDR = 68;                      // row stride of A, L, T in floats
-constexpr uint32_t SA = BV + 16384;          // f32 [64][LDR]
-constexpr uint32_t SL = SA + 64 * LDR * 4;
-constexpr uint32_t ST = SL + 64 * LDR * 4;
-constexpr uint32_t SBETA = ST + 64 * LDR * 4;        // f32 [3][64]: 1/|q|, 1/|k|, beta (the aux record)
-constexpr uint32_t STOT = SBETA + 768;       // f32 [4][128] running gate totals of the four 16-row groups
-constexpr uint32_t SMIDF = STOT + 2048;      // f32 [4][128] midpoint of every (block, channel) of the cumulative gate
-constexpr uint32_t SPASS = SMIDF + 2048;     // int [4][4]: guard decision of every [16 rows x 32 channels] tile
-constexpr uint32_t TOTAL = SPASS + 64;
-constexpr uint32_t KN = KSC;                 // f32 [64][128] (chunk-swizzled rows): k_j 2^(m - G_j), live only during the diagonal phase
-constexpr uint32_t T_D = 0, T_W = 96, T_U = 160, TMEM_COLS = 256;
+constexpr int D = 128, NTHR = 256;
+constexpr int LDR = 68, LDA = 20;            // row strides in floats: L / T, partial diagonal blocks of Aqk
+constexpr uint32_t SQ = 0;                   // q rows, then q^ bf16 [64][128] (swz_bf16); later beta k^ 2^G
+constexpr uint32_t SK = SQ + 16384;          // k rows, then k^
+constexpr uint32_t SV = SK + 16384;          // v rows, then beta v (swz_bf16)
+constexpr uint32_t SG = SV + 16384;          // G f32 [64][128] (swz_f32)
+constexpr uint32_t SM = SG + 32768;          // gate rows bf16 [64][128] as they arrive; then f32 [64][LDR]: L, T;
+                                             // partial blocks of Aqk above the diagonal
+constexpr uint32_t SU = SM + 64 * LDR * 4;   // 8 KB: gate totals of the four 16-row groups f32 [4][128] | partial
+                                             // diagonal blocks of Aqk | inner products of the inverse | T bf16 cm(i, j; 64)
+constexpr uint32_t TAPS = SG;                // when G is dead: the filter taps of the next unit, f32 [3][8][16][4]
+constexpr uint32_t SMID = SU + 8192;         // f32 [8][128] midpoint of every (eight rows, channel)
+constexpr uint32_t SBETA = SMID + 4096;      // f32 [3][64]: 1/|q|, 1/|k|, beta (the aux record)
+constexpr uint32_t SMODE = SBETA + 768;      // int [4][2]: how the diagonal block may be evaluated, per 64 channels
+constexpr uint32_t SBAR = SMODE + 32;        // four mbarriers, the tensor-memory base
+constexpr uint32_t HALO = SBAR + 48;         // fused convolution: rows -3 .. -1 of q, k, v, bf16 [3][3][128]
+constexpr uint32_t TOTAL = HALO, TOTAL_CONV = HALO + 9 * 256;
+static_assert(TOTAL_CONV <= 115712, "two CTAs per SM");
+constexpr uint32_t T_W = 0, T_U = 64, TMEM_COLS = 128;
+enum { MIDPOINT = 0, LEVELS = 1, PAIRS = 2 };
+// Largest span of eight rows for their midpoint: the factors reach 2^(+-100), the low parts of the operands stay normal numbers.
+constexpr float MAX_SPAN = 200.f;
 }  // namespace fi
 using fi::LDR;
 
-// T = (I + diag(beta) L)^-1 by blocks, FP32.  sL holds L (strictly lower), sT receives T (zero above the diagonal blocks on
-// entry); both have rows of LDR floats on 16-byte boundaries.  The four 16 x 16 diagonal blocks are inverted by forward
-// substitution, one warp each (a dependent chain of 16 rows, lane = column), by the four warps that have no share in the
-// accumulator read-back; everything below them is products: T_ba = -T_bb (beta L)_ba T_aa for the block pairs (0, 1) and
-// (2, 3), then the same with 32 x 32 halves.  A thread's tile is 2 x 2, in the small products with the inner index split
-// over two lanes; sY (32 rows of LDY floats) takes the inner products between two barriers.  Eight warps do them: the
-// others write the Aqk record and issue the next unit's copies, which hold an issuing warp up for 0.7-0.9 us.  (One
-// column after the other down all blocks was a chain three block levels long, 2.6 us of a unit's 15.5; with all sixteen
-// warps in the products a training step's stores delayed them: 978 us against 988 for 3072 units, forward and backward.)
+// T = (I + diag(beta) L)^-1 by blocks, in place: M holds L (strictly lower) and receives T on and below the diagonal blocks; rows
+// of LDR floats.  The four 16 x 16 diagonal blocks are inverted by forward substitution in FP32, one warp each (a dependent
+// chain of 16 rows, lane = column); everything below them is products, T_ba = -T_bb (beta L)_ba T_aa for the block pairs (0, 1)
+// and (2, 3), then the same with 32 x 32 halves, in FP32-class TF32 passes of split operands.  sY (32 rows of LDY floats) takes
+// the inner products.
 constexpr int LDY = 36;
 
-// a 2 x 2 tile over `K4` groups of four inner elements: rows of A (float4 along k), rows k of B (two columns)
-template <int K4>
-__device__ __forceinline__ void tile22(float2 (&acc)[2], const float* A0, const float* A1, const float* B, int ldb, int kstep) {
-#pragma unroll 2
-    for (int m = 0; m < K4; ++m) {
-        const float4 a0 = *reinterpret_cast<const float4*>(A0 + m * kstep), a1 = *reinterpret_cast<const float4*>(A1 + m * kstep);
-        const float x0[4] = {a0.x, a0.y, a0.z, a0.w}, x1[4] = {a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 b = *reinterpret_cast<const float2*>(B + (m * kstep + j) * ldb);
-            acc[0] = __ffma2_rn(make_float2(x0[j], x0[j]), b, acc[0]);
-            acc[1] = __ffma2_rn(make_float2(x1[j], x1[j]), b, acc[1]);
-        }
-    }
-}
-template <int LANES>
-__device__ __forceinline__ void sum22(float2 (&acc)[2]) {
-#pragma unroll
-    for (int o = 1; o < LANES; o <<= 1)
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            acc[i].x += __shfl_xor_sync(0xffffffffu, acc[i].x, o);
-            acc[i].y += __shfl_xor_sync(0xffffffffu, acc[i].y, o);
-        }
-}
-
-__device__ __forceinline__ void invert_diagonal(const float* sL, float* sT, const float* sbeta, int blk, int lane) {
+__device__ __forceinline__ void invert_diagonal(float* M, const float* sbeta, int blk, int lane) {
     const int col = lane & 15;
     float t[16];
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
-        const float* lrow = sL + (16 * blk + r) * LDR + 16 * blk;
+        const float* lrow = M + (16 * blk + r) * LDR + 16 * blk;
         float s0 = 0.f, s1 = 0.f;
 #pragma unroll
         for (int j = 0; j < r; j += 4) {
@@ -105,91 +81,132 @@ __device__ __forceinline__ void invert_diagonal(const float* sL, float* sT, cons
         t[r] = (r == col ? 1.f : 0.f) - sbeta[16 * blk + r] * (s0 + s1);
         if (r < col) t[r] = 0.f;
     }
+    __syncwarp();
     if (lane < 16) {
 #pragma unroll
-        for (int r = 0; r < 16; ++r) sT[(16 * blk + r) * LDR + 16 * blk + col] = t[r];
+        for (int r = 0; r < 16; ++r) M[(16 * blk + r) * LDR + 16 * blk + col] = t[r];
     }
 }
 
-__device__ __forceinline__ void invert_products(const float* sL, float* sT, const float* sbeta, float* sY, int warp, int lane) {
-    float2 acc[2] = {};
-    {   // pairs of 16 x 16 blocks: four warps each, inner index over two lanes (alternating groups of four)
-        const int pr = warp >> 2, a = 32 * pr, b = a + 16, i = lane & 1;
-        const int r0 = 4 * (warp & 3) + 2 * (lane >> 4), c0 = 2 * ((lane >> 1) & 7), k0 = 4 * i;
-        tile22<2>(acc, sL + (b + r0) * LDR + a + k0, sL + (b + r0 + 1) * LDR + a + k0, sT + (a + k0) * LDR + a + c0, LDR, 8);
-        sum22<2>(acc);
-        const float be = sbeta[b + r0 + i];
-        *reinterpret_cast<float2*>(sY + (16 * pr + r0 + i) * LDY + c0) = make_float2(be * (i ? acc[1].x : acc[0].x), be * (i ? acc[1].y : acc[0].y));
-        bar_sync(1, 256);
-        acc[0] = acc[1] = make_float2(0.f, 0.f);
-        tile22<2>(acc, sT + (b + r0) * LDR + b + k0, sT + (b + r0 + 1) * LDR + b + k0, sY + (16 * pr + k0) * LDY + c0, LDY, 8);
-        sum22<2>(acc);
-        *reinterpret_cast<float2*>(sT + (b + r0 + i) * LDR + a + c0) = make_float2(-(i ? acc[1].x : acc[0].x), -(i ? acc[1].y : acc[0].y));
-        bar_sync(1, 256);
-    }
-    {   // the 32 x 32 halves: a warp has four rows
-        const int r0 = 4 * warp + 2 * (lane >> 4), c0 = 2 * (lane & 15);
-        acc[0] = acc[1] = make_float2(0.f, 0.f);
-        tile22<8>(acc, sL + (32 + r0) * LDR, sL + (33 + r0) * LDR, sT + c0, LDR, 4);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const float be = sbeta[32 + r0 + i];
-            *reinterpret_cast<float2*>(sY + (r0 + i) * LDY + c0) = make_float2(be * acc[i].x, be * acc[i].y);
-        }
-        bar_sync(1, 256);
-        acc[0] = acc[1] = make_float2(0.f, 0.f);
-        tile22<8>(acc, sT + (32 + r0) * LDR + 32, sT + (33 + r0) * LDR + 32, sY + c0, LDY, 4);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) *reinterpret_cast<float2*>(sT + (32 + r0 + i) * LDR + c0) = make_float2(-acc[i].x, -acc[i].y);
-    }
+
+// mma.sync fragments (lane = 4 g + t).  The contracted index may be dealt out in any order that both operands share: of sixteen
+// channels a lane holds 4 t .. 4 t + 3, one 16-byte word of G and one 8-byte word of q^ and k^, for one BF16 step or two TF32
+// steps.  Row (and key) number g of a tile stands for row bit_reverse(g): with the row swizzle of the tiles (swz_f32,
+// swz_bf16) the loads of a quarter warp then fall into different banks.
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_tf32(float (&c)[4], float a0, float a1, float a2, float a3, float b0, float b1) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(a2)), "r"(__float_as_uint(a3)),
+                   "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+}
+// x = hi + lo: hi the 11 significant bits that TF32 keeps, lo rounded to as many (the multiplier drops the low 13 bits; half of the
+// last place it keeps is added before): x to 2^-21, without a bias
+__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
+    hi = __uint_as_float(__float_as_uint(x) & 0xffffe000u);
+    lo = __uint_as_float(__float_as_uint(x - hi) + 0x1000u);
+}
+struct Split2 { float h[2], l[2]; };  // the two B elements of a lane, split
+// c += a b with split operands: lo hi + hi lo + hi hi
+__device__ __forceinline__ void mma_tf32x3(float (&c)[4], float a0, float a1, float a2, float a3, const Split2& b) {
+    float h[4], l[4];
+    split_tf32(a0, h[0], l[0]);
+    split_tf32(a1, h[1], l[1]);
+    split_tf32(a2, h[2], l[2]);
+    split_tf32(a3, h[3], l[3]);
+    mma_tf32(c, l[0], l[1], l[2], l[3], b.h[0], b.h[1]);
+    mma_tf32(c, h[0], h[1], h[2], h[3], b.l[0], b.l[1]);
+    mma_tf32(c, h[0], h[1], h[2], h[3], b.h[0], b.h[1]);
+}
+__device__ __forceinline__ void exp2_diff(const float4& a, const float4& b, float (&f)[4]) {  // 2^(a - b)
+    f[0] = ex2_approx(a.x - b.x); f[1] = ex2_approx(a.y - b.y); f[2] = ex2_approx(a.z - b.z); f[3] = ex2_approx(a.w - b.w);
+}
+__device__ __forceinline__ void unpack4(const uint2& u, float (&f)[4]) {
+    f[0] = __uint_as_float(u.x << 16); f[1] = __uint_as_float(u.x & 0xffff0000u);
+    f[2] = __uint_as_float(u.y << 16); f[3] = __uint_as_float(u.y & 0xffff0000u);
 }
 
-// Off-diagonal blocks from tensor memory into sA (Aqk, scaled) and sL: accumulator column
-// 32 (I - 1) + n holds, for key row j (lane), the product with q row n (n < 16) or k row n - 16 of
-// block I.  One call covers the 32 columns of block I = CBASE / 32 + 1; CBASE is a template argument
-// so that every block / row index is a constant.
-template <int CBASE>
-__device__ __forceinline__ void read_offdiag(uint32_t tmem_d, int qd, int lane, float* sA, float* sL, float scale) {
-    const int j = 16 * qd + (lane & 15);
+// a 16 x 8 tile of A B over 8 KS inner elements; A: row g, column t, B: row t, column g of this lane's fragments
+template <int KS>
+__device__ __forceinline__ void tile_product(float (&c)[4], const float* A, const float* B, int ldb) {
+    float c1[4] = {}, c2[4] = {};  // three independent chains
 #pragma unroll
-    for (int cc = 0; cc < 32; cc += 16) {
-        uint32_t r[16];
-        tmem_ld16(tmem_d + ((uint32_t)(32 * qd) << 16) + CBASE + cc, r);
-        tmem_wait_ld();
-        if (lane < 16) {
-#pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                const int col = CBASE + cc + u, I = (col >> 5) + 1, nn = col & 31;
-                if (j < 16 * I) {
-                    const float val = __uint_as_float(r[u]);
-                    if (nn < 16) sA[(16 * I + nn) * LDR + j] = val * scale;
-                    else sL[(16 * I + nn - 16) * LDR + j] = val;
-                }
-            }
-        }
+    for (int k = 0; k < KS; ++k) {
+        float h[4], l[4], bh[2], bl[2];
+        split_tf32(A[8 * k], h[0], l[0]);
+        split_tf32(A[8 * k + 8 * LDR], h[1], l[1]);
+        split_tf32(A[8 * k + 4], h[2], l[2]);
+        split_tf32(A[8 * k + 4 + 8 * LDR], h[3], l[3]);
+        split_tf32(B[8 * k * ldb], bh[0], bl[0]);
+        split_tf32(B[(8 * k + 4) * ldb], bh[1], bl[1]);
+        mma_tf32(c1, l[0], l[1], l[2], l[3], bh[0], bh[1]);
+        mma_tf32(c2, h[0], h[1], h[2], h[3], bl[0], bl[1]);
+        mma_tf32(c, h[0], h[1], h[2], h[3], bh[0], bh[1]);
     }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) c[x] += c1[x] + c2[x];
+}
+__device__ __forceinline__ void store_tile(float* dst, int ld, const float (&c)[4], float f0, float f1) {
+    *reinterpret_cast<float2*>(dst) = make_float2(f0 * c[0], f0 * c[1]);
+    *reinterpret_cast<float2*>(dst + 8 * ld) = make_float2(f1 * c[2], f1 * c[3]);
+}
+__device__ __forceinline__ void invert_products(float* M, const float* sbeta, float* sY, int warp, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    if (warp < 4) {  // pairs of 16 x 16 blocks: a warp has eight columns of one, so the inner product stays with it
+        const int pr = warp >> 1, n8 = 8 * (warp & 1), a = 32 * pr, b = a + 16;
+        float y[4] = {}, c[4] = {};
+        tile_product<2>(y, M + (b + g) * LDR + a + t, M + (a + t) * LDR + a + n8 + g, LDR);
+        store_tile(sY + (16 * pr + g) * LDY + n8 + 2 * t, LDY, y, sbeta[b + g], sbeta[b + g + 8]);
+        bar_sync(1 + pr, 64);  // both warps of the pair have read L_ba
+        tile_product<2>(c, M + (b + g) * LDR + b + t, sY + (16 * pr + t) * LDY + n8 + g, LDY);
+        store_tile(M + (b + g) * LDR + a + n8 + 2 * t, LDR, c, -1.f, -1.f);
+    }
+    __syncthreads();
+    // the 32 x 32 halves: a warp has one 16 x 8 tile.  (Blocks above the diagonal hold other things: their products are left out.)
+    const int n8 = 8 * (warp & 3), m16 = 16 * (warp >> 2);
+    const float* A = M + (32 + m16 + g) * LDR + t;
+    float y[4] = {}, c[4] = {};
+    if (n8 < 16) tile_product<4>(y, A, M + t * LDR + n8 + g, LDR);
+    else tile_product<2>(y, A + 16, M + (16 + t) * LDR + n8 + g, LDR);
+    store_tile(sY + (m16 + g) * LDY + n8 + 2 * t, LDY, y, sbeta[32 + m16 + g], sbeta[40 + m16 + g]);
+    __syncthreads();
+    if (m16) tile_product<4>(c, A + 32, sY + t * LDY + n8 + g, LDY);
+    else tile_product<2>(c, A + 32, sY + t * LDY + n8 + g, LDY);
+    store_tile(M + (32 + m16 + g) * LDR + n8 + 2 * t, LDR, c, -1.f, -1.f);
 }
 
 template <bool CONV>
-__global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams p, const __grid_constant__ RowMaps maps) {
+__global__ void __launch_bounds__(fi::NTHR, 2) kda_fwd_intra_tc(const KdaParams p, const __grid_constant__ RowMaps maps, const WsLayout L) {
     using namespace fi;
-    extern __shared__ __align__(128) unsigned char dyn[];
-    __shared__ uint64_t bar, bar2, rowbar, vbar;
-    __shared__ uint32_t tmem_s;
+    extern __shared__ __align__(1024) unsigned char dyn[];
     __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(dyn + SQ);
     __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(dyn + SK);
     float* sG = reinterpret_cast<float*>(dyn + SG);
-    __nv_bfloat16* sKB = reinterpret_cast<__nv_bfloat16*>(dyn + KB);
-    __nv_bfloat16* sBV = reinterpret_cast<__nv_bfloat16*>(dyn + BV);
-    float* sA = reinterpret_cast<float*>(dyn + SA);
-    float* sL = reinterpret_cast<float*>(dyn + SL);
-    float* sT = reinterpret_cast<float*>(dyn + ST);
+    __nv_bfloat16* sV = reinterpret_cast<__nv_bfloat16*>(dyn + SV);
+    __nv_bfloat16* sRG = reinterpret_cast<__nv_bfloat16*>(dyn + SM);
+    float* sM = reinterpret_cast<float*>(dyn + SM);
+    float* stot = reinterpret_cast<float*>(dyn + SU);
+    float* sAd = reinterpret_cast<float*>(dyn + SU);
+    float* sY = reinterpret_cast<float*>(dyn + SU);
+    __nv_bfloat16* sTB = reinterpret_cast<__nv_bfloat16*>(dyn + SU);
+    float4* sW = reinterpret_cast<float4*>(dyn + TAPS);
+    float* smid = reinterpret_cast<float*>(dyn + SMID);
     float* saux = reinterpret_cast<float*>(dyn + SBETA);
     float* sbeta = saux + 2 * C;
-    float* stot = reinterpret_cast<float*>(dyn + STOT);
+    int* smode = reinterpret_cast<int*>(dyn + SMODE);
+    uint64_t* kbar = reinterpret_cast<uint64_t*>(dyn + SBAR);  // k (and every halo row)
+    uint64_t* qbar = kbar + 1;  // q, v
+    uint64_t* gbar = kbar + 2;  // gate
+    uint64_t* wbar = kbar + 3;  // W and U products
+    uint32_t* tmem_s = reinterpret_cast<uint32_t*>(kbar + 4);
+    __nv_bfloat16* sHalo = reinterpret_cast<__nv_bfloat16*>(dyn + HALO);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (warp-uniform: roles and MMA issue)
     char* ws = (char*)p.workspace;
     const __nv_bfloat16* q = (const __nv_bfloat16*)p.q;
     const __nv_bfloat16* k = (const __nv_bfloat16*)p.k;
@@ -201,107 +218,111 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
 
     KDA_PHASE_BEGIN();
     if (warp == 0) {
-        tmem_alloc(&tmem_s, TMEM_COLS);
+        tmem_alloc(tmem_s, TMEM_COLS);
         tmem_relinquish();
     }
-    if (tid == 0) {
-        mbar_init(&bar, 3);   // three issuing threads commit the off-diagonal products
-        mbar_init(&bar2, 2);  // two issuing threads commit the W and U products
-        mbar_init(&rowbar, 1);
-        mbar_init(&vbar, 1);
+    if (tid >= 64 && tid < 68) prefetch_map(&maps.m[tid - 64]);
+    if (tid == 32) {
+        mbar_init(kbar, 1);
+        mbar_init(gbar, 1);
+        mbar_init(qbar, 2);  // (the threads that issue q and v)
+        mbar_init(wbar, 2);  // two issuing threads commit the W and U products
         mbar_fence_init();
     }
     pdl_wait();
+    tc_fence_before();
     __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem0 = *tmem_s;
 
-    // ---- 0: a unit's inputs arrive as bulk-tensor tile copies (row by row for partial chunks), completing on two
-    //      mbarriers.  The CTA walks the units blockIdx.x, blockIdx.x + gridDim.x, ... and requests the inputs of
-    //      its NEXT unit while it still works on the current one, into space that is dead by then: the gate, q and
-    //      k rows (q, k: ROWS each, three halo rows first when the convolution is fused; the halo rows of v too)
-    //      go to the operand space behind the first key tile once the off-diagonal products have been read, some
-    //      8 us ahead of their use; the v rows, which are needed last, go to the L tile once T is solved; the few
-    //      scalars travel in registers.  Rows past the end of the sequence are zero-filled by the thread that
-    //      would have requested them.
-    constexpr int HALO = CONV ? 3 : 0, ROWS = C + HALO;
-    constexpr uint32_t RGATE = KSC + 16384, RQ = RGATE + C * D * 2, RK = RQ + ROWS * D * 2, RVH = RK + ROWS * D * 2, TAPS = ST;
-    static_assert(RVH + HALO * D * 2 <= KB, "staging overruns the operand space");
-    __nv_bfloat16* sRG = reinterpret_cast<__nv_bfloat16*>(dyn + RGATE);
-    __nv_bfloat16* sRq = reinterpret_cast<__nv_bfloat16*>(dyn + RQ);    // rows -HALO .. 63 of q
-    __nv_bfloat16* sRk = reinterpret_cast<__nv_bfloat16*>(dyn + RK);
-    __nv_bfloat16* sRvh = reinterpret_cast<__nv_bfloat16*>(dyn + RVH);  // rows -3 .. -1 of v (fused convolution only)
-    __nv_bfloat16* sRv = reinterpret_cast<__nv_bfloat16*>(dyn + SL);    // rows 0 .. 63 of v
-    const int quarter = tid >> 7, dch = tid & 127;  // gate: thread = (16-row group, channel)
-    const int hw = tid >> 4, c8 = (tid & 15) * 8;   // rows: half warp = row, lane = 8 channels
-    auto zero_row = [&](__nv_bfloat16* dst) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) reinterpret_cast<uint4*>(dst)[j] = make_uint4(0, 0, 0, 0);
-    };
-    const bool tiles = maps.ok != 0;  // whole [64 x 128] tiles with one bulk-tensor copy each (full chunks only)
+    // thread roles of the element-wise stages
+    const int hw = tid >> 4, c8r = (tid & 15) * 8;               // rows: a half warp has the rows 4 hw .. 4 hw + 3, a lane 8 channels
+    const int qt = warp >> 1, gh = warp & 1, gd = 64 * gh + 2 * lane;  // gate: 16-row group, half, the first of two channels
+    const bool tiles = maps.ok != 0;  // whole tiles with bulk-tensor copies; rows past the end of the sequence are masked when read
     auto row_src = [&](const __nv_bfloat16* base, const ChunkInfo& ci, int h, int i) { return base + ((size_t)(ci.tok0 + i) * p.H + h) * D; };
-    auto request_rows = [&](const ChunkInfo& ci, int h) {  // gate, q, k (and every halo row)
-        // (issued from the last warp, which has no diagonal block to invert after the in-loop request: the
-        //  issuing warp is held up while the copy unit works through its requests)
-        if (tid == NTHR - 32) mbar_expect_tx(&rowbar, (uint32_t)(3 * ci.len + ((CONV && ci.lc > 0) ? 9 : 0)) * 256u);
-        if (tiles && ci.len == C) {
-            if (tid == NTHR - 32) tma_load_tile(sRG, &maps.m[3], h * D, (int)ci.tok0, &rowbar);
-            if (tid == NTHR - 31) tma_load_tile(sRq + HALO * D, &maps.m[0], h * D, (int)ci.tok0, &rowbar);
-            if (tid == NTHR - 30) tma_load_tile(sRk + HALO * D, &maps.m[1], h * D, (int)ci.tok0, &rowbar);
-        } else if (tid < 3 * C) {
-            const int t3 = tid >> 6, i = tid & 63;
-            __nv_bfloat16* dst = (t3 == 0 ? sRG : t3 == 1 ? sRq + HALO * D : sRk + HALO * D) + i * D;
-            if (i < ci.len) tma_load_1d(dst, row_src(t3 == 0 ? g : t3 == 1 ? q : k, ci, h, i), 256, &rowbar);
-            else zero_row(dst);
-        }
-        if (CONV && lane == 0 && warp >= 6 && warp < 15) {  // three rows before the chunk (one copy each from nine warps):
-            const int t3 = (warp - 6) / 3, r = (warp - 6) % 3;  // they exist unless the chunk starts its sequence
-            __nv_bfloat16* dst = (t3 == 0 ? sRq : t3 == 1 ? sRk : sRvh) + r * D;
-            if (ci.lc > 0) tma_load_1d(dst, row_src(t3 == 0 ? q : t3 == 1 ? k : v, ci, h, r - 3), 256, &rowbar);
-            else zero_row(dst);
+    // (a thread is held up by every copy it issues: each tile has its own)
+    auto load_rows = [&](uint32_t dst, const CUtensorMap* m, const ChunkInfo& ci, int h, uint64_t* bar, uint32_t more) {
+        mbar_expect_tx(bar, C * D * 2 + more);
+        tma_load_tile(dyn + dst, m, h * D, (int)ci.tok0, bar);
+        tma_load_tile(dyn + dst + 8192, m, h * D + 64, (int)ci.tok0, bar);
+    };
+    auto request_g = [&](const ChunkInfo& ci, int h) {
+        if (tiles && tid == 0) {
+            mbar_expect_tx(gbar, C * D * 2);
+            tma_load_tile(sRG, &maps.m[3], h * D, (int)ci.tok0, gbar);
         }
     };
-    auto request_v = [&](const ChunkInfo& ci, int h) {
-        if (tid == 256) mbar_expect_tx(&vbar, (uint32_t)ci.len * 256u);
-        if (tiles && ci.len == C) {
-            if (tid == 256) tma_load_tile(sRv, &maps.m[2], h * D, (int)ci.tok0, &vbar);
-        } else if (tid >= 256 && tid < 256 + C) {
-            const int i = tid - 256;
-            if (i < ci.len) tma_load_1d(sRv + i * D, row_src(v, ci, h, i), 256, &vbar);
-            else zero_row(sRv + i * D);
-        }
-    };
-    struct Scalars {  // (beta stays in its storage type: a conversion here would wait for the load)
-        float a_log, bias;
-        __nv_bfloat16 rb[2];
-        float4 tap;
-    };
-    auto request_scalars = [&](const ChunkInfo& ci, int h, Scalars& sc) {
-        sc.a_log = gate ? p.A_log[h] : 0.f;
-        sc.bias = (gate && p.dt_bias) ? p.dt_bias[h * D + dch] : 0.f;
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const int i = CONV ? 2 * hw + m : hw + 32 * m;
-            sc.rb[m] = beta[(size_t)(ci.tok0 + (i < ci.len ? i : 0)) * p.H + h];  // (used by lane 0 of the half warp, rows < len)
-        }
-        sc.tap = make_float4(0.f, 0.f, 0.f, 0.f);
-        if constexpr (CONV) {  // filter taps of this head, padded to four: entry e = tensor * 128 + channel
-            const int K = p.conv_ksize;
-            if (tid < 3 * D) {
-                float t4[4] = {0.f, 0.f, 0.f, 0.f};
-                const float* w = (tid < D ? p.conv_q : tid < 2 * D ? p.conv_k : p.conv_v) + (size_t)(h * D + (tid & (D - 1))) * K;
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (j >= 4 - K) t4[j] = w[j - (4 - K)];
-                sc.tap = make_float4(t4[0], t4[1], t4[2], t4[3]);
+    auto request_k = [&](const ChunkInfo& ci, int h) {
+        if (!tiles) return;
+        const bool halo = CONV && ci.lc > 0;
+        if (tid == 32) load_rows(SK, &maps.m[1], ci, h, kbar, halo ? 9 * 256u : 0u);
+        if constexpr (CONV) {  // three rows before the chunk, unless it starts its sequence
+            if (halo) {
+                if (warp == 2 && lane < 9)
+                    tma_load_1d(sHalo + lane * D, row_src(lane < 3 ? q : lane < 6 ? k : v, ci, h, lane % 3 - 3), 256, kbar);
+            } else if (tid < 9 * 16) {
+                reinterpret_cast<uint4*>(sHalo)[tid] = make_uint4(0, 0, 0, 0);
             }
         }
     };
-    // taps: entry (tensor, channel) at [tensor][channel % 8][channel / 8], so that the sixteen lanes of a
-    // half warp read consecutive 16-byte words; they wait in the (dead) T tile for the next unit
-    auto park_taps = [&](const Scalars& sc) {
-        if constexpr (CONV) {
-            float4* sW = reinterpret_cast<float4*>(dyn + TAPS);
-            if (tid < 3 * D) sW[(tid & ~(D - 1)) + (tid & 7) * 16 + ((tid & (D - 1)) >> 3)] = sc.tap;
+    auto request_qv = [&](const ChunkInfo& ci, int h) {
+        if (!tiles) return;
+        if (tid == 64) load_rows(SQ, &maps.m[0], ci, h, qbar, 0);
+        if (tid == 96) load_rows(SV, &maps.m[2], ci, h, qbar, 0);
+    };
+    const uint4 zero4 = make_uint4(0, 0, 0, 0);
+    auto copy_rows = [&](const ChunkInfo& ci, int h) {  // no tensor maps: the same tiles with plain loads, at the start of the unit
+#pragma unroll 1
+        for (int x = tid; x < 4 * C * 16; x += NTHR) {
+            const int t4 = x >> 10, i = (x >> 4) & 63, c8 = (x & 15) * 8;
+            const uint4 u = i < ci.len ? *reinterpret_cast<const uint4*>(row_src(t4 == 0 ? q : t4 == 1 ? k : t4 == 2 ? v : g, ci, h, i) + c8) : zero4;
+            *reinterpret_cast<uint4*>(t4 == 3 ? sRG + i * D + c8 : reinterpret_cast<__nv_bfloat16*>(dyn + SQ) + t4 * C * D + swz_bf16(i, c8)) = u;
         }
+        if (CONV && tid < 9 * 16) {
+            const int r = tid >> 4;
+            reinterpret_cast<uint4*>(sHalo)[tid] =
+                ci.lc > 0 ? *reinterpret_cast<const uint4*>(row_src(r < 3 ? q : r < 6 ? k : v, ci, h, r % 3 - 3) + 8 * (tid & 15)) : zero4;
+        }
+        __syncthreads();
+    };
+    // rows past the end of a partial chunk (the tile copies brought what follows in memory): q, k, v zero, no decay
+    auto clear_tail = [&](int len) {
+#pragma unroll 1
+        for (int x = tid; x < 4 * C * 16; x += NTHR) {
+            const int t4 = x >> 10, i = (x >> 4) & 63, c8 = (x & 15) * 8;
+            const uint32_t w = t4 == 3 && gate ? 0xff80ff80u : 0u;  // softplus(-inf) = 0
+            if (i >= len)
+                *reinterpret_cast<uint4*>(t4 == 3 ? sRG + i * D + c8 : reinterpret_cast<__nv_bfloat16*>(dyn + SQ) + t4 * C * D + swz_bf16(i, c8)) =
+                    make_uint4(w, w, w, w);
+        }
+        __syncthreads();
+    };
+    struct Scalars {  // (beta stays in its storage type: a conversion here would wait for the load)
+        float a_log;
+        float2 bias;
+        __nv_bfloat16 rb;
+    };
+    auto request_scalars = [&](const ChunkInfo& ci, int h, Scalars& sc) {
+        sc.a_log = gate ? p.A_log[h] : 0.f;
+        sc.bias = make_float2(0.f, 0.f);
+        if (gate && p.dt_bias) sc.bias = make_float2(p.dt_bias[h * D + gd], p.dt_bias[h * D + gd + 1]);
+        const int i = 4 * hw + (lane & 3);
+        sc.rb = beta[(size_t)(ci.tok0 + (i < ci.len ? i : 0)) * p.H + h];
+    };
+    // filter taps of a head, padded to four: entry (tensor, channel) at [tensor][channel % 8][channel / 8], so that the sixteen
+    // lanes of a half warp read consecutive 16-byte words
+    auto request_taps = [&](int h) {
+        if constexpr (CONV) {
+#pragma unroll 1
+            for (int e = tid; e < 3 * D; e += NTHR)
+                stage_taps(sW + (e & ~(D - 1)) + (e & 7) * 16 + ((e & (D - 1)) >> 3), e < D ? p.conv_q : e < 2 * D ? p.conv_k : p.conv_v, h, e & (D - 1), p.conv_ksize);
+            cp_async_commit();
+        }
+    };
+    auto load_g8 = [&](int i, int c8, float (&x)[8]) {
+        const float4 a = *reinterpret_cast<const float4*>(sG + swz_f32(i, c8));
+        const float4 b = *reinterpret_cast<const float4*>(sG + swz_f32(i, c8 + 4));
+        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
     };
     const int n_units = p.NT * p.H;
     Scalars nx;
@@ -311,557 +332,550 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
     UnitWalk uw;
     uw.init(blockIdx.x, gridDim.x, p.H);
     ChunkInfo ci = chunk_info(p, blockIdx.x / p.H);
-    request_rows(ci, uw.head());
-    request_v(ci, uw.head());
+    request_g(ci, uw.head());
+    request_k(ci, uw.head());
+    request_qv(ci, uw.head());
     request_scalars(ci, uw.head(), nx);
-    park_taps(nx);
-    __syncthreads();
+    request_taps(uw.head());
+    cp_async_wait<0>();
+    if (CONV) __syncthreads();
     uint32_t it = 0;
     bool ok = true, more = false;
-    for (; uw.unit < n_units; uw.next(), ++it) {
+    for (; uw.unit < n_units; ++it) {
     const int c = uw.c, h = uw.head();
     const size_t rec = (size_t)c * p.H + h;
-    __nv_bfloat16* gW = (__nv_bfloat16*)(ws + L.W) + rec * C * D;
-    __nv_bfloat16* gU = (__nv_bfloat16*)(ws + L.U) + rec * C * D;
-    __nv_bfloat16* gA = (__nv_bfloat16*)(ws + L.Aqk) + rec * C * C;
-    __nv_bfloat16* gQt = (__nv_bfloat16*)(ws + L.Qt) + rec * C * D;
-    __nv_bfloat16* gKh = (__nv_bfloat16*)(ws + L.Kh) + rec * C * D;
-    __nv_bfloat16* gT = (__nv_bfloat16*)(ws + L.Tm) + rec * C * C;
-    float* gGam = (float*)(ws + L.gamC) + rec * D;
-    UnitWalk un = uw;  // the next unit of this CTA
-    un.next();
-    more = un.unit < n_units;
-    ChunkInfo ci_nx = ci;
-    const float a_log_h = nx.a_log, bias = nx.bias;
-    float rb[2];
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-        rb[m] = ((tid & 15) == 0 && (CONV ? 2 * hw + m : hw + 32 * m) < ci.len) ? __bfloat162float(nx.rb[m]) : 0.f;
-    ok = mbar_wait(&rowbar, it & 1, p, 8);
-    KDA_PHASE(13);
-    // ---- 0a: gate, channel-wise: thread (quarter, d) owns rows 16*quarter .. 16*quarter+15 of channel d
-    {
-        const float negA = gate ? -expf(a_log_h) : 0.f;
-        float run = 0.f;
-#pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            const int i = 16 * quarter + r;
-            const float x = __bfloat162float(sRG[i * D + dch]);
-            float gl = 0.f;
-            if (i < ci.len) gl = gate ? negA * softplus_fast(x + bias) : x;
-            run = fmaf(gl, LOG2E, run);  // explicit: both instantiations must round alike
-            sG[swz_f32(i, dch)] = run;
-        }
-        stot[quarter * D + dch] = run;
+    const float a_log_h = nx.a_log;
+    const float2 bias = nx.bias;
+    if (!tiles) copy_rows(ci, h);
+    const int bi = 4 * hw + (lane & 3);
+    const float be = bi < ci.len ? (sig ? sigmoid_f(__bfloat162float(nx.rb)) : __bfloat162float(nx.rb)) : 0.f;  // beta of row bi
+    if ((lane & 15) < 4) sbeta[bi] = be;
+    if (tiles) ok = mbar_wait(gbar, it & 1, p, 8);
+    if (CONV || ci.len < C) {
+        if (tiles) ok = mbar_wait(kbar, it & 1, p, 8) && mbar_wait(qbar, it & 1, p, 8) && ok;
+        if (ci.len < C) clear_tail(ci.len);
     }
     KDA_PHASE(0);
-    ok = mbar_wait(&vbar, it & 1, p, 8) && ok;
-    KDA_PHASE(14);
-    // Rows of a half warp: hw and hw + 32 without the convolution; 2 hw and 2 hw + 1 with it, so that
-    // the five input rows 2 hw - 3 .. 2 hw + 1 serve the two outputs of one thread.
-    uint4 rq4[2], rk4[2], rv4[2];
-    if constexpr (CONV) {
-        // ---- 0c: y[i] = silu(sum_j tap[j] x[i - 3 + j]) for the thread's two rows, rounded to
-        //      BF16 like the stand-alone convolution; the rest of the stage sees only y
-        const float4* sW = reinterpret_cast<const float4*>(dyn + TAPS);
-        // row x of a tensor's window (x = 0 .. 66 stands for token x - 3 of the chunk); the halo rows of v sit apart
-        auto conv_rows = [&](uint4(&out)[2], int tensor) {
-            float win[5][8];
+    // ---- L2 norm of the q and k rows, in place, two rows at a time.  The four sums of squares of a half warp (row m, tensor t) are
+    //      reduced by a transposing exchange, after which four lanes have each and turn it into 1 / norm: one square root and one
+    //      division, long instruction sequences, instead of four
+    auto normalise2 = [&](int i0, uint4 (&x4)[4]) {  // x4: row i0 q, k, row i0 + 1 q, k
+        if (l2) {
+            float s4[4], s2[2];
 #pragma unroll
-            for (int r = 0; r < 5; ++r) {
-                const int x = 2 * hw + r;
-                const __nv_bfloat16* row = tensor == 0 ? sRq + x * D : tensor == 1 ? sRk + x * D : (x < 3 ? sRvh + x * D : sRv + (x - 3) * D);
-                bf16x8_to_f32(*reinterpret_cast<const uint4*>(row + c8), win[r]);
+            for (int m = 0; m < 4; ++m) {
+                float x[8];
+                float2 a = make_float2(0.f, 0.f);
+                bf16x8_to_f32(x4[m], x);
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) {
+                    const float2 x2 = make_float2(x[j], x[j + 1]);
+                    a = __ffma2_rn(x2, x2, a);  // explicit: both instantiations must round alike
+                }
+                s4[m] = a.x + a.y;
             }
-            float y2[2][8];
+            const bool b8 = lane & 8, b4 = lane & 4;
 #pragma unroll
-            for (int j = 0; j < 8; j += 2) {  // two channels in packed FMAs (the order of conv_pre)
-                const float4 wa = sW[tensor * D + j * 16 + (c8 >> 3)], wb = sW[tensor * D + (j + 1) * 16 + (c8 >> 3)];
-                auto x2 = [&](int r) { return make_float2(win[r][j], win[r][j + 1]); };
+            for (int j = 0; j < 2; ++j) s2[j] = (b8 ? s4[2 + j] : s4[j]) + __shfl_xor_sync(0xffffffffu, b8 ? s4[j] : s4[2 + j], 8);
+            float s1 = (b4 ? s2[1] : s2[0]) + __shfl_xor_sync(0xffffffffu, b4 ? s2[0] : s2[1], 4);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
+            const float rn = 1.f / fmaxf(sqrtf(s1), 1e-6f);
+            if ((lane & 3) == 0) saux[(b4 ? C : 0) + i0 + (b8 ? 1 : 0)] = rn;
 #pragma unroll
-                for (int m = 0; m < 2; ++m) {
+            for (int m = 0; m < 4; ++m) {
+                const float n = __shfl_sync(0xffffffffu, rn, (lane & 16) + 4 * m);
+                float x[8];
+                bf16x8_to_f32(x4[m], x);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] *= n;
+                x4[m] = f32_to_bf16x8(x);
+            }
+        } else if ((lane & 3) == 0) {
+            saux[(lane & 4 ? C : 0) + i0 + (lane & 8 ? 1 : 0)] = 1.f;
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m) *reinterpret_cast<uint4*>((m & 1 ? sK : sQ) + swz_bf16(i0 + (m >> 1), c8r)) = x4[m];
+    };
+    auto store_v = [&](int m, const uint4& v4) {  // beta v of row 4 hw + m, the operand of the U product
+        const float b = __shfl_sync(0xffffffffu, be, (lane & 16) + m);
+        float x[8];
+        bf16x8_to_f32(v4, x);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] *= b;
+        *reinterpret_cast<uint4*>(sV + swz_bf16(4 * hw + m, c8r)) = f32_to_bf16x8(x);
+    };
+    if constexpr (CONV) {
+        // ---- 1: y[i] = silu(sum_j tap[j] x[i - 3 + j]) for the thread's four rows, rounded to BF16 like the stand-alone
+        //      convolution; everything after sees only y
+        auto conv_rows = [&](uint4(&out)[4], int tensor) {
+            uint4 win[7];
+#pragma unroll
+            for (int r = 0; r < 7; ++r) {
+                const int x = 4 * hw - 3 + r;
+                win[r] = *reinterpret_cast<const uint4*>(x < 0 ? sHalo + (3 * tensor + x + 3) * D + c8r
+                                                               : reinterpret_cast<__nv_bfloat16*>(dyn + SQ) + tensor * C * D + swz_bf16(x, c8r));
+            }
+            auto pick = [](const uint4& u, int j2) { return j2 == 0 ? u.x : j2 == 1 ? u.y : j2 == 2 ? u.z : u.w; };
+            uint32_t o[4][4];
+#pragma unroll
+            for (int j2 = 0; j2 < 4; ++j2) {  // two channels in packed FMAs (the order of conv_pre)
+                const int j = 2 * j2;
+                const float4 wa = sW[tensor * D + j * 16 + (tid & 15)], wb = sW[tensor * D + (j + 1) * 16 + (tid & 15)];
+                auto x2 = [&](int r) {
+                    const uint32_t w = pick(win[r], j2);
+                    return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+                };
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
                     const float2 pre = __ffma2_rn(make_float2(wa.w, wb.w), x2(m + 3),
                                                   __ffma2_rn(make_float2(wa.z, wb.z), x2(m + 2),
                                                              __ffma2_rn(make_float2(wa.y, wb.y), x2(m + 1), __fmul2_rn(make_float2(wa.x, wb.x), x2(m)))));
-                    y2[m][j] = silu_f(pre.x);
-                    y2[m][j + 1] = silu_f(pre.y);
+                    o[m][j2] = pack_bf16(silu_f(pre.x), silu_f(pre.y));
                 }
             }
 #pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                const float (&y)[8] = y2[m];
-                out[m] = 2 * hw + m < ci.len ? f32_to_bf16x8(y) : make_uint4(0, 0, 0, 0);
-            }
+            for (int m = 0; m < 4; ++m) out[m] = 4 * hw + m < ci.len ? make_uint4(o[m][0], o[m][1], o[m][2], o[m][3]) : zero4;
         };
-        conv_rows(rq4, 0);
-        conv_rows(rk4, 1);
+        uint4 rq4[4], rk4[4], rv4[4];
         conv_rows(rv4, 2);
         if (save) {
             __nv_bfloat16* gVc = (__nv_bfloat16*)(ws + L.Vc) + rec * C * D;
 #pragma unroll
-            for (int m = 0; m < 2; ++m) *reinterpret_cast<uint4*>(gVc + (2 * hw + m) * D + c8) = rv4[m];
+            for (int m = 0; m < 4; ++m) *reinterpret_cast<uint4*>(gVc + (4 * hw + m) * D + c8r) = rv4[m];
         }
-    } else {
+        conv_rows(rq4, 0);
+        conv_rows(rk4, 1);
+        __syncthreads();  // every row has been read
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const int off = (hw + 32 * m) * D + c8;
-            rq4[m] = *reinterpret_cast<const uint4*>(sRq + off);
-            rk4[m] = *reinterpret_cast<const uint4*>(sRk + off);
-            rv4[m] = *reinterpret_cast<const uint4*>(sRv + off);
-        }
-    }
-    // ---- 0b: q, k, v, beta row-wise: a half warp owns two rows, lane c8 the channels 8 c8 ..  The four sums of squares
-    //      (row m, tensor t) are reduced by a transposing exchange (5 shuffles instead of 16, the same additions), after
-    //      which lane 8 m + 4 t of the half warp turns its own into 1 / norm: one square root and one division, long
-    //      instruction sequences, per thread instead of four.  Likewise one sigmoid for the two betas.
-    {
-        auto row_of = [&](int m) { return CONV ? 2 * hw + m : hw + 32 * m; };
-        const int m_l = (lane >> 3) & 1, t_l = (lane >> 2) & 1, base = lane & 16;
-        float qf[2][8], kf[2][8], rn = 1.f;
+        for (int m = 0; m < 4; ++m) store_v(m, rv4[m]);
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            bf16x8_to_f32(rq4[m], qf[m]);
-            bf16x8_to_f32(rk4[m], kf[m]);
-        }
-        float b_l;  // beta of row m_l
-        {
-            const float b0 = __shfl_sync(0xffffffffu, rb[0], base), b1 = __shfl_sync(0xffffffffu, rb[1], base);
-            b_l = m_l ? b1 : b0;
-            if (sig) b_l = row_of(m_l) < ci.len ? sigmoid_f(b_l) : 0.f;
-        }
-        if (l2) {
-            float ss[2][2];  // [row][tensor]
-#pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                ss[m][0] = ss[m][1] = 0.f;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    ss[m][0] = fmaf(qf[m][j], qf[m][j], ss[m][0]);  // explicit: both instantiations must round alike
-                    ss[m][1] = fmaf(kf[m][j], kf[m][j], ss[m][1]);
-                }
-            }
-            float s2[2], s1;
-#pragma unroll
-            for (int t = 0; t < 2; ++t)
-                s2[t] = (m_l ? ss[1][t] : ss[0][t]) + __shfl_xor_sync(0xffffffffu, m_l ? ss[0][t] : ss[1][t], 8);
-            s1 = (t_l ? s2[1] : s2[0]) + __shfl_xor_sync(0xffffffffu, t_l ? s2[0] : s2[1], 4);
-            s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
-            s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
-            rn = 1.f / fmaxf(sqrtf(s1), 1e-6f);
-        }
-        if ((lane & 3) == 0) saux[t_l * C + row_of(m_l)] = rn;
-        if ((lane & 7) == 0) sbeta[row_of(m_l)] = b_l;
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const int i = row_of(m);
-            const float rq = __shfl_sync(0xffffffffu, rn, base + 8 * m), rk = __shfl_sync(0xffffffffu, rn, base + 8 * m + 4);
-            const float b = __shfl_sync(0xffffffffu, b_l, base + 8 * m);
-            float vf[8];
-            bf16x8_to_f32(rv4[m], vf);
-            if (l2) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    qf[m][j] *= rq;
-                    kf[m][j] *= rk;
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) vf[j] *= b;
-            *reinterpret_cast<uint4*>(sQ + swz_bf16(i, c8)) = f32_to_bf16x8(qf[m]);
-            *reinterpret_cast<uint4*>(sK + swz_bf16(i, c8)) = f32_to_bf16x8(kf[m]);
-            *reinterpret_cast<uint4*>(sBV + cm_idx(i, c8, D)) = f32_to_bf16x8(vf);
+        for (int m = 0; m < 4; m += 2) {
+            uint4 x4[4] = {rq4[m], rk4[m], rq4[m + 1], rk4[m + 1]};
+            normalise2(4 * hw + m, x4);
         }
     }
     KDA_PHASE(1);
-    tc_fence_before();
-    __syncthreads();  // the raw gate, q, k rows (operand space) and the raw v rows (L tile) are consumed
-    tc_fence_after();
-    // A and T must read zero above the diagonal: the stages below write A for j <= i only and T from the diagonal
-    // block down, and the records carry whole 64 x 64 tiles.  Row i is cleared from its diagonal block on, four
-    // floats at a time.  (L needs no clearing: the solve uses its diagonal blocks for j < i only, which the
-    // diagonal walks write, and the blocks below them whole, which the accumulator read-back writes.)
-#pragma unroll
-    for (int idx = tid; idx < C * 16; idx += NTHR) {
-        const int i = idx >> 4, q4 = idx & 15;
-        if (q4 >= 4 * (i >> 4)) {
-            *reinterpret_cast<float4*>(sA + i * LDR + 4 * q4) = make_float4(0.f, 0.f, 0.f, 0.f);
-            *reinterpret_cast<float4*>(sT + i * LDR + 4 * q4) = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    }
-    const uint32_t tmem0 = tmem_s;
-    // ---- the later 16-row groups of the cumulative sum pick up the totals of the earlier ones; every thread
-    //      keeps the 16 G values of its (block, channel) and evaluates the span guard of its tile (a warp is one
-    //      [16 rows x 32 channels] tile, k3mini/backends.py:17-19): where it passes, the diagonal block may use the
-    //      midpoint factorisation 2^(G_i - m) 2^(m - G_j) in FP32 (every factor within 2^(+-116)), for which the
-    //      thread leaves k_j 2^(m - G_j) of its rows in the (still free) operand space
-    float* smidf = reinterpret_cast<float*>(dyn + SMIDF);
-    int* spass = reinterpret_cast<int*>(dyn + SPASS);
-    float* sKN = reinterpret_cast<float*>(dyn + KN);
+    // ---- 2: gate.  Thread = (16-row group, two channels): running sums of the group, whose totals are passed on
     {
-        float t = 0.f;
-        if (quarter > 0) t = stot[dch];
-        if (quarter > 1) t += stot[D + dch];
-        if (quarter > 2) t += stot[2 * D + dch];
-        float Gr[16], mid;
+        const float negA = gate ? -expf(a_log_h) : 0.f;
+        const uint32_t* raw = reinterpret_cast<const uint32_t*>(sRG + 16 * qt * D + gd);
+        float2 run = make_float2(0.f, 0.f), Gr[16];
 #pragma unroll
         for (int r = 0; r < 16; ++r) {
-            Gr[r] = sG[swz_f32(16 * quarter + r, dch)] + t;
-            if (quarter > 0) sG[swz_f32(16 * quarter + r, dch)] = Gr[r];
+            const uint32_t w = raw[r * (D / 2)];
+            float2 gl = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+            if (gate) gl = __fmul2_rn(make_float2(negA, negA), softplus_fast2(__fadd2_rn(gl, bias)));
+            run = __ffma2_rn(gl, make_float2(LOG2E, LOG2E), run);  // explicit: both instantiations must round alike
+            Gr[r] = run;
         }
-        const bool tpass = guard_tile(Gr, p.guard_span, mid);
-        smidf[quarter * D + dch] = mid;
-        if (lane == 0) spass[quarter * 4 + (warp & 3)] = tpass ? 1 : 0;
-        if (tpass) {
+        *reinterpret_cast<float2*>(stot + qt * D + gd) = run;
+        KDA_PHASE(2);
+        if constexpr (!CONV) {  // (q is requested last and arrives last)
+            if (tiles && ci.len == C) ok = mbar_wait(kbar, it & 1, p, 8) && mbar_wait(qbar, it & 1, p, 8) && ok;
 #pragma unroll
-            for (int r = 0; r < 16; ++r)
-                sKN[swz_f32(16 * quarter + r, dch)] =
-                    __bfloat162float(sK[swz_bf16(16 * quarter + r, dch)]) * ex2_approx(mid - Gr[r]);
+            for (int m = 0; m < 4; m += 2) {
+                const int i = 4 * hw + m;
+                uint4 x4[4];
+#pragma unroll
+                for (int x = 0; x < 4; ++x) x4[x] = *reinterpret_cast<const uint4*>((x & 1 ? sK : sQ) + swz_bf16(i + (x >> 1), c8r));
+                store_v(m, *reinterpret_cast<const uint4*>(sV + swz_bf16(i, c8r)));
+                store_v(m + 1, *reinterpret_cast<const uint4*>(sV + swz_bf16(i + 1, c8r)));
+                normalise2(i, x4);
+            }
         }
+        __syncthreads();  // the totals of the groups are there
+        float2 base = make_float2(0.f, 0.f);
+        for (int b = 0; b < qt; ++b) base = __fadd2_rn(base, *reinterpret_cast<const float2*>(stot + b * D + gd));
+        // Span guard, after k3mini/backends.py:17-19, of the [8 rows x 64 channels] tiles: every channel monotone non-increasing and
+        // finite (then its span is first - last row), the largest span within the limit.  Where a span is too large the block goes
+        // by levels, where a channel is not monotone by pairs.
+        bool good = true;
+        float span = 0.f;
+        float2 prev = make_float2(INFINITY, INFINITY);
+#pragma unroll
+        for (int r0 = 0; r0 < 16; r0 += 8) {
+            float2 first;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                float2* at = reinterpret_cast<float2*>(sG + swz_f32(16 * qt + r0 + r, gd));
+                const float2 x = __fadd2_rn(Gr[r0 + r], base);
+                *at = x;
+                good = good && x.x <= prev.x && x.y <= prev.y;
+                prev = x;
+                if (r == 0) first = x;
+            }
+            *reinterpret_cast<float2*>(smid + (2 * qt + (r0 >> 3)) * D + gd) = make_float2(0.5f * (first.x + prev.x), 0.5f * (first.y + prev.y));
+            good = good && isfinite(first.x) && isfinite(first.y) && isfinite(prev.x) && isfinite(prev.y);
+            span = fmaxf(span, fmaxf(first.x - prev.x, first.y - prev.y));
+        }
+        good = __all_sync(0xffffffffu, good);
+        const bool narrow = __all_sync(0xffffffffu, span <= fminf(p.guard_span, MAX_SPAN));
+        if (lane == 0) smode[2 * qt + gh] = !good ? PAIRS : !narrow ? LEVELS : MIDPOINT;
     }
     fence_async_smem();
     __syncthreads();
-    KDA_PHASE(2);
-    // ---- diagonal blocks on the CUDA cores: midpoint-factorised where all four tiles of the block passed the
-    //      guard, exact (one exp2 per pair and channel) otherwise.  Thread = (block b, slot, channel slice cs): the eight lanes of a slot split the
-    // 128 channels (16 each: 32 u + 4 cs .. +3), keep their row i in registers, walk key rows j four at a
-    // time, and the eight slices of a pair meet in three shuffles.  Four warps share a block; the 136
-    // pairs (j <= i) of the block are dealt out so that no warp walks more than twelve key rows:
-    //   warps 0, 1 (slot s = 0..7):  row 8 + s            against keys 0..7   (all valid)
-    //   warps 2, 3 (slot s = 0..7):  row 15 - s           against keys 8..15, then row s against keys 0..7
-    // Eight lanes read 128 contiguous bytes of a row: no bank conflicts.
-    {
-        // (role w4 rotates with the block: the four warps of one scheduler, warp % 4 alike, take the four roles,
-        //  two short walks of 8 key rows and two long ones of 12, instead of four of a kind)
-        const int cs = lane & 7, b = warp >> 2, w4 = (warp + b) & 3, slot = 4 * (w4 & 1) + (lane >> 3);
-        // element offsets of this lane's channels 32 u + 4 cs .. + 3 inside the swizzled row r (swz_f32 / swz_bf16
-        // with the row-dependent part computed once per row): FP32 chunk 8 u + cs, BF16 chunk 4 u + cs / 2
-        auto goff = [&](int r, int u) { return 32 * u + 4 * (cs ^ (r & 7)); };
-        auto boff = [&](int r, int u) { return 8 * (((4 * u + (cs >> 1)) ^ (r & 7))) + 4 * (cs & 1); };
-        auto row_against = [&](int i, int jbeg, int jend) {  // jbeg, jend multiples of four, uniform over the warp
-            const int ri = 16 * b + i;
-            float gi[16], qi[16], ki[16];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float4 g4 = *reinterpret_cast<const float4*>(sG + ri * D + goff(ri, u));
-                gi[4 * u] = g4.x; gi[4 * u + 1] = g4.y; gi[4 * u + 2] = g4.z; gi[4 * u + 3] = g4.w;
-                const uint2 q2 = *reinterpret_cast<const uint2*>(sQ + ri * D + boff(ri, u));
-                const uint2 k2 = *reinterpret_cast<const uint2*>(sK + ri * D + boff(ri, u));
-                const float2 qa = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q2.x));
-                const float2 qb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q2.y));
-                const float2 ka = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&k2.x));
-                const float2 kb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&k2.y));
-                qi[4 * u] = qa.x; qi[4 * u + 1] = qa.y; qi[4 * u + 2] = qb.x; qi[4 * u + 3] = qb.y;
-                ki[4 * u] = ka.x; ki[4 * u + 1] = ka.y; ki[4 * u + 2] = kb.x; ki[4 * u + 3] = kb.y;
-            }
-            // four key rows at a time: their eight sums (a and l of each pair) are reduced over the eight
-            // slices by a transposing exchange, 7 shuffles instead of 24, after which lane cs owns sum
-            // number cs and stores it
-#pragma unroll 1
-            for (int j0 = jbeg; j0 < jend; j0 += 4) {
-                float v[8];
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    const int rj = 16 * b + j0 + jj;
-                    float2 av = make_float2(0.f, 0.f), lv = av;  // packed two-wide FMAs: even / odd channels
-                    const int gj0 = goff(rj, 0), kj0 = boff(rj, 0), kj1 = boff(rj, 1);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float4 g4 = *reinterpret_cast<const float4*>(sG + rj * D + gj0 + 32 * u);
-                        const uint2 k2 = *reinterpret_cast<const uint2*>(sK + rj * D + ((u & 1) ? kj1 : kj0) + 64 * (u >> 1));
-                        const float2 ka = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&k2.x));
-                        const float2 kb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&k2.y));
-                        // (rows j > i are computed too but never stored; whatever they overflow to is dropped)
-                        const float2 k01 = __fmul2_rn(ka, make_float2(ex2_approx(gi[4 * u] - g4.x), ex2_approx(gi[4 * u + 1] - g4.y)));
-                        const float2 k23 = __fmul2_rn(kb, make_float2(ex2_approx(gi[4 * u + 2] - g4.z), ex2_approx(gi[4 * u + 3] - g4.w)));
-                        av = __ffma2_rn(make_float2(qi[4 * u], qi[4 * u + 1]), k01, __ffma2_rn(make_float2(qi[4 * u + 2], qi[4 * u + 3]), k23, av));
-                        lv = __ffma2_rn(make_float2(ki[4 * u], ki[4 * u + 1]), k01, __ffma2_rn(make_float2(ki[4 * u + 2], ki[4 * u + 3]), k23, lv));
-                    }
-                    v[2 * jj] = av.x + av.y;
-                    v[2 * jj + 1] = lv.x + lv.y;
-                }
-                const bool b2 = cs & 4, b1 = cs & 2, b0 = cs & 1;
-                float w4s[4], w2s[2];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) w4s[t] = (b2 ? v[t + 4] : v[t]) + __shfl_xor_sync(0xffffffffu, b2 ? v[t] : v[t + 4], 4);
-#pragma unroll
-                for (int t = 0; t < 2; ++t) w2s[t] = (b1 ? w4s[t + 2] : w4s[t]) + __shfl_xor_sync(0xffffffffu, b1 ? w4s[t] : w4s[t + 2], 2);
-                const float sum = (b0 ? w2s[1] : w2s[0]) + __shfl_xor_sync(0xffffffffu, b0 ? w2s[0] : w2s[1], 1);
-                const int j = j0 + (cs >> 1);
-                if (j <= i) {
-                    if (!b0) sA[ri * LDR + 16 * b + j] = sum * p.scale;
-                    else if (j < i) sL[ri * LDR + 16 * b + j] = sum;
-                }
-            }
-        };
-        // guarded variant of the same walk: no exponential in the pair loop, the key rows come pre-scaled
-        auto row_against_mid = [&](int i, int jbeg, int jend) {
-            const int ri = 16 * b + i;
-            float qP[16], kP[16];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int d0 = 32 * u + 4 * cs;
-                const float4 g4 = *reinterpret_cast<const float4*>(sG + ri * D + goff(ri, u));
-                const float4 m4 = *reinterpret_cast<const float4*>(smidf + b * D + d0);
-                const uint2 q2 = *reinterpret_cast<const uint2*>(sQ + ri * D + boff(ri, u));
-                const uint2 k2 = *reinterpret_cast<const uint2*>(sK + ri * D + boff(ri, u));
-                const float2 qa = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q2.x));
-                const float2 qb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q2.y));
-                const float2 ka = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&k2.x));
-                const float2 kb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&k2.y));
-                const float p0 = ex2_approx(g4.x - m4.x), p1 = ex2_approx(g4.y - m4.y), p2 = ex2_approx(g4.z - m4.z),
-                            p3 = ex2_approx(g4.w - m4.w);
-                qP[4 * u] = qa.x * p0; qP[4 * u + 1] = qa.y * p1; qP[4 * u + 2] = qb.x * p2; qP[4 * u + 3] = qb.y * p3;
-                kP[4 * u] = ka.x * p0; kP[4 * u + 1] = ka.y * p1; kP[4 * u + 2] = kb.x * p2; kP[4 * u + 3] = kb.y * p3;
-            }
-#pragma unroll 2
-            for (int j0 = jbeg; j0 < jend; j0 += 4) {
-                float v[8];
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    const int rj = 16 * b + j0 + jj;
-                    const int gj0 = goff(rj, 0);
-                    float2 av = make_float2(0.f, 0.f), lv = av;
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float4 kn = *reinterpret_cast<const float4*>(sKN + rj * D + gj0 + 32 * u);
-                        const float2 k01 = make_float2(kn.x, kn.y), k23 = make_float2(kn.z, kn.w);
-                        av = __ffma2_rn(make_float2(qP[4 * u], qP[4 * u + 1]), k01, __ffma2_rn(make_float2(qP[4 * u + 2], qP[4 * u + 3]), k23, av));
-                        lv = __ffma2_rn(make_float2(kP[4 * u], kP[4 * u + 1]), k01, __ffma2_rn(make_float2(kP[4 * u + 2], kP[4 * u + 3]), k23, lv));
-                    }
-                    v[2 * jj] = av.x + av.y;
-                    v[2 * jj + 1] = lv.x + lv.y;
-                }
-                const bool b2 = cs & 4, b1 = cs & 2, b0 = cs & 1;
-                float w4s[4], w2s[2];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) w4s[t] = (b2 ? v[t + 4] : v[t]) + __shfl_xor_sync(0xffffffffu, b2 ? v[t] : v[t + 4], 4);
-#pragma unroll
-                for (int t = 0; t < 2; ++t) w2s[t] = (b1 ? w4s[t + 2] : w4s[t]) + __shfl_xor_sync(0xffffffffu, b1 ? w4s[t] : w4s[t + 2], 2);
-                const float sum = (b0 ? w2s[1] : w2s[0]) + __shfl_xor_sync(0xffffffffu, b0 ? w2s[0] : w2s[1], 1);
-                const int j = j0 + (cs >> 1);
-                if (j <= i) {
-                    if (!b0) sA[ri * LDR + 16 * b + j] = sum * p.scale;
-                    else if (j < i) sL[ri * LDR + 16 * b + j] = sum;
-                }
-            }
-        };
-        const bool fast = (spass[4 * b] & spass[4 * b + 1] & spass[4 * b + 2] & spass[4 * b + 3]) != 0;  // uniform over the block
-        // warps 0, 1 of a block: row 8 + slot against keys 0..7; warp 2: rows 15 - slot (15..12) against keys 8..15, then
-        // rows slot (0..3) against keys 0..3; warp 3: rows 15 - slot (11..8) against keys 8..11, then rows slot (4..7)
-        // against keys 0..7.
-        if constexpr (CONV) {
-            // One rolled loop over the (at most two) segments keeps a single copy of each walk in the code: with the
-            // convolution the kernel is ~190 KB of instructions otherwise, every unit fetches them anew, and above
-            // that size the fetches started to cost (1.89 -> 1.71 ms on the sublayer workload).
-            const int nseg = w4 < 2 ? 1 : 2;
-#pragma unroll 1
-            for (int sgi = 0; sgi < nseg; ++sgi) {
-                int i, jb, je;
-                if (w4 < 2) { i = 8 + slot; jb = 0; je = 8; }
-                else if (sgi == 0) { i = 15 - slot; jb = 8; je = w4 == 2 ? 16 : 12; }
-                else { i = slot; jb = 0; je = w4 == 2 ? 4 : 8; }
-                if (fast) row_against_mid(i, jb, je);
-                else row_against(i, jb, je);
-            }
-        } else if (fast) {  // (without the convolution the straight-line form fits and is 0.3 us per unit faster)
-            if (w4 < 2) {
-                row_against_mid(8 + slot, 0, 8);
-            } else {
-                row_against_mid(15 - slot, 8, w4 == 2 ? 16 : 12);
-                row_against_mid(slot, 0, w4 == 2 ? 4 : 8);
-            }
-        } else if (w4 < 2) {
-            row_against(8 + slot, 0, 8);
-        } else {
-            row_against(15 - slot, 8, w4 == 2 ? 16 : 12);
-            row_against(slot, 0, w4 == 2 ? 4 : 8);
-        }
-    }
-    __syncthreads();  // the pre-scaled key rows are dead: their space becomes operand space
-    KDA_PHASE(10);
-    // ---- 1: decay-scaled operands of the off-diagonal products.  A warp takes 8 rows x 4 channel groups at a
-    //      time, so that its 16-byte stores into the core-matrix tiles cover four whole 128-byte core matrices
-    //      (no bank conflicts; the row-major loads of q^, k^, G take the conflicts instead, and
-    //      there are fewer of them).  A block's rows serve as queries for their own block and as keys for the later
-    //      ones, so a warp pairs an early combination of rows and channels with a late one.  (Key rows >= 16 I of
-    //      block I's operand keep what was there: their accumulator rows are not read.)
-    auto combo_rows = [&](int it) {
-        const int combo = it ? 31 - warp : warp;
-        return make_int2(8 * (combo >> 2) + (lane & 7), 8 * (4 * (combo & 3) + (lane >> 3)));
-    };
-    auto load_g8 = [&](int i, int c8, float (&x)[8]) {
-        const float4 a = *reinterpret_cast<const float4*>(sG + swz_f32(i, c8));
-        const float4 b = *reinterpret_cast<const float4*>(sG + swz_f32(i, c8 + 4));
-        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-    };
-#pragma unroll 1
-    for (int it = 0; it < 2; ++it) {
-        const int2 ic = combo_rows(it);
-        const int i = ic.x, c8 = ic.y, m = i >> 4;
-        float G8[8], kf[8], o8[8], r[8];
-        load_g8(i, c8, G8);
-        bf16x8_to_f32(*reinterpret_cast<const uint4*>(sK + swz_bf16(i, c8)), kf);
-        if (m >= 1) {  // rows of block m as the N operand of block m's products
-            float qf[8];
-            bf16x8_to_f32(*reinterpret_cast<const uint4*>(sQ + swz_bf16(i, c8)), qf);
-            load_g8(16 * m, c8, r);
-            __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(dyn + XSC + (m - 1) * 8192);
-            float f[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] = ex2_approx(G8[j] - r[j]);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o8[j] = qf[j] * f[j];
-            *reinterpret_cast<uint4*>(xs + cm_idx(i - 16 * m, c8, D)) = f32_to_bf16x8(o8);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o8[j] = kf[j] * f[j];
-            *reinterpret_cast<uint4*>(xs + cm_idx(16 + i - 16 * m, c8, D)) = f32_to_bf16x8(o8);
-        }
-#pragma unroll 1
-        for (int I = m + 1; I <= 3; ++I) {  // keys scaled for the later blocks
-            __nv_bfloat16* ks = reinterpret_cast<__nv_bfloat16*>(dyn + KSC + (I - 1) * 16384);
-            load_g8(16 * I, c8, r);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o8[j] = kf[j] * ex2_approx(r[j] - G8[j]);
-            *reinterpret_cast<uint4*>(ks + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
-        }
-    }
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-
     KDA_PHASE(3);
-    // ---- 2: off-diagonal blocks on the tensor cores, diagonal blocks exactly on the CUDA cores
-    // (lane 0 of warps 0, 1, 2 issues the eight MMAs of block I = warp + 1: the accumulators are
-    //  independent, and no warp starts its share of the diagonal work a whole issue sequence late)
-    if (warp < 3 && lane == 0) {
-        tc_fence_after();
-        const uint32_t sb = smem_u32(dyn);
-        constexpr uint32_t id = make_idesc(64, 32, false, false);
-        const int I = warp + 1;
-#pragma unroll
-        for (int s = 0; s < 8; ++s)
-            mma_ss(tmem0 + T_D + 32 * (I - 1), make_desc(sb + KSC + (I - 1) * 16384 + s * 256, 128, 2048),
-                   make_desc(sb + XSC + (I - 1) * 8192 + s * 256, 128, 2048), id, s > 0);
-        mma_commit(&bar);
-    }
-    if (more) ci_nx = chunk_info(p, un.c);  // (dependent loads: issued well ahead of the requests that need them)
-    // ---- meanwhile: the Qt and Kh records and the operand beta k 2^G of the W product
-#pragma unroll 1
-    for (int it = 0; it < 2; ++it) {
-        const int2 ic = combo_rows(it);
-        const int i = ic.x, c8 = ic.y;
-        float G8[8], qf[8], kf[8], o8[8], eg[8], gl[8];
-        load_g8(i, c8, G8);
-        load_g8(C - 1, c8, gl);
-        bf16x8_to_f32(*reinterpret_cast<const uint4*>(sQ + swz_bf16(i, c8)), qf);
-        bf16x8_to_f32(*reinterpret_cast<const uint4*>(sK + swz_bf16(i, c8)), kf);
-        const float bi = sbeta[i];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) eg[j] = ex2_approx(G8[j]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o8[j] = p.scale * qf[j] * eg[j];
-        *reinterpret_cast<uint4*>(gQt + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o8[j] = bi * kf[j] * eg[j];
-        *reinterpret_cast<uint4*>(sKB + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o8[j] = kf[j] * ex2_approx(gl[j] - G8[j]);
-        *reinterpret_cast<uint4*>(gKh + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
-    }
-    KDA_PHASE(4);
-    ok = mbar_wait(&bar, it & 1, p, 8) && ok;
-    tc_fence_after();
-    KDA_PHASE(11);
-    if (ok) {  // warp (quadrant, group): accumulator columns 32 group .. 32 group + 31 = block I = group + 1
-        const int grp = warp >> 2;
-        if (grp == 0) read_offdiag<0>(tmem0 + T_D, warp & 3, lane, sA, sL, p.scale);
-        else if (grp == 1) read_offdiag<32>(tmem0 + T_D, warp & 3, lane, sA, sL, p.scale);
-        else if (grp == 2) read_offdiag<64>(tmem0 + T_D, warp & 3, lane, sA, sL, p.scale);
-        else invert_diagonal(sL, sT, sbeta, warp & 3, lane);
-    }
-    KDA_PHASE(12);
-    tc_fence_before();
-    __syncthreads();
-    if (more) {  // the operand tiles of the off-diagonal products are dead; the scalars have the inversion to arrive
-        request_rows(ci_nx, un.head());
-        request_scalars(ci_nx, un.head(), nx);
-    }
-    KDA_PHASE(15);
-
-    KDA_PHASE(5);
-    // (issued here rather than before the operand stage, whose shared-memory traffic they would share)
-    if (tid == NTHR - 64 && save) {  // prologue results for the backward: bulk stores straight from shared memory, issued by a
-                                     // thread of a warp that has no diagonal block to invert
-        tma_store_1d((float*)(ws + L.Gc) + rec * C * D, sG, C * D * 4);
-        tma_store_1d((__nv_bfloat16*)(ws + L.Qn) + rec * C * D, sQ, C * D * 2);
-        tma_store_1d((__nv_bfloat16*)(ws + L.Kn) + rec * C * D, sK, C * D * 2);
-        tma_store_1d((float*)(ws + L.aux) + rec * 3 * C, saux, 3 * C * 4);
+    if (save && lane == 0 && warp < 3) {  // prologue results for the backward: bulk stores straight from shared memory
+        if (warp == 0) tma_store_1d((float*)(ws + L.Gc) + rec * C * D, sG, C * D * 4);
+        if (warp == 1) tma_store_1d((__nv_bfloat16*)(ws + L.Qn) + rec * C * D, sQ, C * D * 2);
+        if (warp == 2) {
+            tma_store_1d((__nv_bfloat16*)(ws + L.Kn) + rec * C * D, sK, C * D * 2);
+            tma_store_1d((float*)(ws + L.aux) + rec * 3 * C, saux, 3 * C * 4);
+        }
         tma_store_commit();
     }
-
-    // ---- 3: T = (I + diag(beta) L)^-1; the inner products pass through the space behind T's operand tile
-    if (warp < 8) {
-        invert_products(sL, sT, sbeta, reinterpret_cast<float*>(dyn + KSC + 8192), warp, lane);
-    } else if (warp < 14) {  // the Aqk record; eight lanes = eight adjacent rows of one 8-column group, as below
-        for (int x = tid - 256; x < C * C / 8; x += 192) {
-            const int i = (x & 7) | ((x >> 6) << 3), j8 = ((x >> 3) & 7) * 8;
-            float a8[8];
+    uw.next();  // from here on the next unit of this CTA
+    more = uw.unit < n_units;
+    if (more) ci = chunk_info(p, uw.c);  // (dependent loads: issued well ahead of the requests that need them)
+    // ---- 3: Aqk and L.  Warp = (block I, channel half hf)
+    const int gq = lane >> 2, t = lane & 3;
+    const int I = warp < 4 ? warp : 7 - warp, hf = warp >> 2;  // (a scheduler's two warps share the work of one to four block pairs)
+    const int pr = ((gq & 1) << 2) | (gq & 2) | (gq >> 2), kt = (t >> 1) | ((t & 1) << 1);  // row g; keys 2t and 2t + 1 are kt, kt + 4
+    const int mode = max(smode[2 * I], smode[2 * I + 1]);  // (both halves must agree on where the sums are)
+    float keep[4][8];  // the matrix this warp finishes, Aqk (half 0) or L (half 1): [J][4 n-tile + fragment], keep[3] the diagonal block
+    {
+        float oq[3][2][4] = {}, ol[3][2][4] = {}, dq[2][4] = {}, dl[2][4] = {}, db[4] = {};
+#pragma unroll 1
+        for (int s = 0; s < 4; ++s) {
+            // (every row of this loop is pr mod 8: one swizzled offset for all, a row is a constant away from row pr)
+            const int ch = 64 * hf + 16 * s + 4 * t;
+            const float* pG = sG + swz_f32(pr, ch);
+            const __nv_bfloat16 *pK = sK + swz_bf16(pr, ch), *pQI = pK + (16 * I * 64 - 8192), *pKI = pK + 16 * I * 64;
+            const float4 G0 = *reinterpret_cast<const float4*>(pG + 16 * I * D), G1 = *reinterpret_cast<const float4*>(pG + 16 * I * D + 8 * D);
+            float q0[4], q1[4], k0[4], k1[4];
+            unpack4(*reinterpret_cast<const uint2*>(pQI), q0);
+            unpack4(*reinterpret_cast<const uint2*>(pQI + 8 * 64), q1);
+            unpack4(*reinterpret_cast<const uint2*>(pKI), k0);
+            unpack4(*reinterpret_cast<const uint2*>(pKI + 8 * 64), k1);
+            if (I > 0) {  // earlier blocks: reference r_I (row 16 I, which the swizzle leaves as it is)
+                const float4 rf = *reinterpret_cast<const float4*>(sG + 16 * I * D + ch);
+                float f0[4], f1[4];
+                exp2_diff(G0, rf, f0);
+                exp2_diff(G1, rf, f1);
+                uint32_t aq[4], ak[4];
 #pragma unroll
-            for (int j = 0; j < 8; j += 4) {
-                const float4 a = *reinterpret_cast<const float4*>(sA + i * LDR + j8 + j);
-                a8[j] = a.x, a8[j + 1] = a.y, a8[j + 2] = a.z, a8[j + 3] = a.w;
+                for (int x = 0; x < 2; ++x) {
+                    aq[2 * x] = pack_bf16(q0[2 * x] * f0[2 * x], q0[2 * x + 1] * f0[2 * x + 1]);
+                    aq[2 * x + 1] = pack_bf16(q1[2 * x] * f1[2 * x], q1[2 * x + 1] * f1[2 * x + 1]);
+                    ak[2 * x] = pack_bf16(k0[2 * x] * f0[2 * x], k0[2 * x + 1] * f0[2 * x + 1]);
+                    ak[2 * x + 1] = pack_bf16(k1[2 * x] * f1[2 * x], k1[2 * x + 1] * f1[2 * x + 1]);
+                }
+#pragma unroll
+                for (int J = 0; J < 3; ++J)
+                    if (J < I) {
+#pragma unroll
+                        for (int n = 0; n < 2; ++n) {
+                            float kf[4], f[4];
+                            unpack4(*reinterpret_cast<const uint2*>(pK + (16 * J + 8 * n) * 64), kf);
+                            exp2_diff(rf, *reinterpret_cast<const float4*>(pG + (16 * J + 8 * n) * D), f);
+                            const uint32_t b0 = pack_bf16(kf[0] * f[0], kf[1] * f[1]), b1 = pack_bf16(kf[2] * f[2], kf[3] * f[3]);
+                            mma_bf16(oq[J][n], aq, b0, b1);
+                            mma_bf16(ol[J][n], ak, b0, b1);
+                        }
+                    }
             }
-            *reinterpret_cast<uint4*>(gA + cm_idx(i, j8, C)) = f32_to_bf16x8(a8);
+            if (mode == MIDPOINT) {
+                // the diagonal block: keys 0 .. 7 against all rows with the midpoint of rows 0 .. 7 as reference, keys 8 .. 15 against
+                // rows 8 .. 15 (of q and of k, one operand) with theirs
+                const float4 ma = *reinterpret_cast<const float4*>(smid + 2 * I * D + ch), mb = *reinterpret_cast<const float4*>(smid + (2 * I + 1) * D + ch);
+                float p0[4], p1[4], p2[4], y0[4], y1[4];
+                exp2_diff(G0, ma, p0);
+                exp2_diff(G1, ma, p1);
+                exp2_diff(G1, mb, p2);
+                exp2_diff(ma, G0, y0);
+                exp2_diff(mb, G1, y1);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    y0[j] *= k0[j];
+                    y1[j] *= k1[j];
+                }
+#pragma unroll
+                for (int e = 0; e < 4; e += 2) {  // channels e, e + 1: fragment order (upper row, lower row) of the first, then of the second
+                    Split2 y;
+                    split_tf32(y0[e], y.h[0], y.l[0]);
+                    split_tf32(y0[e + 1], y.h[1], y.l[1]);
+                    mma_tf32x3(dq[0], q0[e] * p0[e], q1[e] * p1[e], q0[e + 1] * p0[e + 1], q1[e + 1] * p1[e + 1], y);
+                    mma_tf32x3(dl[0], k0[e] * p0[e], k1[e] * p1[e], k0[e + 1] * p0[e + 1], k1[e + 1] * p1[e + 1], y);
+                    split_tf32(y1[e], y.h[0], y.l[0]);
+                    split_tf32(y1[e + 1], y.h[1], y.l[1]);
+                    mma_tf32x3(db, q1[e] * p2[e], k1[e] * p2[e], q1[e + 1] * p2[e + 1], k1[e + 1] * p2[e + 1], y);
+                }
+            }
         }
+        if (mode == MIDPOINT) {
+            dq[1][2] = db[0];
+            dq[1][3] = db[1];
+            dl[1][2] = db[2];
+            dl[1][3] = db[3];
+        } else if (mode == LEVELS) {
+            // Halving: the rows of the second half of 16, 8, 4, 2 consecutive rows against the keys of the first, with G at the
+            // second half's first row as reference: every exponent is <= 0.  Eight rows (q and k rows in one operand) and eight keys a
+            // level; what belongs to different halves is dropped.  Half 0 leaves its Aqk above the diagonal of sAd and
+            // its L in place, half 1 its Aqk in place in sAd and its L above the diagonal.
+#pragma unroll 1
+            for (int b = 3; b >= 0; --b) {
+                const int w = 1 << b, key = ((pr >> b) << (b + 1)) | (pr & (w - 1)), row = key | w, ref = (key & ~(w - 1)) | w;
+                float acc[4] = {};
+#pragma unroll 1
+                for (int s = 0; s < 4; ++s) {
+                    const int ch = 64 * hf + 16 * s + 4 * t;
+                    const float4 rf = *reinterpret_cast<const float4*>(sG + swz_f32(16 * I + ref, ch));
+                    float qf[4], kf[4], kk[4], f[4], y[4];
+                    unpack4(*reinterpret_cast<const uint2*>(sQ + swz_bf16(16 * I + row, ch)), qf);
+                    unpack4(*reinterpret_cast<const uint2*>(sK + swz_bf16(16 * I + row, ch)), kf);
+                    unpack4(*reinterpret_cast<const uint2*>(sK + swz_bf16(16 * I + key, ch)), kk);
+                    exp2_diff(*reinterpret_cast<const float4*>(sG + swz_f32(16 * I + row, ch)), rf, f);
+                    exp2_diff(rf, *reinterpret_cast<const float4*>(sG + swz_f32(16 * I + key, ch)), y);
+#pragma unroll
+                    for (int e = 0; e < 4; e += 2) {
+                        Split2 yy;
+                        split_tf32(kk[e] * y[e], yy.h[0], yy.l[0]);
+                        split_tf32(kk[e + 1] * y[e + 1], yy.h[1], yy.l[1]);
+                        mma_tf32x3(acc, qf[e] * f[e], kf[e] * f[e], qf[e + 1] * f[e + 1], kf[e + 1] * f[e + 1], yy);
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int kn = kt + 4 * e, kj = ((kn >> b) << (b + 1)) | (kn & (w - 1));  // key number kn of the level
+                    if ((kn >> b) == (pr >> b)) {
+                        if (hf) {
+                            sAd[(16 * I + row) * LDA + kj] = acc[e];
+                            sM[(16 * I + kj) * LDR + 16 * I + row] = acc[2 + e];
+                        } else {
+                            sAd[(16 * I + kj) * LDA + row] = acc[e];
+                            sM[(16 * I + row) * LDR + 16 * I + kj] = acc[2 + e];
+                        }
+                    }
+                }
+            }
+            // the diagonal of Aqk: products of BF16 numbers
+            float d0[4] = {}, d1[4] = {};
+#pragma unroll 1
+            for (int s = 0; s < 4; ++s) {
+                const int ch = 64 * hf + 16 * s + 4 * t, r0 = 16 * I + pr;
+                const uint2 a = *reinterpret_cast<const uint2*>(sQ + swz_bf16(r0, ch)), b = *reinterpret_cast<const uint2*>(sQ + swz_bf16(r0 + 8, ch));
+                const uint2 x = *reinterpret_cast<const uint2*>(sK + swz_bf16(r0, ch)), y = *reinterpret_cast<const uint2*>(sK + swz_bf16(r0 + 8, ch));
+                const uint32_t a4[4] = {a.x, b.x, a.y, b.y};
+                mma_bf16(d0, a4, x.x, x.y);
+                mma_bf16(d1, a4, y.x, y.y);
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                if (pr == kt + 4 * e) {
+                    sAd[(16 * I + pr) * LDA + (hf ? pr : 16)] = d0[e];
+                    sAd[(16 * I + pr + 8) * LDA + (hf ? pr + 8 : 16)] = d1[2 + e];
+                }
+        } else {  // the pairs one by one: rows pr, pr + 8 against keys kt, kt + 4, kt + 8, kt + 12
+#pragma unroll 1
+            for (int x = 0; x < 16; ++x) {
+                const int ch = 64 * hf + 4 * x;
+                float Gr[2][4], qf[2][4], kf[2][4];
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    const int row = 16 * I + pr + 8 * m;
+                    const float4 G4 = *reinterpret_cast<const float4*>(sG + swz_f32(row, ch));
+                    Gr[m][0] = G4.x; Gr[m][1] = G4.y; Gr[m][2] = G4.z; Gr[m][3] = G4.w;
+                    unpack4(*reinterpret_cast<const uint2*>(sQ + swz_bf16(row, ch)), qf[m]);
+                    unpack4(*reinterpret_cast<const uint2*>(sK + swz_bf16(row, ch)), kf[m]);
+                }
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    const int row = 16 * I + kt + 4 * n;
+                    const float4 G4 = *reinterpret_cast<const float4*>(sG + swz_f32(row, ch));
+                    const float Gk[4] = {G4.x, G4.y, G4.z, G4.w};
+                    float kk[4];
+                    unpack4(*reinterpret_cast<const uint2*>(sK + swz_bf16(row, ch)), kk);
+#pragma unroll
+                    for (int m = n >> 1; m < 2; ++m)  // (keys 8 .. 15 have no pairs with rows 0 .. 7)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            // (pairs j > i are computed too but never used; whatever they overflow to is dropped)
+                            const float e = kk[j] * ex2_approx(Gr[m][j] - Gk[j]);
+                            float &a = dq[n >> 1][2 * m + (n & 1)], &l = dl[n >> 1][2 * m + (n & 1)];
+                            a = fmaf(qf[m][j], e, a);
+                            l = fmaf(kf[m][j], e, l);
+                        }
+                }
+            }
+        }
+        // each half gives the other the partial sums of the matrix that one finishes: L to its place, Aqk to the
+        // mirrored place above the diagonal blocks
+        auto hand_over = [&](int J, const float (&give)[2][4], const float (&own)[2][4], float (&mine)[8]) {
+            float* dst = hf == 0 ? sM + (16 * I + pr) * LDR + 16 * J + kt
+                       : J < I   ? sM + (16 * J + pr) * LDR + 16 * I + kt
+                                 : sAd + (16 * I + pr) * LDA + kt;
+            const int ld = hf && J == I ? LDA : LDR;
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    dst[(x >> 1) * 8 * ld + 8 * n + 4 * (x & 1)] = give[n][x];
+                    mine[4 * n + x] = own[n][x];
+                }
+        };
+        if (hf) {
+            if (mode != LEVELS) hand_over(I, dq, dl, keep[3]);
+#pragma unroll
+            for (int J = 0; J < 3; ++J)
+                if (J < I) hand_over(J, oq[J], ol[J], keep[J]);
+        } else {
+            if (mode != LEVELS) hand_over(I, dl, dq, keep[3]);
+#pragma unroll
+            for (int J = 0; J < 3; ++J)
+                if (J < I) hand_over(J, ol[J], oq[J], keep[J]);
+        }
+    }
+    KDA_PHASE(4);
+    // ---- the Qt, Kh and gamC records.  A warp takes eight rows x four channel chunks at a time (eight lanes = the rows of one core
+    //      matrix: no bank conflicts, whole 128-byte lines); the later its block, the more products it had, the fewer it takes
+    {
+        __nv_bfloat16* gQt = (__nv_bfloat16*)(ws + L.Qt) + rec * C * D;
+        __nv_bfloat16* gKh = (__nv_bfloat16*)(ws + L.Kh) + rec * C * D;
+        const int beg = 16 * hf + (I == 0 ? 0 : I == 1 ? 8 : I == 2 ? 13 : 16), end = 16 * hf + (I == 0 ? 8 : I == 1 ? 13 : 16);
+#pragma unroll 1
+        for (int x = beg; x < end; ++x) {
+            const int i = 8 * (x >> 2) + (lane & 7), c8 = 8 * (4 * (x & 3) + (lane >> 3));
+            float G8[8], x8[8], o8[8], gl[8];
+            load_g8(i, c8, G8);
+            load_g8(C - 1, c8, gl);
+            bf16x8_to_f32(*reinterpret_cast<const uint4*>(sQ + swz_bf16(i, c8)), x8);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o8[j] = p.scale * x8[j] * ex2_approx(G8[j]);
+            *reinterpret_cast<uint4*>(gQt + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
+            bf16x8_to_f32(*reinterpret_cast<const uint4*>(sK + swz_bf16(i, c8)), x8);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o8[j] = x8[j] * ex2_approx(gl[j] - G8[j]);
+            *reinterpret_cast<uint4*>(gKh + cm_idx(i, c8, D)) = f32_to_bf16x8(o8);
+        }
+    }
+    KDA_PHASE(5);
+    if (save && lane == 0 && warp < 3) tma_store_wait_read();  // the bulk stores have read q^, k^, G
+    __syncthreads();
+    KDA_PHASE(6);
+    // ---- 4: the halves' sums: Aqk record (half 0), L and the inverse of its diagonal block (half 1)
+    auto other = [&](int J) { return hf ? sM + (16 * I + pr) * LDR + 16 * J + kt : J < I ? sM + (16 * J + pr) * LDR + 16 * I + kt : sAd + (16 * I + pr) * LDA + kt; };
+    if (hf) {
+#pragma unroll
+        for (int J = 0; J < 4; ++J)
+            if (J < I || J == 3) {
+                float* dst = other(J == 3 ? I : J);
+#pragma unroll
+                for (int x = 0; x < 8; ++x) {
+                    const int m8 = ((x >> 1) & 1) * 8, n8 = 8 * (x >> 2) + 4 * (x & 1);
+                    float* d = dst + m8 * LDR + n8;
+                    if (J == 3 && mode == LEVELS) {
+                        if (kt + n8 < pr + m8) *d += sM[(16 * I + kt + n8) * LDR + 16 * I + pr + m8];
+                    } else {
+                        *d += keep[J][x];
+                    }
+                }
+            }
+        __syncwarp();
+        invert_diagonal(sM, sbeta, I, lane);
+    } else {
+        __nv_bfloat16* gA = (__nv_bfloat16*)(ws + L.Aqk) + rec * C * C;
+#pragma unroll
+        for (int J = 0; J < 4; ++J)
+            if (J < I || J == 3) {
+                const int Jb = J == 3 ? I : J;
+                const float* src = other(Jb);
+                const int ld = J == 3 ? LDA : LDR;
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        float a[2];
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const float* s = src + m * 8 * ld + 8 * n + 4 * e;
+                            float own = keep[J][4 * n + 2 * m + e];
+                            if (J == 3 && mode == LEVELS) {
+                                const int row = pr + 8 * m, key = kt + 4 * e + 8 * n;
+                                own = sAd[key < row ? (16 * I + key) * LDA + row : (16 * I + row) * LDA + 16];
+                            }
+                            a[e] = (own + *s) * p.scale;
+                            if (J == 3 && kt + 4 * e + 8 * n > pr + 8 * m) a[e] = 0.f;
+                        }
+                        // adjacent keys meet in a lane pair: lanes 0, 1 take keys (0, 1), (2, 3), lanes 2, 3 keys (4, 5), (6, 7)
+                        const float got = __shfl_xor_sync(0xffffffffu, t < 2 ? a[1] : a[0], 2);
+                        *reinterpret_cast<uint32_t*>(gA + cm_idx(16 * I + pr + 8 * m, 16 * Jb + 8 * n, C) + 2 * t) =
+                            t < 2 ? pack_bf16(a[0], got) : pack_bf16(got, a[1]);
+                    }
+            }
+        for (int J = I + 1; J < 4; ++J)
+            *reinterpret_cast<uint4*>(gA + cm_idx(16 * I + (lane & 15), 16 * J + 8 * (lane >> 4), C)) = zero4;
+    }
+    KDA_PHASE(7);
+    if (tid < D) ((float*)(ws + L.gamC))[rec * D + tid] = ex2_approx(sG[swz_f32(C - 1, tid)]);
+    // ---- beta k^ 2^G, the operand of the W product, in place of q^
+#pragma unroll 1
+    for (int x = 0; x < 4; ++x) {
+        const int i = 8 * warp + (lane & 7), c8 = 8 * (4 * x + (lane >> 3));
+        float G8[8], kf[8];
+        load_g8(i, c8, G8);
+        bf16x8_to_f32(*reinterpret_cast<const uint4*>(sK + swz_bf16(i, c8)), kf);
+        const float b = sbeta[i];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) kf[j] = b * kf[j] * ex2_approx(G8[j]);
+        *reinterpret_cast<uint4*>(sQ + swz_bf16(i, c8)) = f32_to_bf16x8(kf);
     }
     fence_async_smem();
     __syncthreads();
-    if (more) request_v(ci_nx, un.head());  // L is dead: its tile receives the next unit's v rows
-
-    KDA_PHASE(6);
-    // ---- 4: T record; T as the B operand of the WY products
-    {
-        __nv_bfloat16* sTB = reinterpret_cast<__nv_bfloat16*>(dyn + KSC);
+    KDA_PHASE(12);
+    if (more) {  // k^ is dead
+        request_k(ci, uw.head());
+        request_scalars(ci, uw.head(), nx);
+        request_taps(uw.head());
+    }
+    invert_products(sM, sbeta, sY, warp, lane);
+    __syncthreads();
+    KDA_PHASE(8);
+    // ---- 5: T record; T as the B operand of the WY products (zero above the diagonal blocks, where other things were)
+#pragma unroll 1
+    for (int m = 0; m < 2; ++m) {
         // eight lanes = eight adjacent rows of one 8-column group: one core matrix of the records, 32 distinct banks
-        const int i = (tid & 7) | ((tid >> 6) << 3), j8 = ((tid >> 3) & 7) * 8;
-        float t8[8];
+        const int x = tid + NTHR * m, i = (x & 7) | ((x >> 6) << 3), j8 = ((x >> 3) & 7) * 8;
+        uint4 tb = zero4;
+        if ((j8 >> 4) <= (i >> 4)) {
+            float t8[8];
 #pragma unroll
-        for (int j = 0; j < 8; j += 4) {
-            const float4 t = *reinterpret_cast<const float4*>(sT + i * LDR + j8 + j);
-            t8[j] = t.x, t8[j + 1] = t.y, t8[j + 2] = t.z, t8[j + 3] = t.w;
+            for (int j = 0; j < 8; j += 4) {
+                const float4 t4 = *reinterpret_cast<const float4*>(sM + i * LDR + j8 + j);
+                t8[j] = t4.x, t8[j + 1] = t4.y, t8[j + 2] = t4.z, t8[j + 3] = t4.w;
+            }
+            tb = f32_to_bf16x8(t8);
         }
-        const uint4 tb = f32_to_bf16x8(t8);
-        if (save) *reinterpret_cast<uint4*>(gT + cm_idx(i, j8, C)) = tb;
+        if (save) *reinterpret_cast<uint4*>((__nv_bfloat16*)(ws + L.Tm) + rec * C * C + cm_idx(i, j8, C)) = tb;
         *reinterpret_cast<uint4*>(sTB + cm_idx(i, j8, C)) = tb;
     }
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
-    KDA_PHASE(7);
-    // ---- 5: W^T and U^T (one issuing thread each)
-    if (lane == 0 && warp < 2) {
+    if (more) request_g(ci, uw.head());  // T is dead
+    if (warp < 2 && elect_one()) {  // W^T and U^T (one issuing thread each)
         tc_fence_after();
         const uint32_t sb = smem_u32(dyn);
         constexpr uint32_t id = make_idesc(128, 64, true, false);
-        const uint32_t acc = warp == 0 ? T_W : T_U, a_tile = warp == 0 ? KB : BV;
+        const uint32_t acc = warp == 0 ? T_W : T_U, a_tile = warp == 0 ? SQ : SV;
 #pragma unroll
         for (int s = 0; s < 4; ++s)
-            mma_ss(tmem0 + acc, make_desc(sb + a_tile + s * 4096, 2048, 128), make_desc(sb + KSC + s * 256, 128, 1024), id, s > 0);
-        mma_commit(&bar2);
+            mma_ss(tmem0 + acc, make_desc_sw128(sb + a_tile + s * 2048, 8192, 1024), make_desc(sb + SU + s * 256, 128, 1024), id, s > 0);
+        mma_commit(wbar);
     }
-    if (tid < D) gGam[tid] = ex2_approx(sG[swz_f32(C - 1, tid)]);
-    ok = mbar_wait(&bar2, it & 1, p, 8) && ok;
+    __syncwarp();
+    KDA_PHASE(9);
+    ok = mbar_wait(wbar, it & 1, p, 8) && ok;
     tc_fence_after();
-
-    KDA_PHASE(8);
-    // ---- 6: W and U records: warp (quadrant, group) takes token columns 32 (group % 2) .. +31 of W (groups
-    //      0, 1) or U (groups 2, 3)
+    if (more) request_qv(ci, uw.head());
+    KDA_PHASE(10);
+    // W and U records: warps 0 .. 3 the four quadrants of W, warps 4 .. 7 of U
     if (ok) {
-        const int qd = warp & 3, dd = 32 * qd + lane, grp = warp >> 2;
-        __nv_bfloat16* dst = grp < 2 ? gW : gU;
-        const uint32_t src = tmem0 + ((uint32_t)(32 * qd) << 16) + (grp < 2 ? T_W : T_U);
+        const int qd = warp & 3, dd = 32 * qd + lane;
+        __nv_bfloat16* dst = (__nv_bfloat16*)(ws + (warp < 4 ? L.W : L.U)) + rec * C * D;
+        const uint32_t src = tmem0 + ((uint32_t)(32 * qd) << 16) + (warp < 4 ? T_W : T_U);
 #pragma unroll
-        for (int i0 = 32 * (grp & 1); i0 < 32 * (grp & 1) + 32; i0 += 16) {
+        for (int i0 = 0; i0 < C; i0 += 16) {
             uint32_t r[16];
             tmem_ld16(src + i0, r);
             tmem_wait_ld();
@@ -873,33 +887,36 @@ __global__ void __launch_bounds__(fi::NTHR, 1) kda_fwd_intra_tc(const KdaParams 
                            pack_bf16(__uint_as_float(r[12]), __uint_as_float(r[13])), pack_bf16(__uint_as_float(r[14]), __uint_as_float(r[15])));
         }
     }
-    if (more) park_taps(nx);  // (T has left for its record and its operand tile)
-    if (tid == NTHR - 64) tma_store_wait_all();
+    if constexpr (CONV) cp_async_wait<0>();
     tc_fence_before();
     ok = __syncthreads_and(ok);
-    KDA_PHASE(9);
+    KDA_PHASE(11);
     if (!ok) break;  // a wait gave up (recorded in the status word): no further unit is started
-    ci = ci_nx;
     }
-    if (!ok && more) {  // the next unit's copies are in flight: they must have landed before the CTA leaves
-        mbar_wait(&rowbar, (it + 1) & 1, p, 8);
-        mbar_wait(&vbar, (it + 1) & 1, p, 8);
+    if (!ok && more && tiles) {  // the next unit's copies are in flight: they must have landed before the CTA leaves
+        mbar_wait(kbar, (it + 1) & 1, p, 8);
+        mbar_wait(gbar, (it + 1) & 1, p, 8);
+        mbar_wait(qbar, (it + 1) & 1, p, 8);
     }
+    if (lane == 0 && warp < 3) tma_store_wait_all();
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem_s, TMEM_COLS);
+    if (warp == 0) tmem_dealloc(tmem0, TMEM_COLS);
 }
 
 cudaError_t launch_fwd_intra_tc(const KdaParams& p, cudaStream_t s) {
     auto kern = p.conv_q ? kda_fwd_intra_tc<true> : kda_fwd_intra_tc<false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fi::TOTAL);
+    const uint32_t smem = p.conv_q ? fi::TOTAL_CONV : fi::TOTAL;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int units = p.NT * p.H, sms = sm_count();
+    // (the shared memory is split as for the neighbouring kernels, which fill an SM: another split would cost a drain between them)
+    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) != cudaSuccess) return e;
+    const int units = p.NT * p.H, ctas = 2 * sm_count();
     RowMaps maps = {};
     const long long tokens = (long long)p.B * p.T;
-    maps.ok = !(p.flags & KDA_FLAG_ROW_COPIES) && make_row_map(&maps.m[0], p.q, tokens, p.H, C) && make_row_map(&maps.m[1], p.k, tokens, p.H, C) &&
-              make_row_map(&maps.m[2], p.v, tokens, p.H, C) && make_row_map(&maps.m[3], p.g, tokens, p.H, C);
-    return launch_dependent(kern, units < sms ? units : sms, fi::NTHR, fi::TOTAL, s, p, maps);
+    maps.ok = !(p.flags & KDA_FLAG_ROW_COPIES) && make_row_map(&maps.m[0], p.q, tokens, p.H, C, true) && make_row_map(&maps.m[1], p.k, tokens, p.H, C, true) &&
+              make_row_map(&maps.m[2], p.v, tokens, p.H, C, true) && make_row_map(&maps.m[3], p.g, tokens, p.H, C);
+    return launch_dependent(kern, units < ctas ? units : ctas, fi::NTHR, smem, s, p, maps, ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype));
 }
 
 }  // namespace kda

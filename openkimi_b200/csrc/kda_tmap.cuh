@@ -16,8 +16,9 @@ struct RowMaps {
     int ok;  // 0: the driver's encoder is not available; the kernels then copy row by row
 };
 
-// [tokens][H * 128] BF16 at base, box = [box_rows][128]; false when the encoder is missing or refuses
-bool make_row_map(CUtensorMap* out, const void* base, long long tokens, int H, int box_rows);
+// [tokens][H * 128] BF16 at base, box = [box_rows][128], or [box_rows][64] with the 16-byte chunks of a box row XOR-swizzled by
+// the row (halves); false when the encoder is missing or refuses
+bool make_row_map(CUtensorMap* out, const void* base, long long tokens, int H, int box_rows, bool halves = false);
 
 namespace tc {
 // tile (rows y .. y + box_rows - 1, elements x .. x + 127) -> shared memory (dense, row-major); x * 2 bytes
@@ -27,6 +28,10 @@ __device__ __forceinline__ void tma_load_tile(void* dst_smem, const CUtensorMap*
                      smem_u32(dst_smem)),
                  "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
                  : "memory");
+}
+// a tensor map (a kernel parameter) on its way to the copy unit ahead of its first copy
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
 // shared memory (dense, row-major) -> tile; y must not be negative
 __device__ __forceinline__ void tma_store_tile(const CUtensorMap* map, int x, int y, const void* src_smem) {
