@@ -37,6 +37,7 @@
 #include "kda_common.cuh"
 #include "kda_conv_bwd.cuh"
 #include "kda_tc.cuh"
+#include "kda_tmap.cuh"
 
 namespace kda {
 
@@ -58,12 +59,13 @@ constexpr uint32_t STOT = SMID + 4096;       // f32 [4][128] block totals of dG
 constexpr uint32_t SSCR = STOT + 2048;       // f32 [4][128]
 constexpr uint32_t SRED = SSCR + 2048;       // f32 [16]
 constexpr uint32_t SREJ = SRED + 64;         // int [4][4]: tile (block, channel group) rejected
-constexpr uint32_t FD = SREJ + 64;           // f32 [2][4][16][16] diagonal blocks of dAqk, dM rebuilt for rejected tiles
+constexpr uint32_t FD = SREJ + 64;           // f32 [2][4][16][16] diagonal blocks of dAqk, dM rebuilt for rejected tiles, transposed
 constexpr uint32_t SAUX2 = FD + 8192;        // the aux record of every other unit (requests ahead, CONVB)
 constexpr uint32_t TOTAL = SAUX2 + 768;
 static_assert(TOTAL <= 232448, "shared memory of a CTA");
 // later uses of the dead operand space
 constexpr uint32_t PF = YB;                  // bf16 [3][64][128]: dQt, dKh, dKb (after the MMAs that read Y)
+constexpr uint32_t DG = YB;                  // bf16 [64][128]: the gate's gradient on its way out (after the assembly; not with CONVB)
 constexpr uint32_t STG = SB;                 // f32 [3][64][128] staging of dq, dk, dbeta terms over SB and X (after all MMAs)
 // fused short-convolution backward (CONVB): once their first users are done, Y holds the pre-convolution q and
 // k rows -3 .. 63 (bf16 [67][128] each), and the staging area dq and dk of the convolved rows (bf16, every row in the
@@ -83,15 +85,30 @@ __host__ __device__ constexpr uint32_t rcol(int J) { return 16u * J * (9 - J); }
 __host__ __device__ constexpr uint32_t ccol(int I) { return 320u + 8u * I * (I + 1); }  // accC_I: 16 (I + 1) columns
 }  // namespace bi
 
+// Two neighbouring rows of a channel in packed arithmetic: the kernel is bound by instruction issue and the latencies between its
+// barriers, and the rows lie side by side in the registers of accumulators, hand-over words and G (63 000 -> 49 000 warp
+// instructions a unit; 3072 units 337 -> 313 us, 1536 units with three quarters of the tiles rejected 233 -> 212).
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 ex2_2(float2 x) { return make_float2(ex2_approx(x.x), ex2_approx(x.y)); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, both(-1.f), a); }
+__device__ __forceinline__ float2 bf2(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+
 // eight operand values of one channel -> three BF16 parts, one 16-byte row of a core matrix each
-__device__ __forceinline__ void store_parts(unsigned char* buf, int d, int t0, const float (&v)[8]) {
-    uint32_t p0[4], p1[4], p2[4];
+__device__ __forceinline__ void store_parts(unsigned char* buf, int d, int t0, const float2 (&v)[4]) {
+    uint32_t p[3][4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) split3_bf16(v[2 * j], v[2 * j + 1], p0[j], p1[j], p2[j]);
+    for (int j = 0; j < 4; ++j) {
+        float2 x = v[j];
+#pragma unroll
+        for (int part = 0; part < 3; ++part) {
+            p[part][j] = pack_bf16(x.x, x.y);
+            if (part < 2) x = sub2(x, bf2(p[part][j]));
+        }
+    }
     const uint32_t off = (uint32_t)cm_idx(d, t0, 64) * 2;
-    *reinterpret_cast<uint4*>(buf + off) = make_uint4(p0[0], p0[1], p0[2], p0[3]);
-    *reinterpret_cast<uint4*>(buf + 16384 + off) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
-    *reinterpret_cast<uint4*>(buf + 32768 + off) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
+#pragma unroll
+    for (int part = 0; part < 3; ++part)
+        *reinterpret_cast<uint4*>(buf + part * 16384 + off) = make_uint4(p[part][0], p[part][1], p[part][2], p[part][3]);
 }
 
 // 512 threads: thread (blk, d) = (tid / 128, tid % 128) owns channel d (= TMEM lane d) of the 16-row
@@ -100,10 +117,11 @@ __device__ __forceinline__ void store_parts(unsigned char* buf, int d, int t0, c
 // CONVB: the backward of the short convolutions of q and k runs here too (KdaParams.grad_conv_*): dq, dk of the
 // convolved rows stay in shared memory and grad_q, grad_k receive the gradients of the projections.
 template <bool CONVB>
-__global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) {
+__global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p, const __grid_constant__ RowMaps maps) {
+    const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     using namespace bi;
     extern __shared__ __align__(128) unsigned char dyn[];
-    __shared__ uint64_t barA, barB, barH, mma1, mma2, mma3;
+    __shared__ uint64_t barA, barQ, barB, barH, mma1, mma2, mma3;
     __shared__ uint32_t tmem_s;
     const __nv_bfloat16* sQ = reinterpret_cast<const __nv_bfloat16*>(dyn + SQ);
     const __nv_bfloat16* sK = reinterpret_cast<const __nv_bfloat16*>(dyn + SK);
@@ -123,7 +141,6 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, d = tid & 127, blk = tid >> 7, cg = warp & 3;
     const int wu = __shfl_sync(0xffffffffu, warp, 0);  // the warp index as a warp-uniform value (MMA issue)
     const int b0 = B * blk;
-    const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     char* sc = (char*)p.bwd_scratch;
     const bool l2 = p.flags & KDA_FLAG_QK_L2NORM, gate = p.flags & KDA_FLAG_GATE, sig = p.flags & KDA_FLAG_BETA_SIGMOID;
     const float scale = p.scale;
@@ -133,7 +150,8 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
         tmem_relinquish();
     }
     if (tid == 0) {
-        mbar_init(&barA, 1);
+        mbar_init(&barA, 1);  // (two issuing threads)
+        mbar_init(&barQ, 1);
         mbar_init(&barB, 1);
         mbar_init(&barH, 1);
         mbar_init(&mma1, 4);  // four issuing threads commit each MMA group (one accumulator block each)
@@ -153,12 +171,12 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     // are set up once.  Unit u = (chunk u / H, head (u + chunk) % H), so that the units of one CTA cycle through
     // all heads whatever the stride (heads differ in cost: rejected tiles take the exact path).
     // What the operands are built from: G, the normalised q and k, the row norms and beta kept by the forward.  With the
-    // convolution fused, the NEXT unit's are requested as soon as this one has them in registers or is done with them, a
-    // third of a unit ahead (1667 -> 1595 us at 12288 units; without the convolution that third is too short for the
-    // copies to land, and the registers it takes cost more than it gives: 335 -> 341 us at 3072 units).
+    // convolution fused, the NEXT unit's are requested as soon as this one is done with them, before the convolution's
+    // backward (12288 units: 1530 us; requested before the row stage, with its rows in registers, 1567).
     constexpr bool AHEAD = CONVB;
     auto request_A = [&](size_t r, bool second) {
         const char* ws = (const char*)p.workspace;
+        if (tid != 0) return;
         mbar_expect_tx(&barA, C * D * 4 + 2 * C * D * 2 + 3 * C * 4);
         tma_load_1d(dyn + SG, (const float*)(ws + L.Gc) + r * C * D, C * D * 4, &barA);
         tma_load_1d(dyn + SQ, (const __nv_bfloat16*)(ws + L.Qn) + r * C * D, C * D * 2, &barA);
@@ -175,8 +193,6 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     const float* srq = reinterpret_cast<const float*>(dyn + (AHEAD && par ? SAUX2 : SAUX));  // aux record order: 1/|q|, 1/|k|, beta
     const float* srk = srq + 64;
     const float* sbeta = srq + 128;
-    UnitWalk un = uw;  // the next unit of this CTA (without the requests ahead it is worked out where the hints need it)
-    if constexpr (AHEAD) un.next();
     ahead = false;
     const int c = uw.c, hd = uw.head();
     const ChunkInfo ci = chunk_info(p, c);
@@ -187,8 +203,8 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     //      (G, the normalised q and k, the row norms and beta kept by the forward), on barB the split
     //      dAqk / dM tiles and the diagonal of dAqk from bwd_wy; the three [64][128] hand-over arrays
     //      that only the assembly needs follow on barH once an operand buffer is free
+    if (!AHEAD || it == 0) request_A(rec, false);
     if (tid == 0) {
-        if (!AHEAD || it == 0) request_A(rec, false);
         mbar_expect_tx(&barB, 6 * C * C * 2 + C * 4);
         tma_load_1d(dyn + SB, (const __nv_bfloat16*)(sc + L.dAM) + rec * 6 * C * C, 6 * C * C * 2, &barB);
         tma_load_1d(sdiag, (const float*)(sc + L.dAd) + rec * C, C * 4, &barB);
@@ -199,28 +215,38 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     KDA_PHASE(0);
 
     // ---- my block: G of my channel, guard and references; operand step 1: KN_j = k_j 2^(ref - G_j) -> X
-    float G[B], mid;
+    float mid;
+    float2 G2[B / 2];  // rows 2 i, 2 i + 1
+    bool pass;
+    {
+        float G[B];
 #pragma unroll
-    for (int r = 0; r < B; ++r) G[r] = sG[swz_f32(b0 + r, d)];
+        for (int r = 0; r < B; ++r) G[r] = sG[swz_f32(b0 + r, d)];
+        pass = guard_tile(G, fminf(p.guard_span, TC_SPAN), mid);
+#pragma unroll
+        for (int r = 0; r < B; r += 2) G2[r / 2] = make_float2(G[r], G[r + 1]);
+    }
+    auto k2 = [&](int i) { return make_float2(__bfloat162float(sK[swz_bf16(b0 + 2 * i, d)]), __bfloat162float(sK[swz_bf16(b0 + 2 * i + 1, d)])); };
+    auto q2 = [&](int i) { return make_float2(__bfloat162float(sQ[swz_bf16(b0 + 2 * i, d)]), __bfloat162float(sQ[swz_bf16(b0 + 2 * i + 1, d)])); };
+    auto beta2 = [&](int i) { return *reinterpret_cast<const float2*>(sbeta + b0 + 2 * i); };
     const float gl = sG[swz_f32(C - 1, d)];                          // G of the chunk's last row
     const float gprev = blk > 0 ? sG[swz_f32(b0 - 1, d)] : 0.f;      // G of the row before my block
-    const bool pass = guard_tile(G, fminf(p.guard_span, TC_SPAN), mid);
     {
         // references of my rows as keys / as queries: the midpoint, or first rows when there is none
         // (block 3 has no later rows: zero keys)
-        const float kref = pass ? mid : (blk < 3 ? sG[swz_f32(b0 + B, d)] : -INFINITY), qref = pass ? mid : G[0];
+        const float kref = pass ? mid : (blk < 3 ? sG[swz_f32(b0 + B, d)] : -INFINITY), qref = pass ? mid : G2[0].x;
         smid[blk * D + d] = kref;
         smid[(4 + blk) * D + d] = qref;
         if (lane == 0) srej[blk * 4 + cg] = pass ? 0 : 1;
 #pragma unroll
         for (int g8 = 0; g8 < 2; ++g8) {
-            float v[8];
+            float2 v[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                v[j] = __bfloat162float(sK[swz_bf16(b0 + 8 * g8 + j, d)]) * ex2_approx(kref - G[8 * g8 + j] + SHIFT);
+            for (int j = 0; j < 4; ++j) v[j] = __fmul2_rn(k2(4 * g8 + j), ex2_2(sub2(both(kref + SHIFT), G2[4 * g8 + j])));
             store_parts(dyn + XB, d, b0 + 8 * g8, v);
         }
     }
+    if constexpr (!CONVB) tma_store_wait_read();
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
@@ -258,15 +284,16 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     }
 #pragma unroll
     for (int b = 0; b < 16; ++b) any_rej = any_rej || srej[b] != 0;
-    // ---- operand step 2: QP_i = scale q_i 2^(G_i - ref) -> Y
+    // ---- operand step 2: QP_i = scale q_i 2^(G_i - ref) -> Y (which the last unit's gate gradient has left: the threads that issued
+    //      its copies wait for that before the barrier above)
     {
-        const float qref = pass ? mid : G[0];
+        const float qref = (pass ? mid : G2[0].x) - SHIFT;
 #pragma unroll
         for (int g8 = 0; g8 < 2; ++g8) {
-            float v[8];
+            float2 v[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                v[j] = scale * __bfloat162float(sQ[swz_bf16(b0 + 8 * g8 + j, d)]) * ex2_approx(G[8 * g8 + j] - qref + SHIFT);
+            for (int j = 0; j < 4; ++j)
+                v[j] = __fmul2_rn(__fmul2_rn(both(scale), q2(4 * g8 + j)), ex2_2(__fadd2_rn(G2[4 * g8 + j], both(-qref))));
             store_parts(dyn + YB, d, b0 + 8 * g8, v);
         }
     }
@@ -290,15 +317,13 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     ok = ok && mbar_wait(&mma1, par, p, 64);
     tc_fence_after();
     {
-        const float qref = pass ? mid : G[0];
+        const float qref = (pass ? mid : G2[0].x) - SHIFT;
 #pragma unroll
         for (int g8 = 0; g8 < 2; ++g8) {
-            float v[8];
+            float2 v[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int t = b0 + 8 * g8 + j;
-                v[j] = sbeta[t] * __bfloat162float(sK[swz_bf16(t, d)]) * ex2_approx(G[8 * g8 + j] - qref + SHIFT);
-            }
+            for (int j = 0; j < 4; ++j)
+                v[j] = __fmul2_rn(__fmul2_rn(beta2(4 * g8 + j), k2(4 * g8 + j)), ex2_2(__fadd2_rn(G2[4 * g8 + j], both(-qref))));
             store_parts(dyn + XB, d, b0 + 8 * g8, v);
         }
     }
@@ -320,9 +345,10 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     }
     // ---- row sums of my block from the accumulators while the column-side MMAs run (the pairs inside my
     //      own block only if its tile passed the guard)
-    float a1[B], a2[B], c1[B];
+    float2 a1[B / 2], a2[B / 2], c1[B / 2];
 #pragma unroll
-    for (int r = 0; r < B; ++r) a1[r] = a2[r] = c1[r] = 0.f;
+    for (int i = 0; i < B / 2; ++i) a1[i] = a2[i] = c1[i] = both(0.f);
+    auto pair = [](const uint32_t (&r)[16], int i) { return make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])); };
     if (ok) {
 #pragma unroll
         for (int J = 0; J < 4; ++J)
@@ -333,10 +359,10 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
                 tmem_ld16(col + 64 - B * J, rm);
                 tmem_wait_ld();
 #pragma unroll
-                for (int r = 0; r < B; ++r) {
-                    const float f = ex2_approx(G[r] - kr4[J] - SHIFT);
-                    a1[r] = fmaf(f, __uint_as_float(ra[r]), a1[r]);
-                    a2[r] = fmaf(f, __uint_as_float(rm[r]), a2[r]);
+                for (int i = 0; i < B / 2; ++i) {
+                    const float2 f = ex2_2(__fadd2_rn(G2[i], both(-kr4[J] - SHIFT)));
+                    a1[i] = __ffma2_rn(f, pair(ra, i), a1[i]);
+                    a2[i] = __ffma2_rn(f, pair(rm, i), a2[i]);
                 }
             }
     }
@@ -352,10 +378,8 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     // The next unit of this CTA finds what it needs first in L2: the hints go out here, in the middle of the unit,
     // when the copy unit has nothing else to do (there is no shared memory left to receive the records themselves).
     if (tid == 5 * 32) {
-        if constexpr (!AHEAD) {
-            un = uw;
-            un.next();
-        }
+        UnitWalk un = uw;  // the next unit of this CTA
+        un.next();
         if (un.unit < n_units) {
             const char* ws = (const char*)p.workspace;
             const size_t rn = un.rec();
@@ -376,14 +400,14 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
                 tmem_ld16(tlane + ccol(Ip) + b0, rc);
                 tmem_wait_ld();
 #pragma unroll
-                for (int r = 0; r < B; ++r) c1[r] = fmaf(ex2_approx(qr4[Ip] - G[r] - SHIFT), __uint_as_float(rc[r]), c1[r]);
+                for (int i = 0; i < B / 2; ++i) c1[i] = __ffma2_rn(ex2_2(sub2(both(qr4[Ip] - SHIFT), G2[i])), pair(rc, i), c1[i]);
             }
     }
     KDA_PHASE(6);
     if (any_rej) {  // uniform over the CTA: the diagonal blocks back to FP32 (x = p0 + p1 + p2) for the CUDA-core sums
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const int e = tid + NTHR * u, mat = e >> 10, bb = (e >> 8) & 3, r = (e >> 4) & 15, j = e & 15;
+            const int e = tid + NTHR * u, mat = e >> 10, bb = (e >> 8) & 3, j = (e >> 4) & 15, r = e & 15;
             const __nv_bfloat16* t = sB + mat * 3 * C * C + cm_idx(B * bb + r, B * bb + j, C);
             fD[e] = (__bfloat162float(t[0]) + __bfloat162float(t[C * C])) + __bfloat162float(t[2 * C * C]);
         }
@@ -395,45 +419,51 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     if (ok) {
         // ---- my tile was rejected: the pairs inside the block in FP32 on the CUDA cores, one exp2 per pair.
         //      Pair (r, j), j < r, feeds the row sums of r and the column sum of j with the same decay
-        //      2^(G_r - G_j).  The key row j is the rolled loop (four segments, so that the unrolled rows
-        //      start right below the diagonal instead of being masked off); its column sum goes through my
-        //      own column of the G tile, which nobody else reads (G itself is in registers by now, and rows
-        //      15 / 31 / 47 / 63, which neighbours did read, are never written).
+        //      2^(G_r - G_j).  The key row j is the rolled loop (two segments, so that half of the unrolled rows
+        //      above the diagonal are not masked off but left out); its column sum goes through my
+        //      own column of the G tile, which nobody else reads any more.
         if (!pass) {
             const float* dA = fD + blk * B * B;
             const float* dM = fD + (4 + blk) * B * B;
-            float qs[B], kb[B];
+            float2 qs[B / 2], kb[B / 2];
 #pragma unroll
-            for (int r = 0; r < B; ++r) {
-                qs[r] = scale * __bfloat162float(sQ[swz_bf16(b0 + r, d)]);
-                kb[r] = sbeta[b0 + r] * __bfloat162float(sK[swz_bf16(b0 + r, d)]);
+            for (int i = 0; i < B / 2; ++i) {
+                qs[i] = __fmul2_rn(both(scale), q2(i));
+                kb[i] = __fmul2_rn(beta2(i), k2(i));
             }
-            auto segment = [&](auto r0c, int j0, int j1) {
+            // keys R0 .. R0 + 7 against the rows from R0 on (dA, dM are zero on and above the diagonal; two segments, because four
+            // spill: 1580 against 1530 us with the convolution, 12288 units)
+            auto segment = [&](auto r0c) {
                 constexpr int R0 = decltype(r0c)::value;
 #pragma unroll 1
-                for (int j = j0; j < j1; ++j) {
+                for (int j = R0; j < R0 + 8; ++j) {
                     const float kj = __bfloat162float(sK[swz_bf16(b0 + j, d)]), gj = sG[swz_f32(b0 + j, d)];
-                    float cj = 0.f;
+                    float2 cj = both(0.f);
 #pragma unroll
-                    for (int r = R0; r < B; ++r) {
-                        const float e = r > j ? ex2_approx(G[r] - gj) : 0.f;
-                        const float a = dA[r * B + j], m = dM[r * B + j], kp = kj * e;
-                        a1[r] = fmaf(a, kp, a1[r]);
-                        a2[r] = fmaf(m, kp, a2[r]);
-                        cj = fmaf(fmaf(a, qs[r], m * kb[r]), e, cj);
+                    for (int r = R0; r < B; r += 4) {
+                        const float4 a4 = *reinterpret_cast<const float4*>(dA + j * B + r), m4 = *reinterpret_cast<const float4*>(dM + j * B + r);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int i = r / 2 + h;
+                            const float2 a = h ? make_float2(a4.z, a4.w) : make_float2(a4.x, a4.y), m = h ? make_float2(m4.z, m4.w) : make_float2(m4.x, m4.y);
+                            float2 e = ex2_2(__fadd2_rn(G2[i], both(-gj)));
+                            if (r < R0 + 8) e = make_float2(2 * i > j ? e.x : 0.f, 2 * i + 1 > j ? e.y : 0.f);  // (rows before the key may overflow)
+                            const float2 kp = __fmul2_rn(both(kj), e);
+                            a1[i] = __ffma2_rn(a, kp, a1[i]);
+                            a2[i] = __ffma2_rn(m, kp, a2[i]);
+                            cj = __ffma2_rn(__ffma2_rn(a, qs[i], __fmul2_rn(m, kb[i])), e, cj);
+                        }
                     }
-                    sG[swz_f32(b0 + j, d)] = cj;
+                    sG[swz_f32(b0 + j, d)] = cj.x + cj.y;
                 }
             };
-            segment(std::integral_constant<int, 1>{}, 0, 4);
-            segment(std::integral_constant<int, 5>{}, 4, 8);
-            segment(std::integral_constant<int, 9>{}, 8, 12);
-            segment(std::integral_constant<int, 13>{}, 12, 15);
+            segment(std::integral_constant<int, 0>{});
+            segment(std::integral_constant<int, 8>{});
 #pragma unroll
-            for (int j = 0; j < B - 1; ++j) c1[j] += sG[swz_f32(b0 + j, d)];
+            for (int i = 0; i < B / 2; ++i) c1[i] = __fadd2_rn(c1[i], make_float2(sG[swz_f32(b0 + 2 * i, d)], i < 7 ? sG[swz_f32(b0 + 2 * i + 1, d)] : 0.f));
         }
         KDA_PHASE(8);
-        // ---- assembly of my block, last row first; a1[r] is reused for the running sum of dG
+        // ---- assembly of my block, last row first; a1 is reused for the running sum of dG
         {
             float acc = 0.f, tail = 0.f;
             // my 16 rows of the three hand-over arrays (channel-major, handover_idx): eight rows = one 16-byte word
@@ -442,25 +472,28 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
                 const int o = handover_idx(b0 + 8 * hf, d);
                 const uint4 uq = *reinterpret_cast<const uint4*>(spf + o), ukh = *reinterpret_cast<const uint4*>(spf + C * D + o),
                             ukb = *reinterpret_cast<const uint4*>(spf + 2 * C * D + o);
-                const __nv_bfloat16* hq = reinterpret_cast<const __nv_bfloat16*>(&uq);
-                const __nv_bfloat16* hkh = reinterpret_cast<const __nv_bfloat16*>(&ukh);
-                const __nv_bfloat16* hkb = reinterpret_cast<const __nv_bfloat16*>(&ukb);
+                const uint32_t hq[4] = {uq.x, uq.y, uq.z, uq.w}, hkh[4] = {ukh.x, ukh.y, ukh.z, ukh.w}, hkb[4] = {ukb.x, ukb.y, ukb.z, ukb.w};
 #pragma unroll
-                for (int r8 = 7; r8 >= 0; --r8) {
-                    const int r = 8 * hf + r8, ii = b0 + r;
-                    const float qi = __bfloat162float(sQ[swz_bf16(ii, d)]), ki = __bfloat162float(sK[swz_bf16(ii, d)]);
-                    const float bi_ = sbeta[ii];
-                    const float gam = ex2_approx(G[r]), eta = ex2_approx(gl - G[r]);
-                    const float dQt = __bfloat162float(hq[r8]), dKh = __bfloat162float(hkh[r8]), dKb = __bfloat162float(hkb[r8]);
-                    const float diag = scale * sdiag[ii];
-                    const float dq_in = scale * a1[r], dk_row = bi_ * a2[r], dKt = bi_ * dKb;
-                    stg[(0 * C + ii) * D + d] = dq_in + diag * ki + scale * dQt * gam;
-                    stg[(1 * C + ii) * D + d] = dk_row + c1[r] + diag * qi + dKt * gam + dKh * eta;
-                    stg[(2 * C + ii) * D + d] = ki * a2[r] + dKb * (ki * gam);
-                    const float khe = dKh * (ki * eta);
-                    tail += khe;  // the last row also collects sum_i dKh_i Kh_i
-                    acc += qi * dq_in + ki * dk_row - ki * c1[r] + dQt * (scale * qi * gam) + dKt * (ki * gam) - khe;
-                    a1[r] = acc;
+                for (int r2 = 3; r2 >= 0; --r2) {
+                    const int i = 4 * hf + r2, ii = b0 + 2 * i;
+                    const float2 qi = q2(i), ki = k2(i), be = beta2(i), dg = __fmul2_rn(both(scale), *reinterpret_cast<const float2*>(sdiag + ii));
+                    const float2 gam = ex2_2(G2[i]), he = __fmul2_rn(bf2(hkh[r2]), ex2_2(sub2(both(gl), G2[i])));  // dKh 2^(G_last - G)
+                    const float2 kg = __fmul2_rn(bf2(hkb[r2]), gam);                                               // d(beta K~) 2^G
+                    const float2 rq = __fmul2_rn(both(scale), __ffma2_rn(bf2(hq[r2]), gam, a1[i]));                 // row side of dq
+                    const float2 am = __fadd2_rn(a2[i], kg), rk = __fmul2_rn(be, am), cs = __fadd2_rn(c1[i], he);   // row side of dk, the rest
+                    const float2 dq = __ffma2_rn(dg, ki, rq), dk = __fadd2_rn(__ffma2_rn(dg, qi, rk), cs), db = __fmul2_rn(ki, am);
+                    const float2 khe = __fmul2_rn(ki, he);  // the last row also collects sum_i dKh_i Kh_i
+                    const float2 term = __ffma2_rn(qi, rq, __fmul2_rn(ki, sub2(rk, cs)));
+                    stg[(0 * C + ii) * D + d] = dq.x;
+                    stg[(0 * C + ii + 1) * D + d] = dq.y;
+                    stg[(1 * C + ii) * D + d] = dk.x;
+                    stg[(1 * C + ii + 1) * D + d] = dk.y;
+                    stg[(2 * C + ii) * D + d] = db.x;
+                    stg[(2 * C + ii + 1) * D + d] = db.y;
+                    tail += khe.x + khe.y;
+                    a1[i].y = acc + term.y;
+                    acc = a1[i].y + term.x;
+                    a1[i].x = acc;
                 }
             }
             stot[blk * D + d] = acc;
@@ -468,22 +501,7 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
         }
         KDA_PHASE(9);
         const int c4 = (tid & 15) * 4;
-        uint2 qrow[2][2], krow[2][2];  // q^ and k^ of the two rows this half warp finishes below
-        if constexpr (AHEAD) {
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
-                    qrow[m][hf] = *reinterpret_cast<const uint2*>(sQ + swz_bf16((tid >> 4) + 32 * m, 64 * hf + c4));
-                    krow[m][hf] = *reinterpret_cast<const uint2*>(sK + swz_bf16((tid >> 4) + 32 * m, 64 * hf + c4));
-                }
-            fence_async_smem();
-        }
         __syncthreads();
-        if constexpr (AHEAD) {
-            ahead = un.unit < n_units;
-            if (ahead && tid == NTHR - 32) request_A(un.rec(), par == 0);
-        }
         KDA_PHASE(10);
         if constexpr (CONVB) {  // the hand-over arrays in Y are dead: fetch the projection rows the convolution backward needs
             const __nv_bfloat16* xq = (const __nv_bfloat16*)p.q;
@@ -508,24 +526,44 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
 #pragma unroll
             for (int b = 1; b < 4; ++b)
                 if (b > blk) base += stot[b * D + d];
-            const float negA = -expA, rcpA = 1.f / expA;
+            const float negA = -expA, arg = LOG2E / expA;
+            float2 dA2 = both(0.f), dbias2 = both(0.f);
             // (rows past the end of a partial chunk have a constant G, hence a zero decay and zero terms:
             //  only their stores are masked, so that the rows do not end up in sixteen basic blocks)
             __nv_bfloat16* dgp = (__nv_bfloat16*)p.grad_g + tok(b0) * D + d;
+            __nv_bfloat16* sdg = reinterpret_cast<__nv_bfloat16*>(dyn + DG) + b0 * D + d;
             const size_t rstride = (size_t)p.H * D;
 #pragma unroll
-            for (int r = B - 1; r >= 0; --r) {
-                const float run = base + a1[r];
-                float outv = run;
+            for (int i = B / 2 - 1; i >= 0; --i) {
+                const float2 run = __fadd2_rn(both(base), a1[i]);
+                float2 outv = run;
                 if (gate) {
                     // per-token log decay g = (G_i - G_{i-1}) ln 2; sigmoid(x + b) = 1 - exp(-softplus) = -expm1(g / e^A)
-                    const float gnat = (G[r] - (r > 0 ? G[r > 0 ? r - 1 : 0] : gprev)) * 0.6931471805599453f;
-                    dA_acc = fmaf(run, gnat, dA_acc);
-                    outv = run * negA * (1.f - ex2_approx(gnat * rcpA * LOG2E));
-                    dbias_acc += outv;
+                    const float2 gnat = __fmul2_rn(sub2(G2[i], make_float2(i > 0 ? G2[i > 0 ? i - 1 : 0].y : gprev, G2[i].x)), both(0.6931471805599453f));
+                    dA2 = __ffma2_rn(run, gnat, dA2);
+                    outv = __fmul2_rn(__fmul2_rn(run, both(negA)), sub2(both(1.f), ex2_2(__fmul2_rn(gnat, both(arg)))));
+                    dbias2 = __fadd2_rn(dbias2, outv);
                 }
-                if (b0 + r < ci.len) dgp[r * rstride] = __float2bfloat16_rn(outv);
+                if constexpr (!CONVB) {
+                    sdg[2 * i * D] = __float2bfloat16_rn(outv.x);
+                    sdg[(2 * i + 1) * D] = __float2bfloat16_rn(outv.y);
+                } else {
+                    if (b0 + 2 * i < ci.len) dgp[2 * i * rstride] = __float2bfloat16_rn(outv.x);
+                    if (b0 + 2 * i + 1 < ci.len) dgp[(2 * i + 1) * rstride] = __float2bfloat16_rn(outv.y);
+                }
             }
+            dA_acc = dA2.x + dA2.y;
+            dbias_acc = dbias2.x + dbias2.y;
+        }
+        if constexpr (!CONVB) {  // (one copy of the tile; sixteen 2-byte stores per thread took 0.6 us longer)
+            fence_async_smem();
+            __syncthreads();
+            if (maps.ok && ci.len == C) {
+                if (tid == NTHR - 32) tma_store_tile(&maps.m[0], hd * D, (int)ci.tok0, dyn + DG);
+            } else if (tid >= NTHR - C && tid - (NTHR - C) < ci.len) {
+                tma_store_1d((__nv_bfloat16*)p.grad_g + tok(tid - (NTHR - C)) * D, dyn + DG + (tid - (NTHR - C)) * D * 2, D * 2);
+            }
+            tma_store_commit();
         }
         KDA_PHASE(11);
         // ---- row-wise (one half warp per row, 64 rows): L2-norm chain, beta gradient.  Lane l of the half
@@ -544,8 +582,8 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
                     const float4 a = *reinterpret_cast<const float4*>(stg + (0 * C + ii) * D + ch);
                     const float4 b = *reinterpret_cast<const float4*>(stg + (1 * C + ii) * D + ch);
                     const float4 e = *reinterpret_cast<const float4*>(stg + (2 * C + ii) * D + ch);
-                    const uint2 qu = AHEAD ? qrow[m][hf] : *reinterpret_cast<const uint2*>(sQ + swz_bf16(ii, ch));
-                    const uint2 ku = AHEAD ? krow[m][hf] : *reinterpret_cast<const uint2*>(sK + swz_bf16(ii, ch));
+                    const uint2 qu = *reinterpret_cast<const uint2*>(sQ + swz_bf16(ii, ch));
+                    const uint2 ku = *reinterpret_cast<const uint2*>(sK + swz_bf16(ii, ch));
                     const float2 q01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qu.x));
                     const float2 q23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qu.y));
                     const float2 k01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ku.x));
@@ -611,7 +649,12 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
             // ---- backward of the short convolutions of q and k: thread (channel, 16-row block) walks its rows of both
             //      tensors; dx replaces dy in shared memory and leaves in whole rows
             cp_async_wait<0>();
-            __syncthreads();  // the projection rows have landed, dq / dk of the convolved rows are complete
+            fence_async_smem();
+            __syncthreads();  // the projection rows have landed, dq / dk of the convolved rows are complete; G, q^ and k^ are dead
+            UnitWalk un = uw;
+            un.next();
+            ahead = un.unit < n_units;
+            if (ahead) request_A(un.rec(), par == 0);
             const __nv_bfloat16* sxq = reinterpret_cast<const __nv_bfloat16*>(dyn + CXQ);
             const __nv_bfloat16* sxk = reinterpret_cast<const __nv_bfloat16*>(dyn + CXK);
             __nv_bfloat16* sdyq = reinterpret_cast<__nv_bfloat16*>(dyn + CDYQ);
@@ -620,7 +663,8 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
             int c0s, ncs;
             seq_chunks(p, ci.seq, c0s, ncs);
             const bool has_next = ci.lc + 1 < ncs;
-            float wq[4], wk[4], dwq[4] = {0.f, 0.f, 0.f, 0.f}, dwk[4] = {0.f, 0.f, 0.f, 0.f}, oq[16], ok_[16];
+            float wq[4], wk[4], dwq[4] = {0.f, 0.f, 0.f, 0.f}, dwk[4] = {0.f, 0.f, 0.f, 0.f};
+            uint32_t oq[8], ok_[8];
             {
                 const float4 tq = reinterpret_cast<const float4*>(dyn + CTAPS)[d], tk = reinterpret_cast<const float4*>(dyn + CTAPS)[D + d];
                 wq[0] = tq.x; wq[1] = tq.y; wq[2] = tq.z; wq[3] = tq.w;
@@ -628,15 +672,21 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
             }
             float* cvh = (float*)(sc + L.cv_head) + (rec * 3 * 3) * D;
             float* cvt = (float*)(sc + L.cv_tail) + (rec * 3 * 3) * D;
-            conv_bwd_block<CDS>(sxq, sxq + 3 * D, sdyq, wq, d, blk, cvh, cvt, dwq, oq);
-            conv_bwd_block<CDS>(sxk, sxk + 3 * D, sdyk, wk, d, blk, cvh + 3 * D, cvt + 3 * D, dwk, ok_);
+            auto walk = [&](const __nv_bfloat16* sx, const __nv_bfloat16* sdy, const float(&w)[4], int tensor, float(&dw)[4], uint32_t(&o)[8]) {
+                float out[16];
+                conv_bwd_block<CDS>(sx, sx + 3 * D, sdy, w, d, blk, cvh + tensor * 3 * D, cvt + tensor * 3 * D, dw, out);
+#pragma unroll
+                for (int r = 0; r < 8; ++r) o[r] = pack_bf16(out[2 * r], out[2 * r + 1]);
+            };
+            walk(sxq, sdyq, wq, 0, dwq, oq);
+            walk(sxk, sdyk, wk, 1, dwk, ok_);
             *reinterpret_cast<float4*>(sdw + (blk * D + d) * 4) = make_float4(dwq[0], dwq[1], dwq[2], dwq[3]);
             *reinterpret_cast<float4*>(sdw + ((4 + blk) * D + d) * 4) = make_float4(dwk[0], dwk[1], dwk[2], dwk[3]);
             __syncthreads();  // every read of dy is done, the filter-gradient shares are visible
 #pragma unroll
             for (int r = 0; r < B; ++r) {
-                sdyq[(b0 + r) * CDS + d] = __float2bfloat16_rn(oq[r]);
-                sdyk[(b0 + r) * CDS + d] = __float2bfloat16_rn(ok_[r]);
+                reinterpret_cast<unsigned short*>(sdyq)[(b0 + r) * CDS + d] = (unsigned short)(oq[r / 2] >> (16 * (r & 1)));
+                reinterpret_cast<unsigned short*>(sdyk)[(b0 + r) * CDS + d] = (unsigned short)(ok_[r / 2] >> (16 * (r & 1)));
             }
             if (blk < 2) {  // block 0 threads reduce the q filter, block 1 threads the k filter (fixed order)
                 const float* src = sdw + (4 * blk * D + d) * 4;
@@ -681,7 +731,10 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p) 
     ok = __syncthreads_and(ok);
     if (!ok) break;  // a wait gave up (recorded in the status word): no further unit is started
     }
-    if (!ok && ahead) mbar_wait(&barA, (it + 1) & 1, p, 64);  // the next unit's copies are in flight
+    if constexpr (!CONVB) tma_store_wait_all();
+    if (!ok && ahead) {  // the next unit's copies are in flight
+        mbar_wait(&barA, (it + 1) & 1, p, 64);
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem0, TMEM_COLS);
@@ -764,7 +817,9 @@ cudaError_t launch_bwd_intra(const KdaParams& p, cudaStream_t s) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bi::TOTAL);
     if (e != cudaSuccess) return e;
     const int units = p.NT * p.H, sms = sm_count();
-    if ((e = launch_dependent(kern, units < sms ? units : sms, bi::NTHR, bi::TOTAL, s, p)) != cudaSuccess) return e;
+    RowMaps maps = {};
+    maps.ok = !(p.flags & KDA_FLAG_ROW_COPIES) && make_row_map(&maps.m[0], p.grad_g, (long long)p.B * p.T, p.H, C);
+    if ((e = launch_dependent(kern, units < sms ? units : sms, bi::NTHR, bi::TOTAL, s, p, maps)) != cudaSuccess) return e;
     if (convb) {
         if ((e = launch_dependent(conv_bwd_fixup_kernel, dim3((p.NT + 3) / 4, p.H, 3), 128, 0, s, p)) != cudaSuccess) return e;
         if ((e = launch_dependent(conv_bwd_reduce_kernel, dim3(p.H, 3, 8), 1024, 0, s, p)) != cudaSuccess) return e;
