@@ -4,6 +4,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <atomic>
+
 #include "kda_common.cuh"
 #include "kda_tmap.cuh"
 
@@ -27,6 +29,26 @@ static thread_local char g_last_error[256] = "";
 int fail_cuda(cudaError_t e) {
     snprintf(g_last_error, sizeof(g_last_error), "%s: %s", cudaGetErrorName(e), cudaGetErrorString(e));
     return KDA_ERR_LAUNCH;
+}
+
+cudaError_t allow_smem(const void* kern, int bytes, bool max_carveout) {
+    // a kernel's slot is claimed by its address; bytes is published after the runtime has been told (threads that meet tell it twice)
+    struct Slot { std::atomic<const void*> kern; std::atomic<int> bytes; };
+    constexpr int DEVICES = 64, SLOTS = 64;
+    static Slot table[DEVICES][SLOTS];
+    int dev = 0;
+    Slot* slot = nullptr;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < DEVICES)
+        for (int i = 0; i < SLOTS && !slot; ++i) {
+            const void* k = table[dev][i].kern.load(std::memory_order_acquire);
+            if (k == nullptr && table[dev][i].kern.compare_exchange_strong(k, kern)) k = kern;
+            if (k == kern) slot = &table[dev][i];
+        }
+    if (slot && slot->bytes.load(std::memory_order_acquire) >= bytes) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && max_carveout) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess && slot) slot->bytes.store(bytes, std::memory_order_release);
+    return e;
 }
 
 // The tensor-map encoder is a driver function; it is looked up through the runtime so that the library

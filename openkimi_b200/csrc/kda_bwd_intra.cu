@@ -814,7 +814,7 @@ __global__ void __launch_bounds__(1024) conv_bwd_reduce_kernel(const KdaParams p
 cudaError_t launch_bwd_intra(const KdaParams& p, cudaStream_t s) {
     const bool convb = p.grad_conv_q != nullptr;
     auto kern = convb ? kda_bwd_intra<true> : kda_bwd_intra<false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bi::TOTAL);
+    cudaError_t e = allow_smem(kern, (int)bi::TOTAL);
     if (e != cudaSuccess) return e;
     const int units = p.NT * p.H, sms = sm_count();
     RowMaps maps = {};

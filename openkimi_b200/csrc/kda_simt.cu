@@ -881,7 +881,7 @@ constexpr size_t smem_bwd_chunk() {
 
 template <typename K>
 static cudaError_t set_smem(K kernel, size_t bytes) {
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return allow_smem(kernel, (int)bytes);
 }
 
 template <typename T, int D>

@@ -337,7 +337,7 @@ template <typename T, int D, int BV>
 static cudaError_t launch_state(const KdaParams& p, bool bwd, cudaStream_t s) {
     auto kern = bwd ? kda_bwd_state_simt<T, D, BV> : kda_fwd_state_simt<T, D, BV>;
     constexpr int smem = ss::Smem<T, D, BV>::TOTAL;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     return launch_dependent(kern, dim3(D / BV, p.H, p.N), ss::NT, smem, s, p);
 }

@@ -362,13 +362,13 @@ cudaError_t launch_seg_combine(const KdaParams& p, const StateSegs& segs, bool b
     auto kern = bwd ? (two ? kda_seg_combine<true, 1> : kda_seg_combine<true, 2>)
                     : (two ? kda_seg_combine<false, 1> : kda_seg_combine<false, 2>);
     const int smem = (int)sc::total(two ? 1 : 2);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     return launch_dependent(kern, dim3(sc::D / sc::ROWS, p.H, p.N), sc::NTHR, smem, s, p, segs);
 }
 
 cudaError_t launch_fwd_segments(const KdaParams& p, const StateSegs& segs, cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(kda_fwd_segment_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sg::TOTAL);
+    cudaError_t e = allow_smem(kda_fwd_segment_tc, (int)sg::TOTAL);
     if (e != cudaSuccess) return e;
     if ((e = launch_dependent(kda_fwd_segment_tc, dim3(p.H, segs.count), sg::NTHR, sg::TOTAL, s, p, segs)) != cudaSuccess) return e;
     return launch_seg_combine(p, segs, false, s);

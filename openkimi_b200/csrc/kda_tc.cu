@@ -707,7 +707,7 @@ cudaError_t tc_fwd(const KdaParams& p, cudaStream_t s) {
         const StateSegs segs = state_segs(p, false);
         if (segs.len > 0 && !(p.flags & KDA_FLAG_BORDERS_READY) && (e = launch_fwd_segments(p, segs, s)) != cudaSuccess) return e;
         constexpr int smem = fs::TOTAL;
-        if ((e = cudaFuncSetAttribute(kda_fwd_state_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
+        if ((e = allow_smem(kda_fwd_state_tc, smem)) != cudaSuccess)
             return e;
         RowMaps maps = {};
         maps.ok = !(p.flags & KDA_FLAG_ROW_COPIES) && make_row_map(&maps.m[0], p.o, (long long)p.B * p.T, p.H, C);
@@ -724,11 +724,11 @@ cudaError_t tc_bwd(const KdaParams& p, cudaStream_t s) {
         if ((e = simt_stage(p, ST_BWD_STATE, s)) != cudaSuccess) return e;
     } else {
         constexpr int smem = 3 * bs::STAGE;
-        if ((e = cudaFuncSetAttribute(kda_bwd_state_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
+        if ((e = allow_smem(kda_bwd_state_tc<false>, smem)) != cudaSuccess)
             return e;
         const StateSegs segs = state_segs(p, true);
         if (segs.len > 0) {
-            if ((e = cudaFuncSetAttribute(kda_bwd_state_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
+            if ((e = allow_smem(kda_bwd_state_tc<true>, smem)) != cudaSuccess)
                 return e;
             if ((e = launch_dependent(kda_bwd_state_tc<true>, dim3(p.H, segs.count), bs::NTHR, smem, s, p, segs)) != cudaSuccess) return e;
             if ((e = launch_seg_combine(p, segs, true, s)) != cudaSuccess) return e;

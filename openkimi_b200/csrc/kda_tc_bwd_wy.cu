@@ -557,7 +557,7 @@ cudaError_t launch_bwd_wy_tc(const KdaParams& p, cudaStream_t s) {
     maps.ok = !(p.flags & KDA_FLAG_ROW_COPIES) && make_row_map(&maps.m[0], p.grad_v, (long long)p.B * p.T, p.H, C);
     auto kern = convb ? kda_bwd_wy_tc_pf<true> : kda_bwd_wy_tc_pf<false>;
     const int smem = convb ? (int)bp::TOTAL_CONVB : (int)bp::TOTAL;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     return launch_dependent(kern, units < sms ? units : sms, bp::NTHR, smem, s, p, maps);
 }

@@ -907,10 +907,8 @@ __global__ void __launch_bounds__(fi::NTHR, 2) kda_fwd_intra_tc(const KdaParams 
 cudaError_t launch_fwd_intra_tc(const KdaParams& p, cudaStream_t s) {
     auto kern = p.conv_q ? kda_fwd_intra_tc<true> : kda_fwd_intra_tc<false>;
     const uint32_t smem = p.conv_q ? fi::TOTAL_CONV : fi::TOTAL;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem(kern, (int)smem, true);
     if (e != cudaSuccess) return e;
-    // (the shared memory is split as for the neighbouring kernels, which fill an SM: another split would cost a drain between them)
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) != cudaSuccess) return e;
     const int units = p.NT * p.H, ctas = 2 * sm_count();
     RowMaps maps = {};
     const long long tokens = (long long)p.B * p.T;
