@@ -332,22 +332,14 @@ __device__ __forceinline__ float conv_pre(float w0, float w1, float w2, float w3
 // softplus with torch's threshold of 20 (F.softplus, k3mini/model.py:220)
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + expf(-x)); }
-// softplus for the BF16 path: max(x, 0) + log(1 + e^-|x|) with hardware exp / log; the logarithm's absolute error is at most
-// 2.9e-7 (a decay e^-softplus measures 2.1e-7 relative), which is what matters for a log-decay
-__device__ __forceinline__ float softplus_fast(float x) {
-    const float t = exp_ftz(-fabsf(x));
-    const float l = t < 1e-3f ? t * fmaf(t, fmaf(0.33333334f, t, -0.5f), 1.f) : ln_ftz(1.f + t);
-    return fmaxf(x, 0.f) + l;
-}
-
-__device__ __forceinline__ float2 softplus_fast2(float2 x) {  // the same of two, in packed arithmetic, bit for bit
+// softplus of two numbers for the BF16 path: max(x, 0) + log(1 + e^-|x|) with hardware exp / log, in packed arithmetic; the
+// logarithm's absolute error is at most 2.9e-7 (a decay e^-softplus measures 2.1e-7 relative), which is what matters for a
+// log-decay; for small t = e^-|x| its series
+__device__ __forceinline__ float2 softplus_fast(float2 x) {
     const float2 u = __fmul2_rn(make_float2(-fabsf(x.x), -fabsf(x.y)), make_float2(LOG2E, LOG2E));
-    const float2 t = make_float2(ex2_ftz(u.x), ex2_ftz(u.y)), o = make_float2(1.f, 1.f), s = __fadd2_rn(o, t);
-    float a, b;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(s.x));
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(b) : "f"(s.y));
-    const float2 l = __fmul2_rn(make_float2(a, b), make_float2(0.6931471805599453f, 0.6931471805599453f));
-    const float2 q = __fmul2_rn(t, __ffma2_rn(t, __ffma2_rn(make_float2(0.33333334f, 0.33333334f), t, make_float2(-0.5f, -0.5f)), o));
+    const float2 t = make_float2(ex2_ftz(u.x), ex2_ftz(u.y)), one = make_float2(1.f, 1.f), s = __fadd2_rn(one, t);
+    const float2 l = make_float2(ln_ftz(s.x), ln_ftz(s.y));
+    const float2 q = __fmul2_rn(t, __ffma2_rn(t, __ffma2_rn(make_float2(0.33333334f, 0.33333334f), t, make_float2(-0.5f, -0.5f)), one));
     return __fadd2_rn(make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)), make_float2(t.x < 1e-3f ? q.x : l.x, t.y < 1e-3f ? q.y : l.y));
 }
 

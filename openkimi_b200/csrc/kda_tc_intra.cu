@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(fi::NTHR, 2) kda_fwd_intra_tc(const KdaParams 
         for (int r = 0; r < 16; ++r) {
             const uint32_t w = raw[r * (D / 2)];
             float2 gl = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-            if (gate) gl = __fmul2_rn(make_float2(negA, negA), softplus_fast2(__fadd2_rn(gl, bias)));
+            if (gate) gl = __fmul2_rn(make_float2(negA, negA), softplus_fast(__fadd2_rn(gl, bias)));
             run = __ffma2_rn(gl, make_float2(LOG2E, LOG2E), run);  // explicit: both instantiations must round alike
             Gr[r] = run;
         }
