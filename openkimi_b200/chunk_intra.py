@@ -6,8 +6,8 @@ path unless that module carries the three attributes below with these exact valu
 experiments/kda_sm90/patch_fla_guarded_intra.py:229-242).  This module is the object a
 maintainer hands to ``_validated_kda_backend_name`` for the B200 kernels.
 
-``_OPENKIMI_GUARD_MAX_LOG2_SPAN`` is read at every backward call, so validators can set it
-to ``-1.0`` to force the exact pairwise evaluation of every diagonal tile without
+``_OPENKIMI_GUARD_MAX_LOG2_SPAN`` is read at every forward and every backward call, so validators
+can set it to ``-1.0`` to force the exact pairwise evaluation of every diagonal tile without
 recompiling (experiments/kda_sm90/validate_fla_guarded_integration.py:257-267).
 """
 

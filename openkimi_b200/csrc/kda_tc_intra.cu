@@ -8,9 +8,8 @@
 //   3  Aqk and L: warp = (16-row block I, 64 channels), operands made in registers for mma.sync.  Earlier blocks: x_i 2^(G_i - r_I)
 //      against k_j 2^(r_I - G_j), r_I = G at the first row of block I, every exponent <= 0, one BF16 pass.  The diagonal block, whose
 //      products stay FP32-class (three TF32 passes of split operands), by eight rows: with their midpoint m as reference,
-//      x_i 2^(G_i - m) against k_j 2^(m - G_j), where the tile passes the guard; else by halving (reference: the second half's
-//      first row, every exponent <= 0); pair by pair with one exp2 each where G is not monotone.  The two channel halves
-//      meet in shared memory.  The Qt and Kh records
+//      x_i 2^(G_i - m) against k_j 2^(m - G_j), where the tile passes the guard; else pair by pair, one exp2 each.  The two
+//      channel halves meet in shared memory.  The Qt and Kh records
 //   4  Aqk record; T = (I + diag(beta) L)^-1; the operand beta*k*2^G
 //   5  T record; W^T = (beta k 2^G)^T T^T and U^T = (beta v)^T T^T as tcgen05 MMAs (M = 128 channels); W, U records
 //
@@ -50,7 +49,7 @@ constexpr uint32_t HALO = SBAR + 48;         // fused convolution: rows -3 .. -1
 constexpr uint32_t TOTAL = HALO, TOTAL_CONV = HALO + 9 * 256;
 static_assert(TOTAL_CONV <= 115712, "two CTAs per SM");
 constexpr uint32_t T_W = 0, T_U = 64, TMEM_COLS = 128;
-enum { MIDPOINT = 0, LEVELS = 1, PAIRS = 2 };
+enum { MIDPOINT = 0, PAIRS = 1 };
 // Largest span of eight rows for their midpoint: the factors reach 2^(+-100), the low parts of the operands stay normal numbers.
 constexpr float MAX_SPAN = 200.f;
 }  // namespace fi
@@ -488,8 +487,8 @@ __global__ void __launch_bounds__(fi::NTHR, 2) kda_fwd_intra_tc(const KdaParams 
         float2 base = make_float2(0.f, 0.f);
         for (int b = 0; b < qt; ++b) base = __fadd2_rn(base, *reinterpret_cast<const float2*>(stot + b * D + gd));
         // Span guard, after k3mini/backends.py:17-19, of the [8 rows x 64 channels] tiles: every channel monotone non-increasing and
-        // finite (then its span is first - last row), the largest span within the limit.  Where a span is too large the block goes
-        // by levels, where a channel is not monotone by pairs.
+        // finite (then its span is first - last row), the largest span within the limit.  A block with any other tile goes pair by
+        // pair (a negative limit: every block).
         bool good = true;
         float span = 0.f;
         float2 prev = make_float2(INFINITY, INFINITY);
@@ -511,7 +510,7 @@ __global__ void __launch_bounds__(fi::NTHR, 2) kda_fwd_intra_tc(const KdaParams 
         }
         good = __all_sync(0xffffffffu, good);
         const bool narrow = __all_sync(0xffffffffu, span <= fminf(p.guard_span, MAX_SPAN));
-        if (lane == 0) smode[2 * qt + gh] = !good ? PAIRS : !narrow ? LEVELS : MIDPOINT;
+        if (lane == 0) smode[2 * qt + gh] = good && narrow ? MIDPOINT : PAIRS;
     }
     fence_async_smem();
     __syncthreads();
@@ -608,64 +607,6 @@ __global__ void __launch_bounds__(fi::NTHR, 2) kda_fwd_intra_tc(const KdaParams 
             dq[1][3] = db[1];
             dl[1][2] = db[2];
             dl[1][3] = db[3];
-        } else if (mode == LEVELS) {
-            // Halving: the rows of the second half of 16, 8, 4, 2 consecutive rows against the keys of the first, with G at the
-            // second half's first row as reference: every exponent is <= 0.  Eight rows (q and k rows in one operand) and eight keys a
-            // level; what belongs to different halves is dropped.  Half 0 leaves its Aqk above the diagonal of sAd and
-            // its L in place, half 1 its Aqk in place in sAd and its L above the diagonal.
-#pragma unroll 1
-            for (int b = 3; b >= 0; --b) {
-                const int w = 1 << b, key = ((pr >> b) << (b + 1)) | (pr & (w - 1)), row = key | w, ref = (key & ~(w - 1)) | w;
-                float acc[4] = {};
-#pragma unroll 1
-                for (int s = 0; s < 4; ++s) {
-                    const int ch = 64 * hf + 16 * s + 4 * t;
-                    const float4 rf = *reinterpret_cast<const float4*>(sG + swz_f32(16 * I + ref, ch));
-                    float qf[4], kf[4], kk[4], f[4], y[4];
-                    unpack4(*reinterpret_cast<const uint2*>(sQ + swz_bf16(16 * I + row, ch)), qf);
-                    unpack4(*reinterpret_cast<const uint2*>(sK + swz_bf16(16 * I + row, ch)), kf);
-                    unpack4(*reinterpret_cast<const uint2*>(sK + swz_bf16(16 * I + key, ch)), kk);
-                    exp2_diff(*reinterpret_cast<const float4*>(sG + swz_f32(16 * I + row, ch)), rf, f);
-                    exp2_diff(rf, *reinterpret_cast<const float4*>(sG + swz_f32(16 * I + key, ch)), y);
-#pragma unroll
-                    for (int e = 0; e < 4; e += 2) {
-                        Split2 yy;
-                        split_tf32(kk[e] * y[e], yy.h[0], yy.l[0]);
-                        split_tf32(kk[e + 1] * y[e + 1], yy.h[1], yy.l[1]);
-                        mma_tf32x3(acc, qf[e] * f[e], kf[e] * f[e], qf[e + 1] * f[e + 1], kf[e + 1] * f[e + 1], yy);
-                    }
-                }
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int kn = kt + 4 * e, kj = ((kn >> b) << (b + 1)) | (kn & (w - 1));  // key number kn of the level
-                    if ((kn >> b) == (pr >> b)) {
-                        if (hf) {
-                            sAd[(16 * I + row) * LDA + kj] = acc[e];
-                            sM[(16 * I + kj) * LDR + 16 * I + row] = acc[2 + e];
-                        } else {
-                            sAd[(16 * I + kj) * LDA + row] = acc[e];
-                            sM[(16 * I + row) * LDR + 16 * I + kj] = acc[2 + e];
-                        }
-                    }
-                }
-            }
-            // the diagonal of Aqk: products of BF16 numbers
-            float d0[4] = {}, d1[4] = {};
-#pragma unroll 1
-            for (int s = 0; s < 4; ++s) {
-                const int ch = 64 * hf + 16 * s + 4 * t, r0 = 16 * I + pr;
-                const uint2 a = *reinterpret_cast<const uint2*>(sQ + swz_bf16(r0, ch)), b = *reinterpret_cast<const uint2*>(sQ + swz_bf16(r0 + 8, ch));
-                const uint2 x = *reinterpret_cast<const uint2*>(sK + swz_bf16(r0, ch)), y = *reinterpret_cast<const uint2*>(sK + swz_bf16(r0 + 8, ch));
-                const uint32_t a4[4] = {a.x, b.x, a.y, b.y};
-                mma_bf16(d0, a4, x.x, x.y);
-                mma_bf16(d1, a4, y.x, y.y);
-            }
-#pragma unroll
-            for (int e = 0; e < 2; ++e)
-                if (pr == kt + 4 * e) {
-                    sAd[(16 * I + pr) * LDA + (hf ? pr : 16)] = d0[e];
-                    sAd[(16 * I + pr + 8) * LDA + (hf ? pr + 8 : 16)] = d1[2 + e];
-                }
         } else {  // the pairs one by one: rows pr, pr + 8 against keys kt, kt + 4, kt + 8, kt + 12
 #pragma unroll 1
             for (int x = 0; x < 16; ++x) {
@@ -715,12 +656,12 @@ __global__ void __launch_bounds__(fi::NTHR, 2) kda_fwd_intra_tc(const KdaParams 
                 }
         };
         if (hf) {
-            if (mode != LEVELS) hand_over(I, dq, dl, keep[3]);
+            hand_over(I, dq, dl, keep[3]);
 #pragma unroll
             for (int J = 0; J < 3; ++J)
                 if (J < I) hand_over(J, oq[J], ol[J], keep[J]);
         } else {
-            if (mode != LEVELS) hand_over(I, dl, dq, keep[3]);
+            hand_over(I, dl, dq, keep[3]);
 #pragma unroll
             for (int J = 0; J < 3; ++J)
                 if (J < I) hand_over(J, ol[J], oq[J], keep[J]);
@@ -763,12 +704,7 @@ __global__ void __launch_bounds__(fi::NTHR, 2) kda_fwd_intra_tc(const KdaParams 
 #pragma unroll
                 for (int x = 0; x < 8; ++x) {
                     const int m8 = ((x >> 1) & 1) * 8, n8 = 8 * (x >> 2) + 4 * (x & 1);
-                    float* d = dst + m8 * LDR + n8;
-                    if (J == 3 && mode == LEVELS) {
-                        if (kt + n8 < pr + m8) *d += sM[(16 * I + kt + n8) * LDR + 16 * I + pr + m8];
-                    } else {
-                        *d += keep[J][x];
-                    }
+                    dst[m8 * LDR + n8] += keep[J][x];
                 }
             }
         __syncwarp();
@@ -789,12 +725,7 @@ __global__ void __launch_bounds__(fi::NTHR, 2) kda_fwd_intra_tc(const KdaParams 
 #pragma unroll
                         for (int e = 0; e < 2; ++e) {
                             const float* s = src + m * 8 * ld + 8 * n + 4 * e;
-                            float own = keep[J][4 * n + 2 * m + e];
-                            if (J == 3 && mode == LEVELS) {
-                                const int row = pr + 8 * m, key = kt + 4 * e + 8 * n;
-                                own = sAd[key < row ? (16 * I + key) * LDA + row : (16 * I + row) * LDA + 16];
-                            }
-                            a[e] = (own + *s) * p.scale;
+                            a[e] = (keep[J][4 * n + 2 * m + e] + *s) * p.scale;
                             if (J == 3 && kt + 4 * e + 8 * n > pr + 8 * m) a[e] = 0.f;
                         }
                         // adjacent keys meet in a lane pair: lanes 0, 1 take keys (0, 1), (2, 3), lanes 2, 3 keys (4, 5), (6, 7)

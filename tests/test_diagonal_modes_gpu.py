@@ -1,7 +1,8 @@
-"""The three ways the BF16 forward evaluates a diagonal 16 x 16 block (midpoint of eight rows, halving, pair by pair), each
-against the CPU oracle, and the first two against each other: both form the FP32-class products of the same BF16 rows
-(operands split to 2^-21, three terms), so their Aqk and L differ by a few 2^-20 before they are rounded to BF16 records; a
-flipped rounding (2^-9 of an element, about one in 2^9 of them) moves the outputs by 2^-9 sqrt(2^-9) = 9e-5 relative."""
+"""The two ways the BF16 forward evaluates a diagonal 16 x 16 block, by the midpoints of eight rows or pair by pair, each against
+the CPU oracle and against the other: their Aqk and L differ by a few 2^-22 (one or two approximated exponentials and a few
+FP32 roundings each) before they are rounded to BF16 records; a flipped rounding (2^-9 of an element, fewer than one in 2^9 of
+them) moves the outputs by 2^-9 sqrt(2^-9) = 9e-5 relative.  And which blocks go pair by pair: those that the guard
+rejects, and all with a negative limit."""
 import math
 
 import pytest
@@ -38,16 +39,16 @@ SPANS = {
 
 @pytest.mark.parametrize("name", SPANS)
 @pytest.mark.parametrize("T", [16, 64, 135])
-def test_midpoint_and_halving(name, T):
+def test_midpoint_and_pairs(name, T):
     inp = _inputs(T, SPANS[name], seed=7 + T)
     ref = run_oracle(inp, fused=False)
     with _guard(232.0):
         mid = run_device(inp, fused=False)
     with _guard(-1.0):
-        lev = run_device(inp, fused=False)
-    for dev in (mid, lev):
+        pairs = run_device(inp, fused=False)
+    for dev in (mid, pairs):
         assert_rows(compare(dev, ref, tol_max=2e-2, tol_l2=7e-3, abs_escape=5e-5, names=("o", "ht")))
-    assert rel_l2(mid["o"], lev["o"]) <= 4 * 9e-5
+    assert rel_l2(mid["o"], pairs["o"]) <= 4 * 9e-5
 
 
 @pytest.mark.parametrize("T", [16, 64, 135])
@@ -57,3 +58,24 @@ def test_rising_gate_by_pairs(T, rise):
     decay = lambda s, gen: torch.where(torch.rand(s, generator=gen) < 0.2, torch.tensor(-rise), 2 * rise * torch.rand(s, generator=gen))
     inp = _inputs(T, decay, seed=11 + T)
     assert_rows(compare(run_device(inp, fused=False), run_oracle(inp, fused=False), tol_max=2e-2, tol_l2=7e-3, names=("o", "ht")))
+
+
+@pytest.mark.parametrize("decay", [0.05, 40.0])
+@pytest.mark.parametrize("T", [64, 1031])
+def test_negative_limit_and_rejected_blocks_go_pair_by_pair(decay, T):
+    """Two channels (one per half) carry no q and k.  Where their gate rises, every block is evaluated pair by pair, and nothing
+    else changes: a negative limit, and the limit of a wide gate, have to give the bits of that run."""
+    inp = _inputs(T, lambda s, gen: decay * torch.rand(s, generator=gen), seed=23 + T, batch=4)
+    for n in ("q", "k"):
+        inp[n][..., 5::64] = 0
+    rising = dict(inp, g=inp["g"].clone())
+    rising["g"][..., 5::64] = 0.01
+    with _guard(232.0):
+        want = run_device(rising, fused=False)
+        kept = run_device(inp, fused=False)
+    with _guard(-1.0):
+        exact = run_device(inp, fused=False)
+    for n in ("o", "ht"):
+        assert torch.equal(exact[n], want[n]), n
+        if decay > 1:  # the eight-row tiles span 200 and more in some channel of every half
+            assert torch.equal(kept[n], want[n]), n
