@@ -66,4 +66,13 @@ def test_segments_with_the_fused_convolution(name, recompute):
     dev = _run(t, True, disable_recompute=not recompute, **kw)
     _same(dev, _run(t, False, disable_recompute=not recompute, **kw))
     ref = _run(t, False, fp32_math=True, **kw)
-    assert_rows(compare(dev, ref, tol_max=2e-2, tol_l2=1.5e-2, names=tuple(ref)))
+    # dA_log of a head is the sum of dg softplus / sigmoid over its elements, terms of both signs.  What a rounded record moves stays in
+    # the state for the n tokens of the head's memory, so n terms move alike: their sum with a standard deviation of
+    # 2.5 2^-9 sqrt(n) root-sum-square(terms) (the rms of 96 heads of other seeds).  Four of them are allowed where that is
+    # more than the limit of the other outputs: a head of n = 50 draws 2.5e-2 of its dA here, whichever way single records round.
+    x = (t["g"].float() + t["dt_bias"].view(1, 1, 2, 128)).double()
+    terms = ref["dg"].double() * torch.nn.functional.softplus(x) / torch.sigmoid(x)
+    memory = 1 / (t["A_log"].double().exp() * torch.nn.functional.softplus(x).mean((0, 1, 3)))
+    bound = 10 * 2.0 ** -9 * memory.clamp_min(1).sqrt() * terms.pow(2).sum((0, 1, 3)).sqrt()
+    assert ((dev["dA"] - ref["dA"]).double().abs() <= bound.clamp_min(1.5e-2 * ref["dA"].double().norm())).all()
+    assert_rows(compare(dev, ref, tol_max=2e-2, tol_l2=1.5e-2, names=tuple(n for n in ref if n != "dA")))
