@@ -80,9 +80,9 @@ typedef struct KdaParams {
     int32_t flags;         /* KDA_FLAG_* */
     float scale;           /* k3mini/model.py:208 */
     float guard_span;      /* log2 span limit of the guarded diagonal (k3mini/backends.py:18): tiles of
-                              16 rows x 32 channels in the backward, of 8 rows x 64 channels (and never
-                              above 200) in the BF16 forward; what it rejects is evaluated pair by pair.
-                              Negative forces the exact pairwise path everywhere */
+                              16 rows x 32 channels, in the BF16 forward the diagonal block of all four;
+                              what it rejects is evaluated pair by pair.  Negative forces the exact
+                              pairwise path everywhere */
     /* forward inputs */
     const void *q, *k, *v, *g, *beta;
     const float *A_log, *dt_bias;

@@ -5,21 +5,22 @@
 //      CONV instantiation reads the pre-convolution projections instead (three halo rows before the chunk included) and applies
 //      the causal depthwise filter + SiLU of k3mini/model.py:76-88,181-185 before anything else sees the rows
 //   2  gate channel-wise: activation, within-chunk cumulative sum G (log2), span guard
-//   3  Aqk and L: warp = (16-row block I, 64 channels), operands made in registers for mma.sync.  Earlier blocks: x_i 2^(G_i - r_I)
-//      against k_j 2^(r_I - G_j), r_I = G at the first row of block I, every exponent <= 0, one BF16 pass.  The diagonal block, whose
-//      products stay FP32-class (three TF32 passes of split operands), by eight rows: with their midpoint m as reference,
-//      x_i 2^(G_i - m) against k_j 2^(m - G_j), where the tile passes the guard; else pair by pair, one exp2 each.  The two
-//      channel halves meet in shared memory.  The Qt and Kh records
+//   3  Aqk and L: warp = (16-row block I, 64 channels).  The diagonal block in FP32 multiply-adds: with the midpoint m of its rows as
+//      reference, x_i 2^(G_i - m) against k_j 2^(m - G_j), where the block passes the guard; else pair by pair, one exp2 each.
+//      Earlier blocks on mma.sync with operands made in registers, one BF16 pass: x_i 2^(G_i - r_I) against k_j 2^(r_I - G_j),
+//      r_I = G at the first row of block I, every exponent <= 0.  The two channel halves meet in shared memory.  The Qt and
+//      Kh records
 //   4  Aqk record; T = (I + diag(beta) L)^-1; the operand beta*k*2^G
 //   5  T record; W^T = (beta k 2^G)^T T^T and U^T = (beta v)^T T^T as tcgen05 MMAs (M = 128 channels); W, U records
 //
-// What bounds it: one unit is a chain of short dependent stages (a dozen barriers, 14 us alone), and at 40 000 warp
-// instructions it needs 5.3 us of the four schedulers.  Two CTAs share an SM so that one unit's waits are the other's issue
-// slots (9.4 us a unit, half of the slots used).  A unit lives in 110 KB for that: the products' operands never touch shared
-// memory, L turns into T in place, beta v and beta k 2^G are MMA operands where the tile copies left v and q, and the next unit's
-// rows are requested as their places fall free.  Operand tiles in shared memory and the diagonal blocks as FP32 FMAs took
-// one CTA of 512 threads and 14.5 us a unit (3072 units 304 -> 206 us, 1536 units of one sequence 162 -> 115, 192 units
-// 40.5 -> 24; with the convolution 12288 units 1434 -> 1052).
+// What bounds it: one unit is a chain of short dependent stages (a dozen barriers).  Two CTAs share an SM so that one unit's waits are
+// the other's issue slots.  A unit lives in 110 KB for that: the off-diagonal products' operands never touch shared memory, the
+// diagonal blocks' scaled rows lie where the partial sums go afterwards, L turns into T in place, beta v and beta k 2^G are MMA
+// operands where the tile copies left v and q, and the next unit's rows are requested as their places fall free.  Operand tiles in
+// shared memory took one CTA of 512 threads (3072 units 304 -> 226 us, twice 1536 units of wide spans 353 -> 265; with
+// the convolution 12288 units 1443 -> 1103).  The diagonal blocks as TF32 products of operands split in two are faster (204 us)
+// and three times as far from 64-bit sums: the share of their BF16 records that come out rounded the other way is 3e-4
+// against 1e-4.
 #include "kda_common.cuh"
 #include "kda_conv_bwd.cuh"
 #include "kda_tc.cuh"
@@ -36,22 +37,21 @@ constexpr uint32_t SQ = 0;                   // q rows, then q^ bf16 [64][128] (
 constexpr uint32_t SK = SQ + 16384;          // k rows, then k^
 constexpr uint32_t SV = SK + 16384;          // v rows, then beta v (swz_bf16)
 constexpr uint32_t SG = SV + 16384;          // G f32 [64][128] (swz_f32)
-constexpr uint32_t SM = SG + 32768;          // gate rows bf16 [64][128] as they arrive; then f32 [64][LDR]: L, T;
-                                             // partial blocks of Aqk above the diagonal
-constexpr uint32_t SU = SM + 64 * LDR * 4;   // 8 KB: gate totals of the four 16-row groups f32 [4][128] | partial
-                                             // diagonal blocks of Aqk | inner products of the inverse | T bf16 cm(i, j; 64)
+constexpr uint32_t SM = SG + 32768;          // gate rows bf16 [64][128] as they arrive; the diagonal blocks' scaled rows; then
+                                             // f32 [64][LDR]: L, T; partial blocks of Aqk above the diagonal
+constexpr uint32_t SU = SM + 64 * LDR * 4;   // 8 KB: gate totals of the four 16-row groups f32 [4][128] | the rest of the
+                                             // scaled rows | partial diagonal blocks of Aqk | inner products of the inverse | T bf16 cm(i, j; 64)
 constexpr uint32_t TAPS = SG;                // when G is dead: the filter taps of the next unit, f32 [3][8][16][4]
-constexpr uint32_t SMID = SU + 8192;         // f32 [8][128] midpoint of every (eight rows, channel)
-constexpr uint32_t SBETA = SMID + 4096;      // f32 [3][64]: 1/|q|, 1/|k|, beta (the aux record)
-constexpr uint32_t SMODE = SBETA + 768;      // int [4][2]: how the diagonal block may be evaluated, per 64 channels
-constexpr uint32_t SBAR = SMODE + 32;        // four mbarriers, the tensor-memory base
+constexpr uint32_t SMID = SU + 8192;         // f32 [4][128] midpoint of every (16-row block, channel)
+constexpr uint32_t SBETA = SMID + 2048;      // f32 [3][64]: 1/|q|, 1/|k|, beta (the aux record)
+constexpr uint32_t SPASS = SBETA + 768;      // int [4][2]: guard decision of every block, per 64 channels
+constexpr uint32_t SBAR = SPASS + 32;        // four mbarriers, the tensor-memory base
 constexpr uint32_t HALO = SBAR + 48;         // fused convolution: rows -3 .. -1 of q, k, v, bf16 [3][3][128]
 constexpr uint32_t TOTAL = HALO, TOTAL_CONV = HALO + 9 * 256;
 static_assert(TOTAL_CONV <= 115712, "two CTAs per SM");
 constexpr uint32_t T_W = 0, T_U = 64, TMEM_COLS = 128;
-enum { MIDPOINT = 0, PAIRS = 1 };
-// Largest span of eight rows for their midpoint: the factors reach 2^(+-100), the low parts of the operands stay normal numbers.
-constexpr float MAX_SPAN = 200.f;
+constexpr int LDS = 20;                      // row stride in floats of a warp's scaled rows: [2][16][LDS], over SM and SU
+static_assert(8 * 2 * 16 * LDS * 4 <= SMID - SM, "scaled rows of eight warps");
 }  // namespace fi
 using fi::LDR;
 
@@ -87,7 +87,6 @@ __device__ __forceinline__ void invert_diagonal(float* M, const float* sbeta, in
     }
 }
 
-
 // mma.sync fragments (lane = 4 g + t).  The contracted index may be dealt out in any order that both operands share: of sixteen
 // channels a lane holds 4 t .. 4 t + 3, one 16-byte word of G and one 8-byte word of q^ and k^, for one BF16 step or two TF32
 // steps.  Row (and key) number g of a tile stands for row bit_reverse(g): with the row swizzle of the tiles (swz_f32,
@@ -108,18 +107,6 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], float a0, float a1, floa
 __device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
     hi = __uint_as_float(__float_as_uint(x) & 0xffffe000u);
     lo = __uint_as_float(__float_as_uint(x - hi) + 0x1000u);
-}
-struct Split2 { float h[2], l[2]; };  // the two B elements of a lane, split
-// c += a b with split operands: lo hi + hi lo + hi hi
-__device__ __forceinline__ void mma_tf32x3(float (&c)[4], float a0, float a1, float a2, float a3, const Split2& b) {
-    float h[4], l[4];
-    split_tf32(a0, h[0], l[0]);
-    split_tf32(a1, h[1], l[1]);
-    split_tf32(a2, h[2], l[2]);
-    split_tf32(a3, h[3], l[3]);
-    mma_tf32(c, l[0], l[1], l[2], l[3], b.h[0], b.h[1]);
-    mma_tf32(c, h[0], h[1], h[2], h[3], b.l[0], b.l[1]);
-    mma_tf32(c, h[0], h[1], h[2], h[3], b.h[0], b.h[1]);
 }
 __device__ __forceinline__ void exp2_diff(const float4& a, const float4& b, float (&f)[4]) {  // 2^(a - b)
     f[0] = ex2_approx(a.x - b.x); f[1] = ex2_approx(a.y - b.y); f[2] = ex2_approx(a.z - b.z); f[3] = ex2_approx(a.w - b.w);
@@ -196,7 +183,7 @@ __global__ void __launch_bounds__(fi::NTHR, 2) kda_fwd_intra_tc(const KdaParams 
     float* smid = reinterpret_cast<float*>(dyn + SMID);
     float* saux = reinterpret_cast<float*>(dyn + SBETA);
     float* sbeta = saux + 2 * C;
-    int* smode = reinterpret_cast<int*>(dyn + SMODE);
+    int* spass = reinterpret_cast<int*>(dyn + SPASS);
     uint64_t* kbar = reinterpret_cast<uint64_t*>(dyn + SBAR);  // k (and every halo row)
     uint64_t* qbar = kbar + 1;  // q, v
     uint64_t* gbar = kbar + 2;  // gate
@@ -486,31 +473,25 @@ __global__ void __launch_bounds__(fi::NTHR, 2) kda_fwd_intra_tc(const KdaParams 
         __syncthreads();  // the totals of the groups are there
         float2 base = make_float2(0.f, 0.f);
         for (int b = 0; b < qt; ++b) base = __fadd2_rn(base, *reinterpret_cast<const float2*>(stot + b * D + gd));
-        // Span guard, after k3mini/backends.py:17-19, of the [8 rows x 64 channels] tiles: every channel monotone non-increasing and
-        // finite (then its span is first - last row), the largest span within the limit.  A block with any other tile goes pair by
-        // pair (a negative limit: every block).
+        // Span guard, after k3mini/backends.py:17-19, of the block's 16 rows: every channel monotone non-increasing and finite (then its
+        // span is first - last row), the largest span within the limit.  A block goes pair by pair unless both its halves pass
+        // (a negative limit: every block).
         bool good = true;
-        float span = 0.f;
-        float2 prev = make_float2(INFINITY, INFINITY);
+        float2 first, prev = make_float2(INFINITY, INFINITY);
 #pragma unroll
-        for (int r0 = 0; r0 < 16; r0 += 8) {
-            float2 first;
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                float2* at = reinterpret_cast<float2*>(sG + swz_f32(16 * qt + r0 + r, gd));
-                const float2 x = __fadd2_rn(Gr[r0 + r], base);
-                *at = x;
-                good = good && x.x <= prev.x && x.y <= prev.y;
-                prev = x;
-                if (r == 0) first = x;
-            }
-            *reinterpret_cast<float2*>(smid + (2 * qt + (r0 >> 3)) * D + gd) = make_float2(0.5f * (first.x + prev.x), 0.5f * (first.y + prev.y));
-            good = good && isfinite(first.x) && isfinite(first.y) && isfinite(prev.x) && isfinite(prev.y);
-            span = fmaxf(span, fmaxf(first.x - prev.x, first.y - prev.y));
+        for (int r = 0; r < 16; ++r) {
+            float2* at = reinterpret_cast<float2*>(sG + swz_f32(16 * qt + r, gd));
+            const float2 x = __fadd2_rn(Gr[r], base);
+            *at = x;
+            good = good && x.x <= prev.x && x.y <= prev.y;
+            prev = x;
+            if (r == 0) first = x;
         }
+        *reinterpret_cast<float2*>(smid + qt * D + gd) = make_float2(0.5f * (first.x + prev.x), 0.5f * (first.y + prev.y));
+        good = good && isfinite(first.x) && isfinite(first.y) && isfinite(prev.x) && isfinite(prev.y) &&
+               fmaxf(first.x - prev.x, first.y - prev.y) <= p.guard_span;
         good = __all_sync(0xffffffffu, good);
-        const bool narrow = __all_sync(0xffffffffu, span <= fminf(p.guard_span, MAX_SPAN));
-        if (lane == 0) smode[2 * qt + gh] = good && narrow ? MIDPOINT : PAIRS;
+        if (lane == 0) spass[2 * qt + gh] = good;
     }
     fence_async_smem();
     __syncthreads();
@@ -531,10 +512,102 @@ __global__ void __launch_bounds__(fi::NTHR, 2) kda_fwd_intra_tc(const KdaParams 
     const int gq = lane >> 2, t = lane & 3;
     const int I = warp < 4 ? warp : 7 - warp, hf = warp >> 2;  // (a scheduler's two warps share the work of one to four block pairs)
     const int pr = ((gq & 1) << 2) | (gq & 2) | (gq >> 2), kt = (t >> 1) | ((t & 1) << 1);  // row g; keys 2t and 2t + 1 are kt, kt + 4
-    const int mode = max(smode[2 * I], smode[2 * I + 1]);  // (both halves must agree on where the sums are)
     float keep[4][8];  // the matrix this warp finishes, Aqk (half 0) or L (half 1): [J][4 n-tile + fragment], keep[3] the diagonal block
     {
-        float oq[3][2][4] = {}, ol[3][2][4] = {}, dq[2][4] = {}, dl[2][4] = {}, db[4] = {};
+        // The diagonal block, in FP32: rows pr, pr + 8 against keys kt + 4 n.  With the midpoint m of its rows as reference: row factors
+        // 2^(G_i - m) and scaled key rows k_j 2^(m - G_j) (within 2^(+-116)) of sixteen channels at a time, made once each and kept in the
+        // warp's part of SM / SU; or pair by pair, one exponential each.  Pairs j > i are computed too but never used; whatever they
+        // overflow to is dropped.  Sums as chains of eight that meet in a tree.
+        float dq[2][4] = {}, dl[2][4] = {}, hq[2][4], hl[2][4];
+        const bool pass = spass[2 * I] & spass[2 * I + 1];
+        float* sF = reinterpret_cast<float*>(dyn + SM) + warp * (2 * 16 * LDS);
+        float* sKY = sF + 16 * LDS;
+#pragma unroll 1
+        for (int s = 0; s < 4; ++s) {
+            float2 av[2][4] = {}, lv[2][4] = {};
+            if (pass) {
+                const int ch = 64 * hf + 16 * s + 4 * t;
+                const float4 mid = *reinterpret_cast<const float4*>(smid + I * D + ch);
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    const int row = 16 * I + pr + 8 * m;
+                    const float4 G4 = *reinterpret_cast<const float4*>(sG + swz_f32(row, ch));
+                    float f[4], y[4], kf[4];
+                    unpack4(*reinterpret_cast<const uint2*>(sK + swz_bf16(row, ch)), kf);
+                    exp2_diff(G4, mid, f);
+                    exp2_diff(mid, G4, y);
+                    *reinterpret_cast<float4*>(sF + (pr + 8 * m) * LDS + 4 * t) = make_float4(f[0], f[1], f[2], f[3]);
+                    *reinterpret_cast<float4*>(sKY + (pr + 8 * m) * LDS + 4 * t) = make_float4(kf[0] * y[0], kf[1] * y[1], kf[2] * y[2], kf[3] * y[3]);
+                }
+                __syncwarp();
+#pragma unroll 2
+                for (int u = 0; u < 4; ++u) {
+                    float2 qf[2][2], kf[2][2];
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        const float4 f = *reinterpret_cast<const float4*>(sF + (pr + 8 * m) * LDS + 4 * u);
+                        const int at = swz_bf16(16 * I + pr + 8 * m, 64 * hf + 16 * s + 4 * u);
+                        float a[4], b[4];
+                        unpack4(*reinterpret_cast<const uint2*>(sQ + at), a);
+                        unpack4(*reinterpret_cast<const uint2*>(sK + at), b);
+                        qf[m][0] = __fmul2_rn(make_float2(a[0], a[1]), make_float2(f.x, f.y));
+                        qf[m][1] = __fmul2_rn(make_float2(a[2], a[3]), make_float2(f.z, f.w));
+                        kf[m][0] = __fmul2_rn(make_float2(b[0], b[1]), make_float2(f.x, f.y));
+                        kf[m][1] = __fmul2_rn(make_float2(b[2], b[3]), make_float2(f.z, f.w));
+                    }
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) {
+                        const float4 y = *reinterpret_cast<const float4*>(sKY + (kt + 4 * n) * LDS + 4 * u);
+#pragma unroll
+                        for (int m = n >> 1; m < 2; ++m) {  // (keys 8 .. 15 have no pairs with rows 0 .. 7)
+                            av[m][n] = __ffma2_rn(qf[m][0], make_float2(y.x, y.y), __ffma2_rn(qf[m][1], make_float2(y.z, y.w), av[m][n]));
+                            lv[m][n] = __ffma2_rn(kf[m][0], make_float2(y.x, y.y), __ffma2_rn(kf[m][1], make_float2(y.z, y.w), lv[m][n]));
+                        }
+                    }
+                }
+                __syncwarp();
+            } else {
+#pragma unroll 1
+                for (int u = 0; u < 4; ++u) {
+                    const int ch = 64 * hf + 16 * s + 4 * u;
+                    float4 Gr[2];
+                    float qf[2][4], kf[2][4];
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        const int row = 16 * I + pr + 8 * m;
+                        Gr[m] = *reinterpret_cast<const float4*>(sG + swz_f32(row, ch));
+                        unpack4(*reinterpret_cast<const uint2*>(sQ + swz_bf16(row, ch)), qf[m]);
+                        unpack4(*reinterpret_cast<const uint2*>(sK + swz_bf16(row, ch)), kf[m]);
+                    }
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) {
+                        const int key = 16 * I + kt + 4 * n;
+                        const float4 Gk = *reinterpret_cast<const float4*>(sG + swz_f32(key, ch));
+                        float kk[4];
+                        unpack4(*reinterpret_cast<const uint2*>(sK + swz_bf16(key, ch)), kk);
+#pragma unroll
+                        for (int m = n >> 1; m < 2; ++m) {
+                            float e[4];
+                            exp2_diff(Gr[m], Gk, e);
+                            const float2 y0 = __fmul2_rn(make_float2(kk[0], kk[1]), make_float2(e[0], e[1])), y1 = __fmul2_rn(make_float2(kk[2], kk[3]), make_float2(e[2], e[3]));
+                            av[m][n] = __ffma2_rn(make_float2(qf[m][0], qf[m][1]), y0, __ffma2_rn(make_float2(qf[m][2], qf[m][3]), y1, av[m][n]));
+                            lv[m][n] = __ffma2_rn(make_float2(kf[m][0], kf[m][1]), y0, __ffma2_rn(make_float2(kf[m][2], kf[m][3]), y1, lv[m][n]));
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int m = n >> 1; m < 2; ++m) {
+                    float &a = dq[n >> 1][2 * m + (n & 1)], &l = dl[n >> 1][2 * m + (n & 1)], &ha = hq[n >> 1][2 * m + (n & 1)], &hb = hl[n >> 1][2 * m + (n & 1)];
+                    const float a16 = av[m][n].x + av[m][n].y, l16 = lv[m][n].x + lv[m][n].y;
+                    if (s & 1) a += ha + a16, l += hb + l16;
+                    else ha = a16, hb = l16;
+                }
+        }
+        __syncthreads();  // the scaled rows are dead: their place takes the partial sums
+        float oq[3][2][4] = {}, ol[3][2][4] = {};
 #pragma unroll 1
         for (int s = 0; s < 4; ++s) {
             // (every row of this loop is pr mod 8: one swizzled offset for all, a row is a constant away from row pr)
@@ -573,71 +646,6 @@ __global__ void __launch_bounds__(fi::NTHR, 2) kda_fwd_intra_tc(const KdaParams 
                             mma_bf16(ol[J][n], ak, b0, b1);
                         }
                     }
-            }
-            if (mode == MIDPOINT) {
-                // the diagonal block: keys 0 .. 7 against all rows with the midpoint of rows 0 .. 7 as reference, keys 8 .. 15 against
-                // rows 8 .. 15 (of q and of k, one operand) with theirs
-                const float4 ma = *reinterpret_cast<const float4*>(smid + 2 * I * D + ch), mb = *reinterpret_cast<const float4*>(smid + (2 * I + 1) * D + ch);
-                float p0[4], p1[4], p2[4], y0[4], y1[4];
-                exp2_diff(G0, ma, p0);
-                exp2_diff(G1, ma, p1);
-                exp2_diff(G1, mb, p2);
-                exp2_diff(ma, G0, y0);
-                exp2_diff(mb, G1, y1);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    y0[j] *= k0[j];
-                    y1[j] *= k1[j];
-                }
-#pragma unroll
-                for (int e = 0; e < 4; e += 2) {  // channels e, e + 1: fragment order (upper row, lower row) of the first, then of the second
-                    Split2 y;
-                    split_tf32(y0[e], y.h[0], y.l[0]);
-                    split_tf32(y0[e + 1], y.h[1], y.l[1]);
-                    mma_tf32x3(dq[0], q0[e] * p0[e], q1[e] * p1[e], q0[e + 1] * p0[e + 1], q1[e + 1] * p1[e + 1], y);
-                    mma_tf32x3(dl[0], k0[e] * p0[e], k1[e] * p1[e], k0[e + 1] * p0[e + 1], k1[e + 1] * p1[e + 1], y);
-                    split_tf32(y1[e], y.h[0], y.l[0]);
-                    split_tf32(y1[e + 1], y.h[1], y.l[1]);
-                    mma_tf32x3(db, q1[e] * p2[e], k1[e] * p2[e], q1[e + 1] * p2[e + 1], k1[e + 1] * p2[e + 1], y);
-                }
-            }
-        }
-        if (mode == MIDPOINT) {
-            dq[1][2] = db[0];
-            dq[1][3] = db[1];
-            dl[1][2] = db[2];
-            dl[1][3] = db[3];
-        } else {  // the pairs one by one: rows pr, pr + 8 against keys kt, kt + 4, kt + 8, kt + 12
-#pragma unroll 1
-            for (int x = 0; x < 16; ++x) {
-                const int ch = 64 * hf + 4 * x;
-                float Gr[2][4], qf[2][4], kf[2][4];
-#pragma unroll
-                for (int m = 0; m < 2; ++m) {
-                    const int row = 16 * I + pr + 8 * m;
-                    const float4 G4 = *reinterpret_cast<const float4*>(sG + swz_f32(row, ch));
-                    Gr[m][0] = G4.x; Gr[m][1] = G4.y; Gr[m][2] = G4.z; Gr[m][3] = G4.w;
-                    unpack4(*reinterpret_cast<const uint2*>(sQ + swz_bf16(row, ch)), qf[m]);
-                    unpack4(*reinterpret_cast<const uint2*>(sK + swz_bf16(row, ch)), kf[m]);
-                }
-#pragma unroll
-                for (int n = 0; n < 4; ++n) {
-                    const int row = 16 * I + kt + 4 * n;
-                    const float4 G4 = *reinterpret_cast<const float4*>(sG + swz_f32(row, ch));
-                    const float Gk[4] = {G4.x, G4.y, G4.z, G4.w};
-                    float kk[4];
-                    unpack4(*reinterpret_cast<const uint2*>(sK + swz_bf16(row, ch)), kk);
-#pragma unroll
-                    for (int m = n >> 1; m < 2; ++m)  // (keys 8 .. 15 have no pairs with rows 0 .. 7)
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            // (pairs j > i are computed too but never used; whatever they overflow to is dropped)
-                            const float e = kk[j] * ex2_approx(Gr[m][j] - Gk[j]);
-                            float &a = dq[n >> 1][2 * m + (n & 1)], &l = dl[n >> 1][2 * m + (n & 1)];
-                            a = fmaf(qf[m][j], e, a);
-                            l = fmaf(kf[m][j], e, l);
-                        }
-                }
             }
         }
         // each half gives the other the partial sums of the matrix that one finishes: L to its place, Aqk to the

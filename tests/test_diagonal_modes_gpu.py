@@ -1,5 +1,5 @@
-"""The two ways the BF16 forward evaluates a diagonal 16 x 16 block, by the midpoints of eight rows or pair by pair, each against
-the CPU oracle and against the other: their Aqk and L differ by a few 2^-22 (one or two approximated exponentials and a few
+"""The two ways the BF16 forward evaluates a diagonal 16 x 16 block, with the midpoint of its rows or pair by pair, each against the
+CPU oracle and against the other: their Aqk and L differ by a few 2^-22 (one or two approximated exponentials and a few
 FP32 roundings each) before they are rounded to BF16 records; a flipped rounding (2^-9 of an element, fewer than one in 2^9 of
 them) moves the outputs by 2^-9 sqrt(2^-9) = 9e-5 relative.  And which blocks go pair by pair: those that the guard
 rejects, and all with a negative limit."""
@@ -30,6 +30,8 @@ SPANS = {
     "weak": lambda s, gen: 0.05 * torch.rand(s, generator=gen),
     "eight rows at 190": lambda s, gen: (190 / 7 * math.log(2.0)) * (0.98 + 0.02 * torch.rand(s, generator=gen)),
     "eight rows at 210": lambda s, gen: (210 / 7 * math.log(2.0)) * (1.0 + 0.02 * torch.rand(s, generator=gen)),
+    "sixteen rows at 228": lambda s, gen: (228 / 15 * math.log(2.0)) * (0.98 + 0.02 * torch.rand(s, generator=gen)),
+    "sixteen rows at 236": lambda s, gen: (236 / 15 * math.log(2.0)) * (1.0 + 0.02 * torch.rand(s, generator=gen)),
     "one wide channel half": lambda s, gen: torch.rand(s, generator=gen) * torch.cat([torch.ones(64), torch.full((64,), 60.0)]),
     "wide": lambda s, gen: 100 * torch.rand(s, generator=gen),
     "steps": lambda s, gen: 300 * (torch.rand(s, generator=gen) < 0.05).float(),
@@ -77,5 +79,5 @@ def test_negative_limit_and_rejected_blocks_go_pair_by_pair(decay, T):
         exact = run_device(inp, fused=False)
     for n in ("o", "ht"):
         assert torch.equal(exact[n], want[n]), n
-        if decay > 1:  # the eight-row tiles span 200 and more in some channel of every half
+        if decay > 1:  # sixteen rows span more than 232 in some channel of every block
             assert torch.equal(kept[n], want[n]), n
