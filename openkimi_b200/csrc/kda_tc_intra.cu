@@ -17,10 +17,10 @@
 // the other's issue slots.  A unit lives in 110 KB for that: the off-diagonal products' operands never touch shared memory, the
 // diagonal blocks' scaled rows lie where the partial sums go afterwards, L turns into T in place, beta v and beta k 2^G are MMA
 // operands where the tile copies left v and q, and the next unit's rows are requested as their places fall free.  Operand tiles in
-// shared memory took one CTA of 512 threads (3072 units 304 -> 226 us, twice 1536 units of wide spans 353 -> 265; with
-// the convolution 12288 units 1443 -> 1103).  The diagonal blocks as TF32 products of operands split in two are faster (204 us)
-// and three times as far from 64-bit sums: the share of their BF16 records that come out rounded the other way is 3e-4
-// against 1e-4.
+// shared memory took one CTA of 512 threads (3072 units 304 -> 231 us, twice 1536 units of wide spans 353 -> 271; with
+// the convolution 12288 units 1443 -> 1131).  The diagonal blocks as TF32 products of operands split in two are faster (3072
+// units by 22 us) and three times as far from 64-bit sums: the share of their BF16 records that come out rounded the other way is
+// 3e-4 against 1e-4.  So are the inverse's products (5 us): 2.3e-3 against 1.4e-3 of T where keys are alike.
 #include "kda_common.cuh"
 #include "kda_conv_bwd.cuh"
 #include "kda_tc.cuh"
@@ -58,8 +58,7 @@ using fi::LDR;
 // T = (I + diag(beta) L)^-1 by blocks, in place: M holds L (strictly lower) and receives T on and below the diagonal blocks; rows
 // of LDR floats.  The four 16 x 16 diagonal blocks are inverted by forward substitution in FP32, one warp each (a dependent
 // chain of 16 rows, lane = column); everything below them is products, T_ba = -T_bb (beta L)_ba T_aa for the block pairs (0, 1)
-// and (2, 3), then the same with 32 x 32 halves, in FP32-class TF32 passes of split operands.  sY (32 rows of LDY floats) takes
-// the inner products.
+// and (2, 3), then the same with 32 x 32 halves, in FP32 multiply-adds.  sY (32 rows of LDY floats) takes the inner products.
 constexpr int LDY = 36;
 
 __device__ __forceinline__ void invert_diagonal(float* M, const float* sbeta, int blk, int lane) {
@@ -88,25 +87,12 @@ __device__ __forceinline__ void invert_diagonal(float* M, const float* sbeta, in
 }
 
 // mma.sync fragments (lane = 4 g + t).  The contracted index may be dealt out in any order that both operands share: of sixteen
-// channels a lane holds 4 t .. 4 t + 3, one 16-byte word of G and one 8-byte word of q^ and k^, for one BF16 step or two TF32
-// steps.  Row (and key) number g of a tile stands for row bit_reverse(g): with the row swizzle of the tiles (swz_f32,
+// channels a lane holds 4 t .. 4 t + 3, one 16-byte word of G and one 8-byte word of q^ and k^, for one step.  Row (and key) number g of a tile stands for row bit_reverse(g): with the row swizzle of the tiles (swz_f32,
 // swz_bf16) the loads of a quarter warp then fall into different banks.
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_tf32(float (&c)[4], float a0, float a1, float a2, float a3, float b0, float b1) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(a2)), "r"(__float_as_uint(a3)),
-                   "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
-}
-// x = hi + lo: hi the 11 significant bits that TF32 keeps, lo rounded to as many (the multiplier drops the low 13 bits; half of the
-// last place it keeps is added before): x to 2^-21, without a bias
-__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
-    hi = __uint_as_float(__float_as_uint(x) & 0xffffe000u);
-    lo = __uint_as_float(__float_as_uint(x - hi) + 0x1000u);
 }
 __device__ __forceinline__ void exp2_diff(const float4& a, const float4& b, float (&f)[4]) {  // 2^(a - b)
     f[0] = ex2_approx(a.x - b.x); f[1] = ex2_approx(a.y - b.y); f[2] = ex2_approx(a.z - b.z); f[3] = ex2_approx(a.w - b.w);
@@ -116,53 +102,59 @@ __device__ __forceinline__ void unpack4(const uint2& u, float (&f)[4]) {
     f[2] = __uint_as_float(u.y << 16); f[3] = __uint_as_float(u.y & 0xffff0000u);
 }
 
-// a 16 x 8 tile of A B over 8 KS inner elements; A: row g, column t, B: row t, column g of this lane's fragments
-template <int KS>
-__device__ __forceinline__ void tile_product(float (&c)[4], const float* A, const float* B, int ldb) {
-    float c1[4] = {}, c2[4] = {};  // three independent chains
+// a 2 x 2 tile over `K4` groups of four inner elements: rows of A (float4 along k), rows k of B (two columns)
+template <int K4>
+__device__ __forceinline__ void tile22(float2 (&acc)[2], const float* A, const float* B, int ldb, int kstep) {
+#pragma unroll 2
+    for (int m = 0; m < K4; ++m) {
+        const float4 a0 = *reinterpret_cast<const float4*>(A + m * kstep), a1 = *reinterpret_cast<const float4*>(A + LDR + m * kstep);
+        const float x0[4] = {a0.x, a0.y, a0.z, a0.w}, x1[4] = {a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-    for (int k = 0; k < KS; ++k) {
-        float h[4], l[4], bh[2], bl[2];
-        split_tf32(A[8 * k], h[0], l[0]);
-        split_tf32(A[8 * k + 8 * LDR], h[1], l[1]);
-        split_tf32(A[8 * k + 4], h[2], l[2]);
-        split_tf32(A[8 * k + 4 + 8 * LDR], h[3], l[3]);
-        split_tf32(B[8 * k * ldb], bh[0], bl[0]);
-        split_tf32(B[(8 * k + 4) * ldb], bh[1], bl[1]);
-        mma_tf32(c1, l[0], l[1], l[2], l[3], bh[0], bh[1]);
-        mma_tf32(c2, h[0], h[1], h[2], h[3], bl[0], bl[1]);
-        mma_tf32(c, h[0], h[1], h[2], h[3], bh[0], bh[1]);
+        for (int j = 0; j < 4; ++j) {
+            const float2 b = *reinterpret_cast<const float2*>(B + (m * kstep + j) * ldb);
+            acc[0] = __ffma2_rn(make_float2(x0[j], x0[j]), b, acc[0]);
+            acc[1] = __ffma2_rn(make_float2(x1[j], x1[j]), b, acc[1]);
+        }
     }
-#pragma unroll
-    for (int x = 0; x < 4; ++x) c[x] += c1[x] + c2[x];
 }
-__device__ __forceinline__ void store_tile(float* dst, int ld, const float (&c)[4], float f0, float f1) {
-    *reinterpret_cast<float2*>(dst) = make_float2(f0 * c[0], f0 * c[1]);
-    *reinterpret_cast<float2*>(dst + 8 * ld) = make_float2(f1 * c[2], f1 * c[3]);
+// row i of a tile whose inner index was split over lanes i = 0, 1
+__device__ __forceinline__ float2 sum_row(const float2 (&acc)[2], int i) {
+    const float2 give = i ? acc[0] : acc[1], own = i ? acc[1] : acc[0];
+    return make_float2(own.x + __shfl_xor_sync(0xffffffffu, give.x, 1), own.y + __shfl_xor_sync(0xffffffffu, give.y, 1));
 }
 __device__ __forceinline__ void invert_products(float* M, const float* sbeta, float* sY, int warp, int lane) {
-    const int g = lane >> 2, t = lane & 3;
-    if (warp < 4) {  // pairs of 16 x 16 blocks: a warp has eight columns of one, so the inner product stays with it
-        const int pr = warp >> 1, n8 = 8 * (warp & 1), a = 32 * pr, b = a + 16;
-        float y[4] = {}, c[4] = {};
-        tile_product<2>(y, M + (b + g) * LDR + a + t, M + (a + t) * LDR + a + n8 + g, LDR);
-        store_tile(sY + (16 * pr + g) * LDY + n8 + 2 * t, LDY, y, sbeta[b + g], sbeta[b + g + 8]);
-        bar_sync(1 + pr, 64);  // both warps of the pair have read L_ba
-        tile_product<2>(c, M + (b + g) * LDR + b + t, sY + (16 * pr + t) * LDY + n8 + g, LDY);
-        store_tile(M + (b + g) * LDR + a + n8 + 2 * t, LDR, c, -1.f, -1.f);
+    float2 acc[2] = {};
+    {   // pairs of 16 x 16 blocks: four warps each, inner index over two lanes (alternating groups of four)
+        const int pr = warp >> 2, a = 32 * pr, b = a + 16, i = lane & 1;
+        const int r0 = 4 * (warp & 3) + 2 * (lane >> 4), c0 = 2 * ((lane >> 1) & 7), k0 = 4 * i;
+        tile22<2>(acc, M + (b + r0) * LDR + a + k0, M + (a + k0) * LDR + a + c0, LDR, 8);
+        const float2 y = sum_row(acc, i);
+        const float be = sbeta[b + r0 + i];
+        *reinterpret_cast<float2*>(sY + (16 * pr + r0 + i) * LDY + c0) = make_float2(be * y.x, be * y.y);
+        bar_sync(1 + pr, 128);  // the pair's warps have read L_ba
+        acc[0] = acc[1] = make_float2(0.f, 0.f);
+        tile22<2>(acc, M + (b + r0) * LDR + b + k0, sY + (16 * pr + k0) * LDY + c0, LDY, 8);
+        const float2 x = sum_row(acc, i);
+        *reinterpret_cast<float2*>(M + (b + r0 + i) * LDR + a + c0) = make_float2(-x.x, -x.y);
     }
     __syncthreads();
-    // the 32 x 32 halves: a warp has one 16 x 8 tile.  (Blocks above the diagonal hold other things: their products are left out.)
-    const int n8 = 8 * (warp & 3), m16 = 16 * (warp >> 2);
-    const float* A = M + (32 + m16 + g) * LDR + t;
-    float y[4] = {}, c[4] = {};
-    if (n8 < 16) tile_product<4>(y, A, M + t * LDR + n8 + g, LDR);
-    else tile_product<2>(y, A + 16, M + (16 + t) * LDR + n8 + g, LDR);
-    store_tile(sY + (m16 + g) * LDY + n8 + 2 * t, LDY, y, sbeta[32 + m16 + g], sbeta[40 + m16 + g]);
+    // the 32 x 32 halves: a warp has eight rows and sixteen columns.  (Blocks above the diagonal hold other things: their products
+    // are left out.)
+    const int r0 = 8 * (warp >> 1) + 2 * (lane >> 3), c16 = 16 * (warp & 1), c0 = c16 + 2 * (lane & 7);
+    acc[0] = acc[1] = make_float2(0.f, 0.f);
+    if (c16) tile22<4>(acc, M + (32 + r0) * LDR + 16, M + 16 * LDR + c0, LDR, 4);
+    else tile22<8>(acc, M + (32 + r0) * LDR, M + c0, LDR, 4);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const float be = sbeta[32 + r0 + i];
+        *reinterpret_cast<float2*>(sY + (r0 + i) * LDY + c0) = make_float2(be * acc[i].x, be * acc[i].y);
+    }
     __syncthreads();
-    if (m16) tile_product<4>(c, A + 32, sY + t * LDY + n8 + g, LDY);
-    else tile_product<2>(c, A + 32, sY + t * LDY + n8 + g, LDY);
-    store_tile(M + (32 + m16 + g) * LDR + n8 + 2 * t, LDR, c, -1.f, -1.f);
+    acc[0] = acc[1] = make_float2(0.f, 0.f);
+    if (warp < 4) tile22<4>(acc, M + (32 + r0) * LDR + 32, sY + c0, LDY, 4);
+    else tile22<8>(acc, M + (32 + r0) * LDR + 32, sY + c0, LDY, 4);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) *reinterpret_cast<float2*>(M + (32 + r0 + i) * LDR + c0) = make_float2(-acc[i].x, -acc[i].y);
 }
 
 template <bool CONV>

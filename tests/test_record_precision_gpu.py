@@ -94,3 +94,25 @@ def test_diagonal_blocks(gate, guard):
     differ = _differ(_diagonal(A), exact, LOW.cuda()), _differ(_diagonal(T), exact_t, STRICT.cuda())
     print(gate, guard, differ)
     assert differ[0] <= 2e-4 and differ[1] <= 2.5e-4, differ
+
+
+@pytest.mark.parametrize("common,limits", [(0.0, (8e-5, 1.1e-4, 1.5e-4)), (0.5, (8e-5, 2.6e-4, 3.7e-4)), (1.5, (8e-4, 1.9e-3, 2e-3))])
+def test_inverse(common, limits):
+    """Without a gate L is a product of BF16 rows, so all of T is the inverse in FP32.  `common`: how much the keys of a chunk share;
+    the limits, for the diagonal blocks and the two levels of products below them, lie above the shares that FP32
+    multiply-adds show (5e-5, 8e-5, 1.2e-4; 5e-5, 2.0e-4, 3.2e-4; 5e-4, 1.5e-3, 1.6e-3 over a million entries and more) and for
+    alike keys below those of operands of 22 bits (3.3e-4, 4.1e-4; 2.3e-3, 2.5e-3)."""
+    q, k, v, g, beta = _inputs(65536, 4, 5, 0.0)
+    kf = k.float() + common * k.float().view(1, -1, CH, 4, D)[:, :, :1].expand(-1, -1, CH, -1, -1).reshape(k.shape)
+    k = (kf / kf.norm(dim=-1, keepdim=True)).bfloat16()
+    _, T, _, _, kn, be = _records(q, k, v, g, beta, D ** -0.5)
+    differ = [0.0, 0.0, 0.0]
+    index = torch.arange(CH, device="cuda")
+    level = torch.where(index[:, None] // 16 == index // 16, 0, torch.where(index[:, None] // 32 == index // 32, 1, 2))
+    for b in range(0, len(T), 1024):
+        kb, lower = kn[b:b + 1024].double(), torch.ones(CH, CH, dtype=torch.bool, device="cuda").tril(-1)
+        exact = torch.linalg.inv(torch.eye(CH, dtype=torch.float64, device="cuda") + be[b:b + 1024].double()[:, :, None] * (kb @ kb.transpose(1, 2)).tril(-1))
+        for x in range(3):
+            differ[x] += _differ(T[b:b + 1024], exact, lower & (level == x)) / (len(T) / 1024)
+    print(common, differ)
+    assert all(d <= m for d, m in zip(differ, limits)), differ
