@@ -31,42 +31,49 @@ int fail_cuda(cudaError_t e) {
     return KDA_ERR_LAUNCH;
 }
 
+// Driver functions are looked up through the runtime, so that the library has no link-time dependency on the driver.
+template <class F>
+static F driver_function(const char* name) {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult qr;
+    return cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &qr) == cudaSuccess && qr == cudaDriverEntryPointSuccess ? (F)f : nullptr;
+}
+
+// number of the current context: no two contexts of a process have the same, nor one before and after cudaDeviceReset; 0: none yet
+static unsigned long long context_id() {
+    typedef CUresult (*IdFn)(CUcontext, unsigned long long*);
+    static const IdFn fn = driver_function<IdFn>("cuCtxGetId");
+    unsigned long long id = 0;
+    return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 cudaError_t allow_smem(const void* kern, int bytes, bool max_carveout) {
-    // a kernel's slot is claimed by its address; bytes is published after the runtime has been told (threads that meet tell it twice)
-    struct Slot { std::atomic<const void*> kern; std::atomic<int> bytes; };
+    // A slot per kernel and device holds the context whose limit is set (a kernel always asks for the same bytes): claimed by the kernel's
+    // address, published after the runtime has been told; threads that meet tell it twice, contexts that share a device in turn
+    struct Slot { std::atomic<const void*> kern; std::atomic<unsigned long long> context; };
     constexpr int DEVICES = 64, SLOTS = 64;
     static Slot table[DEVICES][SLOTS];
     int dev = 0;
     Slot* slot = nullptr;
-    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < DEVICES)
+    const unsigned long long id = context_id();
+    if (id && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < DEVICES)
         for (int i = 0; i < SLOTS && !slot; ++i) {
             const void* k = table[dev][i].kern.load(std::memory_order_acquire);
             if (k == nullptr && table[dev][i].kern.compare_exchange_strong(k, kern)) k = kern;
             if (k == kern) slot = &table[dev][i];
         }
-    if (slot && slot->bytes.load(std::memory_order_acquire) >= bytes) return cudaSuccess;
+    if (slot && slot->context.load(std::memory_order_acquire) == id) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess && max_carveout) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess && slot) slot->bytes.store(bytes, std::memory_order_release);
+    if (e == cudaSuccess && slot) slot->context.store(id, std::memory_order_release);
     return e;
 }
 
-// The tensor-map encoder is a driver function; it is looked up through the runtime so that the library
-// has no link-time dependency on the driver.
 bool make_row_map(CUtensorMap* out, const void* base, long long tokens, int H, int box_rows, bool halves) {
     typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static EncodeFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &qr) == cudaSuccess &&
-            qr == cudaDriverEntryPointSuccess)
-            fn = (EncodeFn)f;
-        tried = true;
-    }
+    static const EncodeFn fn = driver_function<EncodeFn>("cuTensorMapEncodeTiled");
     if (!fn || !base || tokens <= 0) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)H * 128, (cuuint64_t)tokens};
     const cuuint64_t strides[1] = {(cuuint64_t)H * 128 * 2};

@@ -20,9 +20,9 @@ inline int launch_status() {
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? KDA_OK : fail_cuda(e);
 }
-// Lets `kern` use `bytes` of dynamic shared memory on the current device.  The runtime is told once per kernel and device (0.5 us a call, up to
-// nine kernels a pass, which counts where the host is what bounds a pass), again if a kernel needs more.  max_carveout: split the SM's
-// memory as for kernels that fill it, where a smaller CTA would get another split and a drain between the two.
+// Lets `kern` use `bytes` of dynamic shared memory in the current context.  The runtime is told once per kernel and context (0.5 us
+// a call, up to nine kernels a pass, which counts where the host is what bounds a pass).  max_carveout: split the SM's memory as
+// for kernels that fill it, where a smaller CTA would get another split and a drain between the two.
 cudaError_t allow_smem(const void* kern, int bytes, bool max_carveout = false);
 template <class... P>
 inline cudaError_t allow_smem(void (*kern)(P...), int bytes, bool max_carveout = false) {
