@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p, 
     const WsLayout L = ws_layout(p.NT, p.H, p.dk, p.dv, p.dtype);
     using namespace bi;
     extern __shared__ __align__(128) unsigned char dyn[];
-    __shared__ uint64_t barA, barQ, barB, barH, mma1, mma2, mma3;
+    __shared__ uint64_t barA, barB, barH, mma1, mma2, mma3;
     __shared__ uint32_t tmem_s;
     const __nv_bfloat16* sQ = reinterpret_cast<const __nv_bfloat16*>(dyn + SQ);
     const __nv_bfloat16* sK = reinterpret_cast<const __nv_bfloat16*>(dyn + SK);
@@ -150,8 +150,7 @@ __global__ void __launch_bounds__(bi::NTHR, 1) kda_bwd_intra(const KdaParams p, 
         tmem_relinquish();
     }
     if (tid == 0) {
-        mbar_init(&barA, 1);  // (two issuing threads)
-        mbar_init(&barQ, 1);
+        mbar_init(&barA, 1);
         mbar_init(&barB, 1);
         mbar_init(&barH, 1);
         mbar_init(&mma1, 4);  // four issuing threads commit each MMA group (one accumulator block each)
