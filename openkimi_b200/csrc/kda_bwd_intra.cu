@@ -86,8 +86,9 @@ __host__ __device__ constexpr uint32_t ccol(int I) { return 320u + 8u * I * (I +
 }  // namespace bi
 
 // Two neighbouring rows of a channel in packed arithmetic: the kernel is bound by instruction issue and the latencies between its
-// barriers, and the rows lie side by side in the registers of accumulators, hand-over words and G (63 000 -> 49 000 warp
-// instructions a unit; 3072 units 337 -> 313 us, 1536 units with three quarters of the tiles rejected 233 -> 212).
+// barriers, and the rows lie side by side in the registers of accumulators, hand-over words and G (with four-wide coefficients for
+// rejected tiles and the gate's gradient leaving by tile copy 57 500 -> 43 000 warp instructions a unit; 3072 units 337 -> 302 us,
+// 1536 units with three quarters of the tiles rejected 235 -> 206).
 __device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
 __device__ __forceinline__ float2 ex2_2(float2 x) { return make_float2(ex2_approx(x.x), ex2_approx(x.y)); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, both(-1.f), a); }

@@ -83,8 +83,8 @@ LOW, STRICT = (torch.ones(16, 16, dtype=torch.bool).tril(d) for d in (0, -1))
 @pytest.mark.parametrize("guard", [232.0, -1.0])
 @pytest.mark.parametrize("gate", [0.01, 1.0, 5.0, 9.0, 12.0, 40.0])
 def test_diagonal_blocks(gate, guard):
-    """Spans of sixteen rows from 0.2 to 1100, blocks on both sides of the guard.  FP32 multiply-adds differ in 4e-5 to 1.4e-4 of
-    the entries of Aqk and 1.0e-4 to 1.9e-4 of T (700 000 entries: the counts spread by a tenth); operands of 22 bits in
+    """Spans of sixteen rows from 0.2 to 1100, blocks on both sides of the guard.  FP32 multiply-adds differ in 4e-5 to 1.2e-4 of
+    the entries of Aqk and 9e-5 to 1.8e-4 of T (700 000 entries: the counts spread by a tenth); operands of 22 bits in
     3e-4 and 4e-4, exponentials that flush before their product does in 1e-2."""
     q, k, v, g, beta = _inputs(20480, 4, 3, gate)
     A, T, G, qn, kn, be = _records(q, k, v, g, beta, D ** -0.5, guard)
